@@ -370,6 +370,8 @@ void fill_sys(const pimc_system& s, DevSys& d) {
   }
   d.rcut2 *= 0.25;
   d.rcut2_lo = (float)(d.rcut2 * (1.0 - 1e-5));
+  d.rcut2_hi = (float)(d.rcut2 * (1.0 + 1e-5));
+  for (int a = 0; a < 3; ++a) d.cellb_f[a] = (float)d.cellb[a];
   d.spring = s.spring;
   d.coulomb = s.coulomb;
   d.ewald = s.ewald;

@@ -68,11 +68,10 @@ __device__ double link_utau(const DevSys& s, const double* path, int ip, int t,
         if (s.mixed) {
           const float fx = (float)ex, fy = (float)ey, fz = (float)ez;
           const float gx = (float)px, gy = (float)py, gz = (float)pz;
-          const float r = sqrtf(fx * fx + fy * fy + fz * fz);
-          const float rp = sqrtf(gx * gx + gy * gy + gz * gz);
+          const float r = sqrtf(norm2_f(fx, fy, fz));
+          const float rp = sqrtf(norm2_f(gx, gy, gz));
           const float q = 0.5f * (r + rp);
-          const float sx = fx - gx, sy = fy - gy, sz = fz - gz;
-          const float s2 = __fdividef(sx * sx + sy * sy + sz * sz, q * q);
+          const float s2 = __fdividef(norm2_f(fx - gx, fy - gy, fz - gz), __fmul_rn(q, q));
           up += 0.5 * (double)tab_uk0d_tau_f(tb, q, s2);
           continue;
         }
@@ -109,6 +108,19 @@ struct ThermoParams {
 // term differs between the two orderings.  Both from one product cellb v per
 // component: the image and the tie test share it.
 __device__ __forceinline__ bool pbc_and_tie(const DevSys& s, double& x, double& y, double& z) {
+  const float fx = abs_f32_trunc(x), fy = abs_f32_trunc(y), fz = abs_f32_trunc(z);
+  const float r2 = fx * fx + fy * fy + fz * fz;
+  if (r2 < s.rcut2_lo) return false;
+  bool ok = r2 > s.rcut2_hi;  // certain on the FP32 pipe (pbc): far from every tie too
+  const double cx = image_shift(s.cell[0], s.cellb_f[0], x, fx, ok);
+  const double cy = image_shift(s.cell[1], s.cellb_f[1], y, fy, ok);
+  const double cz = image_shift(s.cell[2], s.cellb_f[2], z, fz, ok);
+  if (ok) {
+    x = __dsub_rn(x, cx);
+    y = __dsub_rn(y, cy);
+    z = __dsub_rn(z, cz);
+    return false;
+  }
   if (!(dot3(x, y, z, x, y, z) > s.rcut2)) return false;
   double v[3] = {x, y, z};
   bool tie = false;
@@ -133,13 +145,12 @@ __device__ __forceinline__ double pair_utau_images(const DevSys& s, const DevTab
                                                    double ey, double ez, double px, double py,
                                                    double pz) {
   if (s.mixed) {
-    const float fx = (float)ex, fy = (float)ey, fz = (float)ez;
-    const float gx = (float)px, gy = (float)py, gz = (float)pz;
-    const float r = sqrtf(fx * fx + fy * fy + fz * fz);
-    const float rp = sqrtf(gx * gx + gy * gy + gz * gz);
+    const float fx = f32_rn(ex), fy = f32_rn(ey), fz = f32_rn(ez);
+    const float gx = f32_rn(px), gy = f32_rn(py), gz = f32_rn(pz);
+    const float r = sqrtf(norm2_f(fx, fy, fz));
+    const float rp = sqrtf(norm2_f(gx, gy, gz));
     const float q = 0.5f * (r + rp);
-    const float sx = fx - gx, sy = fy - gy, sz = fz - gz;
-    const float s2 = __fdividef(sx * sx + sy * sy + sz * sz, q * q);
+    const float s2 = __fdividef(norm2_f(fx - gx, fy - gy, fz - gz), __fmul_rn(q, q));
     return (double)tab_uk0d_tau_f(tb, q, s2);
   }
   const double r = sqrt(dot3(ex, ey, ez, ex, ey, ez));

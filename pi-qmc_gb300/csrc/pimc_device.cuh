@@ -52,7 +52,9 @@ struct DevSys {
   int dr;
   double dr_sigma[kMaxSpecies], dr_inv2s2[kMaxSpecies];
   double cell[3], cellb[3], rcut2;
-  float rcut2_lo;  // the mixed form's FP32 pre-test of pbc (pbc_f): rcut2 (1 - 1e-5)
+  // FP32 pre-tests of the minimum image (pbc): rcut2 (1 - 1e-5) and rcut2 (1 + 1e-5),
+  // and the reciprocal box sides
+  float rcut2_lo, rcut2_hi, cellb_f[3];
   int spring, coulomb, ewald, mover, fixed_node;
   int mixed;  // PIMC_PREC_MIXED: pair-action terms in FP32, accumulated in FP64
   double epsilon;
@@ -94,9 +96,34 @@ __device__ __forceinline__ double dot3(double ax, double ay, double az, double b
   return __dadd_rn(__dadd_rn(__dmul_rn(ax, bx), __dmul_rn(ay, by)), __dmul_rn(az, bz));
 }
 
+// GB300's FP64 pipe takes 19 clocks of the SM for every warp instruction, and
+// conversions and floor run on it too (16 clocks each); integer and FP32
+// instructions take about a quarter of a clock.  So what decides (whether a
+// vector is imaged, by which multiple of the box) runs on the integer and FP32
+// pipes wherever the answer is certain there, and FP64 does only the arithmetic
+// of the result.
+
+// |v| cut to an FP32 from the high word: in [|v| (1 - 2^-20), |v|]; infinities,
+// NaN and values past FP32's range give infinity or NaN.
+__device__ __forceinline__ float abs_f32_trunc(double v) {
+  const int h = (__double2hiint(v) & 0x7fffffff) - (896 << 20);
+  return __int_as_float(min(max(h, 0), 0x0fffffff) << 3);
+}
+
+// (float)v, rounded to nearest even, on the integer pipe; zero, subnormal and
+// out-of-range results take the conversion instruction.
+__device__ __forceinline__ float f32_rn(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned m = hi & 0x7fffffffu;
+  if (m - (897u << 20) >= (253u << 20)) return (float)v;
+  unsigned b = __funnelshift_l(lo, m - (896u << 20), 3);  // the kept bits
+  b += (lo << 3) + (b & 1u) > 0x80000000u;                // the 29 cut ones, ties to even
+  return __uint_as_float(b | (hi & 0x80000000u));
+}
+
 // SuperCell::pbc (src/util/SuperCell.cc:25-34): minimum image, only applied
 // when |v|^2 exceeds a quarter of the shortest side squared.
-__device__ __forceinline__ void pbc(const DevSys& s, double& x, double& y, double& z) {
+static __device__ __noinline__ double3 pbc_exact(const DevSys& s, double x, double y, double z) {
   if (dot3(x, y, z, x, y, z) > s.rcut2) {
     const double ix = floor(__dadd_rn(__dmul_rn(s.cellb[0], x), 1000.5)) - 1000;
     const double iy = floor(__dadd_rn(__dmul_rn(s.cellb[1], y), 1000.5)) - 1000;
@@ -105,24 +132,72 @@ __device__ __forceinline__ void pbc(const DevSys& s, double& x, double& y, doubl
     y = __dsub_rn(y, __dmul_rn(s.cell[1], iy));
     z = __dsub_rn(z, __dmul_rn(s.cell[2], iz));
   }
+  return make_double3(x, y, z);
+}
+
+// The box side to subtract from component v of |v| ~ f (abs_f32_trunc) for its
+// minimum image: 0 or +-L; ok is cleared where the rounding of v / L is not
+// certain (within 4e-5 of a half-integer: the FP32 quotient errs by under 3e-6)
+// or where it is beyond one box.
+__device__ __forceinline__ double image_shift(double cell, float cellb, double v, float f,
+                                              bool& ok) {
+  const float u = f * cellb;
+  ok &= fabsf(u - 0.5f) > 4e-5f && u < 1.4999f;  // (false for NaN)
+  return u > 0.5f ? copysign(cell, v) : 0.0;
+}
+
+// pbc_exact with its test and its image numbers taken on the FP32 pipe where
+// they are certain there: the same bits.  What is left of FP64 is nothing for a
+// vector inside the cutoff (was 6 instructions) and three subtractions for an
+// imaged one (was 24).  A step of 152 electron gases (N = 54, M = 512, 64 attempts)
+// 115 -> 97 ms, of 9728 two-electron dots (32 attempts) 59.2 -> 53.2 ms.
+__device__ __forceinline__ double3 pbc_far(const DevSys& s, double x, double y, double z,
+                                           float fx, float fy, float fz, float r2) {
+  bool ok = r2 > s.rcut2_hi;
+  const double cx = image_shift(s.cell[0], s.cellb_f[0], x, fx, ok);
+  const double cy = image_shift(s.cell[1], s.cellb_f[1], y, fy, ok);
+  const double cz = image_shift(s.cell[2], s.cellb_f[2], z, fz, ok);
+  return ok ? make_double3(__dsub_rn(x, cx), __dsub_rn(y, cy), __dsub_rn(z, cz))
+            : pbc_exact(s, x, y, z);
+}
+
+// (a call: one copy for the movers' many images)
+static __device__ __noinline__ double3 pbc_far_call(const DevSys& s, double x, double y, double z,
+                                                    float fx, float fy, float fz, float r2) {
+  return pbc_far(s, x, y, z, fx, fy, fz, r2);
+}
+
+__device__ __forceinline__ void pbc(const DevSys& s, double& x, double& y, double& z) {
+  const float fx = abs_f32_trunc(x), fy = abs_f32_trunc(y), fz = abs_f32_trunc(z);
+  const float r2 = fx * fx + fy * fy + fz * fz;
+  if (!(r2 < s.rcut2_lo)) {
+    const double3 v = pbc_far_call(s, x, y, z, fx, fy, fz, r2);
+    x = v.x;
+    y = v.y;
+    z = v.z;
+  }
+}
+
+// |v|^2 of the FP32 terms, every rounding written out: the same bits in every
+// kernel, however the compiler would contract the sum.
+__device__ __forceinline__ float norm2_f(float x, float y, float z) {
+  return __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x)));
 }
 
 // The mixed form's minimum image of an FP64 difference, rounded to FP32 for
-// its FP32 terms: pbc()'s decision taken in FP32 first, against rcut2 less
-// 1e-5 relative (the FP32 sum of three rounded squares errs by under 5e-7
-// relative, all terms positive), so every vector pbc() would image passes
-// the pre-test and then takes pbc()'s own FP64 test and image; the others
-// skip its FP64 dot product.
+// its FP32 terms (pbc's image, then the rounding, both without FP64
+// conversions).
 __device__ __forceinline__ void pbc_f(const DevSys& s, double x, double y, double z, float& fx,
                                       float& fy, float& fz) {
-  fx = (float)x;
-  fy = (float)y;
-  fz = (float)z;
-  if (fx * fx + fy * fy + fz * fz > s.rcut2_lo) {
-    pbc(s, x, y, z);
-    fx = (float)x;
-    fy = (float)y;
-    fz = (float)z;
+  fx = f32_rn(x);
+  fy = f32_rn(y);
+  fz = f32_rn(z);
+  const float r2 = fx * fx + fy * fy + fz * fz;
+  if (!(r2 < s.rcut2_lo)) {
+    const double3 v = pbc_far(s, x, y, z, fabsf(fx), fabsf(fy), fabsf(fz), r2);
+    fx = f32_rn(v.x);
+    fy = f32_rn(v.y);
+    fz = f32_rn(v.z);
   }
 }
 
@@ -238,7 +313,7 @@ __device__ __forceinline__ float tab_uk0_f(const DevTable& t, float q, float s2,
 // FP32 tau derivative of the off-diagonal series (uk0CalcDerivatives' utau).
 __device__ __forceinline__ float tab_uk0d_tau_f(const DevTable& t, float q, float s2) {
   q *= (float)t.rgridinv;
-  float x = __logf(q) * (float)t.logrratioinv;
+  float x = __fmul_rn(__logf(q), (float)t.logrratioinv);
   int i;  // range tests before the conversion, as tab_locate
   if (!(q >= 1.f)) {
     i = 0;
@@ -248,7 +323,7 @@ __device__ __forceinline__ float tab_uk0d_tau_f(const DevTable& t, float q, floa
     x = 1.f;
   } else {
     i = (int)x;
-    x -= i;
+    x = __fsub_rn(x, (float)i);
   }
   const float* g0 = t.ugrid32 + (size_t)i * 2 * t.ndata + t.ndata;
   const float* g1 = g0 + 2 * t.ndata;
