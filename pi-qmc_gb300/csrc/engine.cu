@@ -310,9 +310,16 @@ void fill_sys(const pimc_system& s, DevSys& d) {
       const double sinhwt = std::sinh(w * 0.5 / T);
       d.node_c[i] = s.spec_mass[i] * 0.5 * w / sinhwt;
     } else if (s.node_kind[i] == PIMC_NODES_FREE) {
-      for (int a = 0; a < 3; ++a)
-        pg_params(s.spec_mass[i] * s.node_temperature, s.cell[a], d.pg_nome[i][a], d.pg_pref[i][a],
-                  d.pg_k[i][a], d.pg_nmax[i][a]);
+      d.pg_alpha[i] = s.spec_mass[i] * s.node_temperature;
+      d.pg_images[i] = 1;
+      for (int a = 0; a < 3; ++a) {
+        pg_params(d.pg_alpha[i], s.cell[a], d.pg_nome[i][a], d.pg_pref[i][a], d.pg_k[i][a],
+                  d.pg_nmax[i][a]);
+        d.pg_al[i][a] = d.pg_alpha[i] * s.cell[a];
+        const double al2 = d.pg_al[i][a] * s.cell[a];
+        if (!(al2 >= 20.0)) d.pg_images[i] = 0;
+        d.pg_c[i][a] = al2 < 40.0 ? std::exp(-2.0 * al2) : 0.0;
+      }
     }
   }
   d.tau = s.tau;

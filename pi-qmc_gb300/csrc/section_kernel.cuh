@@ -176,15 +176,20 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
     } else {
       double dx = rjx - rix, dy = rjy - riy, dz = rjz - riz;
       pbc(s, dx, dy, dz);
-      double g0, g1, g2;
-      const double v0 = pg_eval(s.pg_nome[sp][0], s.pg_pref[sp][0], s.pg_k[sp][0], s.pg_nmax[sp][0], dx, &g0);
-      const double v1v = pg_eval(s.pg_nome[sp][1], s.pg_pref[sp][1], s.pg_k[sp][1], s.pg_nmax[sp][1], dy, &g1);
-      const double v2v = pg_eval(s.pg_nome[sp][2], s.pg_pref[sp][2], s.pg_k[sp][2], s.pg_nmax[sp][2], dz, &g2);
-      const double val = v0 * v1v * v2v;
-      double gx = g0 / (v0 + 1e-300), gy = g1 / (v1v + 1e-300), gz = g2 / (v2v + 1e-300);
-      gx *= v0; gy *= v0; gz *= v0;
-      gx *= v1v; gy *= v1v; gz *= v1v;
-      gx *= v2v; gy *= v2v; gz *= v2v;
+      double val, gx, gy, gz;
+      if (s.pg_images[sp]) {
+        val = pg_images_eval(s, sp, dx, dy, dz, gx, gy, gz);
+      } else {
+        double g0, g1, g2;
+        const double v0 = pg_eval(s.pg_nome[sp][0], s.pg_pref[sp][0], s.pg_k[sp][0], s.pg_nmax[sp][0], dx, &g0);
+        const double v1v = pg_eval(s.pg_nome[sp][1], s.pg_pref[sp][1], s.pg_k[sp][1], s.pg_nmax[sp][1], dy, &g1);
+        const double v2v = pg_eval(s.pg_nome[sp][2], s.pg_pref[sp][2], s.pg_k[sp][2], s.pg_nmax[sp][2], dz, &g2);
+        val = v0 * v1v * v2v;
+        gx = g0 / (v0 + 1e-300), gy = g1 / (v1v + 1e-300), gz = g2 / (v2v + 1e-300);
+        gx *= v0; gy *= v0; gz *= v0;
+        gx *= v1v; gy *= v1v; gz *= v1v;
+        gx *= v2v; gy *= v2v; gz *= v2v;
+      }
       if (to_cache) {
         ecache[j * n + i] = val;
         ecache[nn + j * n + i] = gx;

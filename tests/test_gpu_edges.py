@@ -63,3 +63,48 @@ def test_minimum_image_edges(pimc, cell):
     mixed = pimc.Engine(kw, 1, tabs, precision=pimc.PIMC_PREC_MIXED)
     mixed.upload_paths([x])
     assert abs(mixed.thermo_energy()[0] - want) <= 1e-5 * abs(want)
+
+
+def _pg_images(al, cell, x):
+    """Periodic Gaussian and its derivative by nine images: every term positive."""
+    m = np.arange(-4, 5)[:, None, None, None, None]
+    g = np.exp(-al * (x - m * cell) ** 2)
+    return g.sum(0), (-2 * al * (x - m * cell) * g).sum(0)
+
+
+@pytest.mark.parametrize("al2", [8.0, 19.999999, 20.000001, 39.999999, 40.000001, 400.0])
+@pytest.mark.parametrize("n", [2, 9, 17])
+def test_periodic_gaussian_images(pimc, al2, n):
+    # Free-particle nodes on both sides of the line between the series and the
+    # images, and with and without the second one, with separations up to exactly
+    # half the box.  Forward error of the determinant and of the gradients: n eps
+    # of the norms that enter.
+    cell = 16.0
+    kw = W.heg54(n=2 * n, nslice=64, nlevel=3, coulomb=0, ewald=0, cell=cell, beta=2.0,
+                 node_temperature=al2 / cell ** 2)
+    rng = np.random.default_rng(n)
+    nb = 12
+    r1 = rng.uniform(-cell / 2, cell / 2, size=(nb, 2 * n, 3))
+    r2 = r1 + 0.15 * cell * rng.normal(size=r1.shape) / np.sqrt(al2)
+    r2[0, 0] = r1[0, 1] + [cell / 2, 0.3 * cell, 0.0]
+    r2[1, 1] = r1[1, 0] + [cell / 2, -cell / 2, cell / 2]
+    r2[2, 0] = r1[2, 0]
+    e = pimc.Engine(kw, 1)
+    err, det, d1, _ = e.node_evaluate(0, r1, r2)
+    x = r1[:, None, :n] - r2[:, :n, None]  # [b][i of r2][j of r1]
+    x = x - cell * np.floor(x / cell + 0.5)
+    v, dv = _pg_images(al2 / cell ** 2, cell, x)
+    rho = v.prod(-1)
+    grad = np.stack([dv[..., 0] * v[..., 1] * v[..., 2], v[..., 0] * dv[..., 1] * v[..., 2],
+                     v[..., 0] * v[..., 1] * dv[..., 2]], -1)
+    cond = np.linalg.cond(rho)
+    # the series errs by ~1e-13 of its largest element where it cancels
+    tol = (1e-12 if al2 < 20 else 1e-13) * n * cond
+    assert not err.any()
+    assert np.all(np.abs(det - np.linalg.det(rho)) <= tol * np.abs(det))
+    inv = np.linalg.inv(rho)
+    log = np.einsum("bji,bijd->bjd", inv, grad)
+    ref = np.sqrt(2 / (kw["beta"] / 64 * ((log ** 2).sum(-1) + 1e-15)))
+    size = np.einsum("bji,bijd->bjd", np.abs(inv), np.abs(grad)).sum(-1)
+    slack = tol[:, None] * size * np.sqrt(kw["beta"] / 64 / 2) * ref ** 2 + 1e-12 * ref
+    assert np.all(np.abs(d1[:, :n] - ref) <= slack)
