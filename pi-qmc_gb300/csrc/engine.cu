@@ -130,6 +130,8 @@ struct LayoutOpts {
   bool scratch_global = false;  // per-warp Slater scratch in global memory even when it fits
   bool cold_global = false;     // its cold parts in global memory even when all of it fits
   bool full_ewald_tables = false;  // Ewald tables for every bead (full evalLongRange sums)
+  bool single_levels = false;      // action differences of one level at a time only
+  bool no_actions = false;         // no buffers for the action differences (displacement moves)
 };
 
 struct pimc_engine {
@@ -466,7 +468,7 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
   L.mv = take(3 * nsec);
   L.nrm = take(3 * nsec);
   L.red = take(64);
-  L.vred = take(9 * kWarps);
+  L.old = take(nsec);
   L.q = take(np);
   L.dm = take(kMaxSpecies * nsec);
   L.ndm = take(nsec);
@@ -534,6 +536,25 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
   L.nodescr = L.nodescr_in_smem ? take(nwarps * L.nodescr_stride) : -1;
   const int gwarp = L.split ? cold : (L.nodescr_in_smem ? 0 : full);
   L.gcta = nwarps * gwarp + (L.ncol_global ? ncol_size : 0);
+  // the action differences' buffers: the warps' Slater scratch where that is in
+  // shared memory (a warp is done with it by then), else their own
+  if (!opts.no_actions) {
+    int need = 0;
+    for (const DevSys& d : sys) {
+      // (a launch of all levels together alone needs no buffer for a single one)
+      const bool single = opts.single_levels || d.fixed_node || d.dr || d.ewald;
+      need = std::max(need, action_buffer(d.nlevel, single, d.mixed != 0));
+    }
+    if (L.nodescr_in_smem && L.nodescr_stride >= need) {
+      L.act = -1;
+      L.act_stride = L.nodescr_stride;
+    } else {
+      L.act_stride = need;
+      L.act_global = off + nwarps * need > limit;
+      L.act = L.act_global ? -1 : take(nwarps * need);
+      if (L.act_global) L.gcta += nwarps * need;
+    }
+  }
   L.total = off;
   ok = L.total <= limit;
   return L;
@@ -577,7 +598,9 @@ Layout estimator_layout(const std::vector<DevSys>& sys, const int* ikmax_extra) 
   L.mv = take(3 * nsec);
   L.nrm = L.mv;
   L.red = take(64);
-  L.vred = L.red;
+  L.old = L.red;
+  L.act = 0;
+  L.act_stride = L.act_global = 0;
   L.q = take(np);
   L.ewt = take(2 * ((ik[0] + 1) + (2 * ik[1] + 1) + (2 * ik[2] + 1)) * (np + 1));
   L.ictl = take(C_NCTL + 2);
@@ -1348,6 +1371,7 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
   // (full Ewald tables: every slice's evalLongRange is summed here)
   LayoutOpts dopt;
   dopt.full_ewald_tables = true;
+  dopt.no_actions = true;
   bool lok = false;
   Layout L = make_layout(e->hsys, nwarps, lok, dopt);
   if (!lok || (size_t)(L.total + nwarps * stage) * 8 > (size_t)kSmemLimit) {
@@ -1520,12 +1544,15 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   LayoutOpts aopt;
   aopt.scratch_global = true;
   aopt.full_ewald_tables = true;
+  aopt.single_levels = true;
   bool lok = false;
   const Layout alay = make_layout(e->hsys, kBlock / 32, lok, aopt);
   if (!lok) return fail(PIMC_ERR_CAPACITY, "working set does not fit in shared memory");
   const size_t nsecd = (size_t)nbatch * s.nsec * s.npart * 3, nmovd = (size_t)nbatch * s.nsec * 3;
-  double *d_sec = nullptr, *d_mov = nullptr, *d_ds = nullptr;
+  double *d_sec = nullptr, *d_mov = nullptr, *d_ds = nullptr, *d_scr = nullptr;
   int* d_ip = nullptr;
+  if (alay.act_global)
+    CU(cudaMallocAsync(&d_scr, (size_t)nbatch * alay.gcta * 8, e->stream));
   CU(cudaMallocAsync(&d_sec, nsecd * 8, e->stream));
   CU(cudaMallocAsync(&d_mov, nmovd * 8, e->stream));
   CU(cudaMallocAsync(&d_ds, nbatch * 8, e->stream));
@@ -1541,10 +1568,12 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   P.ds = d_ds;
   P.level = level;
   P.lay = alay;
+  P.scratch = d_scr;
   action_diff_kernel<<<nbatch, kBlock, P.lay.total * 8, e->stream>>>(P);
   e->launches++;
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(ds, d_ds, nbatch * 8, cudaMemcpyDeviceToHost, e->stream));
+  if (d_scr) CU(cudaFreeAsync(d_scr, e->stream));
   CU(cudaFreeAsync(d_sec, e->stream));
   CU(cudaFreeAsync(d_mov, e->stream));
   CU(cudaFreeAsync(d_ds, e->stream));

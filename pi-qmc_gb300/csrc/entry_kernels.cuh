@@ -572,6 +572,7 @@ struct ActionDiffParams {
   double* ds;
   int level;
   Layout lay;
+  double* scratch;  // the layout's global area per CTA (null: none)
 };
 
 __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P) {
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   }
   __syncthreads();
   const DevSys& s = S;
-  Smem m = carve(smem, P.lay, s, nullptr);
+  Smem m = carve(smem, P.lay, s, P.scratch);
   const int b = blockIdx.x, np = s.npart, nsec = s.nsec;
   const double* sec = P.section + (size_t)b * nsec * np * 3;
   const double* mov = P.moving + (size_t)b * nsec * 3;
@@ -602,7 +603,16 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
   __syncthreads();
   const int ip = P.ipart[b];
-  double ds = block_sum(action_partial(s, m, ip, P.level, threadIdx.x, blockDim.x), m.red);
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, d = s.nlevel - P.level;
+  double* lds = m.red + kWarps + 8;
+  if (s.mixed)
+    action_warp<true>(s, m, ip, d, d, warp, nw, m.act + warp * m.act_stride);
+  else
+    action_warp<false>(s, m, ip, d, d, warp, nw, m.act + warp * m.act_stride);
+  __syncthreads();
+  action_reduce(s, m.act, m.act_stride, d, d, nw, lds);
+  __syncthreads();
+  double ds = lds[P.level];
   if (s.ewald && s.coulomb && P.level == 0)
     for (int t = 1; t < nsec - 1; ++t) ds += ewald_slice_diff(s, m, ip, t);
   if (threadIdx.x == 0) P.ds[b] = ds;

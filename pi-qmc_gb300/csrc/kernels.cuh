@@ -2,7 +2,7 @@
 // fixed-node set-up and levels, and the persistent kernel itself.
 #pragma once
 #include "../../include/pimc_gb300.h"
-#include "section_kernel.cuh"
+#include "actions.cuh"
 
 namespace pimc {
 
@@ -12,7 +12,9 @@ struct Layout {
   int s1, s2, mv, red, q, dm, ndm, dist, ndist, ewt, nodescr, ictl, ecache, ncol;
   int ncol_stride;
   int nrm;  // the attempt's normals, 3 per movable slice
-  int vred;             // vector reductions: [8][kWarps] partials, then 8 sums
+  int old;  // the mover's terms of the old beads
+  int act, act_stride, act_global;  // per-warp buffers of the action differences: offset
+                                    // (-1: the warps' Slater scratch, or the CTA's global area)
   int nodescr_in_smem;  // the node scratch (its hot parts when split) in shared memory
   int nodescr_stride;   // doubles per warp of that scratch
   int split;            // cold parts apart, in the CTA's global area
@@ -62,7 +64,7 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
   m.my = m.mx + s.nsec;
   m.mz = m.my + s.nsec;
   m.red = base + L.red;
-  m.vred = base + L.vred;
+  m.old = base + L.old;
   m.qpart = base + L.q;
   m.dm = base + L.dm;
   m.ndm = base + L.ndm;
@@ -85,14 +87,10 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
   m.ncol_stride = L.ncol_stride;
   m.nodescr_stride = L.nodescr_stride;
   m.nodescr = L.nodescr_in_smem ? base + L.nodescr : gbase;
+  m.act = L.act >= 0 ? base + L.act
+                     : (L.act_global ? gbase + (L.gcta - nw * L.act_stride) : m.nodescr);
+  m.act_stride = L.act_stride;
   return m;
-}
-
-__device__ __forceinline__ int species_of(const DevSys& s, int p) {
-  int r = 0;
-  for (int k = 0; k < s.nspecies; ++k)
-    if (p >= s.spec_first[k] && p < s.spec_first[k] + s.spec_count[k]) r = k;
-  return r;
 }
 
 // Section slice k of a section starting at ifirst, in path slice numbering with
@@ -182,35 +180,222 @@ static __device__ __noinline__ void store_section(const DevSys& s, double* path,
   }
 }
 
-// FreeMover::makeMove (src/advancer/mover/FreeMover.cc:59-124) and
-// FreeMoverPBC::makeMove (src/advancer/mover/FreeMoverPBC.cc:59-152) for one
-// moving particle at one level; threads own moved slices.  Returns ln(T_old/T_new).
 // Every normal the attempt's mover can use, drawn in parallel before the
 // levels: moved slice `ord` (0 .. 2^L - 2 in FreeMover's order) takes Box-Muller
 // pairs 2 ord and 2 ord + 1 and uses the first three values.  Both precision
 // forms draw the same FP64 normals, so a mixed-form chain makes the FP64
 // chain's proposals and its action differences can be compared with the FP64
-// form's on identical moves.
+// form's on identical moves.  Whole warps draw the first or the second pairs.
 static __device__ __noinline__ void attempt_normals(const DevSys& s, const Smem& m, uint64_t seed,
                                        uint32_t rep, uint32_t att) {
   // (with delayed rejection one more: the second proposal at level nlevel - 1
   // takes order 1, the slices after it one order later)
-  const int nord = (1 << s.nlevel) - 1 + (s.dr ? 1 : 0);
-  for (int o = threadIdx.x; o < nord; o += blockDim.x) {
-    double z0, z1, z2, z3;
-    stream_normal_pair(seed, rep, att, 2u * o, &z0, &z1);
-    stream_normal_pair(seed, rep, att, 2u * o + 1u, &z2, &z3);
-    m.nrm[3 * o] = z0;
-    m.nrm[3 * o + 1] = z1;
-    m.nrm[3 * o + 2] = z2;
+  const int nord = (1 << s.nlevel) - 1 + (s.dr ? 1 : 0), pad = (nord + 31) & ~31;
+  for (int it = threadIdx.x; it < 2 * pad; it += blockDim.x) {
+    const int second = it >= pad, o = it - second * pad;
+    if (o >= nord) continue;
+    double z0, z1;
+    stream_normal_pair(seed, rep, att, 2u * o + second, &z0, &z1);
+    if (second) {
+      m.nrm[3 * o + 2] = z0;
+    } else {
+      m.nrm[3 * o] = z0;
+      m.nrm[3 * o + 1] = z1;
+    }
   }
 }
 
+// The uniform-stream index of the first uniform consumed at `level`
+// (image choices of FreeMoverPBC, then the Metropolis uniform).
+__device__ __forceinline__ uint32_t level_uniform_base(const DevSys& s, int level) {
+  uint32_t u = (s.fixed_node ? 2u : 1u) + 1u;  // section choice + particle choice
+  const uint32_t pbcu = s.mover == PIMC_MOVER_FREE_PBC ? 3u : 0u;
+  for (int l = s.nlevel; l > level; --l) {
+    const uint32_t nmov = (l == s.nlevel) ? 0u : (1u << (s.nlevel - l - 1));
+    u += pbcu * nmov + 1u;
+  }
+  return u;
+}
+
+// FreeMoverPBC's image choice of a midpoint offset md (half the separation of the
+// neighbouring beads): md or md + L/2 with probabilities w1 = exp(-md^2 / 2 sigma^2)
+// against w2.  |md + L/2| >= L/2 - |md|, so when ((L/2 - |md|)^2 - md^2) / 2 sigma^2
+// > 40 on every axis w2 is below 2^-57 w1, w1 / (w1 + w2) rounds to 1 (or is 0/0)
+// and no uniform exceeds it: the exponentials and uniforms are left out.  That is
+// every choice in a box much wider than the level's sigma.
+__device__ __forceinline__ void mover_image(const DevSys& s, double md[3], double inv2Sigma2,
+                                            uint64_t seed, uint32_t rep, uint32_t att,
+                                            uint32_t u0) {
+  const float w = (float)inv2Sigma2;
+  bool sure = true;
+  for (int d = 0; d < 3; ++d) {
+    const float c = (float)s.cell[d], a = abs_f32_trunc(md[d]) * 1.000002f;
+    sure &= w * (c * (0.25f * c - a)) > 40.f * 1.0001f;
+  }
+  if (sure) return;
+  double m2[3] = {md[0] + 0.5 * s.cell[0], md[1] + 0.5 * s.cell[1], md[2] + 0.5 * s.cell[2]};
+  pbc(s, m2[0], m2[1], m2[2]);
+  for (int d = 0; d < 3; ++d) {
+    // No periodic Gaussian on the mover path (the engine rejects boxes that need one).
+    const double w1 = exp(-inv2Sigma2 * md[d] * md[d]);
+    const double w2 = exp(-inv2Sigma2 * m2[d] * m2[d]);
+    const double u = stream_uniform(seed, rep, att, u0 + d);
+    if (u > w1 / (w1 + w2)) md[d] = m2[d];
+  }
+}
+
+// FreeMover::makeMove (src/advancer/mover/FreeMover.cc:59-124) and
+// FreeMoverPBC::makeMove (src/advancer/mover/FreeMoverPBC.cc:59-152) for one moving
+// particle at every level.  Moved slices are the nodes of a binary heap: slot n >= 1
+// of depth d = floor(log2 n) is moved at level nlevel - 1 - d, and takes normals
+// n - 1.  What does not depend on the new beads (the old beads' terms here, the
+// proposals' own in mover_all) runs on one lane per slice of every level; only the
+// midpoints go level by level.  (Level by level with everything in it, each level
+// cost the FP64 pipe the same 55 instructions for its 1, 2, 4 ... slices.)
+__device__ __forceinline__ void moved_slice(int L, int slot, int& level, int& t, int& k) {
+  const int d = 31 - __clz(slot);
+  level = L - 1 - d;
+  k = slot - (1 << d);
+  t = (2 * k + 1) << level;
+}
+
+// The old beads' part of ln(T_old / T_new), per moved slice into m.old.  One warp.
+static __device__ __noinline__ void mover_old(const DevSys& s, const Smem& m, int ipart) {
+  const int np = s.npart, sp = species_of(s, ipart);
+  for (int slot = threadIdx.x & 31; slot < (1 << s.nlevel); slot += 32) {
+    if (slot == 0) continue;
+    int level, t, k;
+    moved_slice(s.nlevel, slot, level, t, k);
+    const int tp = t - (1 << level), tn = t + (1 << level);
+    const double inv2Sigma2 = s.mov_inv2s2[level][sp];
+    const double ox = m.s1x[t * np + ipart], oy = m.s1y[t * np + ipart], oz = m.s1z[t * np + ipart];
+    const double opx = m.s1x[tp * np + ipart], opy = m.s1y[tp * np + ipart], opz = m.s1z[tp * np + ipart];
+    const double onx = m.s1x[tn * np + ipart], ony = m.s1y[tn * np + ipart], onz = m.s1z[tn * np + ipart];
+    double acc = 0.0;
+    if (s.mover == PIMC_MOVER_FREE) {
+      double ax = onx - opx, ay = ony - opy, az = onz - opz;
+      pbc(s, ax, ay, az);
+      ax = __fma_rn(ax, 0.5, opx);  // (halving is exact)
+      ay = __fma_rn(ay, 0.5, opy);
+      az = __fma_rn(az, 0.5, opz);
+      pbc(s, ax, ay, az);
+      double ex = ox - ax, ey = oy - ay, ez = oz - az;
+      pbc(s, ex, ey, ez);
+      acc -= ex * ex * inv2Sigma2;
+      acc -= ey * ey * inv2Sigma2;
+      acc -= ez * ez * inv2Sigma2;
+    } else {
+      double po[3] = {ox - opx, oy - opy, oz - opz}, no[3] = {ox - onx, oy - ony, oz - onz};
+      double dol[3] = {onx - opx, ony - opy, onz - opz};
+      pbc(s, po[0], po[1], po[2]);
+      pbc(s, no[0], no[1], no[2]);
+      pbc(s, dol[0], dol[1], dol[2]);
+      for (int d = 0; d < 3; ++d) {
+        acc -= po[d] * po[d] * inv2Sigma2 * 0.5;
+        acc -= no[d] * no[d] * inv2Sigma2 * 0.5;
+        acc += dol[d] * dol[d] * inv2Sigma2 * 0.25;
+      }
+    }
+    m.old[slot] = acc;
+  }
+}
+
+// The new beads of every level, and ln(T_old / T_new) per level into llt.  One
+// warp; reads the section's end beads in m.mx, m.nrm and m.old.
+static __device__ __noinline__ void mover_all(const DevSys& s, const Smem& m, int ipart,
+                                              uint64_t seed, uint32_t att, double* llt) {
+  const int L = s.nlevel, lane = threadIdx.x & 31, sp = species_of(s, ipart);
+  if (lane == 0) llt[L] = 0.0;  // the top level moves nothing
+  for (int c = 0; 32 * c < (1 << L); ++c) {
+    const int slot = 32 * c + lane;
+    const bool on = slot > 0 && slot < (1 << L);
+    int level, t, k;
+    moved_slice(L, on ? slot : 1, level, t, k);
+    const int tp = t - (1 << level), tn = t + (1 << level), ord = on ? slot - 1 : 0;
+    const double sigma = s.mov_sigma[level][sp], inv2Sigma2 = s.mov_inv2s2[level][sp];
+    const double z0 = m.nrm[3 * ord], z1 = m.nrm[3 * ord + 1], z2 = m.nrm[3 * ord + 2];
+    double acc = 0.0;
+    const int dlo = c ? 5 : 0, dhi = c ? 5 : min(4, L - 1);
+    if (s.mover == PIMC_MOVER_FREE) {
+      double dx = __dmul_rn(z0, sigma), dy = __dmul_rn(z1, sigma), dz = __dmul_rn(z2, sigma);
+      pbc(s, dx, dy, dz);
+      acc += dx * dx * inv2Sigma2;
+      acc += dy * dy * inv2Sigma2;
+      acc += dz * dz * inv2Sigma2;
+      for (int d = dlo; d <= dhi; ++d) {
+        if (on && level == L - 1 - d) {
+          const double mpx = m.mx[tp], mpy = m.my[tp], mpz = m.mz[tp];
+          double x = m.mx[tn] - mpx, y = m.my[tn] - mpy, z = m.mz[tn] - mpz;
+          pbc(s, x, y, z);
+          x = __fma_rn(x, 0.5, mpx);
+          y = __fma_rn(y, 0.5, mpy);
+          z = __fma_rn(z, 0.5, mpz);
+          pbc(s, x, y, z);
+          x = __dadd_rn(x, dx);
+          y = __dadd_rn(y, dy);
+          z = __dadd_rn(z, dz);
+          pbc(s, x, y, z);
+          m.mx[t] = x;
+          m.my[t] = y;
+          m.mz[t] = z;
+        }
+        __syncwarp();
+      }
+    } else {
+      for (int d = dlo; d <= dhi; ++d) {
+        if (on && level == L - 1 - d) {
+          const double mpx = m.mx[tp], mpy = m.my[tp], mpz = m.mz[tp];
+          double md[3] = {m.mx[tn] - mpx, m.my[tn] - mpy, m.mz[tn] - mpz};
+          pbc(s, md[0], md[1], md[2]);
+          md[0] *= 0.5; md[1] *= 0.5; md[2] *= 0.5;
+          mover_image(s, md, inv2Sigma2, seed, s.stream_id, att,
+                      level_uniform_base(s, level) + 3u * k);
+          double x = __fma_rn(z0, sigma, __dadd_rn(md[0], mpx));
+          double y = __fma_rn(z1, sigma, __dadd_rn(md[1], mpy));
+          double z = __fma_rn(z2, sigma, __dadd_rn(md[2], mpz));
+          pbc(s, x, y, z);
+          m.mx[t] = x;
+          m.my[t] = y;
+          m.mz[t] = z;
+        }
+        __syncwarp();
+      }
+      if (on) {
+        const double nx = m.mx[t], ny = m.my[t], nz = m.mz[t];
+        const double mpx = m.mx[tp], mpy = m.my[tp], mpz = m.mz[tp];
+        const double mnx = m.mx[tn], mny = m.my[tn], mnz = m.mz[tn];
+        double pn[3] = {nx - mpx, ny - mpy, nz - mpz}, nn[3] = {nx - mnx, ny - mny, nz - mnz};
+        double dn[3] = {mnx - mpx, mny - mpy, mnz - mpz};
+        pbc(s, pn[0], pn[1], pn[2]);
+        pbc(s, nn[0], nn[1], nn[2]);
+        pbc(s, dn[0], dn[1], dn[2]);
+        for (int d = 0; d < 3; ++d) {
+          acc += pn[d] * pn[d] * inv2Sigma2 * 0.5;
+          acc += nn[d] * nn[d] * inv2Sigma2 * 0.5;
+          acc -= dn[d] * dn[d] * inv2Sigma2 * 0.25;
+        }
+      }
+    }
+    double x = on ? acc + m.old[slot] : 0.0;
+    if (c == 0) {
+      x = fold_by_depth(x, min(32, 1 << L));
+      const int d = 31 - __clz(max(lane, 1));
+      if (on && lane == (1 << d)) llt[L - 1 - d] = x;
+    } else {
+      x = fold_warp(x);
+      if (lane == 0) llt[L - 6] = x;
+    }
+  }
+  __syncwarp();
+}
+
+// The movers' makeMove for one moving particle at one level (delayed rejection,
+// whose second proposal shifts the normals and uniforms of the levels under it);
+// threads own moved slices.  Returns ln(T_old/T_new).
 // oshift: moved-slice orders taken by a delayed-rejection proposal before
 // this level; second: the delayed-rejection proposal itself (its width).
 static __device__ __noinline__ double mover_level_part(const DevSys& s, const Smem& m, int ipart, int level,
-                              uint64_t seed, uint32_t rep, uint32_t att, uint32_t ubase,
-                              int oshift = 0, bool second = false) {
+                              int oshift, bool second) {
   const int L = s.nlevel, np = s.npart;
   const int nStride = 1 << level;
   const int nmov = (level == L) ? 0 : (1 << (L - level - 1));
@@ -230,99 +415,40 @@ static __device__ __noinline__ double mover_level_part(const DevSys& s, const Sm
     const double mpx = m.mx[tp], mpy = m.my[tp], mpz = m.mz[tp];
     const double mnx = m.mx[tn], mny = m.my[tn], mnz = m.mz[tn];
     double acc = 0.0;
-    if (s.mover == PIMC_MOVER_FREE) {
-      double mdx = mnx - mpx, mdy = mny - mpy, mdz = mnz - mpz;
-      pbc(s, mdx, mdy, mdz);
-      mdx *= 0.5; mdy *= 0.5; mdz *= 0.5;
-      mdx += mpx; mdy += mpy; mdz += mpz;
-      pbc(s, mdx, mdy, mdz);
-      double dx = z0 * sigma, dy = z1 * sigma, dz = z2 * sigma;
-      pbc(s, dx, dy, dz);
-      double nx = mdx + dx, ny = mdy + dy, nz = mdz + dz;
-      pbc(s, nx, ny, nz);
-      m.mx[t] = nx;
-      m.my[t] = ny;
-      m.mz[t] = nz;
-      acc += dx * dx * inv2Sigma2;
-      acc += dy * dy * inv2Sigma2;
-      acc += dz * dz * inv2Sigma2;
-      double ax = onx - opx, ay = ony - opy, az = onz - opz;
-      pbc(s, ax, ay, az);
-      ax *= 0.5; ay *= 0.5; az *= 0.5;
-      ax += opx; ay += opy; az += opz;
-      pbc(s, ax, ay, az);
-      double ex = ox - ax, ey = oy - ay, ez = oz - az;
-      pbc(s, ex, ey, ez);
-      acc -= ex * ex * inv2Sigma2;
-      acc -= ey * ey * inv2Sigma2;
-      acc -= ez * ez * inv2Sigma2;
-    } else {
-      double md[3] = {mnx - mpx, mny - mpy, mnz - mpz};
-      pbc(s, md[0], md[1], md[2]);
-      md[0] *= 0.5; md[1] *= 0.5; md[2] *= 0.5;
-      double m2[3] = {md[0] + 0.5 * s.cell[0], md[1] + 0.5 * s.cell[1], md[2] + 0.5 * s.cell[2]};
-      pbc(s, m2[0], m2[1], m2[2]);
-      for (int d = 0; d < 3; ++d) {
-        // No periodic Gaussian on the mover path (the engine rejects boxes that need one).
-        const double w1 = exp(-inv2Sigma2 * md[d] * md[d]);
-        const double w2 = exp(-inv2Sigma2 * m2[d] * m2[d]);
-        const double u = stream_uniform(seed, rep, att, ubase + 3u * k + d);
-        if (u > w1 / (w1 + w2)) md[d] = m2[d];
-      }
-      double nx = md[0] + mpx + z0 * sigma, ny = md[1] + mpy + z1 * sigma, nz = md[2] + mpz + z2 * sigma;
-      pbc(s, nx, ny, nz);
-      m.mx[t] = nx;
-      m.my[t] = ny;
-      m.mz[t] = nz;
-      double pn[3] = {nx - mpx, ny - mpy, nz - mpz}, nn[3] = {nx - mnx, ny - mny, nz - mnz};
-      double dn[3] = {mnx - mpx, mny - mpy, mnz - mpz};
-      double po[3] = {ox - opx, oy - opy, oz - opz}, no[3] = {ox - onx, oy - ony, oz - onz};
-      double dol[3] = {onx - opx, ony - opy, onz - opz};
-      pbc(s, pn[0], pn[1], pn[2]);
-      pbc(s, nn[0], nn[1], nn[2]);
-      pbc(s, dn[0], dn[1], dn[2]);
-      pbc(s, po[0], po[1], po[2]);
-      pbc(s, no[0], no[1], no[2]);
-      pbc(s, dol[0], dol[1], dol[2]);
-      for (int d = 0; d < 3; ++d) {
-        acc -= po[d] * po[d] * inv2Sigma2 * 0.5;
-        acc -= no[d] * no[d] * inv2Sigma2 * 0.5;
-        acc += pn[d] * pn[d] * inv2Sigma2 * 0.5;
-        acc += nn[d] * nn[d] * inv2Sigma2 * 0.5;
-        acc += dol[d] * dol[d] * inv2Sigma2 * 0.25;
-        acc -= dn[d] * dn[d] * inv2Sigma2 * 0.25;
-      }
-    }
+    double mdx = mnx - mpx, mdy = mny - mpy, mdz = mnz - mpz;
+    pbc(s, mdx, mdy, mdz);
+    mdx *= 0.5; mdy *= 0.5; mdz *= 0.5;
+    mdx += mpx; mdy += mpy; mdz += mpz;
+    pbc(s, mdx, mdy, mdz);
+    double dx = z0 * sigma, dy = z1 * sigma, dz = z2 * sigma;
+    pbc(s, dx, dy, dz);
+    double nx = mdx + dx, ny = mdy + dy, nz = mdz + dz;
+    pbc(s, nx, ny, nz);
+    m.mx[t] = nx;
+    m.my[t] = ny;
+    m.mz[t] = nz;
+    acc += dx * dx * inv2Sigma2;
+    acc += dy * dy * inv2Sigma2;
+    acc += dz * dz * inv2Sigma2;
+    double ax = onx - opx, ay = ony - opy, az = onz - opz;
+    pbc(s, ax, ay, az);
+    ax *= 0.5; ay *= 0.5; az *= 0.5;
+    ax += opx; ay += opy; az += opz;
+    pbc(s, ax, ay, az);
+    double ex = ox - ax, ey = oy - ay, ez = oz - az;
+    pbc(s, ex, ey, ez);
+    acc -= ex * ex * inv2Sigma2;
+    acc -= ey * ey * inv2Sigma2;
+    acc -= ez * ez * inv2Sigma2;
     part += acc;
   }
   return part;
 }
 
-// FreeMover(PBC)::makeMove for one level: the beads, and ln(T_old/T_new) summed over the block.
+// FreeMover::makeMove for one level: the beads, and ln(T_old/T_new) summed over the block.
 static __device__ double mover_level(const DevSys& s, const Smem& m, int ipart, int level,
-                              uint64_t seed, uint32_t rep, uint32_t att, uint32_t ubase,
-                              int oshift = 0, bool second = false) {
-  return block_sum(mover_level_part(s, m, ipart, level, seed, rep, att, ubase, oshift, second),
-                   m.red);
-}
-
-
-// Block sums of nv per-thread values (nv <= 8) in a fixed order: warp trees,
-// then the warps in turn; out[v] is visible to every thread on return.
-__device__ __forceinline__ void block_sum_vec(const double* v, int nv, double* buf, double* out) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int k = 0; k < nv; ++k) {
-    double x = v[k];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (l == 0) buf[k * kWarps + w] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < nv) {
-    double x = 0.0;
-    for (int i = 0; i < nw; ++i) x += buf[threadIdx.x * kWarps + i];
-    out[threadIdx.x] = x;
-  }
-  __syncthreads();
+                                     int oshift = 0, bool second = false) {
+  return block_sum(mover_level_part(s, m, ipart, level, oshift, second), m.red);
 }
 
 // Evaluates one slice pair per lane group (group width W from the species size).
@@ -398,10 +524,12 @@ __device__ __forceinline__ double* cache_entry(const DevSys& s, double* cache, i
 // One pass of the set-up over slices [start, nsec) of one node species (only_sp)
 // or of all of them (only_sp < 0): cached results are copied, the others are
 // evaluated, the species' warps side by side.  Determinants go to dm[sp][t],
-// error flags to errs[sp][t], the moving species' distances to dist.
+// error flags to errs[sp][t], the moving species' distances to dist.  With llt,
+// the last warp makes the attempt's proposals beside it (mover_all).
 static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& m, const double* scale,
                                       const int* epoch, int msp, double* cache, int ifirst1,
-                                      int only_sp, int start) {
+                                      int only_sp, int start, int ipart, uint64_t seed,
+                                      uint32_t att, double* llt) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int nsec = s.nsec, M = s.nslice, nsm = s.ns_max;
   int* errs = m.ictl + C_NCTL;                 // [kMaxSpecies][nsec]
@@ -440,6 +568,7 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     ntask += (nmiss[sp] + Gs[sp] - 1) / Gs[sp];
   }
   first[s.nspecies] = ntask;
+  if (llt && warp == nwarps - 1) mover_all(s, m, ipart, seed, att, llt);
   for (int wt = warp; wt < ntask; wt += nwarps) {
     int sp = 0;
     while (wt >= first[sp + 1]) ++sp;
@@ -495,13 +624,14 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
 // leaves [1e-50, 1e50] its loop is replayed sequentially, and its later
 // slices are re-evaluated.
 static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem& m, double* scale, int* epoch,
-                                int msp, uint32_t* status, double* cache, int ifirst1) {
+                                int msp, uint32_t* status, double* cache, int ifirst1, int ipart,
+                                uint64_t seed, uint32_t att, double* llt) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nsec = s.nsec, M = s.nslice;
   const int nsm = s.ns_max;
   int* errs = m.ictl + C_NCTL;  // [kMaxSpecies][nsec]
   const double NaN = __longlong_as_double(0x7ff8000000000000LL);
-  node_init_pass(s, m, scale, epoch, msp, cache, ifirst1, -1, 0);
+  node_init_pass(s, m, scale, epoch, msp, cache, ifirst1, -1, 0, ipart, seed, att, llt);
   for (int sp = 0; sp < s.nspecies; ++sp) {
     if (!s.node_kind[sp]) continue;
     const int n = s.spec_count[sp];
@@ -512,7 +642,8 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
     int* er = errs + sp * nsec;
     int start = 0;
     for (int round = 0; round < 64; ++round) {
-      if (round > 0) node_init_pass(s, m, scale, epoch, msp, cache, ifirst1, sp, start);
+      if (round > 0)
+        node_init_pass(s, m, scale, epoch, msp, cache, ifirst1, sp, start, ipart, seed, att, nullptr);
       if (threadIdx.x == 0) {
         int k = -1;
         for (int t = start; t < nsec; ++t) {
@@ -581,70 +712,10 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
   __syncthreads();
 }
 
-// FixedNodeAction::getActionDifference (src/fixednode/FixedNodeAction.cc:39-131)
-// for the moving species at one level.
-static __device__ __noinline__ double node_level(const DevSys& s, const Smem& m, double scale, int msp, int ipart,
-                             int level, double* cache, int ifirst1, int ep) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+// FixedNodeAction::getActionDifference's nodal action over the section
+// (src/fixednode/FixedNodeAction.cc:96-131), after level 0's evaluations.
+static __device__ __noinline__ double nodal_action(const DevSys& s, const Smem& m, int n) {
   const int nsec = s.nsec, nsm = s.ns_max;
-  const int nStride = 1 << (level + 1);
-  const int n = s.spec_count[msp];
-  const int ntask = (nsec - 1 - nStride / 2) / nStride + 1;
-  if (nStride / 2 == nsec - 1) {
-    // The top level's only slice is the section's fixed end: its Slater
-    // matrix is the set-up one, so its determinant and distances are copied.
-    const int t = nsec - 1;
-    for (int i = threadIdx.x; i < 2 * nsm; i += blockDim.x) m.ndist[t * 2 * nsm + i] = m.dist[t * 2 * nsm + i];
-    if (threadIdx.x == 0) {
-      m.ndm[t] = m.dm[msp * nsec + t];
-      m.ictl[C_FLAG] = (m.ndm[t] * m.dm[msp * nsec + 0] <= 1e-200) ? 1 : 0;
-    }
-    __syncthreads();
-    return m.ictl[C_FLAG] ? 2e100 : 0.0;
-  }
-  // lane groups of the species' width, packed (32 / W matrices a warp): the
-  // SM's narrow FP64 pipe, shared by every resident warp, is the limit, and a
-  // packed warp instruction serves several matrices
-  const int W = node_group_width(n), G = 32 / W, g = lane / W;
-  const bool sho = s.node_kind[msp] == PIMC_NODES_SHO;
-  double* scr = group_scr(m, warp, g, n, !sho);
-  double* cold = group_cold(m, warp, g, n, !sho);
-  const int jcol = ipart - s.spec_first[msp];
-  if (threadIdx.x == 0) m.ictl[C_FLAG] = 0;
-  __syncthreads();
-  for (int base = warp * G; base < ntask; base += nwarps * G) {
-    const int task = base + g;
-    const bool act = task < ntask;
-    const int t = nStride / 2 + (act ? task : base) * nStride;
-    SliceView v1{m.s1x, m.s1y, m.s1z, s.npart, t, ipart, m.mx[t], m.my[t], m.mz[t]};
-    SliceView v2{m.s2x, m.s2y, m.s2z, s.npart, t, -1, 0, 0, 0};
-    double det = 0;
-    int err = 0;
-    double* ec = nullptr;
-    const double* xb = nullptr;  // mixed form: the entry's inverse block
-    double det_in = 0.0;
-    if (cache) {
-      double* e = cache_entry(s, cache, msp, wrap_slice(ifirst1 + t, s.nslice));
-      ec = e + 2 + 2 * n;
-      if (sm_species(s, msp) && m.xstage) {
-        xb = e + cache_x_slot(s, msp);
-        det_in = e[1];
-      }
-    } else if (sho && m.ecache) {
-      ec = m.ecache + (size_t)t * n * n;
-    }
-    node_eval_dispatch(W, s, msp, v1, v2, scale, scr, 1, ec, jcol, act, det, err,
-                       m.ndist + (t * 2) * nsm, m.ndist + (t * 2 + 1) * nsm,
-                       cache ? m.ncol + t * m.ncol_stride : nullptr, 0u, cold, xb, det_in,
-                       xb ? m.xstage + (size_t)t * m.xstage_stride : nullptr, (double)ep);
-    if (act && (lane & (W - 1)) == 0) {
-      m.ndm[t] = det;
-      if (err || det * m.dm[msp * nsec + 0] <= 1e-200) atomicOr(&m.ictl[C_FLAG], 1);
-    }
-  }
-  __syncthreads();
-  if (m.ictl[C_FLAG]) return 2e100;
-  if (level != 0) return 0.0;
   double part = 0.0;
   FSum fpart;
   for (int it = threadIdx.x; it < (nsec - 1) * n; it += blockDim.x) {
@@ -671,125 +742,107 @@ static __device__ __noinline__ double node_level(const DevSys& s, const Smem& m,
   return block_sum(s.mixed ? fpart.value() : part, m.red);
 }
 
-// The uniform-stream index of the first uniform consumed at `level`
-// (image choices of FreeMoverPBC, then the Metropolis uniform).
-__device__ __forceinline__ uint32_t level_uniform_base(const DevSys& s, int level) {
-  uint32_t u = (s.fixed_node ? 2u : 1u) + 1u;  // section choice + particle choice
-  const uint32_t pbcu = s.mover == PIMC_MOVER_FREE_PBC ? 3u : 0u;
-  for (int l = s.nlevel; l > level; --l) {
-    const uint32_t nmov = (l == s.nlevel) ? 0u : (1u << (s.nlevel - l - 1));
-    u += pbcu * nmov + 1u;
-  }
-  return u;
-}
-
-// The top bisection levels lo .. hi (all above 0) at once: the movers, level
-// by level (a level's midpoints are the beads of the levels above), then the
-// changed slices of every level in the range on the first warps, side by side,
-// while the remaining warps compute the levels' action differences (a level's
-// proposal does not depend on the decisions above it).  Per level l: lds[l]
-// the action difference, llt[l] the mover's ln(T_old/T_new), lnd[l] the
-// fixed-node difference (2e100 when a changed slice crosses a node, else 0).
+// Bisection levels lo .. hi of the attempt at once, after its proposals (a
+// level's proposal does not depend on the decisions above it).  The changed
+// slices of the levels go to the first warps, side by side; the other warps
+// take the action differences of levels alo .. ahi (all of them together down from
+// the top, ahi = nlevel, or one; none with alo > ahi), or every warp does after
+// its node work when that takes more than half of them.  Per level l: lds[l] the
+// action difference, lnd[l] the fixed-node difference
+// (FixedNodeAction::getActionDifference, src/fixednode/FixedNodeAction.cc:39-131:
+// 2e100 when a changed slice crosses a node; on level 0, alone, the nodal action).
 // The caller applies pi-qmc's level-by-level decisions to them.
-static __device__ __noinline__ void top_levels(const DevSys& s, const Smem& m, double scale, int msp,
-                                  int ipart, int lo, int hi, bool mynode, double* cache,
-                                  int ifirst1, int ep, uint64_t seed, uint32_t att, double* lds,
-                                  double* llt, double* lnd) {
+static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, double scale, int msp,
+                                  int ipart, int lo, int hi, int alo, int ahi, bool mynode,
+                                  double* cache, int ifirst1, int ep, double* lds, double* lnd) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int nsec = s.nsec, nsm = s.ns_max, L = s.nlevel;
-  // hi - lo + 1 <= 4 levels: v[0..3] mover terms, v[4..7] action terms
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int level = hi; level >= lo; --level) {
-    const double p = mover_level_part(s, m, ipart, level, seed, s.stream_id, att,
-                                      level_uniform_base(s, level));
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (k == hi - level) v[k] = p;
-    __syncthreads();  // this level's beads before the next level's midpoints
-  }
   const int n = mynode ? s.spec_count[msp] : 1;
   const int top = hi == L ? L - 1 : hi;
   int ntask = 0;
   if (mynode)
     for (int l = top; l >= lo; --l) ntask += (nsec - 1 - (1 << l)) / (1 << (l + 1)) + 1;
+  // lane groups of the species' width, packed (32 / W matrices a warp): the
+  // SM's narrow FP64 pipe, shared by every resident warp, is the limit, and a
+  // packed warp instruction serves several matrices
   const int W = node_group_width(n), G = 32 / W, g = lane / W;
   const int nodeW = min(nwarps, (ntask + G - 1) / G);
-  if (threadIdx.x == 0) m.ictl[C_FLAG] = 0;
-  if (mynode && hi == L) {
-    // the top level's only slice is the section's fixed end: copied from the set-up
-    const int t = nsec - 1;
-    for (int i = threadIdx.x; i < 2 * nsm; i += blockDim.x) m.ndist[t * 2 * nsm + i] = m.dist[t * 2 * nsm + i];
-  }
-  __syncthreads();
-  if (mynode && hi == L && threadIdx.x == 0) {
-    const int t = nsec - 1;
-    m.ndm[t] = m.dm[msp * nsec + t];
-    if (m.ndm[t] * m.dm[msp * nsec + 0] <= 1e-200) atomicOr(&m.ictl[C_FLAG], 1 << L);
-  }
-  if (warp < nodeW) {
-    const bool sho = s.node_kind[msp] == PIMC_NODES_SHO;
-    double* scr = group_scr(m, warp, g, n, !sho);
-    double* cold = group_cold(m, warp, g, n, !sho);
-    const int jcol = ipart - s.spec_first[msp];
-    for (int base = warp * G; base < ntask; base += nodeW * G) {
-      const int task = base + g;
-      const bool act = task < ntask;
-      int k = act ? task : base, l = top;  // task -> (level, slice)
-      for (;;) {
-        const int nl = (nsec - 1 - (1 << l)) / (1 << (l + 1)) + 1;
-        if (k < nl || l == lo) break;
-        k -= nl;
-        --l;
-      }
-      const int t = (1 << l) + k * (1 << (l + 1));
-      SliceView v1{m.s1x, m.s1y, m.s1z, s.npart, t, ipart, m.mx[t], m.my[t], m.mz[t]};
-      SliceView v2{m.s2x, m.s2y, m.s2z, s.npart, t, -1, 0, 0, 0};
-      double det = 0;
-      int err = 0;
-      double* ec = nullptr;
-      const double* xb = nullptr;  // mixed form: the entry's inverse block
-      double det_in = 0.0;
-      if (cache) {
-        double* e = cache_entry(s, cache, msp, wrap_slice(ifirst1 + t, s.nslice));
-        ec = e + 2 + 2 * n;
-        if (sm_species(s, msp) && m.xstage) {
-          xb = e + cache_x_slot(s, msp);
-          det_in = e[1];
+  if (mynode) {
+    if (threadIdx.x == 0) m.ictl[C_FLAG] = 0;
+    if (hi == L) {
+      // the top level's only slice is the section's fixed end: copied from the set-up
+      const int t = nsec - 1;
+      for (int i = threadIdx.x; i < 2 * nsm; i += blockDim.x) m.ndist[t * 2 * nsm + i] = m.dist[t * 2 * nsm + i];
+    }
+    __syncthreads();
+    if (hi == L && threadIdx.x == 0) {
+      const int t = nsec - 1;
+      m.ndm[t] = m.dm[msp * nsec + t];
+      if (m.ndm[t] * m.dm[msp * nsec + 0] <= 1e-200) atomicOr(&m.ictl[C_FLAG], 1 << L);
+    }
+    if (warp < nodeW) {
+      const bool sho = s.node_kind[msp] == PIMC_NODES_SHO;
+      double* scr = group_scr(m, warp, g, n, !sho);
+      double* cold = group_cold(m, warp, g, n, !sho);
+      const int jcol = ipart - s.spec_first[msp];
+      for (int base = warp * G; base < ntask; base += nodeW * G) {
+        const int task = base + g;
+        const bool act = task < ntask;
+        int k = act ? task : base, l = top;  // task -> (level, slice)
+        for (;;) {
+          const int nl = (nsec - 1 - (1 << l)) / (1 << (l + 1)) + 1;
+          if (k < nl || l == lo) break;
+          k -= nl;
+          --l;
         }
-      } else if (sho && m.ecache) {
-        ec = m.ecache + (size_t)t * n * n;
-      }
-      node_eval_dispatch(W, s, msp, v1, v2, scale, scr, 1, ec, jcol, act, det, err,
-                         m.ndist + (t * 2) * nsm, m.ndist + (t * 2 + 1) * nsm,
-                         cache ? m.ncol + t * m.ncol_stride : nullptr, 0u, cold, xb, det_in,
-                         xb ? m.xstage + (size_t)t * m.xstage_stride : nullptr, (double)ep);
-      if (act && (lane & (W - 1)) == 0) {
-        m.ndm[t] = det;
-        if (err || det * m.dm[msp * nsec + 0] <= 1e-200) atomicOr(&m.ictl[C_FLAG], 1 << l);
+        const int t = (1 << l) + k * (1 << (l + 1));
+        SliceView v1{m.s1x, m.s1y, m.s1z, s.npart, t, ipart, m.mx[t], m.my[t], m.mz[t]};
+        SliceView v2{m.s2x, m.s2y, m.s2z, s.npart, t, -1, 0, 0, 0};
+        double det = 0;
+        int err = 0;
+        double* ec = nullptr;
+        const double* xb = nullptr;  // mixed form: the entry's inverse block
+        double det_in = 0.0;
+        if (cache) {
+          double* e = cache_entry(s, cache, msp, wrap_slice(ifirst1 + t, s.nslice));
+          ec = e + 2 + 2 * n;
+          if (sm_species(s, msp) && m.xstage) {
+            xb = e + cache_x_slot(s, msp);
+            det_in = e[1];
+          }
+        } else if (sho && m.ecache) {
+          ec = m.ecache + (size_t)t * n * n;
+        }
+        node_eval_dispatch(W, s, msp, v1, v2, scale, scr, 1, ec, jcol, act, det, err,
+                           m.ndist + (t * 2) * nsm, m.ndist + (t * 2 + 1) * nsm,
+                           cache ? m.ncol + t * m.ncol_stride : nullptr, 0u, cold, xb, det_in,
+                           xb ? m.xstage + (size_t)t * m.xstage_stride : nullptr, (double)ep);
+        if (act && (lane & (W - 1)) == 0) {
+          m.ndm[t] = det;
+          if (err || det * m.dm[msp * nsec + 0] <= 1e-200) atomicOr(&m.ictl[C_FLAG], 1 << l);
+        }
       }
     }
   }
-  // the action differences on the other warps (on all of them when the node
-  // tasks take every warp, after those)
-  if (nodeW == nwarps) __syncthreads();
-  const int a0 = nodeW == nwarps ? 0 : nodeW * 32;
-  if ((int)threadIdx.x >= a0)
-    for (int level = lo; level <= hi; ++level) {
-      const double a = action_partial(s, m, ipart, level, threadIdx.x - a0, blockDim.x - a0);
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (k == level - lo) v[4 + k] = a;
+  const int a0 = 2 * nodeW > nwarps ? 0 : nodeW, dmax = L - alo, dmin = ahi == L ? 0 : dmax;
+  if (alo <= ahi) {
+    if (warp >= a0) {
+      double* buf = m.act + (size_t)warp * m.act_stride;
+      if (s.mixed)
+        action_warp<true>(s, m, ipart, dmin, dmax, warp - a0, nwarps - a0, buf);
+      else
+        action_warp<false>(s, m, ipart, dmin, dmax, warp - a0, nwarps - a0, buf);
     }
+    __syncthreads();
+    action_reduce(s, m.act + (size_t)a0 * m.act_stride, m.act_stride, dmin, dmax, nwarps - a0, lds);
+  }
   __syncthreads();
-  const int flags = m.ictl[C_FLAG];
-  double* out = m.vred + 8 * kWarps;
-  block_sum_vec(v, 8, m.vred, out);
+  const int flags = mynode ? m.ictl[C_FLAG] : 0;
+  double nodal = 0.0;
+  if (mynode && lo == 0 && !(flags & 1)) nodal = nodal_action(s, m, n);
   if (threadIdx.x == 0)
-    for (int level = lo; level <= hi; ++level) {
-      llt[level] = out[hi - level];
-      lds[level] = out[4 + level - lo];
-      lnd[level] = ((flags >> level) & 1) ? 2e100 : 0.0;
-    }
+    for (int level = lo; level <= hi; ++level)
+      lnd[level] = ((flags >> level) & 1) ? 2e100 : (level == 0 ? nodal : 0.0);
   __syncthreads();
 }
 
@@ -821,16 +874,19 @@ static __device__ __noinline__ void delayed_rejection(const DevSys& s, const Sme
   }
   __syncthreads();
   // C: FreeMover::makeMove with factor = newFactor and the next normals
-  const double lnTC = mover_level(s, m, ipart, level, seed, s.stream_id, att, uacc, 1, true);
-  double dsC = block_sum(action_partial(s, m, ipart, level, threadIdx.x, blockDim.x), m.red);
+  const double lnTC = mover_level(s, m, ipart, level, 1, true);
+  double* lds = m.red + kWarps + 8;
+  double* lnd = lds + 2 * kMaxLevels;
+  eval_levels(s, m, scale, msp, ipart, level, level, level, level, mynode, cache, ifirst1, ep, lds,
+              lnd);
+  double dsC = lds[level];
   if (s.ewald && s.coulomb && level == 0) {
     if (ek)
       dsC += ewald_level0_cached(s, m, ipart, ifirst1, ek, ekstage);
     else
       for (int k = 1; k < nsec - 1; ++k) dsC += ewald_slice_diff(s, m, ipart, k);
   }
-  double dsnC = 0.0;
-  if (mynode) dsnC = node_level(s, m, scale, msp, ipart, level, cache, ifirst1, ep);
+  const double dsnC = lnd[level];
   if (threadIdx.x == 0) {
     const double piRatioBoA = m.red[kWarps + 3], accRatioA2B = m.red[kWarps + 4];
     const double sigma = s.mov_sigma[level][sp], inv2Sigma2 = s.mov_inv2s2[level][sp];
@@ -974,33 +1030,43 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
       if (fixed) load_section(s, path, ifirst2, m.s2x, m.s2y, m.s2z);
       attempt_normals(s, m, P.seed, s.stream_id, att);
       __syncthreads();
+      double* lds = m.red + kWarps + 8;  // [kMaxLevels] per level: action difference,
+      double* llt = lds + kMaxLevels;     // mover ln T,
+      double* lnd = llt + kMaxLevels;     // fixed-node difference
       for (int t = threadIdx.x; t < nsec; t += blockDim.x) {
         m.mx[t] = m.s1x[t * np + ipart];
         m.my[t] = m.s1y[t * np + ipart];
         m.mz[t] = m.s1z[t * np + ipart];
       }
+      if (!s.dr && (threadIdx.x >> 5) == (blockDim.x >> 5) - 1) mover_old(s, m, ipart);
       const int msp = species_of(s, ipart);
       const bool mynode = fixed && s.node_kind[msp];
-      if (fixed)
-        node_initialize(s, m, scale, epoch, mynode ? msp : -1, &status, cache, ifirst1);
+      // the proposals of every level: beside the node set-up, or now
+      if (fixed) {
+        node_initialize(s, m, scale, epoch, mynode ? msp : -1, &status, cache, ifirst1, ipart,
+                        P.seed, att, s.dr ? nullptr : llt);
+      } else {
+        __syncthreads();
+        if (!s.dr && threadIdx.x < 32) mover_all(s, m, ipart, P.seed, att, llt);
+      }
       __syncthreads();
       pimc_move_record* rec = P.rec ? P.rec + (size_t)r * P.nattempt + a : nullptr;
       double oldDS = 0.0;
       int reject = -1;
-      // The top levels (L down to lb) are proposed and evaluated together,
-      // their Slater matrices side by side; the decisions then follow level by
-      // level exactly as below.  Work done for levels under a rejection is
-      // discarded.
+      // The top levels (L down to lb) are evaluated together, their Slater
+      // matrices side by side; the decisions then follow level by level exactly as
+      // below.  Work done for levels under a rejection is discarded.  Without node
+      // work or Ewald sums that is every level; else the lower levels, whose
+      // slices make up most of the work, wait for the decisions above them (the
+      // mixed form's FP32 action terms are cheap and all come with the top ones).
       // (with delayed rejection every level is taken in turn: a second proposal
       // at level L - 1 changes the normals and uniforms of the levels under it)
-      const int lb = (L >= 2 && !s.dr) ? max(1, L - 3) : L + 1;
+      const bool longr = s.ewald && s.coulomb;
+      const int lb = s.dr ? L + 1 : ((mynode || longr) ? max(1, L - 3) : 0);
+      const int alb = s.mixed ? 0 : lb;  // the lowest level whose action comes with them
       if (lb <= L) {
-        double* lds = m.red + kWarps + 8;  // [kMaxLevels] per level: action difference,
-        double* llt = lds + kMaxLevels;     // mover ln T,
-        double* lnd = llt + kMaxLevels;     // fixed-node difference
-        top_levels(s, m, scale[msp], msp, ipart, lb, L, mynode, cache, ifirst1, epoch[msp], P.seed,
-                   att, lds, llt, lnd);
-        __syncthreads();
+        eval_levels(s, m, scale[msp], msp, ipart, lb, L, alb, L, mynode, cache, ifirst1,
+                    epoch[msp], lds, lnd);
         if (threadIdx.x < 32) {
           // Lane i takes level L - i: every level's acceptance probability
           // exp(lnT - total + total of the level above) and uniform at once
@@ -1048,16 +1114,18 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
       uint32_t ushift = 0;  // proposal took before the level
       for (int level = min(L, lb - 1); level >= 0 && reject < 0; --level) {
         const uint32_t ubase = level_uniform_base(s, level) + ushift;
-        const double lnT = mover_level(s, m, ipart, level, P.seed, s.stream_id, att, ubase, oshift);
-        double ds = block_sum(action_partial(s, m, ipart, level, threadIdx.x, blockDim.x), m.red);
-        if (s.ewald && s.coulomb && level == 0) {
+        const double lnT = s.dr ? mover_level(s, m, ipart, level, oshift) : llt[level];
+        const bool done = level >= alb && lb <= L;
+        eval_levels(s, m, scale[msp], msp, ipart, level, level, done ? 1 : level, done ? 0 : level,
+                    mynode, cache, ifirst1, epoch[msp], lds, lnd);
+        double ds = lds[level];
+        if (longr && level == 0) {
           if (ek)
             ds += ewald_level0_cached(s, m, ipart, ifirst1, ek, ekstage);
           else
             for (int t = 1; t < nsec - 1; ++t) ds += ewald_slice_diff(s, m, ipart, t);
         }
-        double dsn = 0.0;
-        if (mynode) dsn = node_level(s, m, scale[msp], msp, ipart, level, cache, ifirst1, epoch[msp]);
+        const double dsn = lnd[level];
         if (threadIdx.x == 0) {
           const double total = fixed ? ds + dsn : ds;
           const uint32_t nmov = (level == L) ? 0u : (1u << (L - level - 1));

@@ -186,6 +186,13 @@ __device__ __forceinline__ void pbc(const DevSys& s, double& x, double& y, doubl
 __device__ __forceinline__ float norm2_f(float x, float y, float z) {
   return __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x)));
 }
+// The moves' order of the same (x and y fused the other way round), and of a.b.
+__device__ __forceinline__ float dot_f(float ax, float ay, float az, float bx, float by, float bz) {
+  return __fmaf_rn(az, bz, __fmaf_rn(ax, bx, __fmul_rn(ay, by)));
+}
+__device__ __forceinline__ float norm2_move_f(float x, float y, float z) {
+  return dot_f(x, y, z, x, y, z);
+}
 
 // The mixed form's minimum image of an FP64 difference, rounded to FP32 for
 // its FP32 terms (pbc's image, then the rounding, both without FP64
@@ -343,7 +350,7 @@ __device__ __forceinline__ void tab_uk0d(const DevTable& t, double q, double s2,
 // FP32 variants for the mixed-precision form (same grid, FP32 coefficients).
 __device__ __forceinline__ float tab_uk0_f(const DevTable& t, float q, float s2, int norder_eff) {
   q *= (float)t.rgridinv;
-  float x = __logf(q) * (float)t.logrratioinv;
+  float x = __fmul_rn(__logf(q), (float)t.logrratioinv);
   int i;  // range tests before the conversion, as tab_locate
   if (!(q >= 1.f)) {
     i = 0;
@@ -353,7 +360,7 @@ __device__ __forceinline__ float tab_uk0_f(const DevTable& t, float q, float s2,
     x = 1.f;
   } else {
     i = (int)x;
-    x -= i;
+    x = __fsub_rn(x, (float)i);
   }
   const float* g0 = t.ugrid32 + (size_t)i * 2 * t.ndata;
   const float* g1 = g0 + 2 * t.ndata;

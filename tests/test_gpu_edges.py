@@ -108,3 +108,54 @@ def test_periodic_gaussian_images(pimc, al2, n):
     size = np.einsum("bji,bijd->bjd", np.abs(inv), np.abs(grad)).sum(-1)
     slack = tol[:, None] * size * np.sqrt(kw["beta"] / 64 / 2) * ref ** 2 + 1e-12 * ref
     assert np.all(np.abs(d1[:, :n] - ref) <= slack)
+
+
+@pytest.mark.parametrize("nlevel", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("counts,block", [([1], 32), ([1, 1], 64), ([3, 2], 32), ([4, 5], 256),
+                                          ([17, 18], 128)])
+def test_every_level_at_once(pimc, nlevel, counts, block):
+    # The levels' links share a warp's lanes: one to six levels, fewer partners than
+    # a warp takes at once up to several rounds of them, one to eight warps.
+    kw = W.dot2(counts=counts, sho_omega=[1.0] * len(counts), nslice=64, beta=3.0, nlevel=nlevel)
+    tabs, _ = pimc.coulomb_tables(kw)
+    cfg = O.make_config(**kw)
+    x = W.initial_path(cfg, "gauss", seed=3)
+    port = O.PortOracle(cfg, tabs)
+    port.set_path(x)
+    ref = port.run(60)
+    e = pimc.Engine(kw, 1, tabs)
+    e.configure(block, 0, 0, 2)
+    e.upload_paths([x])
+    rec = e.run_sections(60, records=True)
+    for k in ("ifirst1", "ipart", "reject_level"):
+        assert np.array_equal(rec[k][0], ref[k]), k
+    for k in ("ds", "lnt"):
+        a, b = rec[k][0][:, :nlevel + 1], ref[k][:, :nlevel + 1]
+        assert np.all(np.abs(a - b) <= 1e-12 * np.maximum(np.abs(b), 1.0)), k
+    assert np.abs(e.download_paths()[0] - port.get_path()).max() <= 1e-12
+
+
+@pytest.mark.parametrize("nlevel,cell", [(3, 4.3), (4, 6.1), (5, 8.6), (6, 12.2), (4, 30.0)])
+def test_periodic_mover_images(pimc, nlevel, cell):
+    # Boxes at the smallest width the periodic mover takes, where its image choices
+    # need their exponentials, and one where they are certain.
+    kw = W.dot2(counts=[2, 1], sho_omega=[0.0, 0.0], nslice=128, beta=128 * 0.02, nlevel=nlevel,
+                cell=cell, mover=1)
+    tabs, _ = pimc.coulomb_tables(kw)
+    cfg = O.make_config(**kw)
+    rng = np.random.default_rng(1)
+    x = np.cumsum(rng.normal(size=(128, 3, 3)) * 0.14, axis=0)
+    x -= np.linspace(0, 1, 128)[:, None, None] * x[-1]
+    x += rng.uniform(-cell / 2, cell / 2, size=(1, 3, 3))
+    x -= cell * np.floor(x / cell + 0.5)
+    port = O.PortOracle(cfg, tabs)
+    port.set_path(x)
+    ref = port.run(200)
+    e = pimc.Engine(kw, 1, tabs)
+    e.upload_paths([x])
+    rec = e.run_sections(200, records=True)
+    for k in ("ifirst1", "ipart", "reject_level"):
+        assert np.array_equal(rec[k][0], ref[k]), k
+    a, b = rec["lnt"][0][:, :nlevel + 1], ref["lnt"][:, :nlevel + 1]
+    assert np.all(np.abs(a - b) <= 1e-12 * np.maximum(np.abs(b), 1.0))
+    assert np.abs(e.download_paths()[0] - port.get_path()).max() <= 1e-12
