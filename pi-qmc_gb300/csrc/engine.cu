@@ -131,7 +131,6 @@ struct LayoutOpts {
   bool cold_global = false;     // its cold parts in global memory even when all of it fits
   bool full_ewald_tables = false;  // Ewald tables for every bead (full evalLongRange sums)
   bool single_levels = false;      // action differences of one level at a time only
-  bool no_actions = false;         // no buffers for the action differences (displacement moves)
 };
 
 struct pimc_engine {
@@ -538,7 +537,7 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
   L.gcta = nwarps * gwarp + (L.ncol_global ? ncol_size : 0);
   // the action differences' buffers: the warps' Slater scratch where that is in
   // shared memory (a warp is done with it by then), else their own
-  if (!opts.no_actions) {
+  {
     int need = 0;
     for (const DevSys& d : sys) {
       // (a launch of all levels together alone needs no buffer for a single one)
@@ -612,6 +611,64 @@ Layout estimator_layout(const std::vector<DevSys>& sys, const int* ikmax_extra) 
   L.split = L.ncol_global = L.gcta = L.nodecold_stride = 0;
   L.total = off;
   return L;
+}
+
+// Shared memory of the displacement kernel: the Slater scratch of the node pass and
+// the Ewald tables share their space (a barrier lies between their phases); the
+// scratch goes to global memory, cold part first, and the tables' batch shrinks,
+// until it fits.
+bool displace_layout(const std::vector<DevSys>& sys, int nwarps, int nmoving, DisplaceLayout& out) {
+  int np = 1, per = 0, perfull = 0, stage = 0, full = 0, hot = 0, cold = 0;
+  for (const DevSys& d : sys) {
+    np = std::max(np, d.npart);
+    if (d.ewald) {
+      const int p = d.ikmax[0] + 1 + 2 * d.ikmax[1] + 1 + 2 * d.ikmax[2] + 1;
+      (d.ek_offset >= 0 ? per : perfull) = std::max(d.ek_offset >= 0 ? per : perfull, p);
+    }
+    for (int i = 0; i < d.nspecies; ++i)
+      if (d.node_kind[i]) {
+        const int n = d.spec_count[i], G = 32 / node_group_width(n);
+        const bool fr = d.node_kind[i] == PIMC_NODES_FREE;
+        stage = std::max(stage, G * 6 * n);
+        full = std::max(full, G * node_group_scratch(n, fr));
+        hot = std::max(hot, G * node_group_hot(n));
+        cold = std::max(cold, G * node_group_cold(n, fr));
+      }
+  }
+  const int limit = kSmemLimit / 8;
+  for (int place = 0; place < 3; ++place)
+    for (int batch = 8; batch >= 1; batch /= 2) {
+      DisplaceLayout L{};
+      int off = 0;
+      auto take = [&](int n) {
+        const int o = off;
+        off += (n + 1) & ~1;
+        return o;
+      };
+      L.red = take(64);
+      L.q = take(np);
+      L.ictl = take(C_NCTL);
+      L.sec = take(perfull ? 6 * np : 0);
+      L.ewt_cols = perfull ? np + 1 : 0;
+      L.ewt = take(2 * perfull * L.ewt_cols);
+      L.stage = take(nwarps * stage);
+      L.split = place == 1;
+      L.in_smem = place < 2;
+      L.nodescr_stride = ((place == 1 ? hot : full) + 1) & ~1;
+      L.nodecold_stride = place == 1 ? (cold + 1) & ~1 : 0;
+      L.gcta = nwarps * (place == 0 ? 0 : (place == 1 ? L.nodecold_stride : L.nodescr_stride));
+      L.ek_batch = batch;
+      L.ek_stride = 2 * per * 2 * nmoving * batch;
+      L.nodescr = L.ek = off;
+      off += nwarps * std::max(L.in_smem ? L.nodescr_stride : 0, L.ek_stride);
+      L.total = off;
+      if (off <= limit) {
+        out = L;
+        return true;
+      }
+      if (!per) break;  // (no tables to shrink)
+    }
+  return false;
 }
 
 int device_check(int& nsm) {
@@ -1354,43 +1411,63 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
     if (d.fixed_node && (d.nslice % 2)) return fail(PIMC_ERR_INVALID, "odd nslice");
   }
   if (nattempt == 0) return PIMC_OK;
-  // shared memory: a section layout (slices staged for the Ewald sums, the
-  // reduction buffer, charges, control words, Slater scratch) plus a slice-pair
-  // staging area per lane group
   const int dthreads = std::min(e->block, kBlock), nwarps = dthreads / 32;
-  int stage = 0, half_max = 1, nsm = 1;
-  for (const DevSys& d : e->hsys) {
-    half_max = std::max(half_max, d.nslice / 2);
-    nsm = std::max(nsm, d.ns_max);
-    for (int i = 0; i < d.nspecies; ++i)
-      if (d.node_kind[i]) {
-        const int n = d.spec_count[i];
-        stage = std::max(stage, (32 / node_group_width(n)) * 6 * n);
-      }
-  }
-  // (full Ewald tables: every slice's evalLongRange is summed here)
-  LayoutOpts dopt;
-  dopt.full_ewald_tables = true;
-  dopt.no_actions = true;
-  bool lok = false;
-  Layout L = make_layout(e->hsys, nwarps, lok, dopt);
-  if (!lok || (size_t)(L.total + nwarps * stage) * 8 > (size_t)kSmemLimit) {
-    dopt.scratch_global = true;
-    L = make_layout(e->hsys, nwarps, lok, dopt);
-  }
-  const int stage_off = L.total;
-  const size_t smem = (size_t)(L.total + nwarps * stage) * 8;
-  if (!lok || smem > (size_t)kSmemLimit)
+  DisplaceLayout L;
+  if (!displace_layout(e->hsys, nwarps, nmoving, L))
     return fail(PIMC_ERR_CAPACITY, "displacement working set too large");
-  if ((size_t)e->grid * L.gcta > e->d_nodescr.n) {
+  const size_t smem = (size_t)L.total * 8;
+  cudaFuncSetAttribute(displace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  // CTAs per replica: the cluster size whose waves over the replicas, shared by its
+  // CTAs, are the fewest (clusters of 8 need 8 free SMs of one GPC, so fewer fit than
+  // the SM count says)
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(dthreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = e->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int clusters = 0, C = 0;
+  double best = 0.0;
+  for (int c = 1; c <= kMaxDisplaceCluster; c *= 2) {
+    attr.val.clusterDim.x = c;
+    cfg.gridDim = dim3(c);
+    int ncl = 0;
+    if (cudaOccupancyMaxActiveClusters(&ncl, displace_kernel, &cfg) != cudaSuccess || ncl < 1) {
+      cudaGetLastError();
+      continue;
+    }
+    ncl = std::min(ncl, e->nrep);
+    const double cost = (double)((e->nrep + ncl - 1) / ncl) / c;
+    if (C == 0 || cost < best) {
+      best = cost;
+      C = c;
+      clusters = ncl;
+    }
+  }
+  if (C == 0) return fail(PIMC_ERR_CAPACITY, "displacement working set too large");
+  attr.val.clusterDim.x = C;
+  cfg.gridDim = dim3(clusters * C);
+  if ((size_t)clusters * C * L.gcta > e->d_nodescr.n) {
     CU(cudaStreamSynchronize(e->stream));
-    if (e->d_nodescr.alloc((size_t)e->grid * L.gcta))
+    if (e->graph) {  // captured with the old scratch
+      cudaGraphExecDestroy(e->graph);
+      e->graph = nullptr;
+    }
+    if (e->d_nodescr.alloc((size_t)clusters * C * L.gcta))
       return fail(PIMC_ERR_CUDA, "cudaMalloc node scratch");
   }
-  const long long sstride = (long long)half_max * (1 + 4 * nsm);
-  const size_t need = (size_t)e->grid * sstride;
-  if (e->d_dscratch.n < need && e->d_dscratch.alloc(need))
-    return fail(PIMC_ERR_CUDA, "cudaMalloc displacement scratch");
+  long long sstride = 0;
+  for (const DevSys& d : e->hsys)
+    if (d.fixed_node)
+      sstride = std::max(sstride, (long long)d.nspecies * (d.nslice / 2) * (1 + 4 * d.ns_max));
+  const size_t need = (size_t)clusters * sstride;
+  if (e->d_dscratch.n < need) {
+    CU(cudaStreamSynchronize(e->stream));
+    if (e->d_dscratch.alloc(need)) return fail(PIMC_ERR_CUDA, "cudaMalloc displacement scratch");
+  }
   pimc_displace_record* d_rec = nullptr;
   if (records) {
     CU(cudaMallocAsync(&d_rec, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt,
@@ -1403,6 +1480,7 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
   P.state = e->d_state.p;
   P.paths = e->d_paths.p;
   P.nodecache = e->d_nodecache.p;
+  P.ekcache = e->d_ekcache.p;
   P.scratch = e->d_dscratch.p;
   P.scratch_stride = sstride;
   P.nodescr_g = e->d_nodescr.p;
@@ -1416,14 +1494,9 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
   P.nmoving = nmoving;
   P.species = species;
   P.lay = L;
-  P.stage_off = stage_off;
-  cudaFuncSetAttribute(displace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
-  displace_kernel<<<e->grid, dthreads, smem, e->stream>>>(P);
+  CU(cudaLaunchKernelEx(&cfg, displace_kernel, P));
   e->launches++;
-  CU(cudaGetLastError());
-  // displaced paths: every slice's structure factors are rebuilt
-  if (int rc = prefill_ewald(e, nullptr, e->nrep)) return rc;
   if (records) {
     CU(cudaMemcpyAsync(records, d_rec, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt,
                        cudaMemcpyDeviceToHost, e->stream));

@@ -455,7 +455,7 @@ static __device__ double mover_level(const DevSys& s, const Smem& m, int ipart, 
 __device__ __forceinline__ void node_eval_dispatch(int W, const DevSys& s, int sp,
                                                    const SliceView& v1, const SliceView& v2,
                                                    double scale, double* scr, int full,
-                                                   double* ecache, int jcol, bool write,
+                                                   double* ecache, unsigned cols, bool write,
                                                    double& det, int& err, double* d1,
                                                    double* d2, double* newcol = nullptr,
                                                    unsigned rowmask = 0xffffffffu,
@@ -466,22 +466,22 @@ __device__ __forceinline__ void node_eval_dispatch(int W, const DevSys& s, int s
   // (xin and xout are the same for every lane of a warp)
   if (xin || xout) {
     if (W == 8)
-      node_eval_group<8, true>(s, sp, v1, v2, scale, scr, full, ecache, jcol, write, det, err,
+      node_eval_group<8, true>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err,
                                d1, d2, newcol, rowmask, cold, xin, det_in, xout, xepoch);
     else if (W == 16)
-      node_eval_group<16, true>(s, sp, v1, v2, scale, scr, full, ecache, jcol, write, det, err,
+      node_eval_group<16, true>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err,
                                 d1, d2, newcol, rowmask, cold, xin, det_in, xout, xepoch);
     else
-      node_eval_group<32, true>(s, sp, v1, v2, scale, scr, full, ecache, jcol, write, det, err,
+      node_eval_group<32, true>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err,
                                 d1, d2, newcol, rowmask, cold, xin, det_in, xout, xepoch);
   } else if (W == 8) {
-    node_eval_group<8>(s, sp, v1, v2, scale, scr, full, ecache, jcol, write, det, err, d1, d2,
+    node_eval_group<8>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2,
                        newcol, rowmask, cold);
   } else if (W == 16) {
-    node_eval_group<16>(s, sp, v1, v2, scale, scr, full, ecache, jcol, write, det, err, d1, d2,
+    node_eval_group<16>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2,
                         newcol, rowmask, cold);
   } else {
-    node_eval_group<32>(s, sp, v1, v2, scale, scr, full, ecache, jcol, write, det, err, d1, d2,
+    node_eval_group<32>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2,
                         newcol, rowmask, cold);
   }
 }
@@ -595,7 +595,7 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     const unsigned rmask = e ? cache_rowmask(e, cache_mask_slot(s, sp)) : 0xffffffffu;
     // mixed form: the entry's inverse, updated for its changed rows when it can be
     double* xb = (e && sm_species(s, sp)) ? e + cache_x_slot(s, sp) : nullptr;
-    node_eval_dispatch(W, s, sp, v1, v2, scale[sp], scrm, full, ec, -1, act, det, err, d1, d2,
+    node_eval_dispatch(W, s, sp, v1, v2, scale[sp], scrm, full, ec, 0u, act, det, err, d1, d2,
                        nullptr, rmask, coldm, xb, e ? e[1] : 0.0, xb, (double)epoch[sp]);
     if (act) {
       if (e && mine && glm < n) {
@@ -681,7 +681,7 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
           SliceView v2{m.s2x, m.s2y, m.s2z, s.npart, k, -1, 0, 0, 0};
           double d = 0;
           int e2 = 0;
-          node_eval_dispatch(W, s, sp, v1, v2, sc2, dsc, mine ? 1 : 0, nullptr, -1, g == 0, d,
+          node_eval_dispatch(W, s, sp, v1, v2, sc2, dsc, mine ? 1 : 0, nullptr, 0u, g == 0, d,
                              e2, m.dist + (k * 2) * nsm, m.dist + (k * 2 + 1) * nsm, nullptr,
                              0xffffffffu, dcold);
           det = __shfl_sync(0xffffffffu, d, 0);
@@ -813,7 +813,7 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
         } else if (sho && m.ecache) {
           ec = m.ecache + (size_t)t * n * n;
         }
-        node_eval_dispatch(W, s, msp, v1, v2, scale, scr, 1, ec, jcol, act, det, err,
+        node_eval_dispatch(W, s, msp, v1, v2, scale, scr, 1, ec, 1u << jcol, act, det, err,
                            m.ndist + (t * 2) * nsm, m.ndist + (t * 2 + 1) * nsm,
                            cache ? m.ncol + t * m.ncol_stride : nullptr, 0u, cold, xb, det_in,
                            xb ? m.xstage + (size_t)t * m.xstage_stride : nullptr, (double)ep);

@@ -142,11 +142,11 @@ __global__ void __launch_bounds__(kBlock) cache_prefill_kernel(PrefillParams P) 
     // (mixed form, free-particle nodes: the inverse block too, the start of
     // its update count)
     if (sm_species(s, sp))
-      node_eval_group<32, true>(s, sp, v1, v2, scale, scr, 1, e + 2 + 2 * n, -1, true, det, err,
+      node_eval_group<32, true>(s, sp, v1, v2, scale, scr, 1, e + 2 + 2 * n, 0u, true, det, err,
                                 e + 2, e + 2 + n, nullptr, 0xffffffffu, cold, nullptr, 0.0,
                                 e + cache_x_slot(s, sp), ep);
     else
-      node_eval_group<32>(s, sp, v1, v2, scale, scr, 1, e + 2 + 2 * n, -1, true, det, err, e + 2,
+      node_eval_group<32>(s, sp, v1, v2, scale, scr, 1, e + 2 + 2 * n, 0u, true, det, err, e + 2,
                           e + 2 + n, nullptr, 0xffffffffu, cold);
     __syncwarp();
     if (lane == 0) {

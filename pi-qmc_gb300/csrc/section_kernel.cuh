@@ -110,6 +110,45 @@ __device__ __forceinline__ double* group_cold(const Smem& m, int warp, int g, in
                     : nullptr;
 }
 
+// One element rho(r1_j, r2_i) of a species' Slater matrix (unscaled), and for
+// free-particle nodes its gradient with respect to r1_j.  Rounded operations: the
+// same bits wherever it is computed.
+struct NodeElement {
+  double v, gx, gy, gz;
+};
+__device__ __forceinline__ NodeElement node_element(const DevSys& s, int sp, const SliceView& v1,
+                                                    const SliceView& v2, int i, int j) {
+  const int f = s.spec_first[sp];
+  double rix, riy, riz, rjx, rjy, rjz;
+  v2.get(f + i, rix, riy, riz);
+  v1.get(f + j, rjx, rjy, rjz);
+  NodeElement r{0.0, 0.0, 0.0, 0.0};
+  if (s.node_kind[sp] == 1) {
+    const double ri2 = dot3(rix, riy, riz, rix, riy, riz);
+    const double rj2 = dot3(rjx, rjy, rjz, rjx, rjy, rjz);
+    const double rirj = dot3(rix, riy, riz, rjx, rjy, rjz);
+    const double q = __dsub_rn(__dmul_rn(__dadd_rn(ri2, rj2), s.node_cosh[sp]),
+                               __dmul_rn(2.0, rirj));
+    r.v = exp(__dmul_rn(-s.node_c[sp], q));
+    return r;
+  }
+  double dx = rjx - rix, dy = rjy - riy, dz = rjz - riz;
+  pbc(s, dx, dy, dz);
+  if (s.pg_images[sp]) {
+    r.v = pg_images_eval(s, sp, dx, dy, dz, r.gx, r.gy, r.gz);
+    return r;
+  }
+  double g0, g1, g2;
+  const double v0 = pg_eval(s.pg_nome[sp][0], s.pg_pref[sp][0], s.pg_k[sp][0], s.pg_nmax[sp][0], dx, &g0);
+  const double v1v = pg_eval(s.pg_nome[sp][1], s.pg_pref[sp][1], s.pg_k[sp][1], s.pg_nmax[sp][1], dy, &g1);
+  const double v2v = pg_eval(s.pg_nome[sp][2], s.pg_pref[sp][2], s.pg_k[sp][2], s.pg_nmax[sp][2], dz, &g2);
+  r.v = v0 * v1v * v2v;
+  r.gx = g0 / (v0 + 1e-300) * v0 * v1v * v2v;
+  r.gy = g1 / (v1v + 1e-300) * v0 * v1v * v2v;
+  r.gz = g2 / (v2v + 1e-300) * v0 * v1v * v2v;
+  return r;
+}
+
 // NodeModel::evaluate (+ evaluateDistance) for one species on one slice pair,
 // executed by a group of W lanes (W = 8, 16 or 32; 32/W groups per warp each
 // take their own slice pair).  Lanes own matrix rows.  LU with partial pivoting
@@ -119,16 +158,17 @@ __device__ __forceinline__ double* group_cold(const Smem& m, int warp, int g, in
 // (src/fixednode/SHONodes.cc:51-170, src/fixednode/FreeParticleNodes.cc:72-234).
 // full = 0: determinant only.  Every lane of the warp must call this (the
 // shuffles span the warp); a group with write = false computes but stores
-// nothing.  For SHONodes, ecache (n*n, or null) holds the slice's exp matrix:
-// jcol < 0 fills it, jcol >= 0 reuses it and recomputes column jcol only (the
-// other columns' inputs are unchanged, so the values are bit-identical).
+// nothing.  ecache (or null) holds the slice pair's element matrix: the rows of
+// rowmask are recomputed, and the columns of `cols` in the other rows (their
+// other inputs are unchanged, so the values are bit-identical); without columns
+// what is recomputed is stored there.
 // kSm: the variant with the mixed form's Sherman-Morrison updates and inverse
 // blocks (xin / xout); without it those arguments are ignored and the
 // evaluation is the plain factorisation.
 template <int W, bool kSm = false>
 static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, const SliceView& v1,
                                 const SliceView& v2, double scale, double* scr, int full,
-                                double* ecache, int jcol, bool write, double& det_out,
+                                double* ecache, unsigned cols, bool write, double& det_out,
                                 int& err_out, double* d1, double* d2,
                                 double* newcol = nullptr, unsigned rowmask = 0xffffffffu,
                                 double* cold = nullptr, const double* xin = nullptr,
@@ -146,75 +186,47 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   double* G = E + n * n;    // 3 n*n gradient factors (free-particle nodes)
   const bool sho = s.node_kind[sp] == 1;
   // --- build the Slater matrix: A(i,j) = scale * rho(r1_j, r2_i)
-  // Elements come from ecache where it holds them (a column update keeps every
-  // column but jcol; a row refresh keeps the rows outside rowmask); the others
-  // are computed.  Whole rows (all of them without a cache, the stale ones on a
+  // Elements come from ecache where it holds them (outside rowmask's rows and the
+  // columns of `cols`); the others are computed.  Whole rows (all of them without a cache, the stale ones on a
   // refresh) go one element per lane and step, so that refreshing one or two
   // rows still spreads over the group; the new column of a column update goes
   // one row per lane.  Every element is the same rounded arithmetic wherever
   // it is computed, so cached and recomputed values agree bit for bit.
   const int nn = n * n;
   const unsigned nmask = n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
-  const unsigned rows_new = !ecache ? nmask : (jcol < 0 ? (rowmask & nmask) : 0u);
+  const unsigned rows_new = !ecache ? nmask : (rowmask & nmask);
   // element (i, j): value into A (scaled), E (SHO) or G (gradients), and into
   // ecache (a refresh) or newcol (the new column) when this group writes
   auto element = [&](int i, int j) {
-    double rix, riy, riz, rjx, rjy, rjz;
-    v2.get(f + i, rix, riy, riz);
-    v1.get(f + j, rjx, rjy, rjz);
-    const bool to_cache = ecache && jcol < 0 && write;
-    const bool to_col = newcol && j == jcol && write;
+    const bool to_cache = ecache && !cols && write;
+    const bool to_col = newcol && ((cols >> j) & 1u) && write;
+    const NodeElement v = node_element(s, sp, v1, v2, i, j);
+    if (to_cache) ecache[j * n + i] = v.v;
+    if (to_col) newcol[i] = v.v;
+    A[j * n + i] = scale * v.v;
     if (sho) {
-      const double ri2 = dot3(rix, riy, riz, rix, riy, riz);
-      const double rj2 = dot3(rjx, rjy, rjz, rjx, rjy, rjz);
-      const double rirj = dot3(rix, riy, riz, rjx, rjy, rjz);
-      const double q = __dsub_rn(__dmul_rn(__dadd_rn(ri2, rj2), s.node_cosh[sp]),
-                                 __dmul_rn(2.0, rirj));
-      const double e = exp(__dmul_rn(-s.node_c[sp], q));
-      if (to_cache) ecache[j * n + i] = e;
-      if (to_col) newcol[i] = e;
-      E[j * n + i] = e;
-      A[j * n + i] = scale * e;
+      E[j * n + i] = v.v;
     } else {
-      double dx = rjx - rix, dy = rjy - riy, dz = rjz - riz;
-      pbc(s, dx, dy, dz);
-      double val, gx, gy, gz;
-      if (s.pg_images[sp]) {
-        val = pg_images_eval(s, sp, dx, dy, dz, gx, gy, gz);
-      } else {
-        double g0, g1, g2;
-        const double v0 = pg_eval(s.pg_nome[sp][0], s.pg_pref[sp][0], s.pg_k[sp][0], s.pg_nmax[sp][0], dx, &g0);
-        const double v1v = pg_eval(s.pg_nome[sp][1], s.pg_pref[sp][1], s.pg_k[sp][1], s.pg_nmax[sp][1], dy, &g1);
-        const double v2v = pg_eval(s.pg_nome[sp][2], s.pg_pref[sp][2], s.pg_k[sp][2], s.pg_nmax[sp][2], dz, &g2);
-        val = v0 * v1v * v2v;
-        gx = g0 / (v0 + 1e-300), gy = g1 / (v1v + 1e-300), gz = g2 / (v2v + 1e-300);
-        gx *= v0; gy *= v0; gz *= v0;
-        gx *= v1v; gy *= v1v; gz *= v1v;
-        gx *= v2v; gy *= v2v; gz *= v2v;
-      }
       if (to_cache) {
-        ecache[j * n + i] = val;
-        ecache[nn + j * n + i] = gx;
-        ecache[2 * nn + j * n + i] = gy;
-        ecache[3 * nn + j * n + i] = gz;
+        ecache[nn + j * n + i] = v.gx;
+        ecache[2 * nn + j * n + i] = v.gy;
+        ecache[3 * nn + j * n + i] = v.gz;
       }
       if (to_col) {
-        newcol[i] = val;
-        newcol[n + i] = gx;
-        newcol[2 * n + i] = gy;
-        newcol[3 * n + i] = gz;
+        newcol[n + i] = v.gx;
+        newcol[2 * n + i] = v.gy;
+        newcol[3 * n + i] = v.gz;
       }
-      A[j * n + i] = scale * val;
-      G[j * n + i] = gx;
-      G[nn + j * n + i] = gy;
-      G[2 * nn + j * n + i] = gz;
+      G[j * n + i] = v.gx;
+      G[nn + j * n + i] = v.gy;
+      G[2 * nn + j * n + i] = v.gz;
     }
   };
   // cached rows (with the new column of a column update), one row per lane
   if (ecache && gl < n && !((rows_new >> gl) & 1u)) {
     const int i = gl;
     for (int j = 0; j < n; ++j) {
-      if (jcol >= 0 && j == jcol) {
+      if ((cols >> j) & 1u) {
         element(i, j);
       } else if (sho) {
         const double e = ecache[j * n + i];
@@ -253,7 +265,8 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
     for (int k = gl; k < nn; k += W) X[k] = xc ? xc[k] : 0.0;
     __syncwarp();
     double det = det_in;
-    if (jcol >= 0) {
+    if (cols) {
+      const int jcol = __ffs(cols) - 1;  // (a level evaluation: one column)
       // column jcol replaced by u = A(:, jcol): w = inv u, ratio = w_jcol,
       // inv'(a, b) = inv(a, b) - (w_a - [a = jcol]) inv(jcol, b) / ratio
       double w = 0.0;
@@ -580,7 +593,7 @@ __host__ __device__ __forceinline__ int node_group_width(int n) {
 static __device__ void node_eval_warp(const DevSys& s, int sp, const SliceView& v1, const SliceView& v2,
                                double scale, double* scr, int full, double& det_out,
                                int& err_out, double* d1, double* d2) {
-  node_eval_group<32>(s, sp, v1, v2, scale, scr, full, nullptr, -1, true, det_out, err_out, d1,
+  node_eval_group<32>(s, sp, v1, v2, scale, scr, full, nullptr, 0u, true, det_out, err_out, d1,
                       d2);
 }
 

@@ -159,3 +159,61 @@ def test_periodic_mover_images(pimc, nlevel, cell):
     a, b = rec["lnt"][0][:, :nlevel + 1], ref["lnt"][:, :nlevel + 1]
     assert np.all(np.abs(a - b) <= 1e-12 * np.maximum(np.abs(b), 1.0))
     assert np.abs(e.download_paths()[0] - port.get_path()).max() <= 1e-12
+
+
+DISPLACE = {
+    # (system, first paths): node models with and without cached entries, Ewald sums
+    # with and without cached structure factors, odd slice counts
+    "dot5_fn": (W.dot20_fn(counts=[3, 2], nslice=40, beta=2.0, nlevel=2, node_temperature=0.5),
+                "const"),
+    "dot5_fn_uncached": (W.dot20_fn(counts=[3, 2], nslice=16, beta=1.0, nlevel=3,
+                                    node_temperature=0.5), "const"),
+    "dot18_fn": (W.dot20_fn(counts=[9, 9], nslice=20, beta=1.0, nlevel=2, node_temperature=0.5),
+                 "const"),
+    "heg10": (W.heg54(n=10, nslice=16, nlevel=2, t_over_tf=1.5), "grid"),
+    "heg10_one_species": (dict(W.heg54(n=10, nslice=16, nlevel=2, t_over_tf=1.5),
+                               node_kind=[2, 0]), "grid"),
+    "heg10_uncached": (W.heg54(n=10, nslice=8, nlevel=2, t_over_tf=3.0), "grid"),
+    "dot3_odd": (W.dot2(counts=[2, 1], nslice=37, beta=2.0, nlevel=2), "gauss"),
+}
+
+
+@pytest.mark.parametrize("nmoving,species", [(1, -1), (3, -1), (2, 0)])
+@pytest.mark.parametrize("nrep", [1, 21, 170])
+@pytest.mark.parametrize("case", list(DISPLACE))
+def test_displacements_then_sections(pimc, case, nrep, nmoving, species):
+    # One to eight CTAs a replica, one to three particles: particles, displacements and
+    # decisions as the restatement's, action differences to the displacement bars of
+    # the golden test; then the sections that follow, whose cached entries and
+    # structure factors the accepted displacements updated.
+    kw, kind = DISPLACE[case]
+    tabs, ew = pimc.coulomb_tables(kw)
+    box = [1.2, 1.2, 1.2]
+    e = pimc.Engine(kw, nrep, tabs, ew, seed=99)
+    x = [W.initial_path(O.make_config(**kw), kind, seed=7 + r) for r in range(nrep)]
+    e.upload_paths(x)
+    e.run_sections(12)
+    start = e.download_paths()
+    scales = [e.replica_state(r)["node_scale"] for r in (0, nrep - 1)]
+    d = e.run_displace(9, box, nmoving, species, records=True)
+    paths = e.download_paths()
+    s = e.run_sections(25, records=True)
+    for r in {0, nrep - 1}:
+        port = O.PortOracle(O.make_config(**dict(kw, seed=99, replica=r)), tabs, ew)
+        port.set_path(x[r])
+        port.run(12)
+        assert np.abs(port.get_path() - start[r]).max() <= 1e-12
+        ref = port.run_displace(9, box, nmoving, species, first_attempt=12)
+        assert np.array_equal(d["ipart"][r], ref["ipart"])
+        assert np.array_equal(d["disp"][r], ref["disp"])
+        assert np.array_equal(d["accepted"][r], ref["accepted"])
+        for k, tol in (("ds", 1e-11), ("ds_node", 1e-9)):
+            assert np.all(np.abs(d[k][r] - ref[k]) <= tol * np.maximum(np.abs(ref[k]), 1.0)), k
+        assert np.abs(port.get_path() - paths[r]).max() <= 1e-12
+        ref = port.run(25, first_attempt=21)
+        for k in ("ifirst1", "ipart", "reject_level"):
+            assert np.array_equal(s[k][r], ref[k]), k
+        nl = kw["nlevel"] + 1
+        for k, tol in (("ds", 1e-11), ("ds_node", 1e-9)):
+            a, b = s[k][r][:, :nl], ref[k][:, :nl]
+            assert np.all(np.abs(a - b) <= tol * np.maximum(np.abs(b), 1.0)), k
