@@ -181,6 +181,7 @@ struct pimc_engine {
   DevBuf<double> d_partial;  // [nrep][kThermoChunks]
   DevBuf<double> d_dscratch;  // displacement moves: node dets and distances per CTA
   DevBuf<double> d_energy;   // [steps][nrep]
+  DevBuf<double> d_forces;   // virial estimator: forces of a pass's replicas (bounded)
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   int graph_attempts = -1, graph_steps = -1;
@@ -199,6 +200,7 @@ struct pimc_engine {
     d_partial.free();
     d_dscratch.free();
     d_energy.free();
+    d_forces.free();
     d_sys.free();
     d_state.free();
     d_paths.free();
@@ -592,16 +594,17 @@ Layout estimator_layout(const std::vector<DevSys>& sys, const int* ikmax_extra) 
     off += (n + 1) & ~1;
     return o;
   };
-  L.s1 = take(3 * nsec * np);
-  L.s2 = L.s1;
-  L.mv = take(3 * nsec);
-  L.nrm = L.mv;
+  L.s1 = L.s2 = L.mv = L.nrm = 0;  // (no section is staged)
   L.red = take(64);
   L.old = L.red;
   L.act = 0;
   L.act_stride = L.act_global = 0;
   L.q = take(np);
   L.ewt = take(2 * ((ik[0] + 1) + (2 * ik[1] + 1) + (2 * ik[2] + 1)) * (np + 1));
+  // their products while three CTAs still share an SM (the 54-electron gas: 57 KB)
+  const int xy = 2 * (ik[0] + 1) * (2 * ik[1] + 1) * np;
+  const bool ewald = ik[0] + ik[1] + ik[2] > 0;
+  L.ewxy = ewald && (off + xy) * 8 <= 74 * 1024 ? take(xy) : 0;
   L.ictl = take(C_NCTL + 2);
   L.dm = L.ndm = L.dist = L.ndist = L.red;
   L.ecache = L.ncol = -1;
@@ -1366,32 +1369,66 @@ int pimc_thermo_energy(pimc_engine* e, double* host_energy) {
 }
 
 namespace {
-// Runs one estimator kernel over every replica (64 chunks each), reduces the
-// partials per replica (÷ M) and copies the energies to the host.
+// Runs one estimator over every replica, reduces the partials per replica (÷ M) and
+// copies the energies to the host.
 enum { kEstVirial = 0, kEstCoulomb = 1 };
 int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L, double* host) {
-  if (e->d_partial.n < (size_t)e->nrep * kThermoChunks &&
-      e->d_partial.alloc((size_t)e->nrep * kThermoChunks))
-    return fail(PIMC_ERR_CUDA, "cudaMalloc energy partials");
+  const int nchunk = which == kEstVirial ? 2 * kThermoChunks : kThermoChunks;
+  if (e->d_partial.n < (size_t)e->nrep * nchunk) {
+    CU(cudaStreamSynchronize(e->stream));
+    if (e->graph) {  // captured with the old buffer
+      cudaGraphExecDestroy(e->graph);
+      e->graph = nullptr;
+    }
+    if (e->d_partial.alloc((size_t)e->nrep * nchunk))
+      return fail(PIMC_ERR_CUDA, "cudaMalloc energy partials");
+  }
   double* d_out = nullptr;
   CU(cudaMallocAsync(&d_out, e->nrep * sizeof(double), e->stream));
   P.sys = e->d_sys.p;
   P.paths = e->d_paths.p;
   P.partial = e->d_partial.p;
-  P.nchunk = kThermoChunks;
+  P.nchunk = nchunk;
   P.nrep = e->nrep;
+  P.ekcache = e->d_ekcache.p;
   P.lay = L;
-  const dim3 grid(kThermoChunks, e->nrep);
+  const int smem_max = 200 * 1024;
   if (which == kEstVirial) {
-    cudaFuncSetAttribute(virial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    virial_kernel<<<grid, kBlock, L.total * 8, e->stream>>>(P);
+    // forces of as many replicas at a time as fit 256 MB (one at least)
+    long long stride = 0;
+    int per_warp = 1;
+    for (const DevSys& d : e->hsys) {
+      stride = std::max(stride, 6LL * d.nslice * d.npart);
+      const int npair = (d.npart + 1) / 2, lpw = npair < 32 ? 32 / npair : 1;
+      per_warp = std::max(per_warp, 6 * lpw * d.npart);
+    }
+    int warps = kBlock / 32;
+    while (warps > 1 && (size_t)warps * per_warp * 8 > (size_t)smem_max) warps /= 2;
+    const int pass = (int)std::max(1LL, std::min((long long)std::min(e->nrep, 65535),
+                                                 (256LL << 20) / (8 * stride)));
+    if (e->d_forces.n < (size_t)pass * stride) {
+      CU(cudaStreamSynchronize(e->stream));
+      if (e->d_forces.alloc((size_t)pass * stride)) return fail(PIMC_ERR_CUDA, "cudaMalloc forces");
+    }
+    P.forces = e->d_forces.p;
+    P.forces_stride = stride;
+    cudaFuncSetAttribute(virial_links_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    cudaFuncSetAttribute(virial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    for (P.rep0 = 0; P.rep0 < e->nrep; P.rep0 += pass) {
+      const dim3 grid(kThermoChunks, std::min(pass, e->nrep - P.rep0));
+      virial_links_kernel<<<grid, 32 * warps, (size_t)warps * per_warp * 8, e->stream>>>(P);
+      virial_kernel<<<grid, kBlock, L.total * 8, e->stream>>>(P);
+      e->launches += 2;
+    }
   } else {
-    cudaFuncSetAttribute(coulomb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    const dim3 grid(kThermoChunks, e->nrep);
+    cudaFuncSetAttribute(coulomb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     coulomb_kernel<<<grid, kBlock, L.total * 8, e->stream>>>(P);
+    e->launches++;
   }
   thermo_reduce_kernel<<<(e->nrep + 127) / 128, 128, 0, e->stream>>>(
-      e->d_sys.p, nullptr, e->d_partial.p, kThermoChunks, e->nrep, d_out);
-  e->launches += 2;
+      e->d_sys.p, nullptr, e->d_partial.p, nchunk, e->nrep, d_out);
+  e->launches++;
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(host, d_out, e->nrep * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
   CU(cudaFreeAsync(d_out, e->stream));
@@ -2030,6 +2067,7 @@ int refresh_order(pimc_engine* e) {
     bool ok = false;
     e->lay = make_layout(live, e->block / 32, ok, e->lay_opts);
     if (!ok) return fail(PIMC_ERR_CAPACITY, "working set does not fit in shared memory");
+    e->est_lay = estimator_layout(live, nullptr);
     int occ = 1;
     occ = section_occupancy(e->minb, e->block, e->lay.total * 8);
     e->grid = std::min(e->nactive, e->num_sms * std::max(occ, 1));
@@ -2298,8 +2336,8 @@ int server_energy(pimc_engine* e, const std::vector<int>& slots, double* out) {
   P.partial = d_part;
   P.nchunk = nchunk;
   P.nrep = n;
-  P.lay = e->lay;
-  thermo_kernel<<<dim3(nchunk, n), kBlock, e->lay.total * 8, e->stream>>>(P);
+  P.lay = e->est_lay;
+  thermo_kernel<<<dim3(nchunk, n), kBlock, e->est_lay.total * 8, e->stream>>>(P);
   e->launches++;
   CU(cudaGetLastError());
   std::vector<double> part((size_t)n * nchunk);

@@ -202,94 +202,125 @@ __device__ __forceinline__ void round_robin_pair(int n, int rd, int k, int& a, i
   }
 }
 
-// ------------------------------------------------------ virial estimator
-// The forces fm, fp of getBeadAction summed over the actions, for the link
-// ending at slice t of particle ip: SpringAction (src/action/SpringAction.cc:112-123),
-// SHOAction (src/action/SHOAction.cc:71-105), PrimSHOAction
-// (src/action/PrimSHOAction.cc:65-81), PairAction (src/action/PairAction.cc:509-599,
-// uk0CalcDerivatives :641-660).  The Ewald term and FixedNodeAction add none.
-static __device__ void bead_forces(const DevSys& s, const double* path, int ip, int t, double* fm,
-                                   double* fp) {
-  const int np = s.npart, M = s.nslice;
-  const int tm = t == 0 ? M - 1 : t - 1, tp = t == M - 1 ? 0 : t + 1;
-  const double* b1 = path + ((size_t)t * np + ip) * 3;
-  const double* b0 = path + ((size_t)tm * np + ip) * 3;
-  const double* b2 = path + ((size_t)tp * np + ip) * 3;
-  const int sp = species_of(s, ip);
-  const double tau = s.tau;
-  for (int d = 0; d < 3; ++d) fm[d] = fp[d] = 0.0;
-  double dmx = b1[0] - b0[0], dmy = b1[1] - b0[1], dmz = b1[2] - b0[2];
-  pbc(s, dmx, dmy, dmz);
-  double dpx = b1[0] - b2[0], dpy = b1[1] - b2[1], dpz = b1[2] - b2[2];
-  pbc(s, dpx, dpy, dpz);
-  const double dm[3] = {dmx, dmy, dmz}, dp[3] = {dpx, dpy, dpz};
-  if (s.spring)
-    for (int d = 0; d < 3; ++d) {
-      fm[d] -= dm[d] / (2 * s.lambda[sp] * tau);
-      fp[d] -= dp[d] / (2 * s.lambda[sp] * tau);
-    }
-  const double om = s.sho_omega[sp];
-  if (om > 0) {
-    const double m = s.mass[sp], cschwt = s.sho_csch[sp], coshwt = s.sho_cosh0[sp];
-    const double tin = 1.0 / tau;
-    for (int d = 0; d < 3; ++d) {
-      fm[d] -= m * om * (b1[d] * coshwt - b0[d]) * cschwt - m * dm[d] * tin;
-      fp[d] -= m * om * (b1[d] * coshwt - b2[d]) * cschwt - m * dp[d] * tin;
-    }
+// evalLongRange summed over slices [t0, t1) from the cached structure factors:
+// sum_k 2 v_k |rho_k|^2 / (2V) + the self energy.  All threads.
+static __device__ double ewald_cached_energy(const DevSys& s, const long long* ekcache, int t0,
+                                             int t1, double* red) {
+  const long long* ek = ekcache + s.ek_offset;
+  const double is = 1.0 / s.ek_scale;
+  const int nt = max(0, t1 - t0), totk = s.totk;
+  double lr = 0.0;
+  for (int it = threadIdx.x; it < nt * totk; it += blockDim.x) {
+    const int t = t0 + it / totk, k = it % totk;
+    const longlong2 v = *(const longlong2*)(ek + ((size_t)t * totk + k) * 2);
+    const double re = __ll2double_rn(v.x) * is, im = __ll2double_rn(v.y) * is;
+    lr += 2 * __ldg(s.vk + k) * (re * re + im * im);
   }
-  if (s.prim_a[sp] != 0 || s.prim_b[sp] != 0) {
-    const double x2 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
-    const double c = -0.5 * (2 * s.prim_a[sp] + 4 * s.prim_b[sp] * x2) * tau;
-    for (int d = 0; d < 3; ++d) {
-      fm[d] += c * b1[d];
-      fp[d] += c * b1[d];
-    }
+  return block_sum(lr, red) * s.one_over_2v + nt * s.self_energy;
+}
+
+// evalLongRange of path slice t (EwaldSum::evalLongRange, src/util/EwaldSum.cc:103-181),
+// charges in m.qpart.  All threads; every thread returns it.  Where the layout has
+// room (m.ewxy), q e^{i kx x} e^{i ky y} is formed once per (kx, ky) and bead instead
+// of once per k-vector: four fused operations a term are left of fourteen.
+static __device__ __noinline__ double ewald_staged_energy(const DevSys& s, const Smem& m,
+                                                          const double* path, int t) {
+  const int np = s.npart, kx0 = s.ikmax[0], ky0 = s.ikmax[1], kz0 = s.ikmax[2];
+  const int nx = kx0 + 1, ny = 2 * ky0 + 1, w = m.ewt_cols;
+  double2* X = (double2*)m.ewt;  // [nx][w]
+  double2* Y = X + nx * w;       // [ny][w]
+  double2* Z = Y + ny * w;       // [nz][w]
+  double2* XY = (double2*)m.ewxy;  // [nx * ny][np]
+  __syncthreads();
+  for (int p = threadIdx.x; p < np; p += blockDim.x) {
+    const double* b = path + ((size_t)t * np + p) * 3;
+    ewald_bead_tables(s, X, Y, Z, w, p, b[0], b[1], b[2]);
   }
-  if (!s.coulomb) return;
-  for (int ti = 0; ti < s.ntab; ++ti) {
-    const DevTable& tb = s.tab[ti];
-    int jb, je;
-    if (ip >= tb.ifirst1 && ip < tb.ifirst1 + tb.npart1) {
-      jb = tb.ifirst2;
-      je = tb.ifirst2 + tb.npart2;
-    } else if (ip >= tb.ifirst2 && ip < tb.ifirst2 + tb.npart2) {
-      jb = tb.ifirst1;
-      je = tb.ifirst1 + tb.npart1;
-    } else {
-      continue;
+  __syncthreads();
+  if (XY) {
+    for (int it = threadIdx.x; it < nx * ny * np; it += blockDim.x) {
+      const int c = it / np, p = it - c * np, kx = c / ny, ky = c - kx * ny;
+      const double2 a = X[kx * w + p], b = Y[ky * w + p];
+      const double q = m.qpart[p], ar = q * a.x, ai = q * a.y;
+      XY[it] = make_double2(ar * b.x - ai * b.y, ar * b.y + ai * b.x);
     }
-    for (int j = jb; j < je; ++j) {
-      if (j == ip) continue;
-      const double* c1 = path + ((size_t)t * np + j) * 3;
-      double delta[3] = {b1[0] - c1[0], b1[1] - c1[1], b1[2] - c1[2]};
-      pbc(s, delta[0], delta[1], delta[2]);
-      const double r = sqrt(dot3(delta[0], delta[1], delta[2], delta[0], delta[1], delta[2]));
-      for (int side = 0; side < 2; ++side) {
-        const double* bo = side == 0 ? b0 : b2;
-        const double* co = path + ((size_t)(side == 0 ? tm : tp) * np + j) * 3;
-        double o[3] = {bo[0] - co[0], bo[1] - co[1], bo[2] - co[2]};
-        pbc(s, o[0], o[1], o[2]);
-        const double ro = sqrt(dot3(o[0], o[1], o[2], o[0], o[1], o[2]));
-        const double q = 0.5 * (r + ro);
-        const double sv[3] = {delta[0] - o[0], delta[1] - o[1], delta[2] - o[2]};
-        const double s2 = dot3(sv[0], sv[1], sv[2], sv[0], sv[1], sv[2]) / (q * q);
-        // uk0CalcDerivatives: the q and s^2 derivatives of the off-diagonal series
-        int i;
-        double x;
-        tab_locate(tb, q, i, x);
-        const double* g0 = tb.ugrid + (size_t)i * 2 * tb.ndata;
-        const double* g1 = g0 + 2 * tb.ndata;
-        double uq = 0, us2 = 0;
-        for (int k = tb.norder; k >= 0; k--) uq = uq * s2 + (__ldg(g1 + k) - __ldg(g0 + k));
-        uq *= tb.logrratioinv * tb.rgridinv / (q * tb.rgridinv);
-        for (int k = tb.norder; k > 0; k--)
-          us2 = us2 * s2 + k * ((1 - x) * __ldg(g0 + k) + x * __ldg(g1 + k));
-        double* f = side == 0 ? fm : fp;
-        for (int d = 0; d < 3; ++d)
-          f[d] -= uq * delta[d] / (2 * r) + us2 * (2 * sv[d] / (q * q) - s2 * delta[d] / (q * r));
+    __syncthreads();
+  }
+  double sum = 0.0;
+  for (int k = threadIdx.x; k < s.totk; k += blockDim.x) {
+    const int kx = __ldg(s.kvec + 3 * k), ky = __ldg(s.kvec + 3 * k + 1) + ky0,
+              kz = __ldg(s.kvec + 3 * k + 2) + kz0;
+    double re = 0.0, im = 0.0;
+    for (int j = 0; j < np; ++j) {
+      double2 u;
+      if (XY) {
+        u = XY[(kx * ny + ky) * np + j];
+      } else {
+        const double2 a = X[kx * w + j], b = Y[ky * w + j];
+        const double q = m.qpart[j], ar = q * a.x, ai = q * a.y;
+        u = make_double2(ar * b.x - ai * b.y, ar * b.y + ai * b.x);
       }
+      const double2 z = Z[kz * w + j];
+      re += u.x * z.x;
+      re -= u.y * z.y;
+      im += u.x * z.y;
+      im += u.y * z.x;
     }
+    sum += 2 * __ldg(s.vk + k) * (re * re + im * im);
   }
+  return block_sum(sum, m.red) * s.one_over_2v + s.self_energy;
+}
+
+// ------------------------------------------------------ virial estimator
+// VirialEnergyEstimator (src/estimator/VirialEnergyEstimator.cc:34-79) in two kernels.
+// The forces fm, fp of getBeadAction (SpringAction src/action/SpringAction.cc:112-123,
+// SHOAction src/action/SHOAction.cc:71-105, PrimSHOAction
+// src/action/PrimSHOAction.cc:65-81, PairAction src/action/PairAction.cc:509-599 and
+// uk0CalcDerivatives :641-660; the Ewald term and FixedNodeAction add none) and utau are
+// sums over links, and a pair's link gives utau and the forces on both particles at
+// both of its ends from one table lookup: virial_links_kernel evaluates every pair
+// once per link.  (One thread per bead and window, every bead going over all
+// partners and both of its links, took six lookups for it, and the windows bounded
+// the threads: 8 electron gases of M = 512 in windows of 16, their four estimators together 34.7 -> 7.2 ms.)
+struct PairForce {
+  double vt;          // d u / d tau
+  double f1[3];       // force on the first particle at the link's end
+  double f0[3];       // and at its start
+};
+
+// One pair's link from the separations e (end) and p (start).
+__device__ __forceinline__ PairForce pair_force(const DevTable& tb, const double* e,
+                                                const double* p) {
+  const double e2 = dot3(e[0], e[1], e[2], e[0], e[1], e[2]);
+  const double p2 = dot3(p[0], p[1], p[2], p[0], p[1], p[2]);
+  const double ri1 = rsqrt(e2), ri0 = rsqrt(p2);
+  const double q = 0.5 * (e2 * ri1 + p2 * ri0), qi = 1.0 / q;
+  const double sv[3] = {e[0] - p[0], e[1] - p[1], e[2] - p[2]};
+  const double s2 = dot3(sv[0], sv[1], sv[2], sv[0], sv[1], sv[2]) * (qi * qi);
+  int i;
+  double x;
+  tab_locate(tb, q, i, x);
+  const double* g0 = tb.ugrid + (size_t)i * 2 * tb.ndata;
+  const double* g1 = g0 + 2 * tb.ndata;
+  double uq = 0.0, us2 = 0.0, vt = 0.0;
+  for (int k = tb.norder; k >= 0; k--) {
+    const double a0 = __ldg(g0 + k), da = __ldg(g1 + k) - a0;
+    uq = uq * s2 + da;
+    if (k > 0) us2 = us2 * s2 + k * (a0 + x * da);
+    vt = vt * s2 + ((1 - x) * __ldg(g0 + tb.ndata + k) + x * __ldg(g1 + tb.ndata + k));
+  }
+  uq *= tb.logrratioinv * qi;
+  // -[uq d / (2 r) + us2 (2 s / q^2 - s2 d / (q r))], d the end's own separation, s
+  // its difference from the other end's
+  const double h = 0.5 * uq - us2 * s2 * qi, w = 2.0 * us2 * (qi * qi);
+  PairForce r;
+  r.vt = vt;
+  const double a1 = h * ri1, a0 = h * ri0;
+  for (int d = 0; d < 3; ++d) {
+    r.f1[d] = -(a1 * e[d] + w * sv[d]);
+    r.f0[d] = -(a0 * p[d] - w * sv[d]);
+  }
+  return r;
 }
 
 struct EstimatorParams {
@@ -299,7 +330,13 @@ struct EstimatorParams {
   int nchunk;
   int nrep;
   Layout lay;
-  int nwindow;  // virial
+  // virial: window, replicas of this pass (blockIdx.y counts from rep0), the forces
+  // fm and fp on every bead, [replica of the pass][nslice_max][npart_max][6]
+  int nwindow;
+  int rep0;
+  double* forces;
+  long long forces_stride;   // doubles per replica
+  const long long* ekcache;  // structure factors of Ewald replicas (null: none)
   // Coulomb estimators: epsilon; with vgrid, the optimized-Ewald form (short
   // range tabulated to rcut, long range from this k-list)
   double epsilon;
@@ -312,26 +349,170 @@ struct EstimatorParams {
   int ikmax[3];
 };
 
-// VirialEnergyEstimator::handleLink / endCalc (src/estimator/VirialEnergyEstimator.cc:34-79).
-// One CTA per (chunk of windows, replica); one thread per (window, particle)
-// runs the window's links in order, so each window's running sums are pi-qmc's.
+// One CTA per (chunk of links, replica); a warp takes as many links at a time as
+// their rounds of disjoint pairs fit its lanes, and keeps those links' forces in
+// shared memory: within a round every (link, particle) belongs to one lane.
+__global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P) {
+  extern __shared__ double smem[];
+  __shared__ DevSys S;
+  const int rep = P.rep0 + blockIdx.y;
+  {
+    const int* src = (const int*)(P.sys + rep);
+    int* dst = (int*)&S;
+    for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x)
+      dst[i] = src[i];
+  }
+  __shared__ signed char tabof[kMaxSpecies][kMaxSpecies];
+  __shared__ double red[64];
+  __syncthreads();
+  const DevSys& s = S;
+  if (threadIdx.x < kMaxSpecies * kMaxSpecies) {
+    const int a = threadIdx.x / kMaxSpecies, b = threadIdx.x % kMaxSpecies;
+    int ti = -1;
+    for (int k = 0; k < s.ntab; ++k)
+      if ((s.tab[k].s1 == a && s.tab[k].s2 == b) || (s.tab[k].s1 == b && s.tab[k].s2 == a)) ti = k;
+    tabof[a][b] = (signed char)ti;
+  }
+  __syncthreads();
+  const double* path = P.paths + s.path_offset;
+  double* forces = P.forces + blockIdx.y * P.forces_stride;
+  const int M = s.nslice, np = s.npart, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nwarps = blockDim.x >> 5;
+  const int nchunk = gridDim.x;
+  const int t0 = (int)((long long)M * blockIdx.x / nchunk);
+  const int t1 = (int)((long long)M * (blockIdx.x + 1) / nchunk);
+  const int ne = np + (np & 1), npair = ne / 2, nrd = s.coulomb && np > 1 ? ne - 1 : 0;
+  const int lpw = npair < 32 ? 32 / npair : 1;  // links a warp takes at once
+  double* F = smem + (size_t)warp * lpw * np * 6;
+  double part = 0.0;
+  for (int tw = t0 + warp * lpw; tw < t1; tw += nwarps * lpw) {
+    const int nl = min(lpw, t1 - tw);
+    __syncwarp();
+    // the beads' own terms start the sums
+    for (int it = lane; it < nl * np; it += 32) {
+      const int t = tw + it / np, ip = it % np, tm = t == 0 ? M - 1 : t - 1;
+      const double* b1 = path + ((size_t)t * np + ip) * 3;
+      const double* b0 = path + ((size_t)tm * np + ip) * 3;
+      part += link_utau(s, path, ip, t, false);
+      const int sp = species_of(s, ip);
+      double fm[3] = {0, 0, 0}, fp[3] = {0, 0, 0};
+      double dm[3] = {b1[0] - b0[0], b1[1] - b0[1], b1[2] - b0[2]};
+      double dp[3] = {b0[0] - b1[0], b0[1] - b1[1], b0[2] - b1[2]};
+      pbc(s, dm[0], dm[1], dm[2]);
+      pbc(s, dp[0], dp[1], dp[2]);
+      if (s.spring) {
+        const double c = 1 / (2 * s.lambda[sp] * s.tau);
+        for (int d = 0; d < 3; ++d) {
+          fm[d] -= dm[d] * c;
+          fp[d] -= dp[d] * c;
+        }
+      }
+      const double om = s.sho_omega[sp];
+      if (om > 0) {
+        const double m = s.mass[sp], csch = s.sho_csch[sp], ch = s.sho_cosh0[sp];
+        const double tin = 1.0 / s.tau;
+        for (int d = 0; d < 3; ++d) {
+          fm[d] -= m * om * (b1[d] * ch - b0[d]) * csch - m * dm[d] * tin;
+          fp[d] -= m * om * (b0[d] * ch - b1[d]) * csch - m * dp[d] * tin;
+        }
+      }
+      if (s.prim_a[sp] != 0 || s.prim_b[sp] != 0) {
+        const double x1 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
+        const double x0 = b0[0] * b0[0] + b0[1] * b0[1] + b0[2] * b0[2];
+        const double c1 = -0.5 * (2 * s.prim_a[sp] + 4 * s.prim_b[sp] * x1) * s.tau;
+        const double c0 = -0.5 * (2 * s.prim_a[sp] + 4 * s.prim_b[sp] * x0) * s.tau;
+        for (int d = 0; d < 3; ++d) {
+          fm[d] += c1 * b1[d];
+          fp[d] += c0 * b0[d];
+        }
+      }
+      for (int d = 0; d < 3; ++d) {
+        F[it * 6 + d] = fm[d];
+        F[it * 6 + 3 + d] = fp[d];
+      }
+    }
+    __syncwarp();
+    for (int rd = 0; rd < nrd; ++rd) {
+      for (int it = lane; it < lpw * npair; it += 32) {
+        const int l = it / npair, k = it - l * npair;
+        int a, b;
+        round_robin_pair(ne, rd, k, a, b);
+        if (l >= nl || a >= np || b >= np) continue;  // (the bye of an odd count)
+        const int ti = tabof[species_of(s, a)][species_of(s, b)];
+        if (ti < 0) continue;
+        const DevTable& tb = s.tab[ti];
+        const int t = tw + l, tm = t == 0 ? M - 1 : t - 1;
+        const double* a1 = path + ((size_t)t * np + a) * 3;
+        const double* a0 = path + ((size_t)tm * np + a) * 3;
+        const double* b1 = path + ((size_t)t * np + b) * 3;
+        const double* b0 = path + ((size_t)tm * np + b) * 3;
+        double e[3] = {a1[0] - b1[0], a1[1] - b1[1], a1[2] - b1[2]};
+        double p[3] = {a0[0] - b0[0], a0[1] - b0[1], a0[2] - b0[2]};
+        const bool tie1 = pbc_and_tie(s, e[0], e[1], e[2]);
+        const bool tie0 = pbc_and_tie(s, p[0], p[1], p[2]);
+        const PairForce fa = pair_force(tb, e, p);
+        PairForce fb;
+        if (tie1 || tie0) {  // the other ordering takes other images
+          for (int d = 0; d < 3; ++d) {
+            e[d] = b1[d] - a1[d];
+            p[d] = b0[d] - a0[d];
+          }
+          pbc(s, e[0], e[1], e[2]);
+          pbc(s, p[0], p[1], p[2]);
+          fb = pair_force(tb, e, p);
+        } else {
+          fb.vt = fa.vt;
+          for (int d = 0; d < 3; ++d) {
+            fb.f1[d] = -fa.f1[d];
+            fb.f0[d] = -fa.f0[d];
+          }
+        }
+        part += 0.5 * fa.vt + 0.5 * fb.vt;
+        double* Fa = F + ((size_t)l * np + a) * 6;
+        double* Fb = F + ((size_t)l * np + b) * 6;
+        for (int d = 0; d < 3; ++d) {
+          Fa[d] += fa.f1[d];
+          Fa[3 + d] += fa.f0[d];
+          Fb[d] += fb.f1[d];
+          Fb[3 + d] += fb.f0[d];
+        }
+      }
+      __syncwarp();
+    }
+    // fm of the link's end bead, fp of its start bead
+    for (int it = lane; it < nl * np * 3; it += 32) {
+      const int q = it / 3, d = it - q * 3, t = tw + q / np, ip = q % np;
+      const int tm = t == 0 ? M - 1 : t - 1;
+      forces[((size_t)t * np + ip) * 6 + d] = F[q * 6 + d];
+      forces[((size_t)tm * np + ip) * 6 + 3 + d] = F[q * 6 + 3 + d];
+    }
+  }
+  double tot = block_sum(part, red);
+  if (s.coulomb && s.ewald && P.ekcache && s.ek_offset >= 0)
+    tot += ewald_cached_energy(s, P.ekcache, t0, t1, red) / s.epsilon;
+  if (threadIdx.x == 0) P.partial[(size_t)rep * P.nchunk + blockIdx.x] = tot;
+}
+
+// VirialEnergyEstimator::handleLink / endCalc's windows.  One CTA per (chunk of
+// windows, replica); one thread per (window, particle) runs the window's links in
+// order, so each window's running sums are pi-qmc's.
 __global__ void __launch_bounds__(kBlock) virial_kernel(EstimatorParams P) {
   extern __shared__ double smem[];
   __shared__ DevSys S;
+  const int rep = P.rep0 + blockIdx.y;
   {
-    const int* src = (const int*)(P.sys + blockIdx.y);
+    const int* src = (const int*)(P.sys + rep);
     int* dst = (int*)&S;
     for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x)
       dst[i] = src[i];
   }
   __syncthreads();
-  if (threadIdx.x == 0) S.mixed = 0;  // the estimator is evaluated in FP64
-  __syncthreads();
   const DevSys& s = S;
   const double* path = P.paths + s.path_offset;
+  const double* forces = P.forces + blockIdx.y * P.forces_stride;
   const int M = s.nslice, np = s.npart, nw = P.nwindow;
   const int nwin = (M + nw - 1) / nw;
-  const int per = (nwin + P.nchunk - 1) / P.nchunk;
+  const int per = (nwin + gridDim.x - 1) / gridDim.x;
   const int w0 = blockIdx.x * per, w1 = min(nwin, w0 + per);
   Smem m = carve(smem, P.lay, s, nullptr);
   const double tau = s.tau, h = 1 / (2 * tau);
@@ -346,39 +527,28 @@ __global__ void __launch_bounds__(kBlock) virial_kernel(EstimatorParams P) {
       const int tm = t == 0 ? M - 1 : t - 1;
       const double* b1 = path + ((size_t)t * np + ip) * 3;
       const double* b0 = path + ((size_t)tm * np + ip) * 3;
+      const double* fr = forces + ((size_t)t * np + ip) * 6;
       double r[3] = {b1[0] - b0[0], b1[1] - b0[1], b1[2] - b0[2]};
       pbc(s, r[0], r[1], r[2]);
-      double fm[3], fp[3];
-      bead_forces(s, path, ip, t, fm, fp);
       double f[3];
       for (int d = 0; d < 3; ++d) {
         rav[d] += r[d];
         r0[d] += (thisWindow - k) * r[d] / thisWindow;
-        f[d] = fm[d] + fp[d];
+        f[d] = fr[d] + fr[3 + d];
         fav[d] += f[d];
       }
-      e += link_utau(s, path, ip, t);
       e += -(1. - 1. / thisWindow) * (3 / (2 * tau)) - h * dot3(f[0], f[1], f[2], rav[0], rav[1], rav[2]);
     }
     e += h * dot3(fav[0], fav[1], fav[2], r0[0], r0[1], r0[2]);
     part += e;
   }
   double tot = block_sum(part, m.red);
-  if (s.coulomb && s.ewald) {  // CoulombAction adds the long-range utau at ipart == 0
+  if (s.coulomb && s.ewald && !(P.ekcache && s.ek_offset >= 0)) {
+    // CoulombAction adds the long-range utau at ipart == 0
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
-    for (int t = w0 * nw; t < min(M, w1 * nw); ++t) {
-      __syncthreads();
-      for (int i = threadIdx.x; i < np; i += blockDim.x) {
-        const double* b = path + ((size_t)t * np + i) * 3;
-        m.s1x[i] = b[0];
-        m.s1y[i] = b[1];
-        m.s1z[i] = b[2];
-      }
-      __syncthreads();
-      tot += ewald_slice_energy(s, m, 0) / s.epsilon;
-    }
+    for (int t = w0 * nw; t < min(M, w1 * nw); ++t) tot += ewald_staged_energy(s, m, path, t) / s.epsilon;
   }
-  if (threadIdx.x == 0) P.partial[(size_t)blockIdx.y * P.nchunk + blockIdx.x] = tot;
+  if (threadIdx.x == 0) P.partial[(size_t)rep * P.nchunk + gridDim.x + blockIdx.x] = tot;
 }
 
 // CoulombEnergyEstimator::handleLink (src/estimator/CoulombEnergyEstimator.cc:30-40) and,
@@ -446,17 +616,7 @@ __global__ void __launch_bounds__(kBlock) coulomb_kernel(EstimatorParams P) {
   double tot = block_sum(part, m.red);
   if (ew) {
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
-    for (int t = t0; t < t1; ++t) {
-      __syncthreads();
-      for (int i = threadIdx.x; i < np; i += blockDim.x) {
-        const double* b = path + ((size_t)t * np + i) * 3;
-        m.s1x[i] = b[0];
-        m.s1y[i] = b[1];
-        m.s1z[i] = b[2];
-      }
-      __syncthreads();
-      tot += ewald_slice_energy(s, m, 0) / eps;
-    }
+    for (int t = t0; t < t1; ++t) tot += ewald_staged_energy(s, m, path, t) / eps;
   }
   if (threadIdx.x == 0) P.partial[(size_t)blockIdx.y * P.nchunk + blockIdx.x] = tot;
 }
@@ -525,40 +685,11 @@ __global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
   }
   double tot = block_sum(part, m.red);
   if (s.coulomb && s.ewald && P.ekcache && s.ek_offset >= 0) {
-    // evalLongRange of every slice from its cached structure factors:
-    // sum_k 2 v_k |rho_k|^2 / (2V) + the self energy
-    const long long* ek = P.ekcache + s.ek_offset;
-    const double is = 1.0 / s.ek_scale;
-    const int nt = max(0, t1 - t0), totk = s.totk;
-    double lr = 0.0;
-    for (int it = threadIdx.x; it < nt * totk; it += blockDim.x) {
-      const int t = t0 + it / totk, k = it % totk;
-      const longlong2 v = *(const longlong2*)(ek + ((size_t)t * totk + k) * 2);
-      const double re = __ll2double_rn(v.x) * is, im = __ll2double_rn(v.y) * is;
-      lr += 2 * __ldg(s.vk + k) * (re * re + im * im);
-    }
-    const double sum = block_sum(lr, m.red);
-    tot += (sum * s.one_over_2v + nt * s.self_energy) / s.epsilon;
+    // evalLongRange of every slice from its cached structure factors
+    tot += ewald_cached_energy(s, P.ekcache, t0, t1, m.red) / s.epsilon;
   } else if (s.coulomb && s.ewald) {
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
-    for (int t = t0; t < t1; ++t) {
-      __syncthreads();
-      for (int i = threadIdx.x; i < np; i += blockDim.x) {
-        const double* b = path + ((size_t)t * np + i) * 3;
-        m.s1x[i] = b[0];
-        m.s1y[i] = b[1];
-        m.s1z[i] = b[2];
-      }
-      if (threadIdx.x == 0) {
-        m.mx[0] = m.s1x[0];
-        m.my[0] = m.s1y[0];
-        m.mz[0] = m.s1z[0];
-      }
-      __syncthreads();
-      // ipart = 0 with the moved bead equal to the old one: new sum == old sum.
-      const double d = ewald_slice_energy(s, m, 0);
-      tot += d / s.epsilon;
-    }
+    for (int t = t0; t < t1; ++t) tot += ewald_staged_energy(s, m, path, t) / s.epsilon;
   }
   if (threadIdx.x == 0) P.partial[(size_t)blockIdx.y * P.nchunk + blockIdx.x] = tot;
 }

@@ -22,6 +22,7 @@ struct Layout {
   int ncol_global;      // the new-column buffer in the CTA's global area
   int gcta;             // doubles of global scratch per CTA
   int ewt_cols;         // bead columns of the Ewald tables area
+  int ewxy;             // their (kx, ky) products (estimators; 0: none)
   int total;  // doubles
 };
 
@@ -83,6 +84,7 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
   m.nodecold = (L.split && gbase) ? gbase : nullptr;
   m.nodecold_stride = L.nodecold_stride;
   m.ewt_cols = L.ewt_cols;
+  m.ewxy = L.ewxy ? base + L.ewxy : nullptr;
   m.nrm = base + L.nrm;
   m.ncol_stride = L.ncol_stride;
   m.nodescr_stride = L.nodescr_stride;

@@ -31,6 +31,7 @@ struct Smem {
   double* dist;             // [nsec][2][ns_max] distances at set-up (moving species)
   double* ndist;            // [nsec][2][ns_max] distances of the new path
   double* ewt;              // Ewald exp(ik.r) tables: [kx, ky, kz rows][ewt_cols]
+  double* ewxy;             // estimators: [kx, ky][npart] products of the tables, or null
   double* qpart;            // [npart] charges
   int* ictl;                // control words
   double* nodescr;          // per-warp node scratch (smem or global)

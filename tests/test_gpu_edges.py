@@ -217,3 +217,47 @@ def test_displacements_then_sections(pimc, case, nrep, nmoving, species):
         for k, tol in (("ds", 1e-11), ("ds_node", 1e-9)):
             a, b = s[k][r][:, :nl], ref[k][:, :nl]
             assert np.all(np.abs(a - b) <= tol * np.maximum(np.abs(b), 1.0)), k
+
+
+ESTIMATE = {
+    "one": W.dot2(counts=[1], sho_omega=[1.0], nslice=37, beta=2.0, nlevel=2, coulomb=0),
+    "dot3_odd": W.dot2(counts=[2, 1], nslice=37, beta=2.0, nlevel=2),
+    "dot67": W.dot2(counts=[40, 27], sho_omega=[1.0, 0.5], nslice=70, beta=3.0, nlevel=3),
+    "dot5_prim": W.dot2(counts=[3, 2], sho_omega=[0.0, 1.0], prim_a=[0.5, 0.0],
+                        prim_b=[0.05, 0.0], nslice=64, beta=3.0, nlevel=3),
+    # grid paths: image ties in every pair; Ewald with and without cached structure factors
+    "heg8_ties": W.heg54(n=8, nslice=128, nlevel=3),
+    "heg10_uncached": W.heg54(n=10, nslice=8, nlevel=2, t_over_tf=3.0),
+}
+
+
+@pytest.mark.parametrize("case", list(ESTIMATE))
+def test_estimators_over_windows(pimc, case):
+    # Windows that divide the path, that do not, and the whole path; sums of
+    # M N^2 terms of mixed sign: 1e-11 of their absolute scale.
+    kw = ESTIMATE[case]
+    tabs, ew = pimc.coulomb_tables(kw)
+    cfg = O.make_config(**kw)
+    x = W.initial_path(cfg, "grid" if kw.get("mover") else "gauss", seed=5)
+    if case == "heg10_uncached":
+        x = x + 0.3 * np.random.default_rng(2).normal(size=x.shape)
+    port = O.PortOracle(cfg, tabs, ew)
+    port.set_path(x)
+    e = pimc.Engine(kw, 3, tabs, ew)
+    e.upload_paths([x] * 3)
+    m = kw["nslice"]
+    for w in (1, 4, 5, m // 2, m):
+        ref = port.virial_energy(w)
+        scale = max(1.0, abs(ref), abs(port.virial_energy(1)))
+        assert np.all(np.abs(e.virial_energy(w) - ref) <= 1e-11 * scale), w
+    if kw["coulomb"]:
+        ref = port.coulomb_energy(1.0)
+        assert np.all(np.abs(e.coulomb_energy(1.0) - ref) <= 1e-12 * abs(ref))
+    if ew is not None:
+        rcut = 0.5 * kw["cell"]
+        est, vg = pimc.ewald_estimator_tables(kw, rcut, kw["ewald_kcut"])
+        ref = port.ewald_coulomb_energy(1.0, rcut, est, vg)
+        assert np.all(np.abs(e.ewald_coulomb_energy(1.0, rcut, est, vg) - ref) <= 1e-11 *
+                      max(1.0, abs(ref)))
+    ref = port.thermo_energy()
+    assert np.all(np.abs(e.thermo_energy() - ref) <= 1e-12 * max(1.0, abs(ref)))
