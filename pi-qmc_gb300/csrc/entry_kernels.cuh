@@ -12,8 +12,7 @@ namespace pimc {
 // SpringAction (src/action/SpringAction.cc:112-123), SHOAction
 // (src/action/SHOAction.cc:71-105), PrimSHOAction (src/action/PrimSHOAction.cc:66-81),
 // PairAction (src/action/PairAction.cc:509-599).  The Ewald term is added per slice.
-__device__ double link_utau(const DevSys& s, const double* path, int ip, int t,
-                            bool with_pairs = true) {
+__device__ double link_utau(const DevSys& s, const double* path, int ip, int t) {
   const int np = s.npart, M = s.nslice;
   const int tm = t == 0 ? M - 1 : t - 1;
   const double* b1 = path + ((size_t)t * np + ip) * 3;
@@ -42,52 +41,6 @@ __device__ double link_utau(const DevSys& s, const double* path, int ip, int t,
     const double x2 = b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2];
     utau += s.prim_a[sp] * x2 + s.prim_b[sp] * x2 * x2;
   }
-  if (s.coulomb && with_pairs) {
-    double uc = 0.0;
-    for (int ti = 0; ti < s.ntab; ++ti) {
-      const DevTable& tb = s.tab[ti];
-      int jb, je;
-      if (ip >= tb.ifirst1 && ip < tb.ifirst1 + tb.npart1) {
-        jb = tb.ifirst2;
-        je = tb.ifirst2 + tb.npart2;
-      } else if (ip >= tb.ifirst2 && ip < tb.ifirst2 + tb.npart2) {
-        jb = tb.ifirst1;
-        je = tb.ifirst1 + tb.npart1;
-      } else {
-        continue;
-      }
-      double up = 0.0;
-      for (int j = jb; j < je; ++j) {
-        if (j == ip) continue;
-        const double* c1 = path + ((size_t)t * np + j) * 3;
-        const double* c0 = path + ((size_t)tm * np + j) * 3;
-        double ex = b1[0] - c1[0], ey = b1[1] - c1[1], ez = b1[2] - c1[2];
-        pbc(s, ex, ey, ez);
-        double px = b0[0] - c0[0], py = b0[1] - c0[1], pz = b0[2] - c0[2];
-        pbc(s, px, py, pz);
-        if (s.mixed) {
-          const float fx = (float)ex, fy = (float)ey, fz = (float)ez;
-          const float gx = (float)px, gy = (float)py, gz = (float)pz;
-          const float r = sqrtf(norm2_f(fx, fy, fz));
-          const float rp = sqrtf(norm2_f(gx, gy, gz));
-          const float q = 0.5f * (r + rp);
-          const float s2 = __fdividef(norm2_f(fx - gx, fy - gy, fz - gz), __fmul_rn(q, q));
-          up += 0.5 * (double)tab_uk0d_tau_f(tb, q, s2);
-          continue;
-        }
-        const double r = sqrt(dot3(ex, ey, ez, ex, ey, ez));
-        const double rp = sqrt(dot3(px, py, pz, px, py, pz));
-        const double q = 0.5 * (r + rp);
-        const double sx = ex - px, sy = ey - py, sz = ez - pz;
-        const double s2 = dot3(sx, sy, sz, sx, sy, sz) / (q * q);
-        double v, vt;
-        tab_uk0d(tb, q, s2, v, vt);
-        up += 0.5 * vt;
-      }
-      uc += up;
-    }
-    utau += uc;
-  }
   return utau;
 }
 
@@ -96,7 +49,7 @@ struct ThermoParams {
   const int* index;  // replicas to measure (null: all, blockIdx.y)
   const double* paths;
   const long long* ekcache;  // structure factors of Ewald replicas (null: none)
-  double* partial;  // [nrep][nchunk]
+  double* partial;  // [nrep][nchunk], the first thermo_chunks of each used
   int nchunk;
   int nrep;
   Layout lay;
@@ -138,54 +91,93 @@ __device__ __forceinline__ bool pbc_and_tie(const DevSys& s, double& x, double& 
   return tie;
 }
 
-// utau of a pair from the minimum images e (link end) and p (link start) of
-// its differences (PairAction's derivative term of the Coulomb pair action,
-// src/action/PairAction.cc:509-599).
-__device__ __forceinline__ double pair_utau_images(const DevSys& s, const DevTable& tb, double ex,
-                                                   double ey, double ez, double px, double py,
-                                                   double pz) {
-  if (s.mixed) {
-    const float fx = f32_rn(ex), fy = f32_rn(ey), fz = f32_rn(ez);
-    const float gx = f32_rn(px), gy = f32_rn(py), gz = f32_rn(pz);
-    const float r = sqrtf(norm2_f(fx, fy, fz));
-    const float rp = sqrtf(norm2_f(gx, gy, gz));
-    const float q = 0.5f * (r + rp);
-    const float s2 = __fdividef(norm2_f(fx - gx, fy - gy, fz - gz), __fmul_rn(q, q));
-    return (double)tab_uk0d_tau_f(tb, q, s2);
+// The separation of a pair at a slice and its length, and whether its image is a tie.
+// (FP64, or rounded to the mixed form's FP32.)
+template <bool kMixed>
+struct PairSep;
+template <>
+struct PairSep<false> : Sep {
+  __device__ __forceinline__ void set(double dx, double dy, double dz) {
+    x = dx;
+    y = dy;
+    z = dz;
+    r = sqrt(dot3(dx, dy, dz, dx, dy, dz));
   }
-  const double r = sqrt(dot3(ex, ey, ez, ex, ey, ez));
-  const double rp = sqrt(dot3(px, py, pz, px, py, pz));
-  const double q = 0.5 * (r + rp);
-  const double sx = ex - px, sy = ey - py, sz = ez - pz;
+};
+template <>
+struct PairSep<true> : SepF {
+  __device__ __forceinline__ void set(double dx, double dy, double dz) {
+    x = f32_rn(dx);
+    y = f32_rn(dy);
+    z = f32_rn(dz);
+    r = sqrtf(norm2_f(x, y, z));
+  }
+};
+
+// (double)f on the integer pipe (f a normal number or zero; else the conversion).
+__device__ __forceinline__ double f64_of(float f) {
+  const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return (double)f;
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + (896u << 20))), (int)(m << 29));
+}
+
+// utau of a pair's link from its separations at the end (e) and the start (p)
+// (PairAction's derivative term of the Coulomb pair action,
+// src/action/PairAction.cc:509-599).
+__device__ __forceinline__ double pair_utau_link(const DevTable& tb, const PairSep<false>& e,
+                                                 const PairSep<false>& p) {
+  const double q = 0.5 * (e.r + p.r);
+  const double sx = e.x - p.x, sy = e.y - p.y, sz = e.z - p.z;
   const double s2 = dot3(sx, sy, sz, sx, sy, sz) / (q * q);
   double v, vt;
   tab_uk0d(tb, q, s2, v, vt);
   return vt;
 }
+__device__ __forceinline__ double pair_utau_link(const DevTable& tb, const PairSep<true>& e,
+                                                 const PairSep<true>& p) {
+  const float q = 0.5f * (e.r + p.r);
+  const float s2 = __fdividef(norm2_f(e.x - p.x, e.y - p.y, e.z - p.z), __fmul_rn(q, q));
+  return f64_of(tab_uk0d_tau_f(tb, q, s2));
+}
 
-// The pair's share of Σ_links utau: pi-qmc adds 0.5 utau for each ordering
-// (PairAction::getBeadAction runs over every partner of every particle); the two
-// orderings agree unless an image tie makes them differ, so one evaluation
-// usually stands for both, and the ordering (j, i) is evaluated only on a tie.
-__device__ double pair_utau(const DevSys& s, const DevTable& tb, const double* path, int i, int j,
-                            int t) {
+// The pair's share of Σ_links utau over the links that end at slices [t0, t1): each
+// separation serves the link that ends there and the one that starts there (152
+// electron gases of a mixed step 5.7 -> 3.3 ms).  pi-qmc
+// adds 0.5 utau for each ordering (PairAction::getBeadAction runs over every partner
+// of every particle); the two orderings agree unless an image tie makes them
+// differ, so one evaluation usually stands for both, and the ordering (j, i) is
+// evaluated only on a tie.
+template <bool kMixed>
+__device__ __forceinline__ double pair_utau_run(const DevSys& s, const DevTable& tb,
+                                                const double* path, int i, int j, int t0, int t1) {
   const int np = s.npart, M = s.nslice;
-  const int tm = t == 0 ? M - 1 : t - 1;
-  const double* b1 = path + ((size_t)t * np + i) * 3;
-  const double* b0 = path + ((size_t)tm * np + i) * 3;
-  const double* c1 = path + ((size_t)t * np + j) * 3;
-  const double* c0 = path + ((size_t)tm * np + j) * 3;
-  double ex = b1[0] - c1[0], ey = b1[1] - c1[1], ez = b1[2] - c1[2];
-  double px = b0[0] - c0[0], py = b0[1] - c0[1], pz = b0[2] - c0[2];
-  const bool tie1 = pbc_and_tie(s, ex, ey, ez);
-  const bool tie0 = pbc_and_tie(s, px, py, pz);
-  const double a = pair_utau_images(s, tb, ex, ey, ez, px, py, pz);
-  if (!(tie1 || tie0)) return a;
-  double fx = c1[0] - b1[0], fy = c1[1] - b1[1], fz = c1[2] - b1[2];
-  double gx = c0[0] - b0[0], gy = c0[1] - b0[1], gz = c0[2] - b0[2];
-  pbc(s, fx, fy, fz);
-  pbc(s, gx, gy, gz);
-  return 0.5 * a + 0.5 * pair_utau_images(s, tb, fx, fy, fz, gx, gy, gz);
+  const auto at = [&](int t, int a, int b, PairSep<kMixed>& sep) {
+    const double* ba = path + ((size_t)t * np + a) * 3;
+    const double* bb = path + ((size_t)t * np + b) * 3;
+    double x = ba[0] - bb[0], y = ba[1] - bb[1], z = ba[2] - bb[2];
+    const bool tie = pbc_and_tie(s, x, y, z);
+    sep.set(x, y, z);
+    return tie;
+  };
+  double sum = 0.0;
+  PairSep<kMixed> p, e;
+  int tm = t0 == 0 ? M - 1 : t0 - 1;
+  bool tie0 = at(tm, i, j, p);
+  for (int t = t0; t < t1; ++t) {
+    const bool tie1 = at(t, i, j, e);
+    double a = pair_utau_link(tb, e, p);
+    if (tie1 || tie0) {
+      PairSep<kMixed> re, rp;
+      at(t, j, i, re);
+      at(tm, j, i, rp);
+      a = 0.5 * a + 0.5 * pair_utau_link(tb, re, rp);
+    }
+    sum += a;
+    p = e;
+    tie0 = tie1;
+    tm = t;
+  }
+  return sum;
 }
 
 // Pair k of round rd of the round-robin schedule over n (even) players: every
@@ -393,7 +385,7 @@ __global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P)
       const int t = tw + it / np, ip = it % np, tm = t == 0 ? M - 1 : t - 1;
       const double* b1 = path + ((size_t)t * np + ip) * 3;
       const double* b0 = path + ((size_t)tm * np + ip) * 3;
-      part += link_utau(s, path, ip, t, false);
+      part += link_utau(s, path, ip, t);
       const int sp = species_of(s, ip);
       double fm[3] = {0, 0, 0}, fp[3] = {0, 0, 0};
       double dm[3] = {b1[0] - b0[0], b1[1] - b0[1], b1[2] - b0[2]};
@@ -624,22 +616,24 @@ __global__ void __launch_bounds__(kBlock) coulomb_kernel(EstimatorParams P) {
 // Per-replica energy from the chunk partials: chunks summed in order, then
 // divided by the slice count (ThermoEnergyEstimator's normalisation).
 __global__ void thermo_reduce_kernel(const DevSys* sys, const int* index, const double* partial,
-                                     int nchunk, int nrow, double* energy) {
+                                     int nchunk, int nrow, double* energy, bool thermo) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nrow) return;
   const int r = index ? index[k] : k;
+  const int used = thermo ? sys[r].thermo_chunks : nchunk;
   double s = 0.0;
-  for (int c = 0; c < nchunk; ++c) s = __dadd_rn(s, partial[(size_t)k * nchunk + c]);
+  for (int c = 0; c < used; ++c) s = __dadd_rn(s, partial[(size_t)k * nchunk + c]);
   energy[r] = __ddiv_rn(s, (double)sys[r].nslice);
 }
 
-// One CTA per (chunk of slices, replica): link utau sums plus, for Coulomb with
-// Ewald, the long-range energy of each slice (CoulombAction::getBeadAction adds
+// One CTA per (chunk of slices, replica; a replica has DevSys::thermo_chunks): link
+// utau sums plus, for Coulomb with Ewald, the long-range energy of each slice (CoulombAction::getBeadAction adds
 // it at ipart == 0, src/action/CoulombAction.cc:165-171).
 __global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
   extern __shared__ double smem[];
   __shared__ DevSys S;
   const int r = P.index ? P.index[blockIdx.y] : blockIdx.y;
+  if ((int)blockIdx.x >= P.sys[r].thermo_chunks) return;
   {
     const int* src = (const int*)(P.sys + r);
     int* dst = (int*)&S;
@@ -650,8 +644,9 @@ __global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
   const DevSys& s = S;
   const double* path = P.paths + s.path_offset;
   const int M = s.nslice, np = s.npart;
-  const int per = (M + P.nchunk - 1) / P.nchunk;
-  const int t0 = blockIdx.x * per, t1 = min(M, t0 + per);
+  const int nchunk = s.thermo_chunks;
+  const int t0 = (int)((long long)M * blockIdx.x / nchunk);
+  const int t1 = (int)((long long)M * (blockIdx.x + 1) / nchunk);
   Smem m = carve(smem, P.lay, s, nullptr);
   // table of each species pair (pairs with no table contribute nothing)
   __shared__ signed char tabof[kMaxSpecies][kMaxSpecies];
@@ -666,21 +661,26 @@ __global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
   double part = 0.0;
   for (int it = threadIdx.x; it < (t1 - t0) * np; it += blockDim.x) {
     const int t = t0 + it / np, ip = it % np;
-    part += link_utau(s, path, ip, t, false);
+    part += link_utau(s, path, ip, t);
   }
   if (s.coulomb && np > 1) {
-    // every pair once per slice: rounds of the round-robin schedule (np rounded up to even)
-    const int ne = np + (np & 1), per_round = ne / 2, nrd = ne - 1;
-    const int items = (t1 - t0) * nrd * per_round;
+    // every pair once: rounds of the round-robin schedule (np rounded up to even).  A
+    // thread takes a run of a pair's links, as long as the threads all have one (a
+    // run of R links forms R + 1 separations).
+    const int ne = np + (np & 1), per_round = ne / 2, nrd = ne - 1, pairs = nrd * per_round;
+    const int len = t1 - t0;
+    const int run = max(1, min(len, len * pairs / (2 * kBlock)));
+    const int items = ((len + run - 1) / run) * pairs;
     for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int t = t0 + it / (nrd * per_round);
-      const int rest = it % (nrd * per_round);
+      const int ta = t0 + it / pairs * run, tb = min(t1, ta + run);
+      const int rest = it % pairs;
       int a, b;
       round_robin_pair(ne, rest / per_round, rest % per_round, a, b);
       if (a >= np || b >= np) continue;  // the bye of an odd count
       const int ti = tabof[species_of(s, a)][species_of(s, b)];
       if (ti < 0) continue;
-      part += pair_utau(s, s.tab[ti], path, a, b, t);
+      part += s.mixed ? pair_utau_run<true>(s, s.tab[ti], path, a, b, ta, tb)
+                      : pair_utau_run<false>(s, s.tab[ti], path, a, b, ta, tb);
     }
   }
   double tot = block_sum(part, m.red);

@@ -69,6 +69,7 @@ struct DevSys {
   double one_over_2v, self_energy, deltak[3];
   int ikmax[3];
   int ns_max;           // largest node-species count
+  int thermo_chunks;    // CTAs of the thermodynamic estimator (kThermoChunks at most)
   uint32_t stream_id;     // random stream of this replica (its replica or request id)
   long long nc_offset;    // doubles into the Slater-result cache pool (-1: no cache)
   int nc_stride;          // doubles per cache entry
