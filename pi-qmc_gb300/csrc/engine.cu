@@ -1655,6 +1655,39 @@ int pimc_run_steps(pimc_engine* e, int nattempt, int nsteps, double* host_energy
   return PIMC_OK;
 }
 
+namespace {
+// Launch shape of a NodeModel-level batch.  A batch with a warp or less per SM runs
+// one-warp CTAs on an SM each, for the shortest time; larger ones pack up to eight
+// warps, and when the whole scratch would keep fewer than 16 warps on an SM (the FP64
+// pipe wants as many), its cold part goes to global memory.
+struct NodeEvalShape {
+  int grid, warps, stage, scratch, cold;  // cold: doubles per warp in global memory (0: none)
+  size_t smem;
+};
+NodeEvalShape node_eval_shape(const DevSys& s, int ispec, int nbatch, int num_sms) {
+  const int n = s.spec_count[ispec], G = 32 / node_group_width(n);
+  const bool fr = s.node_kind[ispec] == PIMC_NODES_FREE;
+  NodeEvalShape r{};
+  const long long warps = (nbatch + G - 1) / G;
+  r.stage = G * 6 * n;
+  r.scratch = (G * node_group_scratch(n, fr) + 1) & ~1;
+  const int per_sm = kSmemLimit / 8 / (r.stage + r.scratch);
+  if (warps > (long long)num_sms * per_sm && per_sm < 16) {
+    r.scratch = (G * node_group_hot(n) + 1) & ~1;
+    r.cold = (G * node_group_cold(n, fr) + 1) & ~1;
+  }
+  r.warps = 1;
+  while (r.warps < 8 && warps > (long long)num_sms * r.warps &&
+         (size_t)2 * r.warps * (r.stage + r.scratch) * 8 <= kSmemLimit / 2)
+    r.warps *= 2;
+  r.smem = (size_t)r.warps * (r.stage + r.scratch) * 8;
+  const int resident = std::max<int>(1, std::min<size_t>(kSmemLimit / r.smem, 32 / r.warps));
+  r.grid = (int)std::min<long long>((warps + r.warps - 1) / r.warps,
+                                    (long long)num_sms * resident);
+  return r;
+}
+}  // namespace
+
 int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* section,
                            const double* moving, const int* ipart, double* ds) {
   if (!e || nbatch <= 0 || !section || !moving || !ipart || !ds)
@@ -1675,10 +1708,15 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   double *d_sec = nullptr, *d_mov = nullptr, *d_ds = nullptr, *d_scr = nullptr;
   int* d_ip = nullptr;
   if (alay.act_global)
-    CU(cudaMallocAsync(&d_scr, (size_t)nbatch * alay.gcta * 8, e->stream));
+    CU(cudaMallocAsync(&d_scr, (size_t)std::min(nbatch, 65535) * alay.gcta * 8, e->stream));
   CU(cudaMallocAsync(&d_sec, nsecd * 8, e->stream));
   CU(cudaMallocAsync(&d_mov, nmovd * 8, e->stream));
-  CU(cudaMallocAsync(&d_ds, nbatch * 8, e->stream));
+  // with Ewald sums the section's slices go to CTAs of their own, as many per entry as
+  // a batch of this size leaves room for (two CTAs an SM), added up here in order
+  int parts = 1;
+  if (s.ewald && s.coulomb && level == 0)
+    parts = 1 + std::max(1, std::min(s.nsec - 2, 2 * e->num_sms / nbatch));
+  CU(cudaMallocAsync(&d_ds, (size_t)nbatch * parts * 8, e->stream));
   CU(cudaMallocAsync(&d_ip, nbatch * 4, e->stream));
   CU(cudaMemcpyAsync(d_sec, section, nsecd * 8, cudaMemcpyHostToDevice, e->stream));
   CU(cudaMemcpyAsync(d_mov, moving, nmovd * 8, cudaMemcpyHostToDevice, e->stream));
@@ -1692,16 +1730,30 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   P.level = level;
   P.lay = alay;
   P.scratch = d_scr;
-  action_diff_kernel<<<nbatch, kBlock, P.lay.total * 8, e->stream>>>(P);
-  e->launches++;
+  std::vector<double> share((size_t)nbatch * parts);
+  for (int b0 = 0; b0 < nbatch; b0 += 65535) {
+    const int nb = std::min(65535, nbatch - b0);
+    ActionDiffParams Q = P;
+    Q.section += (size_t)b0 * s.nsec * s.npart * 3;
+    Q.moving += (size_t)b0 * s.nsec * 3;
+    Q.ipart += b0;
+    Q.ds += (size_t)b0 * parts;
+    action_diff_kernel<<<dim3(parts, nb), kBlock, P.lay.total * 8, e->stream>>>(Q);
+    e->launches++;
+  }
   CU(cudaGetLastError());
-  CU(cudaMemcpyAsync(ds, d_ds, nbatch * 8, cudaMemcpyDeviceToHost, e->stream));
+  CU(cudaMemcpyAsync(share.data(), d_ds, share.size() * 8, cudaMemcpyDeviceToHost, e->stream));
   if (d_scr) CU(cudaFreeAsync(d_scr, e->stream));
   CU(cudaFreeAsync(d_sec, e->stream));
   CU(cudaFreeAsync(d_mov, e->stream));
   CU(cudaFreeAsync(d_ds, e->stream));
   CU(cudaFreeAsync(d_ip, e->stream));
   CU(cudaStreamSynchronize(e->stream));
+  for (int b = 0; b < nbatch; ++b) {
+    double v = share[(size_t)b * parts];
+    for (int k = 1; k < parts; ++k) v += share[(size_t)b * parts + k];
+    ds[b] = v;
+  }
   return PIMC_OK;
 }
 
@@ -1712,7 +1764,7 @@ int pimc_node_evaluate(pimc_engine* e, int ispec, int nbatch, const double* r1, 
   const DevSys& s = e->hsys[0];
   if (ispec < 0 || ispec >= s.nspecies || !s.node_kind[ispec])
     return fail(PIMC_ERR_INVALID, "species has no node model");
-  const int np = s.npart, n = s.spec_count[ispec];
+  const int np = s.npart;
   const size_t nr = (size_t)nbatch * np * 3;
   double *d_r1, *d_r2, *d_det, *d_d1, *d_d2;
   int* d_err;
@@ -1734,12 +1786,20 @@ int pimc_node_evaluate(pimc_engine* e, int ispec, int nbatch, const double* r1, 
   P.d2 = d_d2;
   P.err = d_err;
   P.ispec = ispec;
-  P.lay = e->lay;
-  const int smem = (8 * np + node_group_scratch(n) + 2) * 8;
-  cudaFuncSetAttribute(node_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  node_eval_kernel<<<nbatch, kBlock, smem, e->stream>>>(P);
+  P.nbatch = nbatch;
+  const NodeEvalShape sh = node_eval_shape(s, ispec, nbatch, e->num_sms);
+  P.stage_stride = sh.stage;
+  P.scratch_stride = sh.scratch;
+  P.cold_stride = sh.cold;
+  double* d_cold = nullptr;
+  if (sh.cold)
+    CU(cudaMallocAsync(&d_cold, (size_t)sh.grid * sh.warps * sh.cold * 8, e->stream));
+  P.cold = d_cold;
+  cudaFuncSetAttribute(node_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  node_eval_kernel<<<sh.grid, 32 * sh.warps, sh.smem, e->stream>>>(P);
   e->launches++;
   CU(cudaGetLastError());
+  if (d_cold) CU(cudaFreeAsync(d_cold, e->stream));
   CU(cudaMemcpyAsync(det, d_det, nbatch * 8, cudaMemcpyDeviceToHost, e->stream));
   CU(cudaMemcpyAsync(d1, d_d1, (size_t)nbatch * np * 8, cudaMemcpyDeviceToHost, e->stream));
   CU(cudaMemcpyAsync(d2, d_d2, (size_t)nbatch * np * 8, cudaMemcpyDeviceToHost, e->stream));

@@ -700,12 +700,66 @@ struct ActionDiffParams {
   const double* section;  // [nbatch][nsec][npart][3]
   const double* moving;   // [nbatch][nsec][3]
   const int* ipart;
-  double* ds;
+  double* ds;             // [nbatch][gridDim.x] shares, added by the caller
   int level;
   Layout lay;
-  double* scratch;  // the layout's global area per CTA (null: none)
+  double* scratch;  // the layout's global area per entry (null: none)
 };
 
+// evalLongRange of a section slice with the moved bead less that without it (charges
+// in m.qpart): the structure factors of the slice, four threads a k-vector, and the
+// moved particle's old and new terms.  All threads; every thread returns it.
+static __device__ __noinline__ double ewald_move_energy(const DevSys& s, const Smem& m,
+                                                        const double* sec, const double* mov,
+                                                        int ipart) {
+  const int np = s.npart, kx0 = s.ikmax[0], ky0 = s.ikmax[1], kz0 = s.ikmax[2];
+  const int nx = kx0 + 1, ny = 2 * ky0 + 1, w = m.ewt_cols;  // column np: the moved bead
+  double2* X = (double2*)m.ewt;
+  double2* Y = X + nx * w;
+  double2* Z = Y + ny * w;
+  __syncthreads();
+  for (int p = threadIdx.x; p <= np; p += blockDim.x) {
+    const double* b = p < np ? sec + (size_t)p * 3 : mov;
+    ewald_bead_tables(s, X, Y, Z, w, p, b[0], b[1], b[2]);
+  }
+  __syncthreads();
+  const auto term = [&](int kx, int ky, int kz, int j, double q) {
+    const double2 a = X[kx * w + j], b = Y[ky * w + j], z = Z[kz * w + j];
+    const double ar = q * a.x, ai = q * a.y;
+    const double ur = ar * b.x - ai * b.y, ui = ar * b.y + ai * b.x;
+    return make_double2(ur * z.x - ui * z.y, ur * z.y + ui * z.x);
+  };
+  double sum = 0.0;
+  const int part = threadIdx.x & 3;
+  for (int k0 = 0; k0 < s.totk; k0 += blockDim.x / 4) {  // (whole warps take part)
+    const int k = k0 + (threadIdx.x >> 2);
+    const bool on = k < s.totk;
+    const int kx = on ? __ldg(s.kvec + 3 * k) : 0, ky = (on ? __ldg(s.kvec + 3 * k + 1) : 0) + ky0,
+              kz = (on ? __ldg(s.kvec + 3 * k + 2) : 0) + kz0;
+    double re = 0.0, im = 0.0;
+    for (int j = part; on && j < np; j += 4) {
+      const double2 v = term(kx, ky, kz, j, m.qpart[j]);
+      re += v.x;
+      im += v.y;
+    }
+    for (int o = 1; o < 4; o <<= 1) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    if (on && part == 0) {
+      const double q = m.qpart[ipart];
+      const double2 o = term(kx, ky, kz, ipart, q), n = term(kx, ky, kz, np, q);
+      const double nr = re + (n.x - o.x), ni = im + (n.y - o.y);
+      sum += 2 * __ldg(s.vk + k) * ((nr * nr + ni * ni) - (re * re + im * im));
+    }
+  }
+  return block_sum(sum, m.red) * s.one_over_2v;
+}
+
+// Action differences of independent sections.  CTA (0, b) takes entry b's spring,
+// confinement and pair terms; with Ewald sums on level 0, CTAs (1 .., b) share the
+// section's slices.  (One CTA an entry, slice after slice, each with both sums in
+// full: 3440 us for one section of the electron gas from host arrays, now 312 us.)
 __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P) {
   extern __shared__ double smem[];
   __shared__ DevSys S;
@@ -717,10 +771,21 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   }
   __syncthreads();
   const DevSys& s = S;
-  Smem m = carve(smem, P.lay, s, P.scratch);
-  const int b = blockIdx.x, np = s.npart, nsec = s.nsec;
+  // (the global area serves the action differences, CTA (0, b) alone)
+  Smem m = carve(smem, P.lay, s, P.scratch ? P.scratch + (size_t)blockIdx.y * P.lay.gcta : nullptr);
+  const int b = blockIdx.y, np = s.npart, nsec = s.nsec;
   const double* sec = P.section + (size_t)b * nsec * np * 3;
   const double* mov = P.moving + (size_t)b * nsec * 3;
+  const int ip = P.ipart[b];
+  double* out = P.ds + (size_t)b * gridDim.x + blockIdx.x;
+  if (blockIdx.x > 0) {
+    for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
+    double ds = 0.0;
+    for (int t = blockIdx.x; t < nsec - 1; t += gridDim.x - 1)
+      ds += ewald_move_energy(s, m, sec + (size_t)t * np * 3, mov + (size_t)t * 3, ip);
+    if (threadIdx.x == 0) *out = ds * s.tau / s.epsilon;
+    return;
+  }
   for (int idx = threadIdx.x; idx < nsec * np; idx += blockDim.x) {
     m.s1x[idx] = sec[idx * 3];
     m.s1y[idx] = sec[idx * 3 + 1];
@@ -731,9 +796,7 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
     m.my[t] = mov[t * 3 + 1];
     m.mz[t] = mov[t * 3 + 2];
   }
-  for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
   __syncthreads();
-  const int ip = P.ipart[b];
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, d = s.nlevel - P.level;
   double* lds = m.red + kWarps + 8;
   if (s.mixed)
@@ -743,10 +806,7 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   __syncthreads();
   action_reduce(s, m.act, m.act_stride, d, d, nw, lds);
   __syncthreads();
-  double ds = lds[P.level];
-  if (s.ewald && s.coulomb && P.level == 0)
-    for (int t = 1; t < nsec - 1; ++t) ds += ewald_slice_diff(s, m, ip, t);
-  if (threadIdx.x == 0) P.ds[b] = ds;
+  if (threadIdx.x == 0) *out = lds[P.level];
 }
 
 // ---------------------------------------------------- NodeModel-level entry
@@ -760,9 +820,16 @@ struct NodeEvalParams {
   double* d2;
   int* err;
   int ispec;
-  Layout lay;
+  int nbatch;
+  int stage_stride;    // doubles of staged beads per warp
+  int scratch_stride;  // of Slater scratch per warp (its hot part when split)
+  double* cold;        // the scratch's cold parts in global memory (null: not split)
+  int cold_stride;     // doubles of them per warp
 };
 
+// Warps take as many pairs at a time as their lane groups (one of 32 lanes, two of
+// 16, four of 8 by the species' size).  (One pair a CTA of eight warps, seven of them
+// idle: 1024 27 x 27 evaluations from host arrays 1142 us, now 672 us.)
 __global__ void __launch_bounds__(kBlock) node_eval_kernel(NodeEvalParams P) {
   extern __shared__ double smem[];
   __shared__ DevSys S;
@@ -774,39 +841,43 @@ __global__ void __launch_bounds__(kBlock) node_eval_kernel(NodeEvalParams P) {
   }
   __syncthreads();
   const DevSys& s = S;
-  const int np = s.npart, b = blockIdx.x, sp = P.ispec;
-  double* sx = smem;
-  double* sy = sx + 2 * np;
-  double* sz = sy + 2 * np;
-  double* dd = sz + 2 * np;  // [2][np]
-  double* scr = dd + 2 * np;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    sx[i] = P.r1[((size_t)b * np + i) * 3];
-    sy[i] = P.r1[((size_t)b * np + i) * 3 + 1];
-    sz[i] = P.r1[((size_t)b * np + i) * 3 + 2];
-    sx[np + i] = P.r2[((size_t)b * np + i) * 3];
-    sy[np + i] = P.r2[((size_t)b * np + i) * 3 + 1];
-    sz[np + i] = P.r2[((size_t)b * np + i) * 3 + 2];
-    dd[i] = 200;
-    dd[np + i] = 200;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    SliceView v1{sx, sy, sz, np, 0, -1, 0, 0, 0};
-    SliceView v2{sx, sy, sz, np, 1, -1, 0, 0, 0};
+  const int np = s.npart, sp = P.ispec, n = s.spec_count[sp], f = s.spec_first[sp];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int W = node_group_width(n), G = 32 / W, g = lane / W, gl = lane & (W - 1);
+  const bool free_nodes = s.node_kind[sp] != PIMC_NODES_SHO;
+  const long long gw = (long long)blockIdx.x * nwarps + warp;
+  double* st = smem + (size_t)warp * P.stage_stride + (size_t)g * 6 * n;
+  double* scr = smem + (size_t)nwarps * P.stage_stride + (size_t)warp * P.scratch_stride +
+                (size_t)g * (P.cold ? node_group_hot(n) : node_group_scratch(n, free_nodes));
+  double* cold = P.cold ? P.cold + gw * P.cold_stride + (size_t)g * node_group_cold(n, free_nodes)
+                        : nullptr;
+  const double scale = P.state[0].node_scale[sp];
+  for (long long base = gw * G; base < P.nbatch; base += (long long)gridDim.x * nwarps * G) {
+    const bool act = base + g < P.nbatch;
+    const size_t b = act ? base + g : base;
+    __syncwarp();
+    for (int p = gl; p < n; p += W) {
+      const double* b1 = P.r1 + (b * np + f + p) * 3;
+      const double* b2 = P.r2 + (b * np + f + p) * 3;
+      for (int d = 0; d < 3; ++d) {
+        st[d * n + p] = b1[d];
+        st[(3 + d) * n + p] = b2[d];
+      }
+    }
+    if (act)
+      for (int p = gl; p < np; p += W) P.d1[b * np + p] = P.d2[b * np + p] = 200;
+    __syncwarp();
+    // node_eval_group reads particle f + p: views offset so that it lands on entry p
+    SliceView v1{st - f, st + n - f, st + 2 * n - f, n, 0, -1, 0, 0, 0};
+    SliceView v2{st + 3 * n - f, st + 4 * n - f, st + 5 * n - f, n, 0, -1, 0, 0, 0};
     double det;
     int err;
-    const int f = s.spec_first[sp];
-    node_eval_warp(s, sp, v1, v2, P.state[0].node_scale[sp], scr, 1, det, err, dd + f, dd + np + f);
-    if (threadIdx.x == 0) {
+    node_eval_dispatch(W, s, sp, v1, v2, scale, scr, 1, nullptr, 0u, act, det, err,
+                       P.d1 + b * np + f, P.d2 + b * np + f, nullptr, 0u, cold);
+    if (act && gl == 0) {
       P.det[b] = det;
       P.err[b] = err;
     }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    P.d1[(size_t)b * np + i] = dd[i];
-    P.d2[(size_t)b * np + i] = dd[np + i];
   }
 }
 

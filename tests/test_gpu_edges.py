@@ -261,3 +261,57 @@ def test_estimators_over_windows(pimc, case):
                       max(1.0, abs(ref)))
     ref = port.thermo_energy()
     assert np.all(np.abs(e.thermo_energy() - ref) <= 1e-12 * max(1.0, abs(ref)))
+
+
+@pytest.mark.parametrize("n,heg", [(1, False), (8, False), (9, False), (16, False), (17, True),
+                                   (27, True), (32, False)])
+def test_node_evaluate_batches(pimc, n, heg):
+    # Batches of one pair, part of a warp's lane groups, one wave and more than the
+    # resident warps: each pair's results do not depend on the batch, bit for bit, and
+    # are the restatement's.
+    if heg:
+        kw = W.heg54(n=2 * n, nslice=64, nlevel=3, beta=2.0, coulomb=0, ewald=0)
+    else:
+        kw = W.dot20_fn(counts=[n, 1], nslice=64, beta=4.0, nlevel=3, coulomb=0,
+                        node_temperature=0.5)
+    npart = sum(kw["counts"])
+    rng = np.random.default_rng(n)
+    nb = 3001
+    side = kw["cell"] if heg else 3.0
+    r1 = rng.uniform(-side / 2, side / 2, size=(nb, npart, 3))
+    r2 = r1 + 0.1 * rng.normal(size=r1.shape)
+    e = pimc.Engine(kw, 1)
+    whole = e.node_evaluate(0, r1, r2)
+    for b in (1, 2, 3, 31, 153, 913):
+        part = e.node_evaluate(0, r1[:b], r2[:b])
+        for x, y in zip(part, whole):
+            assert np.array_equal(x, y[:b]), b
+    port = O.PortOracle(O.make_config(**kw))
+    for b in (0, nb - 1):
+        perr, pdet, pd1, pd2 = port.node_eval(0, r1[b], r2[b], 0, False)
+        assert whole[0][b] == perr
+        assert abs(whole[1][b] - pdet) <= 1e-8 * abs(pdet)
+        assert np.all(np.abs(whole[2][b] - pd1) <= 1e-8 * pd1)
+        assert np.all(np.abs(whole[3][b] - pd2) <= 1e-8 * pd2)
+
+
+@pytest.mark.parametrize("nbatch", [1, 3, 40, 400])
+@pytest.mark.parametrize("case", ["heg10", "heg10_uncached", "dot3_odd"])
+def test_action_difference_batches(pimc, case, nbatch):
+    # The section's slices over many CTAs and few, every level.
+    kw, _ = DISPLACE[case]
+    tabs, ew = pimc.coulomb_tables(kw)
+    cfg = O.make_config(**kw)
+    port = O.PortOracle(cfg, tabs, ew)
+    e = pimc.Engine(kw, 1, tabs, ew)
+    rng = np.random.default_rng(4)
+    nsec = (1 << kw["nlevel"]) + 1
+    sec = rng.normal(size=(nbatch, nsec, cfg.npart, 3)) * 2.0
+    ip = rng.integers(0, cfg.npart, nbatch)
+    mov = sec[np.arange(nbatch), :, ip].copy()
+    mov[:, 1:-1] += 0.3 * rng.normal(size=mov[:, 1:-1].shape)
+    for level in range(kw["nlevel"] + 1):
+        ds = e.action_difference(level, sec, mov, ip)
+        for b in list(range(min(nbatch, 3))) + [nbatch - 1]:
+            ref = port.action_diff(level, sec[b], mov[b], int(ip[b]))
+            assert abs(ds[b] - ref) <= 1e-12 * max(abs(ref), 1.0), (level, b)
