@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -184,6 +185,10 @@ struct pimc_engine {
   DevBuf<double> d_dscratch;  // displacement moves: node dets and distances per CTA
   DevBuf<double> d_energy;   // [steps][nrep]
   DevBuf<double> d_forces;   // virial estimator: forces of a pass's replicas (bounded)
+  // host data of the calls that take or return arrays (EntryIo)
+  std::mutex io_mutex;
+  DevBuf<char> io_dev;
+  char* io_host = nullptr;
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   int graph_attempts = -1, graph_steps = -1;
@@ -203,6 +208,8 @@ struct pimc_engine {
     d_dscratch.free();
     d_energy.free();
     d_forces.free();
+    io_dev.free();
+    if (io_host) cudaFreeHost(io_host);
     d_sys.free();
     d_state.free();
     d_paths.free();
@@ -227,6 +234,103 @@ struct pimc_engine {
 };
 
 namespace {
+
+// The arrays of one call between the caller's memory and the device.  A call names
+// its inputs, outputs and scratch, open() places them, dev() gives their device
+// addresses, and close() waits for the stream and delivers the outputs.  Small calls
+// (kIoMapped of inputs and outputs) run on a pinned host block of the engine that the
+// kernels read and write themselves: no copies are queued.  Larger ones copy from
+// and to the caller's memory through a device block, kept up to kIoKeep.  (Allocated
+// from the stream's pool in each call, which gives its memory back at every
+// synchronisation: a node evaluation of one pair took 275 us, now 61.)  The engine's
+// blocks serve one call at a time: a call holds the engine's mutex, and leaves with
+// the stream idle.
+constexpr size_t kIoMapped = 128 << 10, kIoKeep = 64 << 20;
+
+class EntryIo {
+ public:
+  explicit EntryIo(pimc_engine* e) : eng_(e), lock_(e->io_mutex) {}
+  ~EntryIo() {
+    if (own_) cudaFreeAsync(own_, eng_->stream);
+  }
+  int in(const void* p, size_t bytes) { return add(const_cast<void*>(p), bytes, kIn); }
+  // (a table that every CTA reads: to device memory in either case)
+  int in_device(const void* p, size_t bytes) { return add(const_cast<void*>(p), bytes, kInDevice); }
+  int out(void* p, size_t bytes, bool zeroed = false) {
+    return add(p, bytes, zeroed ? kOutZero : kOut);
+  }
+  int scratch(size_t bytes) { return add(nullptr, bytes, kScratch); }
+  int open() {
+    size_t io = 0, tmp = 0;
+    for (const Part& p : parts_) (p.kind >= kInDevice ? tmp : io) += p.bytes;
+    mapped_ = io <= kIoMapped;
+    if (mapped_ && !eng_->io_host &&
+        cudaHostAlloc((void**)&eng_->io_host, kIoMapped, cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      eng_->io_host = nullptr;
+      mapped_ = false;
+    }
+    const size_t need = tmp + (mapped_ ? 0 : io);
+    char* dev = nullptr;
+    if (need > kIoKeep) {
+      CU(cudaMallocAsync(&own_, need, eng_->stream));
+      dev = own_;
+    } else if (need) {
+      if (eng_->io_dev.n < need) {
+        CU(cudaStreamSynchronize(eng_->stream));
+        if (eng_->io_dev.alloc(std::min(kIoKeep, std::max<size_t>(2 * eng_->io_dev.n, need))))
+          return fail(PIMC_ERR_CUDA, "cudaMalloc call buffers");
+      }
+      dev = eng_->io_dev.p;
+    }
+    size_t hoff = 0, doff = 0;
+    for (Part& p : parts_) {
+      const bool on_host = mapped_ && p.kind < kInDevice;
+      size_t& off = on_host ? hoff : doff;
+      p.dev = (on_host ? eng_->io_host : dev) + off;
+      off += p.bytes;
+      if (mapped_ && p.kind == kIn) memcpy(p.dev, p.host, p.size);
+      if (mapped_ && p.kind == kOutZero) memset(p.dev, 0, p.size);
+      if (((!mapped_ && p.kind == kIn) || p.kind == kInDevice) && p.size)
+        CU(cudaMemcpyAsync(p.dev, p.host, p.size, cudaMemcpyHostToDevice, eng_->stream));
+      if (!mapped_ && p.kind == kOutZero) CU(cudaMemsetAsync(p.dev, 0, p.size, eng_->stream));
+    }
+    return PIMC_OK;
+  }
+  template <class T>
+  T* dev(int k) const {
+    return (T*)parts_[k].dev;
+  }
+  int close() {
+    if (!mapped_)
+      for (const Part& p : parts_)
+        if (p.kind == kOut || p.kind == kOutZero)
+          CU(cudaMemcpyAsync(p.host, p.dev, p.size, cudaMemcpyDeviceToHost, eng_->stream));
+    CU(cudaStreamSynchronize(eng_->stream));
+    if (mapped_)
+      for (const Part& p : parts_)
+        if (p.kind == kOut || p.kind == kOutZero) memcpy(p.host, p.dev, p.size);
+    return PIMC_OK;
+  }
+
+ private:
+  enum Kind { kIn, kOut, kOutZero, kInDevice, kScratch };
+  struct Part {
+    void* host;
+    size_t size, bytes;  // bytes: rounded up, so that the next part stays aligned
+    Kind kind;
+    char* dev;
+  };
+  int add(void* p, size_t size, Kind kind) {
+    parts_.push_back({p, size, (size + 255) & ~(size_t)255, kind, nullptr});
+    return (int)parts_.size() - 1;
+  }
+  pimc_engine* eng_;
+  std::lock_guard<std::mutex> lock_;
+  std::vector<Part> parts_;
+  char* own_ = nullptr;
+  bool mapped_ = false;
+};
 
 // PeriodicGaussian constructor constants (src/util/PeriodicGaussian.cc:7-18).
 void pg_params(double alpha, double length, double& nome, double& pref, double& k, int& nmax) {
@@ -580,6 +684,7 @@ void set_smem_caps() {
   cudaFuncSetAttribute(thermo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   cudaFuncSetAttribute(action_diff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        kSmemLimit);
+  cudaFuncSetAttribute(node_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
 }
 
 // Shared memory of the estimator kernels: one staged slice (in the section
@@ -1326,23 +1431,20 @@ void fill_run_params(pimc_engine* e, RunParams& P, int nattempt, pimc_move_recor
 int pimc_run_sections(pimc_engine* e, int nattempt, pimc_move_record* records) {
   if (!e || nattempt < 0) return fail(PIMC_ERR_INVALID, "bad argument");
   if (nattempt == 0) return PIMC_OK;
-  pimc_move_record* d_rec = nullptr;
-  if (records) {
-    CU(cudaMallocAsync(&d_rec, sizeof(pimc_move_record) * (size_t)e->nrep * nattempt, e->stream));
-    CU(cudaMemsetAsync(d_rec, 0, sizeof(pimc_move_record) * (size_t)e->nrep * nattempt, e->stream));
-  }
-  RunParams P;
-  fill_run_params(e, P, nattempt, d_rec);
-  CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
-  CU(section_launch(e->minb, e->grid, e->block, e->lay.total * 8, e->stream, P, e->nodes));
-  e->launches++;
-  if (records) {
-    CU(cudaMemcpyAsync(records, d_rec, sizeof(pimc_move_record) * (size_t)e->nrep * nattempt,
-                       cudaMemcpyDeviceToHost, e->stream));
-    CU(cudaFreeAsync(d_rec, e->stream));
-    CU(cudaStreamSynchronize(e->stream));
-  }
-  return PIMC_OK;
+  const auto launch = [&](pimc_move_record* d_rec) -> int {
+    RunParams P;
+    fill_run_params(e, P, nattempt, d_rec);
+    CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
+    CU(section_launch(e->minb, e->grid, e->block, e->lay.total * 8, e->stream, P, e->nodes));
+    e->launches++;
+    return PIMC_OK;
+  };
+  if (!records) return launch(nullptr);
+  EntryIo io(e);
+  const int rec = io.out(records, sizeof(pimc_move_record) * (size_t)e->nrep * nattempt, true);
+  if (int rc = io.open()) return rc;
+  if (int rc = launch(io.dev<pimc_move_record>(rec))) return rc;
+  return io.close();
 }
 
 int pimc_replica_status(pimc_engine* e, int64_t* accepted, int64_t* attempted, uint32_t* status) {
@@ -1382,10 +1484,10 @@ int pimc_thermo_energy(pimc_engine* e, double* host_energy) {
 }
 
 namespace {
-// Runs one estimator over every replica, reduces the partials per replica (÷ M) and
-// copies the energies to the host.
+// Runs one estimator over every replica and reduces the partials per replica (÷ M)
+// into d_out.
 enum { kEstVirial = 0, kEstCoulomb = 1 };
-int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L, double* host) {
+int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L, double* d_out) {
   const int nchunk = which == kEstVirial ? 2 * kThermoChunks : kThermoChunks;
   if (e->d_partial.n < (size_t)e->nrep * nchunk) {
     CU(cudaStreamSynchronize(e->stream));
@@ -1396,8 +1498,6 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
     if (e->d_partial.alloc((size_t)e->nrep * nchunk))
       return fail(PIMC_ERR_CUDA, "cudaMalloc energy partials");
   }
-  double* d_out = nullptr;
-  CU(cudaMallocAsync(&d_out, e->nrep * sizeof(double), e->stream));
   P.sys = e->d_sys.p;
   P.paths = e->d_paths.p;
   P.partial = e->d_partial.p;
@@ -1443,10 +1543,15 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
       e->d_sys.p, nullptr, e->d_partial.p, nchunk, e->nrep, d_out, false);
   e->launches++;
   CU(cudaGetLastError());
-  CU(cudaMemcpyAsync(host, d_out, e->nrep * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaFreeAsync(d_out, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
   return PIMC_OK;
+}
+// The same with nothing but the energies to return.
+int run_estimator_host(pimc_engine* e, int which, const EstimatorParams& P, double* host) {
+  EntryIo io(e);
+  const int out = io.out(host, e->nrep * sizeof(double));
+  if (int rc = io.open()) return rc;
+  if (int rc = run_estimator(e, which, P, e->est_lay, io.dev<double>(out))) return rc;
+  return io.close();
 }
 }  // namespace
 
@@ -1518,13 +1623,6 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
     CU(cudaStreamSynchronize(e->stream));
     if (e->d_dscratch.alloc(need)) return fail(PIMC_ERR_CUDA, "cudaMalloc displacement scratch");
   }
-  pimc_displace_record* d_rec = nullptr;
-  if (records) {
-    CU(cudaMallocAsync(&d_rec, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt,
-                       e->stream));
-    CU(cudaMemsetAsync(d_rec, 0, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt,
-                       e->stream));
-  }
   DisplaceParams P;
   P.sys = e->d_sys.p;
   P.state = e->d_state.p;
@@ -1534,7 +1632,6 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
   P.scratch = e->d_dscratch.p;
   P.scratch_stride = sstride;
   P.nodescr_g = e->d_nodescr.p;
-  P.rec = d_rec;
   P.order = e->d_order.p;
   P.next = e->d_next.p;
   P.nattempt = nattempt;
@@ -1544,23 +1641,26 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
   P.nmoving = nmoving;
   P.species = species;
   P.lay = L;
-  CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
-  CU(cudaLaunchKernelEx(&cfg, displace_kernel, P));
-  e->launches++;
-  if (records) {
-    CU(cudaMemcpyAsync(records, d_rec, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt,
-                       cudaMemcpyDeviceToHost, e->stream));
-    CU(cudaFreeAsync(d_rec, e->stream));
-    CU(cudaStreamSynchronize(e->stream));
-  }
-  return PIMC_OK;
+  const auto launch = [&](pimc_displace_record* d_rec) -> int {
+    P.rec = d_rec;
+    CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
+    CU(cudaLaunchKernelEx(&cfg, displace_kernel, P));
+    e->launches++;
+    return PIMC_OK;
+  };
+  if (!records) return launch(nullptr);
+  EntryIo io(e);
+  const int rec = io.out(records, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt, true);
+  if (int rc = io.open()) return rc;
+  if (int rc = launch(io.dev<pimc_displace_record>(rec))) return rc;
+  return io.close();
 }
 
 int pimc_virial_energy(pimc_engine* e, int nwindow, double* host_energy) {
   if (!e || e->server || nwindow < 1 || !host_energy) return fail(PIMC_ERR_INVALID, "bad argument");
   EstimatorParams P{};
   P.nwindow = nwindow;
-  return run_estimator(e, kEstVirial, P, e->est_lay, host_energy);
+  return run_estimator_host(e, kEstVirial, P, host_energy);
 }
 
 int pimc_coulomb_energy(pimc_engine* e, double epsilon, double* host_energy) {
@@ -1568,7 +1668,7 @@ int pimc_coulomb_energy(pimc_engine* e, double epsilon, double* host_energy) {
     return fail(PIMC_ERR_INVALID, "bad argument");
   EstimatorParams P{};
   P.epsilon = epsilon;
-  return run_estimator(e, kEstCoulomb, P, e->est_lay, host_energy);
+  return run_estimator_host(e, kEstCoulomb, P, host_energy);
 }
 
 int pimc_ewald_coulomb_energy(pimc_engine* e, double epsilon, double rcut,
@@ -1577,28 +1677,25 @@ int pimc_ewald_coulomb_energy(pimc_engine* e, double epsilon, double rcut,
   if (!e || e->server || !(epsilon > 0) || !(rcut > 0) || !est || !vgrid || !host_energy ||
       est->totk < 0 || (est->totk > 0 && (!est->kvec || !est->vk)))
     return fail(PIMC_ERR_INVALID, "bad argument");
-  DevBuf<int> kv;
-  DevBuf<double> vk, vg;
-  if (kv.alloc(3 * std::max(est->totk, 1)) || vk.alloc(std::max(est->totk, 1)) || vg.alloc(1001))
-    return fail(PIMC_ERR_CUDA, "cudaMalloc estimator tables");
-  if (est->totk > 0) {
-    CU(cudaMemcpy(kv.p, est->kvec, 3 * est->totk * sizeof(int), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(vk.p, est->vk, est->totk * sizeof(double), cudaMemcpyHostToDevice));
-  }
-  CU(cudaMemcpy(vg.p, vgrid, 1001 * sizeof(double), cudaMemcpyHostToDevice));
+  EntryIo io(e);
+  const int kv = io.in_device(est->kvec, 3 * est->totk * sizeof(int));
+  const int vk = io.in_device(est->vk, est->totk * sizeof(double));
+  const int vg = io.in_device(vgrid, 1001 * sizeof(double));
+  const int out = io.out(host_energy, e->nrep * sizeof(double));
+  if (int rc = io.open()) return rc;
   EstimatorParams P{};
   P.epsilon = epsilon;
-  P.vgrid = vg.p;
+  P.vgrid = io.dev<double>(vg);
   P.rcut = rcut;
   P.totk = est->totk;
-  P.kvec = kv.p;
-  P.vk = vk.p;
+  P.kvec = io.dev<int>(kv);
+  P.vk = io.dev<double>(vk);
   P.one_over_2v = est->one_over_2v;
   P.self_energy = est->self_energy;
   for (int a = 0; a < 3; ++a) P.ikmax[a] = est->ikmax[a];
   const Layout L = estimator_layout(e->hsys, est->ikmax);
-  const int rc = run_estimator(e, kEstCoulomb, P, L, host_energy);
-  return rc;
+  if (int rc = run_estimator(e, kEstCoulomb, P, L, io.dev<double>(out))) return rc;
+  return io.close();
 }
 
 int pimc_run_steps(pimc_engine* e, int nattempt, int nsteps, double* host_energy) {
@@ -1705,32 +1802,28 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   const Layout alay = make_layout(e->hsys, kBlock / 32, lok, aopt);
   if (!lok) return fail(PIMC_ERR_CAPACITY, "working set does not fit in shared memory");
   const size_t nsecd = (size_t)nbatch * s.nsec * s.npart * 3, nmovd = (size_t)nbatch * s.nsec * 3;
-  double *d_sec = nullptr, *d_mov = nullptr, *d_ds = nullptr, *d_scr = nullptr;
-  int* d_ip = nullptr;
-  if (alay.act_global)
-    CU(cudaMallocAsync(&d_scr, (size_t)std::min(nbatch, 65535) * alay.gcta * 8, e->stream));
-  CU(cudaMallocAsync(&d_sec, nsecd * 8, e->stream));
-  CU(cudaMallocAsync(&d_mov, nmovd * 8, e->stream));
   // with Ewald sums the section's slices go to CTAs of their own, as many per entry as
   // a batch of this size leaves room for (two CTAs an SM), added up here in order
   int parts = 1;
   if (s.ewald && s.coulomb && level == 0)
     parts = 1 + std::max(1, std::min(s.nsec - 2, 2 * e->num_sms / nbatch));
-  CU(cudaMallocAsync(&d_ds, (size_t)nbatch * parts * 8, e->stream));
-  CU(cudaMallocAsync(&d_ip, nbatch * 4, e->stream));
-  CU(cudaMemcpyAsync(d_sec, section, nsecd * 8, cudaMemcpyHostToDevice, e->stream));
-  CU(cudaMemcpyAsync(d_mov, moving, nmovd * 8, cudaMemcpyHostToDevice, e->stream));
-  CU(cudaMemcpyAsync(d_ip, ipart, nbatch * 4, cudaMemcpyHostToDevice, e->stream));
+  std::vector<double> share((size_t)nbatch * parts);
+  EntryIo io(e);
+  const int sec = io.in(section, nsecd * 8), mov = io.in(moving, nmovd * 8);
+  const int ip = io.in(ipart, nbatch * sizeof(int));
+  const int out = io.out(share.data(), share.size() * 8);
+  const int scr = io.scratch(
+      alay.act_global ? (size_t)std::min(nbatch, 65535) * alay.gcta * 8 : 0);
+  if (int rc = io.open()) return rc;
   ActionDiffParams P;
   P.sys = e->d_sys.p;
-  P.section = d_sec;
-  P.moving = d_mov;
-  P.ipart = d_ip;
-  P.ds = d_ds;
+  P.section = io.dev<double>(sec);
+  P.moving = io.dev<double>(mov);
+  P.ipart = io.dev<int>(ip);
+  P.ds = io.dev<double>(out);
   P.level = level;
   P.lay = alay;
-  P.scratch = d_scr;
-  std::vector<double> share((size_t)nbatch * parts);
+  P.scratch = alay.act_global ? io.dev<double>(scr) : nullptr;
   for (int b0 = 0; b0 < nbatch; b0 += 65535) {
     const int nb = std::min(65535, nbatch - b0);
     ActionDiffParams Q = P;
@@ -1742,13 +1835,7 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
     e->launches++;
   }
   CU(cudaGetLastError());
-  CU(cudaMemcpyAsync(share.data(), d_ds, share.size() * 8, cudaMemcpyDeviceToHost, e->stream));
-  if (d_scr) CU(cudaFreeAsync(d_scr, e->stream));
-  CU(cudaFreeAsync(d_sec, e->stream));
-  CU(cudaFreeAsync(d_mov, e->stream));
-  CU(cudaFreeAsync(d_ds, e->stream));
-  CU(cudaFreeAsync(d_ip, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
+  if (int rc = io.close()) return rc;
   for (int b = 0; b < nbatch; ++b) {
     double v = share[(size_t)b * parts];
     for (int k = 1; k < parts; ++k) v += share[(size_t)b * parts + k];
@@ -1766,48 +1853,32 @@ int pimc_node_evaluate(pimc_engine* e, int ispec, int nbatch, const double* r1, 
     return fail(PIMC_ERR_INVALID, "species has no node model");
   const int np = s.npart;
   const size_t nr = (size_t)nbatch * np * 3;
-  double *d_r1, *d_r2, *d_det, *d_d1, *d_d2;
-  int* d_err;
-  CU(cudaMallocAsync(&d_r1, nr * 8, e->stream));
-  CU(cudaMallocAsync(&d_r2, nr * 8, e->stream));
-  CU(cudaMallocAsync(&d_det, nbatch * 8, e->stream));
-  CU(cudaMallocAsync(&d_d1, (size_t)nbatch * np * 8, e->stream));
-  CU(cudaMallocAsync(&d_d2, (size_t)nbatch * np * 8, e->stream));
-  CU(cudaMallocAsync(&d_err, nbatch * 4, e->stream));
-  CU(cudaMemcpyAsync(d_r1, r1, nr * 8, cudaMemcpyHostToDevice, e->stream));
-  CU(cudaMemcpyAsync(d_r2, r2, nr * 8, cudaMemcpyHostToDevice, e->stream));
+  const NodeEvalShape sh = node_eval_shape(s, ispec, nbatch, e->num_sms);
+  EntryIo io(e);
+  const int a1 = io.in(r1, nr * 8), a2 = io.in(r2, nr * 8);
+  const int odet = io.out(det, nbatch * 8), oerr = io.out(err, nbatch * sizeof(int));
+  const int od1 = io.out(d1, (size_t)nbatch * np * 8), od2 = io.out(d2, (size_t)nbatch * np * 8);
+  const int cold = io.scratch((size_t)sh.grid * sh.warps * sh.cold * 8);
+  if (int rc = io.open()) return rc;
   NodeEvalParams P;
   P.sys = e->d_sys.p;
   P.state = e->d_state.p;
-  P.r1 = d_r1;
-  P.r2 = d_r2;
-  P.det = d_det;
-  P.d1 = d_d1;
-  P.d2 = d_d2;
-  P.err = d_err;
+  P.r1 = io.dev<double>(a1);
+  P.r2 = io.dev<double>(a2);
+  P.det = io.dev<double>(odet);
+  P.d1 = io.dev<double>(od1);
+  P.d2 = io.dev<double>(od2);
+  P.err = io.dev<int>(oerr);
   P.ispec = ispec;
   P.nbatch = nbatch;
-  const NodeEvalShape sh = node_eval_shape(s, ispec, nbatch, e->num_sms);
   P.stage_stride = sh.stage;
   P.scratch_stride = sh.scratch;
   P.cold_stride = sh.cold;
-  double* d_cold = nullptr;
-  if (sh.cold)
-    CU(cudaMallocAsync(&d_cold, (size_t)sh.grid * sh.warps * sh.cold * 8, e->stream));
-  P.cold = d_cold;
-  cudaFuncSetAttribute(node_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  P.cold = sh.cold ? io.dev<double>(cold) : nullptr;
   node_eval_kernel<<<sh.grid, 32 * sh.warps, sh.smem, e->stream>>>(P);
   e->launches++;
   CU(cudaGetLastError());
-  if (d_cold) CU(cudaFreeAsync(d_cold, e->stream));
-  CU(cudaMemcpyAsync(det, d_det, nbatch * 8, cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaMemcpyAsync(d1, d_d1, (size_t)nbatch * np * 8, cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaMemcpyAsync(d2, d_d2, (size_t)nbatch * np * 8, cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaMemcpyAsync(err, d_err, nbatch * 4, cudaMemcpyDeviceToHost, e->stream));
-  for (void* p : {(void*)d_r1, (void*)d_r2, (void*)d_det, (void*)d_d1, (void*)d_d2, (void*)d_err})
-    CU(cudaFreeAsync(p, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
-  return PIMC_OK;
+  return io.close();
 }
 
 int pimc_stream_sample(uint64_t seed, uint32_t replica, uint32_t attempt, int n,
@@ -2398,29 +2469,24 @@ int server_energy(pimc_engine* e, const std::vector<int>& slots, double* out) {
   const int nchunk = kThermoChunks;
   int grid = 1;
   for (int r : slots) grid = std::max(grid, e->hsys[r].thermo_chunks);
-  double* d_part = nullptr;
-  int* d_idx = nullptr;
-  CU(cudaMallocAsync(&d_part, sizeof(double) * (size_t)n * nchunk, e->stream));
-  CU(cudaMallocAsync(&d_idx, sizeof(int) * (size_t)n, e->stream));
-  CU(cudaMemcpyAsync(d_idx, slots.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice,
-                     e->stream));
+  std::vector<double> part((size_t)n * nchunk);
+  EntryIo io(e);
+  const int idx = io.in(slots.data(), sizeof(int) * (size_t)n);
+  const int share = io.out(part.data(), part.size() * 8);
+  if (int rc = io.open()) return rc;
   ThermoParams P;
   P.sys = e->d_sys.p;
-  P.index = d_idx;
+  P.index = io.dev<int>(idx);
   P.paths = e->d_pool.p;
   P.ekcache = nullptr;  // servers take no Ewald systems
-  P.partial = d_part;
+  P.partial = io.dev<double>(share);
   P.nchunk = nchunk;
   P.nrep = n;
   P.lay = e->est_lay;
   thermo_kernel<<<dim3(grid, n), kBlock, e->est_lay.total * 8, e->stream>>>(P);
   e->launches++;
   CU(cudaGetLastError());
-  std::vector<double> part((size_t)n * nchunk);
-  CU(cudaMemcpyAsync(part.data(), d_part, part.size() * 8, cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaFreeAsync(d_part, e->stream));
-  CU(cudaFreeAsync(d_idx, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
+  if (int rc = io.close()) return rc;
   for (int k = 0; k < n; ++k) {
     double s = 0;
     for (int c = 0; c < e->hsys[slots[k]].thermo_chunks; ++c) s += part[(size_t)k * nchunk + c];

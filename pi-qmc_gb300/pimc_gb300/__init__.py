@@ -275,17 +275,17 @@ def ewald_struct(ew):
     return e, [kv, vk]
 
 
+# pimc_move_record and pimc_displace_record as structured arrays
+MOVE_RECORD = np.dtype([("ifirst1", "i4"), ("ifirst2", "i4"), ("ipart", "i4"),
+                        ("reject_level", "i4"), ("ds", "f8", MAXL + 3),
+                        ("ds_node", "f8", MAXL + 3), ("lnt", "f8", MAXL + 3)], align=True)
+DISPLACE_RECORD = np.dtype([("ipart", "i4", 4), ("disp", "f8", (4, 3)), ("ds", "f8"),
+                            ("ds_node", "f8"), ("accepted", "i4")], align=True)
+
+
 def records_to_numpy(recs, n):
-    out = {
-        "ifirst1": np.array([r.ifirst1 for r in recs[:n]], np.int32),
-        "ifirst2": np.array([r.ifirst2 for r in recs[:n]], np.int32),
-        "ipart": np.array([r.ipart for r in recs[:n]], np.int32),
-        "reject_level": np.array([r.reject_level for r in recs[:n]], np.int32),
-        "ds": np.array([list(r.ds) for r in recs[:n]]),
-        "ds_node": np.array([list(r.ds_node) for r in recs[:n]]),
-        "lnt": np.array([list(r.lnt) for r in recs[:n]]),
-    }
-    return out
+    a = np.frombuffer(recs, MOVE_RECORD, n)
+    return {k: np.ascontiguousarray(a[k]) for k in MOVE_RECORD.names}
 
 
 def fp64_peak_tflops():
@@ -453,15 +453,9 @@ class Engine(_Checkpoint):
             n = self.nreplica * nattempt
             recs = (DisplaceRecord * max(n, 1))()
             _check(lib().pimc_run_displace(self.h, nattempt, _dp(b), nmoving, species, recs))
-            out = {
-                "ipart": np.array([[recs[i].ipart[k] for k in range(nmoving)] for i in range(n)],
-                                  np.int32),
-                "disp": np.array([[list(recs[i].disp[k]) for k in range(nmoving)]
-                                  for i in range(n)]),
-                "ds": np.array([recs[i].ds for i in range(n)]),
-                "ds_node": np.array([recs[i].ds_node for i in range(n)]),
-                "accepted": np.array([recs[i].accepted for i in range(n)], np.int32),
-            }
+            a = np.frombuffer(recs, DISPLACE_RECORD, n)
+            out = {k: np.ascontiguousarray(a[k][:, :nmoving] if k in ("ipart", "disp") else a[k])
+                   for k in DISPLACE_RECORD.names}
             return {k: v.reshape((self.nreplica, nattempt) + v.shape[1:]) for k, v in out.items()}
         _check(lib().pimc_run_displace(self.h, nattempt, _dp(b), nmoving, species, None))
         return None
