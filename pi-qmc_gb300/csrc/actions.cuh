@@ -123,33 +123,29 @@ __device__ __forceinline__ void link_terms(const DevSys& s, const Smem& m, int i
       acc.add(__fmaf_rn(pa, d2, __fmul_rn(pb, d4)) * (float)(s.tau * (1 << level)));
     }
   } else {
-    const double inv2Sigma2 = s.spr_inv2s2[level][sp];
-    double dx = n1x - n0x, dy = n1y - n0y, dz = n1z - n0z;
-    double ex = o1x - o0x, ey = o1y - o0y, ez = o1z - o0z;
-    const double om = s.sho_omega[sp];
-    double free_n = 0.0, free_o = 0.0;
-    if (om > 0) {
-      free_n = dx * dx + dy * dy + dz * dz;
-      free_o = ex * ex + ey * ey + ez * ez;
-    }
+    // (the plain differences' squares serve the harmonic term and, but for an image,
+    // the spring)
+    const double dx = n1x - n0x, dy = n1y - n0y, dz = n1z - n0z;
+    const double ex = o1x - o0x, ey = o1y - o0y, ez = o1z - o0z;
+    const double dn = dx * dx + dy * dy + dz * dz, dold = ex * ex + ey * ey + ez * ez;
     if (s.spring) {
-      pbc(s, dx, dy, dz);
-      pbc(s, ex, ey, ez);
-      const double nw = dx * dx * inv2Sigma2 + dy * dy * inv2Sigma2 + dz * dz * inv2Sigma2;
-      const double od = ex * ex * inv2Sigma2 + ey * ey * inv2Sigma2 + ez * ez * inv2Sigma2;
-      acc.add(nw - od);
+      double fx = dx, fy = dy, fz = dz, gx = ex, gy = ey, gz = ez, d2 = dn - dold;
+      if (pbc(s, fx, fy, fz) | pbc(s, gx, gy, gz))
+        d2 = (fx * fx + fy * fy + fz * fz) - (gx * gx + gy * gy + gz * gz);
+      acc.add(s.spr_inv2s2[level][sp] * d2);
     }
+    const double om = s.sho_omega[sp];
     if (om > 0) {
       const double coshwt = s.sho_cosh[level][sp], div1 = s.sho_div1[level][sp];
       const double div2 = s.sho_div2[level], msho = s.mass[sp];
       double r0r0 = n0x * n0x + n0y * n0y + n0z * n0z;
       double r1r1 = n1x * n1x + n1y * n1y + n1z * n1z;
       double r0r1 = n0x * n1x + n0y * n1y + n0z * n1z;
-      const double nw = msho * om * ((r1r1 + r0r0) * coshwt - 2.0 * r0r1) * div1 - msho * free_n * div2;
+      const double nw = msho * om * ((r1r1 + r0r0) * coshwt - 2.0 * r0r1) * div1 - msho * dn * div2;
       r0r0 = o0x * o0x + o0y * o0y + o0z * o0z;
       r1r1 = o1x * o1x + o1y * o1y + o1z * o1z;
       r0r1 = o0x * o1x + o0y * o1y + o0z * o1z;
-      const double od = msho * om * ((r1r1 + r0r0) * coshwt - 2.0 * r0r1) * div1 - msho * free_o * div2;
+      const double od = msho * om * ((r1r1 + r0r0) * coshwt - 2.0 * r0r1) * div1 - msho * dold * div2;
       acc.add(nw - od);
     }
     if (prim) {
@@ -174,7 +170,8 @@ __device__ __forceinline__ double pair_term(const DevTable& t, const Sep& a, con
   const double qq = 0.5 * (a.r + b.r);
   if (!offdiag) return tab_u00(t, qq) * stride;
   const double sx = a.x - b.x, sy = a.y - b.y, sz = a.z - b.z;
-  return tab_uk0(t, qq, dot3(sx, sy, sz, sx, sy, sz) / (qq * qq)) * stride;
+  const double qi = __drcp_rn(qq);
+  return tab_uk0(t, qq, dot3(sx, sy, sz, sx, sy, sz) * (qi * qi)) * stride;
 }
 __device__ __forceinline__ float pair_term(const DevTable& t, const SepF& a, const SepF& b,
                                            bool offdiag, int stride) {

@@ -162,6 +162,7 @@ struct pimc_engine {
   DevBuf<int> d_next;
   DevBuf<double> d_ugrid;
   DevBuf<float> d_ugrid32;
+  DevBuf<double> d_logtab;  // servers: grid_log's table (else the first part of d_ugrid)
   DevBuf<int> d_kvec;
   DevBuf<double> d_vk;
   // serving: slots over one device pool
@@ -228,6 +229,7 @@ struct pimc_engine {
     d_prefill.free();
     d_ugrid.free();
     d_ugrid32.free();
+    d_logtab.free();
     d_kvec.free();
     d_vk.free();
   }
@@ -384,6 +386,31 @@ int validate(const pimc_system& s) {
                       "cell too small: periodic-Gaussian spring/mover images are not supported");
       }
   return 0;
+}
+
+// The table of grid_log: c_j, then e ln 2 - log c_j.
+std::vector<double> log_table() {
+  std::vector<double> t(kLogReciprocals + kLogEntries);
+  for (int j = 0; j < kLogReciprocals; ++j) {
+    // 1 / (middle of the interval) to 13 bits: m c_j - 1 then takes one rounding
+    const double mid = 1.0 + (j + 0.5) / kLogReciprocals;
+    t[j] = std::nearbyint(8192.0 / mid) / 8192.0;
+    const long double lc = -std::log((long double)t[j]);
+    for (int e = 0; e < kLogOctaves; ++e)
+      t[kLogReciprocals + e * kLogReciprocals + j] =
+          (double)(e * 0.693147180559945309417232121458L + lc);
+  }
+  return t;
+}
+
+// The FP64 table a kernel reads: every coefficient beside its difference to the next
+// grid point's.
+void interleave_table(const pimc_pair_table& t, double* out) {
+  const size_t row = 2 * (size_t)(t.norder + 1), n = row * t.ngpts;
+  for (size_t k = 0; k < n; ++k) {
+    out[2 * k] = t.ugrid[k];
+    out[2 * k + 1] = k + row < n ? t.ugrid[k + row] - t.ugrid[k] : 0.0;
+  }
 }
 
 void fill_sys(const pimc_system& s, DevSys& d) {
@@ -817,7 +844,8 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
   e->hdesc.resize(nrep);
   e->path_off.resize(nrep + 1);
   // pair tables: pool the unique table objects in order of appearance
-  std::vector<double> pool;
+  std::vector<float> pool;  // FP32 tables; their FP64 forms take twice the entries
+  std::vector<const pimc_pair_table*> pool_tables;
   std::vector<int> kv;
   std::vector<double> vk;
   long long off = 0;
@@ -869,6 +897,7 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
           po = hit->second;
         } else {
           pool.insert(pool.end(), t.ugrid, t.ugrid + (size_t)t.ngpts * 2 * dt.ndata);
+          pool_tables.push_back(&t);
           pooled[t.ugrid] = po;
         }
         pend.push_back({r, d.ntab, po});
@@ -917,18 +946,27 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
   }
   e->est_lay = estimator_layout(e->hsys, nullptr);
   // device buffers
-  if (e->d_ugrid.alloc(pool.size()) || e->d_ugrid32.alloc(pool.size())) {
+  const std::vector<double> logs = pool.empty() ? std::vector<double>() : log_table();
+  if (e->d_ugrid.alloc(logs.size() + 2 * pool.size()) || e->d_ugrid32.alloc(pool.size())) {
     delete e;
     return fail(PIMC_ERR_CUDA, "cudaMalloc pair tables");
   }
   if (!pool.empty()) {
-    std::vector<float> p32(pool.begin(), pool.end());
-    cudaMemcpy(e->d_ugrid.p, pool.data(), pool.size() * 8, cudaMemcpyHostToDevice);
-    cudaMemcpy(e->d_ugrid32.p, p32.data(), p32.size() * 4, cudaMemcpyHostToDevice);
+    std::vector<double> p64(logs);
+    p64.resize(logs.size() + 2 * pool.size());
+    size_t at = logs.size();
+    for (const pimc_pair_table* t : pool_tables) {
+      interleave_table(*t, p64.data() + at);
+      at += 4 * (size_t)t->ngpts * (t->norder + 1);
+    }
+    cudaMemcpy(e->d_ugrid.p, p64.data(), p64.size() * 8, cudaMemcpyHostToDevice);
+    cudaMemcpy(e->d_ugrid32.p, pool.data(), pool.size() * 4, cudaMemcpyHostToDevice);
   }
   for (const Pending& p : pend) {
-    e->hsys[p.rep].tab[p.slot].ugrid = e->d_ugrid.p + p.pool_off;
-    e->hsys[p.rep].tab[p.slot].ugrid32 = e->d_ugrid32.p + p.pool_off;
+    DevTable& dt = e->hsys[p.rep].tab[p.slot];
+    dt.logtab = e->d_ugrid.p;
+    dt.ugrid = e->d_ugrid.p + logs.size() + 2 * p.pool_off;
+    dt.ugrid32 = e->d_ugrid32.p + p.pool_off;
   }
   if (ewald && e->hsys[0].ewald) {
     if (e->d_kvec.alloc(3 * ewald->totk) || e->d_vk.alloc(ewald->totk)) {
@@ -2282,12 +2320,21 @@ int pimc_server_create(const pimc_server_config* cfg, uint64_t seed, int precisi
     e->xstage_cta = (long long)mx.nsec * (mx.ns_max * mx.ns_max + 2);
   const long long words = (long long)(cfg->hbm_bytes / sizeof(double));
   if (e->d_pool.alloc(words) || e->d_sys.alloc(cfg->slots) || e->d_state.alloc(cfg->slots) ||
-      e->d_order.alloc(cfg->slots) || e->d_next.alloc(1) || e->d_slot_attempts.alloc(cfg->slots) || e->d_ugrid.alloc(1 << 22) ||
+      e->d_order.alloc(cfg->slots) || e->d_next.alloc(1) || e->d_slot_attempts.alloc(cfg->slots) || e->d_ugrid.alloc(2u << 22) ||
       e->d_ugrid32.alloc(1 << 22)) {
     delete e;
     return fail(PIMC_ERR_CUDA, "cudaMalloc server pool");
   }
   e->free_blocks[0] = words;
+  {
+    const std::vector<double> logs = log_table();
+    if (e->d_logtab.alloc(logs.size()) ||
+        cudaMemcpy(e->d_logtab.p, logs.data(), logs.size() * 8, cudaMemcpyHostToDevice) !=
+            cudaSuccess) {
+      delete e;
+      return fail(PIMC_ERR_CUDA, "cudaMalloc server tables");
+    }
+  }
   *out = e;
   return PIMC_OK;
 }
@@ -2340,13 +2387,15 @@ int pimc_server_admit(pimc_engine* e, const pimc_system* sys, const pimc_pair_ta
             std::equal(t.ugrid, t.ugrid + words, it->second.second.begin()))
           toff = it->second.first;
       if (toff == (size_t)-1) {
-        if (e->table_used + words > e->d_ugrid.n) {
+        if (e->table_used + words > e->d_ugrid32.n) {
           pool_free(e, po, pw + cw);
           return fail(PIMC_ERR_INVALID, "server table pool full (distinct pair tables exceed 32 MiB)");
         }
         toff = e->table_used;
         std::vector<float> f(t.ugrid, t.ugrid + words);
-        CU(cudaMemcpy(e->d_ugrid.p + toff, t.ugrid, words * 8, cudaMemcpyHostToDevice));
+        std::vector<double> both(2 * words);
+        interleave_table(t, both.data());
+        CU(cudaMemcpy(e->d_ugrid.p + 2 * toff, both.data(), words * 16, cudaMemcpyHostToDevice));
         CU(cudaMemcpy(e->d_ugrid32.p + toff, f.data(), words * 4, cudaMemcpyHostToDevice));
         e->table_used += words;
         e->table_dev.emplace(t.ugrid, std::make_pair(toff, std::vector<double>(t.ugrid, t.ugrid + words)));
@@ -2363,7 +2412,8 @@ int pimc_server_admit(pimc_engine* e, const pimc_system* sys, const pimc_pair_ta
       dt.npart2 = d.spec_count[t.species2];
       dt.rgridinv = t.rgridinv;
       dt.logrratioinv = t.logrratioinv;
-      dt.ugrid = e->d_ugrid.p + toff;
+      dt.logtab = e->d_logtab.p;
+      dt.ugrid = e->d_ugrid.p + 2 * toff;
       dt.ugrid32 = e->d_ugrid32.p + toff;
     }
     d.ntab = ntables;

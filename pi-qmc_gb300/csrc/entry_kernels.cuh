@@ -129,9 +129,7 @@ __device__ __forceinline__ double pair_utau_link(const DevTable& tb, const PairS
   const double q = 0.5 * (e.r + p.r);
   const double sx = e.x - p.x, sy = e.y - p.y, sz = e.z - p.z;
   const double s2 = dot3(sx, sy, sz, sx, sy, sz) / (q * q);
-  double v, vt;
-  tab_uk0d(tb, q, s2, v, vt);
-  return vt;
+  return tab_uk0_tau(tb, q, s2);
 }
 __device__ __forceinline__ double pair_utau_link(const DevTable& tb, const PairSep<true>& e,
                                                  const PairSep<true>& p) {
@@ -292,14 +290,13 @@ __device__ __forceinline__ PairForce pair_force(const DevTable& tb, const double
   int i;
   double x;
   tab_locate(tb, q, i, x);
-  const double* g0 = tb.ugrid + (size_t)i * 2 * tb.ndata;
-  const double* g1 = g0 + 2 * tb.ndata;
+  const double* g = tb.ugrid + (size_t)i * 4 * tb.ndata;
   double uq = 0.0, us2 = 0.0, vt = 0.0;
   for (int k = tb.norder; k >= 0; k--) {
-    const double a0 = __ldg(g0 + k), da = __ldg(g1 + k) - a0;
-    uq = uq * s2 + da;
-    if (k > 0) us2 = us2 * s2 + k * (a0 + x * da);
-    vt = vt * s2 + ((1 - x) * __ldg(g0 + tb.ndata + k) + x * __ldg(g1 + tb.ndata + k));
+    const double2 a = __ldg((const double2*)g + k);
+    uq = uq * s2 + a.y;
+    if (k > 0) us2 = us2 * s2 + k * fma(x, a.y, a.x);
+    vt = vt * s2 + tab_at(g + 2 * tb.ndata, k, x);
   }
   uq *= tb.logrratioinv * qi;
   // -[uq d / (2 r) + us2 (2 s / q^2 - s2 d / (q r))], d the end's own separation, s

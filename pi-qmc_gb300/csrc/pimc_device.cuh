@@ -17,8 +17,9 @@ constexpr int kMaxBlock = 512;  // largest section-kernel block (64..512 threads
 constexpr int kWarps = kMaxBlock / 32;  // reduction slots
 
 struct DevTable {
-  const double* ugrid;  // (ngpts,2,ndata)
-  const float* ugrid32; // same table in FP32 (mixed precision)
+  const double* ugrid;  // (ngpts,2,ndata,2): coefficient, its difference to the next point's
+  const float* ugrid32; // (ngpts,2,ndata) in FP32 (mixed precision)
+  const double* logtab; // table of the logarithm (grid_log)
   int ngpts, norder, ndata, s1, s2;
   int ifirst1, npart1, ifirst2, npart2;
   double rgridinv, logrratioinv;
@@ -171,15 +172,16 @@ static __device__ __noinline__ double3 pbc_far_call(const DevSys& s, double x, d
   return pbc_far(s, x, y, z, fx, fy, fz, r2);
 }
 
-__device__ __forceinline__ void pbc(const DevSys& s, double& x, double& y, double& z) {
+// (returns whether the vector may have changed)
+__device__ __forceinline__ bool pbc(const DevSys& s, double& x, double& y, double& z) {
   const float fx = abs_f32_trunc(x), fy = abs_f32_trunc(y), fz = abs_f32_trunc(z);
   const float r2 = fx * fx + fy * fy + fz * fz;
-  if (!(r2 < s.rcut2_lo)) {
-    const double3 v = pbc_far_call(s, x, y, z, fx, fy, fz, r2);
-    x = v.x;
-    y = v.y;
-    z = v.z;
-  }
+  if (r2 < s.rcut2_lo) return false;
+  const double3 v = pbc_far_call(s, x, y, z, fx, fy, fz, r2);
+  x = v.x;
+  y = v.y;
+  z = v.z;
+  return true;
 }
 
 // |v|^2 of the FP32 terms, every rounding written out: the same bits in every
@@ -293,59 +295,82 @@ __device__ __forceinline__ double pg_images_eval(const DevSys& s, int sp, double
   return __dmul_rn(e, __dmul_rn(px, pyz));
 }
 
+// log(q) for 1 <= q < 2^20, by table (P. T. P. Tang, "Table-driven implementation of
+// the logarithm function in IEEE floating-point arithmetic", ACM TOMS 16, 1990): 128
+// intervals an octave, c_j near the reciprocal of the interval's middle with few
+// bits, r = m c_j - 1 with |r| < 2^-7.99, and log q = (e ln 2 - log c_j) + log1p(r), the
+// first part tabulated per octave, the second by its series to r^6 (r^7 / 7 < 2^-58).
+// Eight FP64 instructions where log() takes thirty.  The table: kLogReciprocals
+// values c_j, then kLogEntries of e ln 2 - log c_j.
+constexpr int kLogReciprocals = 128, kLogOctaves = 20;
+constexpr int kLogEntries = kLogReciprocals * kLogOctaves;
+__device__ __forceinline__ double grid_log(const double* tab, double q, unsigned k) {
+  const int hi = __double2hiint(q);
+  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(q));
+  const double r = __fma_rn(m, __ldg(tab + (k & (kLogReciprocals - 1))), -1.0);
+  double p = __fma_rn(r, -1.0 / 6, 1.0 / 5);
+  p = __fma_rn(r, p, -1.0 / 4);
+  p = __fma_rn(r, p, 1.0 / 3);
+  p = __fma_rn(r, p, -1.0 / 2);
+  p = __fma_rn(__dmul_rn(r, r), p, r);
+  return __dadd_rn(__ldg(tab + kLogReciprocals + k), p);
+}
+
 // Pair-action table lookup on the logarithmic grid
 // (PairAction::u00 / uk0 / uk0CalcDerivatives, src/action/PairAction.cc:601-655).
-// The range tests come before the conversion to an integer and are written so
-// that a NaN or infinite distance takes a clamped branch: converting NaN to int
-// is not defined to give an in-range index.  For finite q >= 1 the branches
-// are pi-qmc's (i = int(x) > ngpts - 2 exactly when x >= ngpts - 1).
+// Distances below the grid take its first point, those beyond it its last; a NaN or
+// infinite distance ends in a clamped index too.  For finite q >= 1 the branches are
+// pi-qmc's (i = int(x) > ngpts - 2 exactly when x >= ngpts - 1).
 __device__ __forceinline__ void tab_locate(const DevTable& t, double q, int& i, double& x) {
   q *= t.rgridinv;
-  x = log(q) * t.logrratioinv;
-  if (!(q >= 1)) {
-    i = 0;
-    x = 0;
-  } else if (!(x < t.ngpts - 1)) {
+  const unsigned k = (unsigned)(__double2hiint(q) - 0x3ff00000) >> 13;
+  if (k < (unsigned)kLogEntries) {
+    x = grid_log(t.logtab, q, k) * t.logrratioinv;
+  } else {  // below 1 (or negative: NaN paths), past 2^20, infinite or NaN
+    x = q >= 1 ? log(q) * t.logrratioinv : 0.0;
+    if (!(x < 2e9)) x = 2e9;
+  }
+  i = max((int)x, 0);
+  if (i > t.ngpts - 2) {
     i = t.ngpts - 2;
     x = 1;
   } else {
-    i = (int)x;
     x -= i;
   }
+}
+
+// Coefficient k of row (i, which) at x between the grid points.
+__device__ __forceinline__ double tab_at(const double* g, int k, double x) {
+  const double2 v = __ldg((const double2*)g + k);
+  return fma(x, v.y, v.x);
 }
 
 __device__ __forceinline__ double tab_u00(const DevTable& t, double r) {
   int i;
   double x;
   tab_locate(t, r, i, x);
-  const double* g = t.ugrid + (size_t)i * 2 * t.ndata;
-  return (1 - x) * __ldg(g) + x * __ldg(g + 2 * t.ndata);
+  return tab_at(t.ugrid + (size_t)i * 4 * t.ndata, 0, x);
 }
 
 __device__ __forceinline__ double tab_uk0(const DevTable& t, double q, double s2) {
   int i;
   double x;
   tab_locate(t, q, i, x);
-  const double* g0 = t.ugrid + (size_t)i * 2 * t.ndata;
-  const double* g1 = g0 + 2 * t.ndata;
+  const double* g = t.ugrid + (size_t)i * 4 * t.ndata;
   double a = 0;
-  for (int k = t.norder; k >= 0; k--) a = a * s2 + ((1 - x) * __ldg(g0 + k) + x * __ldg(g1 + k));
+  for (int k = t.norder; k >= 0; k--) a = a * s2 + tab_at(g, k, x);
   return a;
 }
 
-__device__ __forceinline__ void tab_uk0d(const DevTable& t, double q, double s2, double& u,
-                                         double& ut) {
+// The tau derivative of the series.
+__device__ __forceinline__ double tab_uk0_tau(const DevTable& t, double q, double s2) {
   int i;
   double x;
   tab_locate(t, q, i, x);
-  const double* g0 = t.ugrid + (size_t)i * 2 * t.ndata;
-  const double* g1 = g0 + 2 * t.ndata;
-  u = 0;
-  ut = 0;
-  for (int k = t.norder; k >= 0; k--) {
-    u = u * s2 + ((1 - x) * __ldg(g0 + k) + x * __ldg(g1 + k));
-    ut = ut * s2 + ((1 - x) * __ldg(g0 + t.ndata + k) + x * __ldg(g1 + t.ndata + k));
-  }
+  const double* g = t.ugrid + (size_t)(i * 2 + 1) * 2 * t.ndata;
+  double a = 0;
+  for (int k = t.norder; k >= 0; k--) a = a * s2 + tab_at(g, k, x);
+  return a;
 }
 
 // FP32 variants for the mixed-precision form (same grid, FP32 coefficients).

@@ -315,3 +315,30 @@ def test_action_difference_batches(pimc, case, nbatch):
         for b in list(range(min(nbatch, 3))) + [nbatch - 1]:
             ref = port.action_diff(level, sec[b], mov[b], int(ip[b]))
             assert abs(ds[b] - ref) <= 1e-12 * max(abs(ref), 1.0), (level, b)
+
+
+@pytest.mark.parametrize("rmin,rmax,ngpts", [(0.005, 20.0, 500), (1.0, 3.0, 2), (1e-4, 300.0, 97)])
+def test_pair_table_grid_edges(pimc, rmin, rmax, ngpts):
+    # Distances at the grid's points and ends, in every octave, below, beyond and far
+    # beyond it, through the Action-level call at a diagonal level (u00 alone) and an
+    # off-diagonal one.  One interpolation of two table values: 1e-12 of the largest.
+    kw = W.dot2(nslice=64, nlevel=4, beta=2.0, sho_omega=[0.0, 0.0], spring=0)
+    tabs, _ = pimc.coulomb_tables(kw, ngpts=ngpts, rmin=rmin, rmax=rmax)
+    t = tabs[0]
+    r = np.concatenate([1.0 / t["rgridinv"] * np.exp(np.arange(ngpts) / t["logrratioinv"]),
+                        rmin * 2.0 ** np.arange(-3, 24), [rmax * (1 + 1e-15), rmax, rmin, 1e-9]])
+    r = np.concatenate([r, r * (1 + 1e-14), r * (1 - 1e-14), r * 1.013])
+    r = r[r < 490.0]  # inside half the cell
+    cfg = O.make_config(**kw)
+    port = O.PortOracle(cfg, tabs)
+    e = pimc.Engine(kw, 1, tabs)
+    sec = np.zeros((len(r), 17, 2, 3))
+    sec[:, :, 0, 0] = r[:, None]
+    sec[:, ::2, 0, 1] = 1e-3 * r[:, None]
+    mov = sec[:, :, 0].copy()
+    mov[:, 1:-1, 0] = np.roll(r, 7)[:, None]
+    size = np.abs(np.asarray(t["ugrid"])[:, 0, 0]).max() * 16
+    for level in (1, 3):
+        ds = e.action_difference(level, sec, mov, np.zeros(len(r), np.int32))
+        ref = np.array([port.action_diff(level, sec[b], mov[b], 0) for b in range(len(r))])
+        assert np.all(np.abs(ds - ref) <= 1e-12 * size), level
