@@ -304,8 +304,8 @@ static __device__ __noinline__ bool displace_nodes(const DevSys& s, const Smem& 
   const int n = s.spec_count[sp], f = s.spec_first[sp], half = s.nslice / 2, nsm = s.ns_max;
   const bool sho = s.node_kind[sp] == PIMC_NODES_SHO;
   const int W = node_group_width(n), G = 32 / W, g = lane / W, gl = lane & (W - 1);
-  double* gscr = group_scr(m, warp, g, n, !sho);
-  double* gcold = group_cold(m, warp, g, n, !sho);
+  double* gscr = group_scr(m, warp * G + g, G, n, !sho);
+  double* gcold = group_cold(m, warp * G + g, G, n, !sho);
   double* st = stage + (size_t)(warp * G + g) * 6 * n;  // [2][3][n]
   const unsigned pm = moved_mask(s, mv, sp);
   bool bad = false;
@@ -412,7 +412,8 @@ static __device__ __noinline__ void displace_commit_nodes(const DevSys& s, const
     const double* b2 = path + ((size_t)ts * np + f + i) * 3;
     SliceView v1{b1 - (f + j), b1 + 1 - (f + j), b1 + 2 - (f + j), 0, 0, -1, 0, 0, 0};
     SliceView v2{b2 - (f + i), b2 + 1 - (f + i), b2 + 2 - (f + i), 0, 0, -1, 0, 0, 0};
-    const NodeElement v = node_element(s, sp, v1, v2, i, j);
+    const NodeElement v = sho ? node_element<true>(s, sp, v1, v2, i, j)
+                              : node_element<false>(s, sp, v1, v2, i, j);
     double* ec = e + 2 + 2 * n + j * n + i;
     ec[0] = v.v;
     if (!sho) {
@@ -492,6 +493,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
       m.nodescr_stride = L.nodescr_stride;
       m.nodecold = L.split ? gbase : nullptr;
       m.nodecold_stride = L.nodecold_stride;
+      m.node_cold_follows = !L.split;
       M_ = m;
       status = P.state[r].status;
       nacc = 0;

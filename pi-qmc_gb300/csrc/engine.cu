@@ -388,8 +388,9 @@ int validate(const pimc_system& s) {
   return 0;
 }
 
-// The table of grid_log: c_j, then e ln 2 - log c_j.
-std::vector<double> log_table() {
+// The table of grid_log: c_j, then e ln 2 - log c_j.  (The same for every engine; made
+// by the first.)
+std::vector<double> make_log_table() {
   std::vector<double> t(kLogReciprocals + kLogEntries);
   for (int j = 0; j < kLogReciprocals; ++j) {
     // 1 / (middle of the interval) to 13 bits: m c_j - 1 then takes one rounding
@@ -400,6 +401,11 @@ std::vector<double> log_table() {
       t[kLogReciprocals + e * kLogReciprocals + j] =
           (double)(e * 0.693147180559945309417232121458L + lc);
   }
+  return t;
+}
+
+const std::vector<double>& log_table() {
+  static const std::vector<double> t = make_log_table();
   return t;
 }
 
@@ -631,19 +637,21 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
     for (int i = 0; i < d.nspecies; ++i) anyfree_col |= d.node_kind[i] == PIMC_NODES_FREE;
   L.ncol_stride = nsm * (anyfree_col ? 4 : 1);
   const int ncol_size = fixed ? nsec * L.ncol_stride : 0;
-  // per-warp Slater scratch: (32 / W) lane groups of node_group_scratch(n)
-  // doubles, or of its hot and cold parts apart (the species present decide
-  // it: a smaller species packs more lane groups per warp)
+  // per-warp Slater scratch: (32 / W) lane groups of node_group_hot(n) doubles, or of
+  // node_group_scratch(n), or of its hot and cold parts apart, when a system of the
+  // launch keeps no cache entries (the species present decide it: a smaller species
+  // packs more lane groups per warp)
   int full = 0, hot = 0, cold = 0;
   for (const DevSys& d : sys)
     for (int i = 0; i < d.nspecies; ++i)
       if (d.node_kind[i]) {
         const int n = d.spec_count[i], G = 32 / node_group_width(n);
         const bool fr = d.node_kind[i] == PIMC_NODES_FREE;
-        full = std::max(full, G * node_group_scratch(n, fr));
+        full = std::max(full, G * (uncached ? node_group_scratch(n, fr) : node_group_hot(n)));
         hot = std::max(hot, G * node_group_hot(n));
-        cold = std::max(cold, G * node_group_cold(n, fr));
+        if (uncached) cold = std::max(cold, G * node_group_cold(n, fr));
       }
+  L.cold_follows = uncached;
   full = (full + 1) & ~1;
   hot = (hot + 1) & ~1;
   cold = (cold + 1) & ~1;
@@ -669,9 +677,11 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
   const bool ncol_smem = place == kAll || place == kHotCol || place == kGlobalCol;
   L.ncol = (fixed && ncol_smem) ? take(ncol_size) : -1;
   L.ncol_global = fixed && !ncol_smem;
-  L.split = place == kHotCol || place == kHot;
-  L.nodescr_in_smem = place == kAll || L.split;
-  L.nodescr_stride = place == kAll ? full : (L.split ? hot : full);
+  // (without cold parts there is nothing to put apart)
+  L.split = uncached && (place == kHotCol || place == kHot);
+  L.nodescr_in_smem = place <= kHot;
+  L.nodescr_stride = L.split ? hot : full;
+  if (L.split) L.cold_follows = 0;
   L.nodecold_stride = L.split ? cold : 0;
   L.nodescr = L.nodescr_in_smem ? take(nwarps * L.nodescr_stride) : -1;
   const int gwarp = L.split ? cold : (L.nodescr_in_smem ? 0 : full);
@@ -1156,33 +1166,23 @@ int prefill_cache(pimc_engine* e, double* cache, const int* d_slots, int nslot,
   P.only_invalid = only_invalid ? 1 : 0;
   P.ntask_per_slot = nsp * mmax;
   P.stage_stride = (6 * nmax + 1) & ~1;
-  // Slater scratch: all of it in shared memory up to 6 KB a warp; else its hot
-  // part (LU, inverse) there up to 24 KB with the cold part in global memory;
-  // else all of it in global memory
-  const int full = (node_group_scratch(nmax, anyfree) + 1) & ~1;
-  const int hot = (node_group_hot(nmax) + 1) & ~1;
-  const int cold = (node_group_cold(nmax, anyfree) + 1) & ~1;
-  const bool all_smem = full * 8 <= 6 * 1024, split = !all_smem && hot * 8 <= 24 * 1024;
-  P.scratch_stride = split ? hot : full;
-  P.cold_stride = split ? cold : 0;
+  // Slater scratch (its hot part: the elements live in the entries) in shared memory
+  // up to 24 KB a warp, else in global memory
+  P.scratch_stride = (node_group_hot(nmax) + 1) & ~1;
+  const bool in_smem = P.scratch_stride * 8 <= 24 * 1024;
   const int nw = kBlock / 32;
   const size_t smem =
-      (size_t)nw * (P.stage_stride + ((all_smem || split) ? P.scratch_stride : 0)) * 8;
+      (size_t)nw * (P.stage_stride + (in_smem ? P.scratch_stride : 0)) * 8;
   const long long ntask = (long long)nslot * P.ntask_per_slot;
   const int grid = (int)std::min<long long>((ntask + nw - 1) / nw, (long long)e->num_sms * 4);
   P.gscratch = nullptr;
-  P.gcold = nullptr;
-  const size_t gper = all_smem ? 0 : (split ? (size_t)cold : (size_t)full);
-  if (gper) {
-    const size_t need = (size_t)grid * nw * gper;
+  if (!in_smem) {
+    const size_t need = (size_t)grid * nw * P.scratch_stride;
     if (e->d_prefill_scr.n < need) {
       CU(cudaStreamSynchronize(e->stream));  // an earlier fill may still use it
       if (e->d_prefill_scr.alloc(need)) return fail(PIMC_ERR_CUDA, "cudaMalloc prefill scratch");
     }
-    if (split)
-      P.gcold = e->d_prefill_scr.p;
-    else
-      P.gscratch = e->d_prefill_scr.p;
+    P.gscratch = e->d_prefill_scr.p;
   }
   cudaFuncSetAttribute(cache_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        200 * 1024);
@@ -2327,7 +2327,7 @@ int pimc_server_create(const pimc_server_config* cfg, uint64_t seed, int precisi
   }
   e->free_blocks[0] = words;
   {
-    const std::vector<double> logs = log_table();
+    const std::vector<double>& logs = log_table();
     if (e->d_logtab.alloc(logs.size()) ||
         cudaMemcpy(e->d_logtab.p, logs.data(), logs.size() * 8, cudaMemcpyHostToDevice) !=
             cudaSuccess) {

@@ -19,6 +19,7 @@ struct Layout {
   int nodescr_stride;   // doubles per warp of that scratch
   int split;            // cold parts apart, in the CTA's global area
   int nodecold_stride;  // doubles per warp of the cold parts
+  int cold_follows;     // each group's cold part follows its hot part
   int ncol_global;      // the new-column buffer in the CTA's global area
   int gcta;             // doubles of global scratch per CTA
   int ewt_cols;         // bead columns of the Ewald tables area
@@ -83,6 +84,7 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
                        : ((L.ncol_global && gbase) ? gbase + (size_t)nw * gwarp : nullptr);
   m.nodecold = (L.split && gbase) ? gbase : nullptr;
   m.nodecold_stride = L.nodecold_stride;
+  m.node_cold_follows = L.cold_follows;
   m.ewt_cols = L.ewt_cols;
   m.ewxy = L.ewxy ? base + L.ewxy : nullptr;
   m.nrm = base + L.nrm;
@@ -453,8 +455,8 @@ static __device__ double mover_level(const DevSys& s, const Smem& m, int ipart, 
   return block_sum(mover_level_part(s, m, ipart, level, oshift, second), m.red);
 }
 
-// Evaluates one slice pair per lane group (group width W from the species size).
-__device__ __forceinline__ void node_eval_dispatch(int W, const DevSys& s, int sp,
+// Evaluates one slice pair per lane group of width W.
+static __device__ __noinline__ void node_eval_dispatch(int W, const DevSys& s, int sp,
                                                    const SliceView& v1, const SliceView& v2,
                                                    double scale, double* scr, int full,
                                                    double* ecache, unsigned cols, bool write,
@@ -466,25 +468,28 @@ __device__ __forceinline__ void node_eval_dispatch(int W, const DevSys& s, int s
                                                    double det_in = 0.0, double* xout = nullptr,
                                                    double xepoch = 0.0) {
   // (xin and xout are the same for every lane of a warp)
-  if (xin || xout) {
-    if (W == 8)
-      node_eval_group<8, true>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err,
-                               d1, d2, newcol, rowmask, cold, xin, det_in, xout, xepoch);
-    else if (W == 16)
-      node_eval_group<16, true>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err,
-                                d1, d2, newcol, rowmask, cold, xin, det_in, xout, xepoch);
-    else
-      node_eval_group<32, true>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err,
-                                d1, d2, newcol, rowmask, cold, xin, det_in, xout, xepoch);
-  } else if (W == 8) {
-    node_eval_group<8>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2,
-                       newcol, rowmask, cold);
-  } else if (W == 16) {
-    node_eval_group<16>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2,
-                        newcol, rowmask, cold);
+  const auto run = [&](auto w, auto sho, auto sm) {
+    node_eval_group<decltype(w)::value, decltype(sho)::value, decltype(sm)::value>(
+        s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2, newcol, rowmask,
+        cold, xin, det_in, xout, xepoch);
+  };
+  const std::integral_constant<int, 8> w8;
+  const std::integral_constant<int, 16> w16;
+  const std::integral_constant<int, 32> w32;
+  const std::true_type yes;
+  const std::false_type no;
+  if (s.node_kind[sp] == PIMC_NODES_SHO) {
+    if (W == 8) run(w8, yes, no);
+    else if (W == 16) run(w16, yes, no);
+    else run(w32, yes, no);
+  } else if (xin || xout) {
+    if (W == 8) run(w8, no, yes);
+    else if (W == 16) run(w16, no, yes);
+    else run(w32, no, yes);
   } else {
-    node_eval_group<32>(s, sp, v1, v2, scale, scr, full, ecache, cols, write, det, err, d1, d2,
-                        newcol, rowmask, cold);
+    if (W == 8) run(w8, no, no);
+    else if (W == 16) run(w16, no, no);
+    else run(w32, no, no);
   }
 }
 
@@ -561,13 +566,11 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   __syncthreads();
   // warp tasks: each warp takes up to G misses of one species (lane groups of
   // a warp must run the same species so that they stay converged)
-  int ntask = 0;
-  int Gs[kMaxSpecies], Ws[kMaxSpecies], first[kMaxSpecies + 1];
+  int ntask = 0, first[kMaxSpecies + 1];
   for (int sp = 0; sp < s.nspecies; ++sp) {
-    Ws[sp] = node_group_width(s.spec_count[sp]);
-    Gs[sp] = 32 / Ws[sp];
+    const int G = 32 / node_group_width(s.spec_count[sp]);
     first[sp] = ntask;
-    ntask += (nmiss[sp] + Gs[sp] - 1) / Gs[sp];
+    ntask += (nmiss[sp] + G - 1) / G;
   }
   first[s.nspecies] = ntask;
   if (llt && warp == nwarps - 1) mover_all(s, m, ipart, seed, att, llt);
@@ -576,13 +579,13 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     while (wt >= first[sp + 1]) ++sp;
     const int n = s.spec_count[sp];
     const bool sho = s.node_kind[sp] == PIMC_NODES_SHO, mine = sp == msp;
-    const int W = Ws[sp], gm = lane / W, glm = lane & (W - 1);
-    const int base = (wt - first[sp]) * Gs[sp];
+    const int W = node_group_width(n), G = 32 / W, gm = lane / W, glm = lane & (W - 1);
+    const int base = (wt - first[sp]) * G;
     const int task = base + gm;
     const bool act = task < nmiss[sp];
     const int t = miss[sp * nsec + (act ? task : base)];
-    double* scrm = group_scr(m, warp, gm, n, !sho);
-    double* coldm = group_cold(m, warp, gm, n, !sho);
+    double* scrm = group_scr(m, warp * G + gm, G, n, !sho);
+    double* coldm = group_cold(m, warp * G + gm, G, n, !sho);
     double* e = cache ? cache_entry(s, cache, sp, wrap_slice(ifirst1 + t, M)) : nullptr;
     SliceView v1{m.s1x, m.s1y, m.s1z, s.npart, t, -1, 0, 0, 0};
     SliceView v2{m.s2x, m.s2y, m.s2z, s.npart, t, -1, 0, 0, 0};
@@ -667,8 +670,12 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
         int err = er[k];
         double sc2 = scale[sp];
         int guard = 0;
-        double* dsc = group_scr(m, warp, g, n, !sho);
-        double* dcold = group_cold(m, warp, g, n, !sho);
+        double* dsc = group_scr(m, g, 32 / W, n, !sho);
+        double* dcold = group_cold(m, g, 32 / W, n, !sho);
+        // (the elements do not depend on the scale: those of the slice's entry, whole
+        // since the pass above)
+        double* ec = cache ? cache_entry(s, cache, sp, wrap_slice(ifirst1 + k, M)) + 2 + 2 * n
+                           : nullptr;
         while (err || fabs(det) < 1e-50 || fabs(det) > 1e50) {
           if (err || ++guard > 2000) {
             if (lane == 0) *status |= err ? (PIMC_STATUS_SINGULAR | PIMC_STATUS_RESCALE_LIMIT)
@@ -683,9 +690,9 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
           SliceView v2{m.s2x, m.s2y, m.s2z, s.npart, k, -1, 0, 0, 0};
           double d = 0;
           int e2 = 0;
-          node_eval_dispatch(W, s, sp, v1, v2, sc2, dsc, mine ? 1 : 0, nullptr, 0u, g == 0, d,
-                             e2, m.dist + (k * 2) * nsm, m.dist + (k * 2 + 1) * nsm, nullptr,
-                             0xffffffffu, dcold);
+          node_eval_dispatch(W, s, sp, v1, v2, sc2, dsc, mine ? 1 : 0, ec, 0u, g == 0, d, e2,
+                             m.dist + (k * 2) * nsm, m.dist + (k * 2 + 1) * nsm, nullptr, 0u,
+                             dcold);
           det = __shfl_sync(0xffffffffu, d, 0);
           err = __shfl_sync(0xffffffffu, e2, 0);
         }
@@ -784,8 +791,8 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
     }
     if (warp < nodeW) {
       const bool sho = s.node_kind[msp] == PIMC_NODES_SHO;
-      double* scr = group_scr(m, warp, g, n, !sho);
-      double* cold = group_cold(m, warp, g, n, !sho);
+      double* scr = group_scr(m, warp * G + g, G, n, !sho);
+      double* cold = group_cold(m, warp * G + g, G, n, !sho);
       const int jcol = ipart - s.spec_first[msp];
       for (int base = warp * G; base < ntask; base += nodeW * G) {
         const int task = base + g;

@@ -42,6 +42,7 @@ struct Smem {
   int nodescr_stride;       // doubles per warp
   double* nodecold;         // cold parts of the node scratch when apart (global), or null
   int nodecold_stride;      // doubles per warp
+  int node_cold_follows;    // each group's cold part follows its hot part
   int ewt_cols;             // bead columns of the Ewald tables area
   double* xstage;           // mixed form: [nsec][xstage_stride] inverse blocks (global), or null
   int xstage_stride;
@@ -78,6 +79,18 @@ struct SliceView {
   }
 };
 
+// a / m for 0 <= a < 2048, 1 <= m <= 32 (an integer division takes some 25 instructions)
+struct SmallReciprocals {
+  unsigned v[33];
+  constexpr SmallReciprocals() : v{} {
+    for (unsigned m = 1; m <= 32; ++m) v[m] = (65536u + m - 1u) / m;
+  }
+};
+static __constant__ SmallReciprocals kSmallReciprocals;
+__device__ __forceinline__ int small_div(int a, int m) {
+  return (int)(((unsigned)a * kSmallReciprocals.v[m]) >> 16);
+}
+
 // ------------------------------------------------------------------ node model
 // The mixed form's Sherman-Morrison updates of cached inverses: at most
 // kSmRefresh updates between two factorisations of a slice pair's matrix, and
@@ -89,10 +102,11 @@ constexpr double kSmRefresh = 16.0;
 constexpr double kSmMinRatio = 0.05;
 constexpr double kSmMaxCond = 1e7;
 // Scratch doubles one lane group needs for an n-particle species: a hot part
-// (the LU and the inverse, rewritten at every elimination step, and the
-// reciprocal pivots) and a cold part (the SHO exp matrix, or the free-particle
-// gradient matrices: written once, read once).
-__host__ __device__ constexpr int node_group_hot(int n) { return 2 * n * n + n + 1; }
+// (the LU and the inverse, rewritten at every elimination step, the reciprocal
+// pivots and the row order), and, for evaluations whose elements are not in a cache
+// entry, a cold part (the SHO exp matrix, or the free-particle gradient matrices:
+// written once, read once).
+__host__ __device__ constexpr int node_group_hot(int n) { return 2 * n * n + n + (n + 1) / 2 + 1; }
 __host__ __device__ constexpr int node_group_cold(int n, bool free_nodes = true) {
   return n * n + (free_nodes ? 3 * n * n : 0);
 }
@@ -100,14 +114,16 @@ __host__ __device__ constexpr int node_group_scratch(int n, bool free_nodes = tr
   return node_group_hot(n) + node_group_cold(n, free_nodes);
 }
 
-// Slater scratch of lane group g of a warp: the hot part (with the cold part
-// after it, unless the layout keeps cold parts apart) and the cold part.
-__device__ __forceinline__ double* group_scr(const Smem& m, int warp, int g, int n, bool free_nodes) {
-  return m.nodescr + (size_t)warp * m.nodescr_stride +
-         g * (m.nodecold ? node_group_hot(n) : node_group_scratch(n, free_nodes));
+// Slater scratch of a lane group: the hot part (with the cold part after it where
+// the layout has one there) and the cold part.  slot counts the groups of every
+// warp, G to a warp.
+__device__ __forceinline__ double* group_scr(const Smem& m, int slot, int G, int n, bool free_nodes) {
+  return m.nodescr + (size_t)(slot / G) * m.nodescr_stride +
+         (slot % G) * (m.node_cold_follows ? node_group_scratch(n, free_nodes) : node_group_hot(n));
 }
-__device__ __forceinline__ double* group_cold(const Smem& m, int warp, int g, int n, bool free_nodes) {
-  return m.nodecold ? m.nodecold + (size_t)warp * m.nodecold_stride + g * node_group_cold(n, free_nodes)
+__device__ __forceinline__ double* group_cold(const Smem& m, int slot, int G, int n, bool free_nodes) {
+  return m.nodecold ? m.nodecold + (size_t)(slot / G) * m.nodecold_stride +
+                          (slot % G) * node_group_cold(n, free_nodes)
                     : nullptr;
 }
 
@@ -117,56 +133,79 @@ __device__ __forceinline__ double* group_cold(const Smem& m, int warp, int g, in
 struct NodeElement {
   double v, gx, gy, gz;
 };
+__device__ __forceinline__ double sho_element(const DevSys& s, int sp, double rix, double riy,
+                                              double riz, double rjx, double rjy, double rjz) {
+  const double ri2 = dot3(rix, riy, riz, rix, riy, riz);
+  const double rj2 = dot3(rjx, rjy, rjz, rjx, rjy, rjz);
+  const double rirj = dot3(rix, riy, riz, rjx, rjy, rjz);
+  const double q = __dsub_rn(__dmul_rn(__dadd_rn(ri2, rj2), s.node_cosh[sp]),
+                             __dmul_rn(2.0, rirj));
+  return exp(__dmul_rn(-s.node_c[sp], q));
+}
+// (a call: boxes too small for pg_images_eval)
+static __device__ __noinline__ NodeElement pg_series_element(const DevSys& s, int sp, double dx,
+                                                             double dy, double dz) {
+  double v[3], g[3];
+  const double d[3] = {dx, dy, dz};
+#pragma unroll 1
+  for (int a = 0; a < 3; ++a)
+    v[a] = pg_eval(s.pg_nome[sp][a], s.pg_pref[sp][a], s.pg_k[sp][a], s.pg_nmax[sp][a], d[a], &g[a]);
+  NodeElement r;
+  r.v = v[0] * v[1] * v[2];
+  r.gx = g[0] / (v[0] + 1e-300) * v[0] * v[1] * v[2];
+  r.gy = g[1] / (v[1] + 1e-300) * v[0] * v[1] * v[2];
+  r.gz = g[2] / (v[2] + 1e-300) * v[0] * v[1] * v[2];
+  return r;
+}
+__device__ __forceinline__ NodeElement free_element(const DevSys& s, int sp, double dx, double dy,
+                                                    double dz) {
+  pbc(s, dx, dy, dz);
+  if (!s.pg_images[sp]) return pg_series_element(s, sp, dx, dy, dz);
+  NodeElement r;
+  r.v = pg_images_eval(s, sp, dx, dy, dz, r.gx, r.gy, r.gz);
+  return r;
+}
+template <bool kSho>
 __device__ __forceinline__ NodeElement node_element(const DevSys& s, int sp, const SliceView& v1,
                                                     const SliceView& v2, int i, int j) {
   const int f = s.spec_first[sp];
   double rix, riy, riz, rjx, rjy, rjz;
   v2.get(f + i, rix, riy, riz);
   v1.get(f + j, rjx, rjy, rjz);
-  NodeElement r{0.0, 0.0, 0.0, 0.0};
-  if (s.node_kind[sp] == 1) {
-    const double ri2 = dot3(rix, riy, riz, rix, riy, riz);
-    const double rj2 = dot3(rjx, rjy, rjz, rjx, rjy, rjz);
-    const double rirj = dot3(rix, riy, riz, rjx, rjy, rjz);
-    const double q = __dsub_rn(__dmul_rn(__dadd_rn(ri2, rj2), s.node_cosh[sp]),
-                               __dmul_rn(2.0, rirj));
-    r.v = exp(__dmul_rn(-s.node_c[sp], q));
-    return r;
-  }
-  double dx = rjx - rix, dy = rjy - riy, dz = rjz - riz;
-  pbc(s, dx, dy, dz);
-  if (s.pg_images[sp]) {
-    r.v = pg_images_eval(s, sp, dx, dy, dz, r.gx, r.gy, r.gz);
-    return r;
-  }
-  double g0, g1, g2;
-  const double v0 = pg_eval(s.pg_nome[sp][0], s.pg_pref[sp][0], s.pg_k[sp][0], s.pg_nmax[sp][0], dx, &g0);
-  const double v1v = pg_eval(s.pg_nome[sp][1], s.pg_pref[sp][1], s.pg_k[sp][1], s.pg_nmax[sp][1], dy, &g1);
-  const double v2v = pg_eval(s.pg_nome[sp][2], s.pg_pref[sp][2], s.pg_k[sp][2], s.pg_nmax[sp][2], dz, &g2);
-  r.v = v0 * v1v * v2v;
-  r.gx = g0 / (v0 + 1e-300) * v0 * v1v * v2v;
-  r.gy = g1 / (v1v + 1e-300) * v0 * v1v * v2v;
-  r.gz = g2 / (v2v + 1e-300) * v0 * v1v * v2v;
-  return r;
+  if constexpr (kSho)
+    return NodeElement{sho_element(s, sp, rix, riy, riz, rjx, rjy, rjz), 0.0, 0.0, 0.0};
+  else
+    return free_element(s, sp, rjx - rix, rjy - riy, rjz - riz);
 }
 
 // NodeModel::evaluate (+ evaluateDistance) for one species on one slice pair,
-// executed by a group of W lanes (W = 8, 16 or 32; 32/W groups per warp each
-// take their own slice pair).  Lanes own matrix rows.  LU with partial pivoting
-// (first largest |pivot|, LAPACK dgetrf semantics), determinant from the U
-// diagonal and pivots, inverse by solving A X = I column per lane (dgetri
-// semantics), then the log-gradient nodal distances
+// executed by a group of W >= n lanes (W = 8, 16 or 32; 32/W groups per warp each
+// take their own slice pair).  LU with
+// partial pivoting (first largest |pivot|, LAPACK dgetrf semantics), determinant from
+// the U diagonal and pivots, inverse (dgetri semantics: the forward substitution runs
+// with the elimination, on the columns of the identity its row interchanges have
+// reached), then the log-gradient nodal distances
 // (src/fixednode/SHONodes.cc:51-170, src/fixednode/FreeParticleNodes.cc:72-234).
 // full = 0: determinant only.  Every lane of the warp must call this (the
 // shuffles span the warp); a group with write = false computes but stores
 // nothing.  ecache (or null) holds the slice pair's element matrix: the rows of
 // rowmask are recomputed, and the columns of `cols` in the other rows (their
 // other inputs are unchanged, so the values are bit-identical); without columns
-// what is recomputed is stored there.
-// kSm: the variant with the mixed form's Sherman-Morrison updates and inverse
-// blocks (xin / xout); without it those arguments are ignored and the
-// evaluation is the plain factorisation.
-template <int W, bool kSm = false>
+// what is recomputed is stored there, a single column goes to newcol.
+// kSho: SHONodes (else FreeParticleNodes).  kSm: the variant with the mixed form's
+// Sherman-Morrison updates and inverse blocks (xin / xout); without it those
+// arguments are ignored and the evaluation is the plain factorisation.
+//
+// FP64 bound: every step deals single elements to the lanes, so that a warp
+// instruction, which costs the SM the same whatever its lanes, has few idle ones.
+// Cached elements are read where they are used, straight from the entry, in
+// coalesced order; only a factorisation copies them (scaled).  The loops are not
+// unrolled and the models are apart: left to the compiler, one instance was 209 KB of
+// code, and warps in different phases waited for instructions.  A step of 304
+// fixed-node dots 157 -> 139 ms, of 152 electron gases 84 -> 62 ms.  (Two particles'
+// rows to a lane, four 10 x 10 matrices a warp on half the warps, would take 20 % fewer
+// FP64 instructions and measured 6 % more time.)
+template <int W, bool kSho, bool kSm = false>
 static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, const SliceView& v1,
                                 const SliceView& v2, double scale, double* scr, int full,
                                 double* ecache, unsigned cols, bool write, double& det_out,
@@ -180,73 +219,55 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   const int n = s.spec_count[sp];
   const int f = s.spec_first[sp];
   // hot part at scr; the cold part follows it unless given apart
-  double* A = scr;          // n*n column-major, LU; after the inverse: the distance weights
+  double* A = scr;          // n*n column-major, LU; after the inverse: work space
   double* X = A + n * n;    // n*n inverse, column-major
   double* R = X + n * n;    // n reciprocals of the U diagonal
-  double* E = cold ? cold : scr + node_group_hot(n);  // n*n exp values (SHO nodes)
-  double* G = E + n * n;    // 3 n*n gradient factors (free-particle nodes)
-  const bool sho = s.node_kind[sp] == 1;
-  // --- build the Slater matrix: A(i,j) = scale * rho(r1_j, r2_i)
-  // Elements come from ecache where it holds them (outside rowmask's rows and the
-  // columns of `cols`); the others are computed.  Whole rows (all of them without a cache, the stale ones on a
-  // refresh) go one element per lane and step, so that refreshing one or two
-  // rows still spreads over the group; the new column of a column update goes
-  // one row per lane.  Every element is the same rounded arithmetic wherever
-  // it is computed, so cached and recomputed values agree bit for bit.
+  int* order = (int*)(R + n + 1);  // the matrix row at each position; then its inverse
+  double* E = cold ? cold : scr + node_group_hot(n);  // elements (and gradients) without a place
+  constexpr bool sho = kSho;
   const int nn = n * n;
   const unsigned nmask = n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
   const unsigned rows_new = !ecache ? nmask : (rowmask & nmask);
-  // element (i, j): value into A (scaled), E (SHO) or G (gradients), and into
-  // ecache (a refresh) or newcol (the new column) when this group writes
-  auto element = [&](int i, int j) {
-    const bool to_cache = ecache && !cols && write;
-    const bool to_col = newcol && ((cols >> j) & 1u) && write;
-    const NodeElement v = node_element(s, sp, v1, v2, i, j);
-    if (to_cache) ecache[j * n + i] = v.v;
-    if (to_col) newcol[i] = v.v;
-    A[j * n + i] = scale * v.v;
-    if (sho) {
-      E[j * n + i] = v.v;
-    } else {
-      if (to_cache) {
-        ecache[nn + j * n + i] = v.gx;
-        ecache[2 * nn + j * n + i] = v.gy;
-        ecache[3 * nn + j * n + i] = v.gz;
-      }
-      if (to_col) {
-        newcol[n + i] = v.gx;
-        newcol[2 * n + i] = v.gy;
-        newcol[3 * n + i] = v.gz;
-      }
-      G[j * n + i] = v.gx;
-      G[nn + j * n + i] = v.gy;
-      G[2 * nn + j * n + i] = v.gz;
-    }
+  // --- build the Slater matrix: A(i,j) = scale * rho(r1_j, r2_i).  The new elements
+  // are computed, one per lane and step (whole rows, then the new columns of the
+  // other rows); the others follow when the matrix is factorised.  Every element is
+  // the same rounded arithmetic wherever it is computed, so cached and recomputed
+  // values agree bit for bit.
+  const bool to_cache = ecache && !cols, to_col = ecache && cols && newcol;
+  // component c (0: value, 1 .. 3: gradient) of element (i, j), k = j n + i
+  auto elem = [&](int c, int i, int j, int k) -> double {
+    if (!ecache) return E[c * nn + k];
+    if (cols && (((cols >> j) | (rows_new >> i)) & 1u)) return newcol ? newcol[c * n + i] : E[c * nn + k];
+    return ecache[c * nn + k];
   };
-  // cached rows (with the new column of a column update), one row per lane
-  if (ecache && gl < n && !((rows_new >> gl) & 1u)) {
-    const int i = gl;
-    for (int j = 0; j < n; ++j) {
-      if ((cols >> j) & 1u) {
-        element(i, j);
-      } else if (sho) {
-        const double e = ecache[j * n + i];
-        E[j * n + i] = e;
-        A[j * n + i] = scale * e;
-      } else {
-        A[j * n + i] = scale * ecache[j * n + i];
-        G[j * n + i] = ecache[nn + j * n + i];
-        G[nn + j * n + i] = ecache[2 * nn + j * n + i];
-        G[2 * nn + j * n + i] = ecache[3 * nn + j * n + i];
+  auto element = [&](int i, int j) {
+    const NodeElement v = node_element<kSho>(s, sp, v1, v2, i, j);
+    double* at = to_cache ? ecache + j * n + i : (to_col ? newcol + i : E + j * n + i);
+    const int step = to_col ? n : nn;
+    if (!to_cache || write) {
+      at[0] = v.v;
+      if (!sho) {
+        at[step] = v.gx;
+        at[2 * step] = v.gy;
+        at[3 * step] = v.gz;
       }
     }
-  }
-  // rows computed in full, one element per lane and step
-  const int nrows = __popc(rows_new);
-  for (int e = gl; e < nrows * n; e += W) {
-    unsigned rm = rows_new;
-    for (int q = e / n; q > 0; --q) rm &= rm - 1u;  // drop the first e/n set rows
-    element(__ffs(rm) - 1, e % n);
+    A[j * n + i] = scale * v.v;
+  };
+  {
+    const int nrows = __popc(rows_new), ncols = ecache ? __popc(cols & nmask) : 0;
+#pragma unroll 1
+    for (int e = gl; e < (nrows + ncols) * n; e += W) {
+      // the q-th new row's element in column x, then the new columns' in row x
+      int q = small_div(e, n);
+      const int x = e - q * n;
+      const bool row = q < nrows;
+      unsigned bits = row ? rows_new : cols & nmask;
+#pragma unroll 1
+      for (q = row ? q : q - nrows; q > 0; --q) bits &= bits - 1u;  // drop the first q
+      const int b = __ffs(bits) - 1;
+      if (row || !((rows_new >> x) & 1u)) element(row ? b : x, row ? x : b);
+    }
   }
   __syncwarp();
   int info = 0;
@@ -263,7 +284,15 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   // (a warp none of whose writing groups can update factorises at once)
   if (kSm && __any_sync(FULL, good && write) && __all_sync(FULL, good || !write)) {
     const double* xc = good ? xin + 2 : nullptr;
-    for (int k = gl; k < nn; k += W) X[k] = xc ? xc[k] : 0.0;
+#pragma unroll 1
+    for (int k0 = gl; k0 < nn; k0 += 8 * W) {  // (eight loads in flight a lane)
+      double v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = xc && k0 + q * W < nn ? xc[k0 + q * W] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (k0 + q * W < nn) X[k0 + q * W] = v[q];
+    }
     __syncwarp();
     double det = det_in;
     if (cols) {
@@ -272,6 +301,7 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
       // inv'(a, b) = inv(a, b) - (w_a - [a = jcol]) inv(jcol, b) / ratio
       double w = 0.0;
       if (gl < n)
+#pragma unroll 1
         for (int i = 0; i < n; ++i) w = __fma_rn(X[i * n + gl], A[jcol * n + i], w);
       const double ratio = __shfl_sync(FULL, w, jcol, W);
       good = good && fabs(ratio) >= kSmMinRatio;
@@ -280,10 +310,11 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
         const double rj = gl < n ? X[gl * n + jcol] : 0.0;  // inv(jcol, b), b = gl
         const double f = gl < n ? (w - (gl == jcol ? 1.0 : 0.0)) / ratio : 0.0;
         __syncwarp();
+#pragma unroll 1
         for (int e0 = 0; e0 < nn; e0 += W) {
           const int e = e0 + gl;
           const bool on = e < nn;
-          const int b = on ? e / n : 0, a = on ? e - b * n : 0;
+          const int b = on ? small_div(e, n) : 0, a = on ? e - b * n : 0;
           const double fa = __shfl_sync(FULL, f, a, W);
           const double rb = __shfl_sync(FULL, rj, b, W);
           if (on) X[b * n + a] = __fma_rn(-fa, rb, X[b * n + a]);
@@ -297,21 +328,24 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
       good = good && nr > 0 && 2 * nr <= n;
       const unsigned nrmax = __reduce_max_sync(FULL, good ? (unsigned)nr : 0u);
       unsigned rm = good ? rows_new : 0u;
+#pragma unroll 1
       for (unsigned k = 0; k < nrmax; ++k) {
         const bool live = rm != 0u;
         const int i = live ? __ffs(rm) - 1 : 0;
         rm &= rm - 1u;
         double z = 0.0;
         if (gl < n)
+#pragma unroll 1
           for (int j = 0; j < n; ++j) z = __fma_rn(A[j * n + i], X[gl * n + j], z);
         const double ratio = __shfl_sync(FULL, z, i, W);
         const double ci = gl < n ? X[i * n + gl] : 0.0;  // inv(a, i), a = gl
         const double g = gl < n ? (z - (gl == i ? 1.0 : 0.0)) / ratio : 0.0;
         __syncwarp();
+#pragma unroll 1
         for (int e0 = 0; e0 < nn; e0 += W) {
           const int e = e0 + gl;
           const bool on = e < nn && live;
-          const int b = e < nn ? e / n : 0, a = e < nn ? e - b * n : 0;
+          const int b = e < nn ? small_div(e, n) : 0, a = e < nn ? e - b * n : 0;
           const double ca = __shfl_sync(FULL, ci, a, W);
           const double gb = __shfl_sync(FULL, g, b, W);
           if (on) X[b * n + a] = __fma_rn(-ca, gb, X[b * n + a]);
@@ -333,152 +367,212 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   // every lane takes part in the shuffles
   const bool xany = kSm && __any_sync(FULL, xout != nullptr);
   if (!use_sm) {
+  if (ecache) {
+    // the cached elements (four loads in flight a lane)
+    int j = small_div(gl, n), i = gl - j * n;
+    const int dj = small_div(W, n), di = W - dj * n;
+#pragma unroll 1
+    for (int k0 = gl; k0 < nn; k0 += 4 * W) {
+      double v[4];
+      unsigned have = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (k0 + q * W < nn && !(((cols >> j) | (rows_new >> i)) & 1u)) {
+          v[q] = ecache[k0 + q * W];
+          have |= 1u << q;
+        }
+        i += di;
+        j += dj;
+        if (i >= n) {
+          i -= n;
+          ++j;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if ((have >> q) & 1u) A[k0 + q * W] = scale * v[q];
+    }
+  }
+#pragma unroll 1
+  for (int k = gl; k < nn; k += W) X[k] = 0.0;
+  if (gl < n) order[gl] = gl;
+  __syncwarp();
   if (xany) {
+#pragma unroll 1
     for (int k = gl; k < nn; k += W) amax = fmax(amax, fabs(A[k]));
 #pragma unroll
     for (int o = W / 2; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(FULL, amax, o, W));
   }
-  // --- LU with partial pivoting (the pivot is the first largest |a|)
-  unsigned pivbits = 0;  // bit j set: row j was interchanged
-  int piv_lane = gl;     // piv[gl] for gl < n
+  // --- LU with partial pivoting (the pivot is the first largest |a|), the identity's
+  // columns beside the matrix: X holds one column per position, in the order in
+  // which the row interchanges bring the rows up, so that step j works on the n
+  // consecutive columns j + 1 .. j + n of [A | X].
+  unsigned pivbits = 0;  // parity of the interchanges
+#pragma unroll 1
   for (int j = 0; j < n; ++j) {
-    // |a| compared through its bit pattern (monotonic for non-negative
-    // doubles), so the search runs on the integer pipe; -1 marks idle lanes
-    long long av = (gl >= j && gl < n)
-                       ? (__double_as_longlong(A[j * n + gl]) & 0x7fffffffffffffffLL)
-                       : -1LL;
-    int ai = gl;
+    // the largest |a| on the integer pipe: bit patterns of non-negative doubles are
+    // ordered like them.  First the upper 26 bits with the row below them (the
+    // smallest row wins a tie); where two rows share those, the whole patterns.
+    const bool live = gl >= j && gl < n;
+    const double aj = live ? A[j * n + gl] : 0.0;
+    const unsigned mine =
+        live ? (((unsigned)__double2hiint(aj) << 1) & ~63u) | (unsigned)(32 - gl) : 0u;
+    unsigned key = mine;
 #pragma unroll
-    for (int o = W / 2; o > 0; o >>= 1) {
-      const long long ov = __shfl_down_sync(FULL, av, o, W);
-      const int oi = __shfl_down_sync(FULL, ai, o, W);
-      if (ov > av || (ov == av && oi < ai)) {
-        av = ov;
-        ai = oi;
+    for (int o = W / 2; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(FULL, key, o, W));
+    int p = 32 - (int)(key & 63u);
+    if (__any_sync(FULL, live && gl != p && ((mine ^ key) >> 6) == 0)) {
+      long long av = live ? (__double_as_longlong(aj) & 0x7fffffffffffffffLL) : -1LL;
+      p = gl;
+#pragma unroll
+      for (int o = W / 2; o > 0; o >>= 1) {
+        const long long ov = __shfl_xor_sync(FULL, av, o, W);
+        const int oi = __shfl_xor_sync(FULL, p, o, W);
+        if (ov > av || (ov == av && oi < p)) {
+          av = ov;
+          p = oi;
+        }
       }
     }
-    const int p = __shfl_sync(FULL, ai, 0, W);
-    if (gl == j) piv_lane = p;
     const double apj = A[j * n + p];
-    if (__double_as_longlong(apj) & 0x7fffffffffffffffLL) {  // apj != 0, on the integer pipe
+    const bool regular = (__double_as_longlong(apj) & 0x7fffffffffffffffLL) != 0;  // apj != 0
+    __syncwarp();  // (every lane has it: the interchange moves it)
+    if (regular) {
+      // (the reciprocal starts on its way beside the interchange)
+      const double rinv = __drcp_rn(apj);  // 1 / a, correctly rounded
       if (p != j) {
-        pivbits |= 1u << j;
-        for (int k = gl; k < n; k += W) {
-          const double t = A[k * n + j];
-          A[k * n + j] = A[k * n + p];
-          A[k * n + p] = t;
+        pivbits ^= 1u;
+        if (gl < n) {  // rows j and p of columns j .. j + n - 1
+          double* col = A + (j + gl) * n;
+          const double t = col[j];
+          col[j] = col[p];
+          col[p] = t;
         }
+      }
+      if (gl == 0) {
+        const int t = order[j];
+        order[j] = order[p];
+        order[p] = t;
+        X[j * n + j] = 1.0;
+        R[j] = rinv;
       }
       __syncwarp();
-      const double rinv = __drcp_rn(A[j * n + j]);  // 1 / a, correctly rounded
-      if (gl == j) R[j] = rinv;
       if (gl > j && gl < n) A[j * n + gl] *= rinv;
-    } else if (info == 0) {
-      info = j + 1;
+    } else {
+      if (info == 0) info = j + 1;
+      __syncwarp();
     }
     __syncwarp();
-    // trailing update, one element per lane and step: a(i,k) -= l(i,j) u(j,k)
-    const int m = n - j - 1;
+    // elimination, one element per lane and step, the operands of two steps loaded at
+    // a time: a(i,k) -= l(i,j) u(j,k).  Each element takes the same FMAs in the same
+    // order as a factorisation and a solve per column.
+    const int m = n - j - 1, cnt = full ? m * n : m * m;
     if (m > 0) {
-      int kk = gl / m, ii = gl - kk * m;
-      const int dk = W / m, di = W - dk * m;
-      for (int e = gl; e < m * m; e += W) {
-        const int row = j + 1 + ii, col = j + 1 + kk;
-        A[col * n + row] -= A[j * n + row] * A[col * n + j];
+      const double* l = A + j * n + j + 1;
+      double* c0 = A + (j + 1) * n + j;  // row j of the first column
+      const int dk = small_div(W, m), di = W - dk * m, step = dk * n + di;
+      int k0 = small_div(gl, m), ii = gl - k0 * m, at = k0 * n + ii;
+#pragma unroll 1
+      for (int e = gl; e < cnt; e += 2 * W) {
+        const bool two = e + W < cnt;
+        const int i0 = ii, a0 = at;
         ii += di;
-        kk += dk;
+        at += step;
         if (ii >= m) {
           ii -= m;
-          ++kk;
+          at += n - m;
+        }
+        const double l0 = l[i0], u0 = c0[a0 - i0], x0 = c0[a0 + 1];
+        if (two) {
+          const double l1 = l[ii], u1 = c0[at - ii], x1 = c0[at + 1];
+          c0[at + 1] = __fma_rn(-l1, u1, x1);
+        }
+        c0[a0 + 1] = __fma_rn(-l0, u0, x0);
+        ii += di;
+        at += step;
+        if (ii >= m) {
+          ii -= m;
+          at += n - m;
         }
       }
     }
     __syncwarp();
   }
-  // --- determinant (sequential product, as the reference)
+  // --- determinant (sequential product, as the reference; the interchanges' signs
+  // are exact wherever they come in)
   double det = 1.0;
-  for (int i = 0; i < n; ++i) {
-    det *= A[i * n + i];
-    // times -1 for an interchanged row: a sign flip, exactly that product
-    if ((pivbits >> i) & 1u) det = __longlong_as_double(__double_as_longlong(det) ^ (1LL << 63));
-  }
+#pragma unroll 4
+  for (int i = 0; i < n; ++i) det = __dmul_rn(det, A[i * n + i]);
+  if (pivbits) det = __longlong_as_double(__double_as_longlong(det) ^ (long long)0x8000000000000000ULL);
   if (write) {
     det_out = det;
     err_out = info != 0;
   }
   if (!full) return;  // the same for every group of the warp
-  // --- inverse: lane c solves A x = e_c
-  int pos = gl;  // e_c after the row interchanges (every lane takes part in the shuffles)
-  for (int j = 0; j < n; ++j) {
-    const int pj = __shfl_sync(FULL, piv_lane, j, W);
-    if (pos == j)
-      pos = pj;
-    else if (pos == pj)
-      pos = j;
-  }
-  // Column c of X starts as e_pos(c); the substitutions then run one element
-  // (column, row) per lane and step.  Every element receives the same FMAs in
-  // the same order as a per-column solve, so the result is that solve's, bit
-  // for bit: the forward steps before pos(c) would only subtract exact zeros
-  // from zeros, and are skipped.
-  const bool inv_ok = info == 0;
-  if (inv_ok && gl < n)
-    for (int i = 0; i < n; ++i) X[gl * n + i] = (i == pos) ? 1.0 : 0.0;
-  int ordc = 0;  // the column whose unit vector sits at row gl
-  for (int c = 0; c < n; ++c)
-    if (__shfl_sync(FULL, pos, c, W) == gl) ordc = c;
-  __syncwarp();
-  for (int j = 0; j < n - 1; ++j) {  // forward: x(i) -= l(i,j) x(j), i > j
-    // the columns nonzero at row j: order[q] for q <= j, rows j+1 .. n-1
-    const int m = n - j - 1, cnt = (j + 1) * m;
-    int q = gl / m, ii = gl - q * m;  // element e = gl + k W: (q, row j + 1 + ii)
-    const int dq = W / m, di = W - dq * m;
-    for (int e0 = 0; e0 < cnt; e0 += W) {
-      const bool on = e0 + gl < cnt;
-      const int c = __shfl_sync(FULL, ordc, on ? q : 0, W);
-      if (inv_ok && on) {
-        const int i = j + 1 + ii;
-        X[c * n + i] -= A[j * n + i] * X[c * n + j];
-      }
-      ii += di;
-      q += dq;
-      if (ii >= m) {
-        ii -= m;
-        ++q;
-      }
-    }
-    __syncwarp();
-  }
+#pragma unroll 1
   for (int j = n - 1; j >= 0; --j) {  // back: x(j) *= 1/u(j,j); x(i) -= u(i,j) x(j), i < j
-    if (inv_ok)
-      for (int c = gl; c < n; c += W) X[c * n + j] *= R[j];
+    const double rj = R[j];
+    if (gl < n) X[gl * n + j] *= rj;
     __syncwarp();
-    if (inv_ok && j > 0) {
-      int c = gl / j, ii = gl - c * j;
-      const int dc = W / j, di = W - dc * j;
-      for (int e = gl; e < n * j; e += W) {
-        X[c * n + ii] -= A[j * n + ii] * X[c * n + j];
+    if (j > 0) {
+      const int dc = small_div(W, j), di = W - dc * j, step = dc * n + di, cnt = n * j;
+      int c0 = small_div(gl, j), ii = gl - c0 * j, at = c0 * n + ii;
+      const double* u = A + j * n;
+#pragma unroll 1
+      for (int e = gl; e < cnt; e += 2 * W) {
+        const bool two = e + W < cnt;
+        const int i0 = ii, a0 = at;
         ii += di;
-        c += dc;
+        at += step;
         if (ii >= j) {
           ii -= j;
-          ++c;
+          at += n - j;
+        }
+        const double u0 = u[i0], t0 = X[a0 - i0 + j], x0 = X[a0];
+        if (two) {
+          const double u1 = u[ii], t1 = X[at - ii + j], x1 = X[at];
+          X[at] = __fma_rn(-u1, t1, x1);
+        }
+        X[a0] = __fma_rn(-u0, t0, x0);
+        ii += di;
+        at += step;
+        if (ii >= j) {
+          ii -= j;
+          at += n - j;
         }
       }
     }
     __syncwarp();
   }
+  // X's columns are solutions for the unit vectors order[0], order[1], ...: turned
+  // into the position of each (SHONodes, whose weights follow it), or sorted
+  // through A (free-particle nodes, which read the inverse more than once)
+  if constexpr (kSho) {
+    const int o = gl < n ? order[gl] : 0;
+    __syncwarp();
+    if (gl < n) order[o] = gl;
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < n; ++c)
+      if (gl < n) A[order[c] * n + gl] = X[c * n + gl];
+    __syncwarp();
+#pragma unroll 1
+    for (int k = gl; k < nn; k += W) X[k] = A[k];
+  }
+  __syncwarp();
   }  // factorisation
   // the inverse and its update count for the cache (mixed form); a fresh
   // factorisation that is too ill-conditioned is marked as used up
   if (xany) {
     double xmax = 0.0;
     if (!use_sm) {
+#pragma unroll 1
       for (int k = gl; k < nn; k += W) xmax = fmax(xmax, fabs(X[k]));
 #pragma unroll
       for (int o = W / 2; o > 0; o >>= 1) xmax = fmax(xmax, __shfl_xor_sync(FULL, xmax, o, W));
     }
     if (write && xout) {
+#pragma unroll 1
       for (int k = gl; k < nn; k += W) xout[2 + k] = X[k];
       if (gl == 0) {
         xout[0] = info == 0 ? xepoch : __longlong_as_double(0x7ff8000000000000LL);
@@ -492,93 +586,149 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   // exit: a singular group simply skips them, so the warp stays converged.)
   const double dk = s.node_dk[sp];
   const bool ok = info == 0;
-  if (sho) {
+  if constexpr (kSho) {
     // weights w(i,j) = inv(j,i) rho(i,j), shared by both gradients
     if (ok) {
-      int j = gl / n, i = gl - j * n;
-      const int dj = W / n, di = W - dj * n;
-      for (int e = gl; e < n * n; e += W) {
-        A[j * n + i] = X[i * n + j] * E[j * n + i];
-        i += di;
-        j += dj;
-        if (i >= n) {
-          i -= n;
-          ++j;
+      int j = small_div(gl, n), i = gl - j * n;
+      const int dj = small_div(W, n), di = W - dj * n;
+#pragma unroll 1
+      for (int e0 = gl; e0 < nn; e0 += 4 * W) {  // (four loads in flight a lane)
+        double v[4], x[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (e0 + q * W < nn) {
+            v[q] = elem(0, i, j, e0 + q * W);
+            x[q] = X[order[i] * n + j];
+          }
+          i += di;
+          j += dj;
+          if (i >= n) {
+            i -= n;
+            ++j;
+          }
         }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (e0 + q * W < nn) A[e0 + q * W] = __dmul_rn(x[q], v[q]);
       }
     }
     __syncwarp();
+    // d1: sum_i w(i,j) 2c (r2_i - ch r1_j), d2: sum_j w(i,j) 2c (r1_j - ch r2_i): with S the
+    // sum of w r and T that of w, S - ch r T
     const double c = s.node_c[sp], ch = s.node_cosh[sp];
     const double fac = 2 * c * scale;
-    // sum_i w(i,j) (r2_i - ch r1_j) = S - ch r1_j T with S = sum_i w(i,j) r2_i and
-    // T = sum_i w(i,j): four FP64 operations a term instead of six
-    if (ok && gl < n) {
-      const int j = gl;  // d1: sum_i w(i,j) 2c (r2_i - ch r1_j)
-      double rjx, rjy, rjz;
-      v1.get(f + j, rjx, rjy, rjz);
-      double sx = 0, sy = 0, sz = 0, tw = 0;
-      for (int i = 0; i < n; ++i) {
-        double rix, riy, riz;
-        v2.get(f + i, rix, riy, riz);
-        const double w = A[j * n + i];
-        sx += w * rix;
-        sy += w * riy;
-        sz += w * riz;
-        tw += w;
+    if (ok)
+#pragma unroll 1
+      for (int q = gl; q < 2 * n; q += W) {
+        const bool first = q < n;
+        const int p = first ? q : q - n;
+        const SliceView& v = first ? v2 : v1;
+        const int at = v.t * v.npart + f, im = v.imov - f;
+        const double* w = A + (first ? p * n : p);
+        const int dw = first ? 1 : n;
+        double sx = 0, sy = 0, sz = 0, tw = 0;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+          const double wk = w[k * dw];
+          sx = __fma_rn(wk, k == im ? v.mxv : v.sx[at + k], sx);
+          sy = __fma_rn(wk, k == im ? v.myv : v.sy[at + k], sy);
+          sz = __fma_rn(wk, k == im ? v.mzv : v.sz[at + k], sz);
+          tw = __dadd_rn(tw, wk);
+        }
+        double rx, ry, rz;
+        (first ? v1 : v2).get(f + p, rx, ry, rz);
+        const double ct = __dmul_rn(ch, tw);
+        const double lx = __dmul_rn(fac, __fma_rn(-ct, rx, sx));
+        const double ly = __dmul_rn(fac, __fma_rn(-ct, ry, sy));
+        const double lz = __dmul_rn(fac, __fma_rn(-ct, rz, sz));
+        const double d = __dmul_rn(dk, rsqrt(__dadd_rn(dot3(lx, ly, lz, lx, ly, lz), 1e-15)));
+        if (write) (first ? d1 : d2)[p] = d;
       }
-      const double ct = ch * tw;
-      const double lx = fac * (sx - ct * rjx), ly = fac * (sy - ct * rjy), lz = fac * (sz - ct * rjz);
-      if (write) d1[j] = dk * rsqrt(dot3(lx, ly, lz, lx, ly, lz) + 1e-15);
-    }
-    if (ok && gl < n) {
-      const int i = gl;  // d2: sum_j w(i,j) 2c (r1_j - ch r2_i)
-      double rix, riy, riz;
-      v2.get(f + i, rix, riy, riz);
-      double sx = 0, sy = 0, sz = 0, tw = 0;
-      for (int j = 0; j < n; ++j) {
-        double rjx, rjy, rjz;
-        v1.get(f + j, rjx, rjy, rjz);
-        const double w = A[j * n + i];
-        sx += w * rjx;
-        sy += w * rjy;
-        sz += w * rjz;
-        tw += w;
-      }
-      const double ct = ch * tw;
-      const double lx = fac * (sx - ct * rix), ly = fac * (sy - ct * riy), lz = fac * (sz - ct * riz);
-      if (write) d2[i] = dk * rsqrt(dot3(lx, ly, lz, lx, ly, lz) + 1e-15);
-    }
   } else {
-    const double* Gx = G;
-    const double* Gy = G + n * n;
-    const double* Gz = G + 2 * n * n;
-    if (ok && gl < n) {
-      const int j = gl;  // d1: sum_i inv(j,i) dA(i,j)/dr1_j
-      double lx = 0, ly = 0, lz = 0;
-      for (int i = 0; i < n; ++i) {
-        const double w = X[i * n + j];
-        lx += w * Gx[j * n + i];
-        ly += w * Gy[j * n + i];
-        lz += w * Gz[j * n + i];
+    // The gradient matrices pass once through A (spent) in tiles of n/3 columns, read
+    // coalesced: lane i adds its row for d2 (sum_j inv(j,i) dA(i,j)/dr2_i, with
+    // dA/dr2_i = -dA/dr1_j), and lanes (component, j) the tile's columns for d1 (sum_i
+    // inv(j,i) dA(i,j)/dr1_j), each kept by its lane until all tiles are done.
+    double l2[3] = {0, 0, 0}, lx = 0, ly = 0, lz = 0;
+    if (n < 3) {  // (no room for a tile: straight from the elements)
+      if (gl < n)
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) {
+          const double w1 = X[k * n + gl], w2 = X[gl * n + k];
+          lx = __fma_rn(w1, elem(1, k, gl, gl * n + k), lx);
+          ly = __fma_rn(w1, elem(2, k, gl, gl * n + k), ly);
+          lz = __fma_rn(w1, elem(3, k, gl, gl * n + k), lz);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) l2[c] = __fma_rn(w2, elem(1 + c, gl, k, k * n + gl), l2[c]);
+        }
+    } else {
+      const int tw = small_div(n, 3), nt = small_div(n + tw - 1, tw);  // 3 to 5 tiles of 3 tw <= W rows
+      double l1[5] = {0, 0, 0, 0, 0};
+#pragma unroll 1
+      for (int t = 0; t < nt; ++t) {
+        const int j0 = t * tw, wd = min(tw, n - j0);
+        __syncwarp();
+        // row r = component * wd + column of the tile, element i on lane i; four rows'
+        // loads in flight
+        const int i = min(gl, n - 1);
+#pragma unroll 1
+        for (int r0 = 0; r0 < 3 * wd; r0 += 4) {
+          double v[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int r = min(r0 + q, 3 * wd - 1), c = 1 + (r >= wd) + (r >= 2 * wd);
+            const int j = j0 + r - (c - 1) * wd;
+            const double* from = (ecache ? ecache : E) + c * nn + j * n;
+            if (cols && (((cols >> j) | (rows_new >> i)) & 1u))
+              from = newcol ? newcol + c * n : E + c * nn + j * n;
+            v[q] = from[i];
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (r0 + q < 3 * wd && gl < n) A[(r0 + q) * n + gl] = v[q];
+        }
+        __syncwarp();
+        if (gl < n)
+#pragma unroll 1
+          for (int jj = 0; jj < wd; ++jj) {
+            const double w = X[gl * n + j0 + jj];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) l2[c] = __fma_rn(w, A[(c * wd + jj) * n + gl], l2[c]);
+          }
+        if (gl < 3 * wd) {
+          const int j = j0 + gl - (gl >= wd) * wd - (gl >= 2 * wd) * wd;
+          double sum = 0.0;
+#pragma unroll 1
+          for (int k = 0; k < n; ++k) sum = __fma_rn(X[k * n + j], A[gl * n + k], sum);
+#pragma unroll
+          for (int q = 0; q < 5; ++q)
+            if (q == t) l1[q] = sum;
+        }
       }
-      lx *= scale;
-      ly *= scale;
-      lz *= scale;
-      if (write) d1[j] = dk * rsqrt(dot3(lx, ly, lz, lx, ly, lz) + 1e-15);
+      // lane j takes its column's three sums from the lanes that hold them
+      const int mine = min(gl, n - 1), mt = small_div(mine, tw), jj = mine - mt * tw;
+#pragma unroll
+      for (int t = 0; t < 5; ++t) {
+        const int wd = max(1, min(tw, n - t * tw));
+        const double a = __shfl_sync(FULL, l1[t], min(jj, W - 1), W);
+        const double b = __shfl_sync(FULL, l1[t], min(wd + jj, W - 1), W);
+        const double c = __shfl_sync(FULL, l1[t], min(2 * wd + jj, W - 1), W);
+        if (t == mt) {
+          lx = a;
+          ly = b;
+          lz = c;
+        }
+      }
     }
     if (ok && gl < n) {
-      const int i = gl;  // d2: sum_j inv(j,i) dA(i,j)/dr2_i, dA/dr2_i = -dA/dr1_j
-      double lx = 0, ly = 0, lz = 0;
-      for (int j = 0; j < n; ++j) {
-        const double w = X[i * n + j];
-        lx += w * Gx[j * n + i];
-        ly += w * Gy[j * n + i];
-        lz += w * Gz[j * n + i];
-      }
       lx *= scale;
       ly *= scale;
       lz *= scale;
-      if (write) d2[i] = dk * rsqrt(dot3(lx, ly, lz, lx, ly, lz) + 1e-15);
+      if (write) d1[gl] = dk * rsqrt(dot3(lx, ly, lz, lx, ly, lz) + 1e-15);
+      lx = l2[0] * scale;
+      ly = l2[1] * scale;
+      lz = l2[2] * scale;
+      if (write) d2[gl] = dk * rsqrt(dot3(lx, ly, lz, lx, ly, lz) + 1e-15);
     }
   }
   __syncwarp();
@@ -594,8 +744,12 @@ __host__ __device__ __forceinline__ int node_group_width(int n) {
 static __device__ void node_eval_warp(const DevSys& s, int sp, const SliceView& v1, const SliceView& v2,
                                double scale, double* scr, int full, double& det_out,
                                int& err_out, double* d1, double* d2) {
-  node_eval_group<32>(s, sp, v1, v2, scale, scr, full, nullptr, 0u, true, det_out, err_out, d1,
-                      d2);
+  if (s.node_kind[sp] == 1)
+    node_eval_group<32, true>(s, sp, v1, v2, scale, scr, full, nullptr, 0u, true, det_out, err_out,
+                              d1, d2);
+  else
+    node_eval_group<32, false>(s, sp, v1, v2, scale, scr, full, nullptr, 0u, true, det_out,
+                               err_out, d1, d2);
 }
 
 __device__ __forceinline__ int species_of(const DevSys& s, int p) {
