@@ -48,6 +48,7 @@ struct SepF {
 __device__ __forceinline__ int pair_partners(const DevSys& s, int ipart) {
   int n = 0;
   if (s.coulomb)
+#pragma unroll 1
     for (int k = 0; k < s.ntab; ++k) {
       const DevTable& t = s.tab[k];
       if (ipart >= t.ifirst1 && ipart < t.ifirst1 + t.npart1)
@@ -59,6 +60,7 @@ __device__ __forceinline__ int pair_partners(const DevSys& s, int ipart) {
 }
 __device__ __forceinline__ int pair_partner(const DevSys& s, int ipart, int p, int& ti) {
   ti = 0;
+#pragma unroll 1
   for (int k = 0; k < s.ntab; ++k) {
     const DevTable& t = s.tab[k];
     int first, n;
@@ -217,10 +219,12 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
   const int total = pair_partners(s, ipart);
   const int P = nl < 32 ? 32 / nl : 1;  // partners a warp takes at once
   S* sep = (S*)buf;
+#pragma unroll 1
   for (int pc = w; pc * P < total; pc += nw) {
     __syncwarp();
     // the partners' separations: entry i <= mid the old path at slice i << sh, entry
     // mid + i the new bead there (the end slices do not move)
+#pragma unroll 1
     for (int e = lane; e < P * nI; e += 32) {
       const int g = e >> (dmax + 1), i = e & (nI - 1);
       int ti;
@@ -242,6 +246,7 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
       }
     }
     __syncwarp();
+#pragma unroll 1
     for (int it = 0; it * 32 < P * nl; ++it) {
       const int li = it * 32 + lane, g = nl < 32 ? li / nl : 0, slot = base + li - g * nl;
       int ti;
@@ -256,14 +261,20 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
       const S& b0 = sg[i0];
       const S& n1 = sg[i1 == mid ? i1 : mid + i1];
       const S& n0 = sg[i0 == 0 ? 0 : mid + i0];
-      const auto vn = pair_term(t, n1, n0, offdiag, 1 << (L - d));
-      const auto vo = pair_term(t, b1, b0, offdiag, 1 << (L - d));
-      add(P > 1 ? 0 : it, vn - vo);
+      decltype(pair_term(t, n1, n0, offdiag, 1)) v[2];
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {  // (one copy of the lookup's code)
+        const auto x = pair_term(t, pass ? b1 : n1, pass ? b0 : n0, offdiag, 1 << (L - d));
+        v[1] = pass ? x : v[1];
+        v[0] = pass ? v[0] : x;
+      }
+      add(P > 1 ? 0 : it, v[0] - v[1]);
     }
   }
   // the links' own terms, on the warp after the last one with a partner
   if (w == ((total + P - 1) / P) % nw) {
     const int sp = species_of(s, ipart);
+#pragma unroll 1
     for (int it = 0; it * 32 < nl; ++it) {
       const int li = it * 32 + lane, slot = base + li;
       if (li >= nl || slot == 0) continue;
@@ -282,8 +293,10 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
 // depth: lane 2^d holds depth d's sum.  Five shuffles for all depths.
 __device__ __forceinline__ double fold_by_depth(double x, int nI) {
   const int lane = threadIdx.x & 31;
+#pragma unroll 1
   for (int o = 16; o >= nI; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   const int slot = lane & (nI - 1);
+#pragma unroll 1
   for (int o = nI / 4; o > 0; o >>= 1) {
     const double y = __shfl_xor_sync(0xffffffffu, x, o);
     if (slot >= 2 * o) x += y;
@@ -291,6 +304,7 @@ __device__ __forceinline__ double fold_by_depth(double x, int nI) {
   return x;
 }
 __device__ __forceinline__ double fold_warp(double x) {
+#pragma unroll 1
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
@@ -301,8 +315,10 @@ __device__ __forceinline__ void action_reduce(const DevSys& s, const double* buf
                                               int dmin, int dmax, int nw, double* lds) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int chunks = (dmin || dmax < 5) ? 1 : dmax - 3;
+#pragma unroll 1
   for (int c = warp; c < chunks; c += nwarps) {
     double x = 0.0;
+#pragma unroll 1
     for (int w = 0; w < nw; ++w) x += buf0[(size_t)w * stride + 32 * c + lane];
     if (dmin || c > 0) {
       x = fold_warp(x);

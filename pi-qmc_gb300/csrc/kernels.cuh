@@ -123,18 +123,18 @@ static __device__ __noinline__ double ewald_level0_cached(const DevSys& s, const
   double2* Z = Y + ny * w;
   const double q = m.qpart[ipart], is = 1.0 / s.ek_scale;
   double acc = 0.0;
+#pragma unroll 1
   for (int t0 = 1; t0 < nsec - 1; t0 += chunk) {
     const int nt = min(chunk, nsec - 1 - t0);
     __syncthreads();
+#pragma unroll 1
     for (int c = threadIdx.x; c < 2 * nt; c += blockDim.x) {
-      const int t = t0 + (c >> 1);
-      if (c & 1)
-        ewald_bead_tables(s, X, Y, Z, w, c, m.mx[t], m.my[t], m.mz[t]);
-      else
-        ewald_bead_tables(s, X, Y, Z, w, c, m.s1x[t * np + ipart], m.s1y[t * np + ipart],
-                          m.s1z[t * np + ipart]);
+      const int t = t0 + (c >> 1), o = t * np + ipart;
+      ewald_bead_tables(s, X, Y, Z, w, c, c & 1 ? m.mx[t] : m.s1x[o], c & 1 ? m.my[t] : m.s1y[o],
+                        c & 1 ? m.mz[t] : m.s1z[o]);
     }
     __syncthreads();
+#pragma unroll 1
     for (int it = threadIdx.x; it < nt * totk; it += blockDim.x) {
       const int tt = it / totk, k = it - tt * totk, t = t0 + tt;
       const int kx = __ldg(s.kvec + 3 * k), ky = __ldg(s.kvec + 3 * k + 1) + ky0,
@@ -158,13 +158,27 @@ static __device__ __noinline__ double ewald_level0_cached(const DevSys& s, const
 static __device__ __noinline__ void load_section(const DevSys& s, const double* path, int ifirst, double* sx,
                              double* sy, double* sz) {
   const int np = s.npart, n = s.nsec * np;
-  for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
-    const int k = idx / np, p = idx - k * np;
-    const int t = wrap_slice(ifirst + k, s.nslice);
-    const double* src = path + ((size_t)t * np + p) * 3;
-    sx[idx] = src[0];
-    sy[idx] = src[1];
-    sz[idx] = src[2];
+#pragma unroll 1
+  for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {  // (four beads' loads in flight)
+    double x[4], y[4], z[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = min(i0 + q * (int)blockDim.x, n - 1);
+      const int k = idx / np, p = idx - k * np;
+      const double* src = path + ((size_t)wrap_slice(ifirst + k, s.nslice) * np + p) * 3;
+      x[q] = src[0];
+      y[q] = src[1];
+      z[q] = src[2];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = i0 + q * blockDim.x;
+      if (idx < n) {
+        sx[idx] = x[q];
+        sy[idx] = y[q];
+        sz[idx] = z[q];
+      }
+    }
   }
 }
 
@@ -172,6 +186,7 @@ static __device__ __noinline__ void load_section(const DevSys& s, const double* 
 static __device__ __noinline__ void store_section(const DevSys& s, double* path, int ifirst, const double* sx,
                               const double* sy, const double* sz) {
   const int np = s.npart, n = s.nsec * np;
+#pragma unroll 1
   for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
     const int k = idx / np, p = idx - k * np;
     const int islice = ifirst + k;
@@ -195,6 +210,7 @@ static __device__ __noinline__ void attempt_normals(const DevSys& s, const Smem&
   // (with delayed rejection one more: the second proposal at level nlevel - 1
   // takes order 1, the slices after it one order later)
   const int nord = (1 << s.nlevel) - 1 + (s.dr ? 1 : 0), pad = (nord + 31) & ~31;
+#pragma unroll 1
   for (int it = threadIdx.x; it < 2 * pad; it += blockDim.x) {
     const int second = it >= pad, o = it - second * pad;
     if (o >= nord) continue;
@@ -214,6 +230,7 @@ static __device__ __noinline__ void attempt_normals(const DevSys& s, const Smem&
 __device__ __forceinline__ uint32_t level_uniform_base(const DevSys& s, int level) {
   uint32_t u = (s.fixed_node ? 2u : 1u) + 1u;  // section choice + particle choice
   const uint32_t pbcu = s.mover == PIMC_MOVER_FREE_PBC ? 3u : 0u;
+#pragma unroll 1
   for (int l = s.nlevel; l > level; --l) {
     const uint32_t nmov = (l == s.nlevel) ? 0u : (1u << (s.nlevel - l - 1));
     u += pbcu * nmov + 1u;
@@ -227,7 +244,7 @@ __device__ __forceinline__ uint32_t level_uniform_base(const DevSys& s, int leve
 // > 40 on every axis w2 is below 2^-57 w1, w1 / (w1 + w2) rounds to 1 (or is 0/0)
 // and no uniform exceeds it: the exponentials and uniforms are left out.  That is
 // every choice in a box much wider than the level's sigma.
-__device__ __forceinline__ void mover_image(const DevSys& s, double md[3], double inv2Sigma2,
+static __device__ __noinline__ void mover_image(const DevSys& s, double md[3], double inv2Sigma2,
                                             uint64_t seed, uint32_t rep, uint32_t att,
                                             uint32_t u0) {
   const float w = (float)inv2Sigma2;
@@ -266,6 +283,7 @@ __device__ __forceinline__ void moved_slice(int L, int slot, int& level, int& t,
 // The old beads' part of ln(T_old / T_new), per moved slice into m.old.  One warp.
 static __device__ __noinline__ void mover_old(const DevSys& s, const Smem& m, int ipart) {
   const int np = s.npart, sp = species_of(s, ipart);
+#pragma unroll 1
   for (int slot = threadIdx.x & 31; slot < (1 << s.nlevel); slot += 32) {
     if (slot == 0) continue;
     int level, t, k;
@@ -310,6 +328,7 @@ static __device__ __noinline__ void mover_all(const DevSys& s, const Smem& m, in
                                               uint64_t seed, uint32_t att, double* llt) {
   const int L = s.nlevel, lane = threadIdx.x & 31, sp = species_of(s, ipart);
   if (lane == 0) llt[L] = 0.0;  // the top level moves nothing
+#pragma unroll 1
   for (int c = 0; 32 * c < (1 << L); ++c) {
     const int slot = 32 * c + lane;
     const bool on = slot > 0 && slot < (1 << L);
@@ -326,6 +345,7 @@ static __device__ __noinline__ void mover_all(const DevSys& s, const Smem& m, in
       acc += dx * dx * inv2Sigma2;
       acc += dy * dy * inv2Sigma2;
       acc += dz * dz * inv2Sigma2;
+#pragma unroll 1
       for (int d = dlo; d <= dhi; ++d) {
         if (on && level == L - 1 - d) {
           const double mpx = m.mx[tp], mpy = m.my[tp], mpz = m.mz[tp];
@@ -346,6 +366,7 @@ static __device__ __noinline__ void mover_all(const DevSys& s, const Smem& m, in
         __syncwarp();
       }
     } else {
+#pragma unroll 1
       for (int d = dlo; d <= dhi; ++d) {
         if (on && level == L - 1 - d) {
           const double mpx = m.mx[tp], mpy = m.my[tp], mpz = m.mz[tp];
@@ -408,6 +429,7 @@ static __device__ __noinline__ double mover_level_part(const DevSys& s, const Sm
   const double sigma = second ? s.dr_sigma[sp] : s.mov_sigma[level][sp];
   const double inv2Sigma2 = second ? s.dr_inv2s2[sp] : s.mov_inv2s2[level][sp];
   double part = 0.0;
+#pragma unroll 1
   for (int k = threadIdx.x; k < nmov; k += blockDim.x) {
     const int t = nStride * (2 * k + 1), tp = t - nStride, tn = t + nStride;
     // the attempt's normals were drawn up front (attempt_normals)
@@ -546,27 +568,38 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   if (threadIdx.x < kMaxSpecies) nmiss[threadIdx.x] = 0;
   __syncthreads();
   const int nt = nsec - start;
+#pragma unroll 1
   for (int it = threadIdx.x; it < s.nspecies * nt; it += blockDim.x) {
     const int sp = it / nt, t = start + (it - sp * nt);
     if (!s.node_kind[sp] || (only_sp >= 0 && sp != only_sp)) continue;
-    const int n = s.spec_count[sp];
     const double* e = cache ? cache_entry(s, cache, sp, wrap_slice(ifirst1 + t, M)) : nullptr;
     if (e && e[0] == (double)epoch[sp]) {
       m.dm[sp * nsec + t] = e[1];
       errs[sp * nsec + t] = 0;
-      if (sp == msp)
-        for (int j = 0; j < n; ++j) {
-          m.dist[(t * 2) * nsm + j] = e[2 + j];
-          m.dist[(t * 2 + 1) * nsm + j] = e[2 + n + j];
-        }
     } else {
       miss[sp * nsec + atomicAdd(&nmiss[sp], 1)] = t;
+    }
+  }
+  // the moving species' distances where the entry is valid (a particle per thread:
+  // as a loop of the slice's own thread this took 8,000-21,000 clocks of load latency)
+  if (cache && msp >= 0 && s.node_kind[msp] && (only_sp < 0 || only_sp == msp)) {
+    const int n = s.spec_count[msp];
+#pragma unroll 1
+    for (int it = threadIdx.x; it < nt * n; it += blockDim.x) {
+      const int t = start + it / n, j = it - (t - start) * n;
+      const double* e = cache_entry(s, cache, msp, wrap_slice(ifirst1 + t, M));
+      const double ep = e[0], a = e[2 + j], b = e[2 + n + j];
+      if (ep == (double)epoch[msp]) {
+        m.dist[(t * 2) * nsm + j] = a;
+        m.dist[(t * 2 + 1) * nsm + j] = b;
+      }
     }
   }
   __syncthreads();
   // warp tasks: each warp takes up to G misses of one species (lane groups of
   // a warp must run the same species so that they stay converged)
   int ntask = 0, first[kMaxSpecies + 1];
+#pragma unroll 1
   for (int sp = 0; sp < s.nspecies; ++sp) {
     const int G = 32 / node_group_width(s.spec_count[sp]);
     first[sp] = ntask;
@@ -574,6 +607,7 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   }
   first[s.nspecies] = ntask;
   if (llt && warp == nwarps - 1) mover_all(s, m, ipart, seed, att, llt);
+#pragma unroll 1
   for (int wt = warp; wt < ntask; wt += nwarps) {
     int sp = 0;
     while (wt >= first[sp + 1]) ++sp;
@@ -628,6 +662,12 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
 // other; they are independent); at a species' first slice whose determinant
 // leaves [1e-50, 1e50] its loop is replayed sequentially, and its later
 // slices are re-evaluated.
+// |x| < lo or |x| > hi (both normal; never for a NaN), on the integer pipe
+__device__ __forceinline__ bool outside_magnitudes(double x, double lo, double hi) {
+  const long long a = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+  return a < __double_as_longlong(lo) || (a > __double_as_longlong(hi) && a <= 0x7ff0000000000000LL);
+}
+
 static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem& m, double* scale, int* epoch,
                                 int msp, uint32_t* status, double* cache, int ifirst1, int ipart,
                                 uint64_t seed, uint32_t att, double* llt) {
@@ -637,6 +677,7 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
   int* errs = m.ictl + C_NCTL;  // [kMaxSpecies][nsec]
   const double NaN = __longlong_as_double(0x7ff8000000000000LL);
   node_init_pass(s, m, scale, epoch, msp, cache, ifirst1, -1, 0, ipart, seed, att, llt);
+#pragma unroll 1
   for (int sp = 0; sp < s.nspecies; ++sp) {
     if (!s.node_kind[sp]) continue;
     const int n = s.spec_count[sp];
@@ -649,20 +690,17 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
     for (int round = 0; round < 64; ++round) {
       if (round > 0)
         node_init_pass(s, m, scale, epoch, msp, cache, ifirst1, sp, start, ipart, seed, att, nullptr);
-      if (threadIdx.x == 0) {
-        int k = -1;
-        for (int t = start; t < nsec; ++t) {
-          const double a = fabs(dm[t]);
-          if (er[t] || a < 1e-50 || a > 1e50) {
-            k = t;
-            break;
-          }
-        }
-        m.ictl[C_SCANK] = k;
+      // (every warp looks for itself, a slice per lane)
+      int k = -1;
+#pragma unroll 1
+      for (int t0 = start; k < 0 && t0 < nsec; t0 += 32) {
+        const int t = t0 + lane;
+        const unsigned bad = __ballot_sync(
+            0xffffffffu, t < nsec && (er[t] || outside_magnitudes(dm[t], 1e-50, 1e50)));
+        if (bad) k = t0 + __ffs(bad) - 1;
       }
-      __syncthreads();
-      const int k = m.ictl[C_SCANK];
       if (k < 0) break;
+      __syncthreads();  // (warp 0 changes what the others have read)
       if (warp == 0) {
         // pi-qmc's do-while rescale loop on slice k, by group 0 of warp 0
         // (the other groups repeat it without storing).
@@ -709,13 +747,16 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
       if (start >= nsec) break;
     }
     // crossing check, as the reference counts errors at set-up
-    if (threadIdx.x == 0) {
-      for (int t = 0; t < nsec; ++t)
-        if (er[t] || dm[t] * dm[0] <= 1e-200) *status |= PIMC_STATUS_INIT_CROSSING;
+    if (warp == 0) {
+      bool crossed = false;
+#pragma unroll 1
+      for (int t = lane; t < nsec; t += 32) crossed = crossed || er[t] || dm[t] * dm[0] <= 1e-200;
+      if (__any_sync(0xffffffffu, crossed) && lane == 0) *status |= PIMC_STATUS_INIT_CROSSING;
     }
   }
   if (msp >= 0 && s.node_kind[msp]) {
     // newDist(0) = dist(0)
+#pragma unroll 1
     for (int i = threadIdx.x; i < 2 * nsm; i += blockDim.x) m.ndist[i] = m.dist[i];
   }
   __syncthreads();
@@ -727,26 +768,26 @@ static __device__ __noinline__ double nodal_action(const DevSys& s, const Smem& 
   const int nsec = s.nsec, nsm = s.ns_max;
   double part = 0.0;
   FSum fpart;
+#pragma unroll 1
   for (int it = threadIdx.x; it < (nsec - 1) * n; it += blockDim.x) {
-    const int t = 1 + it / n, p = it % n;
-    const double* D0 = m.dist + (t * 2) * nsm;
-    const double* Dp0 = m.dist + ((t - 1) * 2) * nsm;
-    const double* N0 = m.ndist + (t * 2) * nsm;
-    const double* Np0 = m.ndist + ((t - 1) * 2) * nsm;
-    if (s.mixed) {
-      // FP32 terms (1 - e^-x through expm1 keeps them accurate near the node),
-      // their sum compensated
-      const float a1 = -expm1f(-(float)(D0[p] * Dp0[p]));
-      const float b1 = -expm1f(-(float)(N0[p] * Np0[p]));
-      const float a2 = -expm1f(-(float)(D0[nsm + p] * Dp0[nsm + p]));
-      const float b2 = -expm1f(-(float)(N0[nsm + p] * Np0[nsm + p]));
-      fpart.add(logf(a1) - logf(b1));
-      fpart.add(logf(a2) - logf(b2));
-      continue;
+    const int t = 1 + it / n, p = it - (t - 1) * n;
+    double num = 1.0, den = 1.0;
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {  // d1, then d2
+      const double* D = m.dist + (t * 2 + side) * nsm + p;
+      const double* N = m.ndist + (t * 2 + side) * nsm + p;
+      const double d = D[0] * D[-2 * nsm], e = N[0] * N[-2 * nsm];
+      if (s.mixed) {
+        // FP32 terms (1 - e^-x through expm1 keeps them accurate near the node),
+        // their sum compensated
+        const float a = -expm1f(-f32_rn(d)), b = -expm1f(-f32_rn(e));
+        fpart.add(logf(a) - logf(b));
+      } else {  // (one logarithm for both sides)
+        num *= 1 - exp(-d);
+        den *= 1 - exp(-e);
+      }
     }
-    double a = log((1 - exp(-D0[p] * Dp0[p])) / (1 - exp(-N0[p] * Np0[p])));
-    a += log((1 - exp(-D0[nsm + p] * Dp0[nsm + p])) / (1 - exp(-N0[nsm + p] * Np0[nsm + p])));
-    part += a;
+    if (!s.mixed) part += log(num / den);
   }
   return block_sum(s.mixed ? fpart.value() : part, m.red);
 }
@@ -770,6 +811,7 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   const int top = hi == L ? L - 1 : hi;
   int ntask = 0;
   if (mynode)
+#pragma unroll 1
     for (int l = top; l >= lo; --l) ntask += (nsec - 1 - (1 << l)) / (1 << (l + 1)) + 1;
   // lane groups of the species' width, packed (32 / W matrices a warp): the
   // SM's narrow FP64 pipe, shared by every resident warp, is the limit, and a
@@ -781,6 +823,7 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
     if (hi == L) {
       // the top level's only slice is the section's fixed end: copied from the set-up
       const int t = nsec - 1;
+#pragma unroll 1
       for (int i = threadIdx.x; i < 2 * nsm; i += blockDim.x) m.ndist[t * 2 * nsm + i] = m.dist[t * 2 * nsm + i];
     }
     __syncthreads();
@@ -794,10 +837,12 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
       double* scr = group_scr(m, warp * G + g, G, n, !sho);
       double* cold = group_cold(m, warp * G + g, G, n, !sho);
       const int jcol = ipart - s.spec_first[msp];
+#pragma unroll 1
       for (int base = warp * G; base < ntask; base += nodeW * G) {
         const int task = base + g;
         const bool act = task < ntask;
         int k = act ? task : base, l = top;  // task -> (level, slice)
+#pragma unroll 1
         for (;;) {
           const int nl = (nsec - 1 - (1 << l)) / (1 << (l + 1)) + 1;
           if (k < nl || l == lo) break;
@@ -850,6 +895,7 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   double nodal = 0.0;
   if (mynode && lo == 0 && !(flags & 1)) nodal = nodal_action(s, m, n);
   if (threadIdx.x == 0)
+#pragma unroll 1
     for (int level = lo; level <= hi; ++level)
       lnd[level] = ((flags >> level) & 1) ? 2e100 : (level == 0 ? nodal : 0.0);
   __syncthreads();
@@ -893,6 +939,7 @@ static __device__ __noinline__ void delayed_rejection(const DevSys& s, const Sme
     if (ek)
       dsC += ewald_level0_cached(s, m, ipart, ifirst1, ek, ekstage);
     else
+#pragma unroll 1
       for (int k = 1; k < nsec - 1; ++k) dsC += ewald_slice_diff(s, m, ipart, k);
   }
   const double dsnC = lnd[level];
@@ -957,6 +1004,20 @@ static __device__ __noinline__ void delayed_rejection(const DevSys& s, const Sme
 // kNodes = false: the variant for launches without node models, whose code
 // leaves the fixed-node phases out (a smaller kernel: fewer instruction-fetch
 // stalls when thousands of one-warp CTAs run different phases).
+// n values by a warp, eight loads in flight a lane
+template <class T>
+__device__ __forceinline__ void copy_warp(T* dst, const T* src, int n) {
+#pragma unroll 1
+  for (int k0 = threadIdx.x & 31; k0 < n; k0 += 256) {
+    T v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = src[min(k0 + 32 * q, n - 1)];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (k0 + 32 * q < n) dst[k0 + 32 * q] = v[q];
+  }
+}
+
 template <int NT, int MINB, bool kNodes = true>
 __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
   extern __shared__ double smem[];
@@ -971,6 +1032,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
   __shared__ Smem M_;
   // Persistent CTAs take replicas from a queue ordered longest-first, so that
   // uneven replicas (different N, M, L) balance across the SMs.
+#pragma unroll 1
   for (;;) {
     if (threadIdx.x == 0) {
       const int k = atomicAdd(P.next, 1);
@@ -982,6 +1044,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
     {
       const int* src = (const int*)(P.sys + r);
       int* dst = (int*)&S;
+#pragma unroll 1
       for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x)
         dst[i] = src[i];
     }
@@ -990,6 +1053,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
                  P.xstage ? P.xstage + (size_t)blockIdx.x * P.xstage_cta : nullptr);
       status = P.state[r].status;
       nacc = 0;
+#pragma unroll 1
       for (int k = 0; k < kMaxSpecies; ++k) {
         scale[k] = P.state[r].node_scale[k];
         epoch[k] = P.state[r].epoch[k];
@@ -1005,15 +1069,18 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
     long long* ekstage = ek ? P.ekstage + (size_t)blockIdx.x * P.ekstage_stride : nullptr;
     const int np = s.npart, nsec = s.nsec, M = s.nslice, L = s.nlevel;
     const bool fixed = kNodes && s.fixed_node;
+#pragma unroll 1
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
     const int nat = P.nattempt_r ? P.nattempt_r[r] : P.nattempt;
+#pragma unroll 1
     for (int a = 0; a < nat; ++a) {
       const uint32_t att = att0 + (uint32_t)a;
       // ---- section choice and moving particle
-      if (threadIdx.x == 0) {
+      if (threadIdx.x < 32) {  // (a uniform per lane)
         int i1, i2 = -2;
-        uint32_t ui = 0;
-        const double x = stream_uniform(P.seed, s.stream_id, att, ui++) * (1 - 1e-8);
+        const double u = stream_uniform(P.seed, s.stream_id, att, min(threadIdx.x, 2));
+        const double u1 = __shfl_sync(0xffffffffu, u, 1), u2 = __shfl_sync(0xffffffffu, u, 2);
+        const double x = __shfl_sync(0xffffffffu, u, 0) * (1 - 1e-8);
         if (!fixed) {
           const int ilo = -1, ihi = M - 1;
           i1 = ilo + (int)((ihi + 1 - ilo) * x);
@@ -1022,15 +1089,17 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
           const int ilo = -1, ihi = M / 2 - 1;
           i1 = ilo + (int)((ihi + 1 - ilo) * x);
           if (i1 > ihi) i1 = ihi;
-          if (stream_uniform(P.seed, s.stream_id, att, ui++) >= 0.5) i1 = (i1 + M / 2 + 1) % M - 1;
+          if (u1 >= 0.5) i1 = (i1 + M / 2 + 1) % M - 1;
           i2 = (i1 + M / 2 + 1) % M - 1;
         }
-        int ip = (int)(np * stream_uniform(P.seed, s.stream_id, att, ui++));
+        int ip = (int)(np * (fixed ? u2 : u1));
         if (ip >= np) ip = np - 1;
-        m.ictl[C_IFIRST1] = i1;
-        m.ictl[C_IFIRST2] = i2;
-        m.ictl[C_IPART] = ip;
-        m.ictl[C_REJECT] = -1;
+        if (threadIdx.x == 0) {
+          m.ictl[C_IFIRST1] = i1;
+          m.ictl[C_IFIRST2] = i2;
+          m.ictl[C_IPART] = ip;
+          m.ictl[C_REJECT] = -1;
+        }
       }
       __syncthreads();
       const int ifirst1 = m.ictl[C_IFIRST1], ifirst2 = m.ictl[C_IFIRST2];
@@ -1042,6 +1111,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
       double* lds = m.red + kWarps + 8;  // [kMaxLevels] per level: action difference,
       double* llt = lds + kMaxLevels;     // mover ln T,
       double* lnd = llt + kMaxLevels;     // fixed-node difference
+#pragma unroll 1
       for (int t = threadIdx.x; t < nsec; t += blockDim.x) {
         m.mx[t] = m.s1x[t * np + ipart];
         m.my[t] = m.s1y[t * np + ipart];
@@ -1121,6 +1191,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
       }
       int oshift = 0;   // moved-slice orders and uniforms a delayed-rejection
       uint32_t ushift = 0;  // proposal took before the level
+#pragma unroll 1
       for (int level = min(L, lb - 1); level >= 0 && reject < 0; --level) {
         const uint32_t ubase = level_uniform_base(s, level) + ushift;
         const double lnT = s.dr ? mover_level(s, m, ipart, level, oshift) : llt[level];
@@ -1132,6 +1203,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
           if (ek)
             ds += ewald_level0_cached(s, m, ipart, ifirst1, ek, ekstage);
           else
+#pragma unroll 1
             for (int t = 1; t < nsec - 1; ++t) ds += ewald_slice_diff(s, m, ipart, t);
         }
         const double dsn = lnd[level];
@@ -1168,6 +1240,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
         oldDS = m.red[kWarps + 2];
       }
       if (reject < 0) {
+#pragma unroll 1
         for (int t = threadIdx.x; t < nsec; t += blockDim.x) {
           m.s1x[t * np + ipart] = m.mx[t];
           m.s1y[t * np + ipart] = m.my[t];
@@ -1176,11 +1249,10 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
         if (threadIdx.x == 0) ++nacc;
         if (ek) {  // the moved slices' structure factors: the staged level-0 values
           const int totk = s.totk;
-          for (int it = threadIdx.x; it < (nsec - 2) * totk; it += blockDim.x) {
-            const int tt = it / totk, k = it - tt * totk;
-            *(longlong2*)(ek + ((size_t)wrap_slice(ifirst1 + 1 + tt, M) * totk + k) * 2) =
-                *(const longlong2*)(ekstage + (size_t)it * 2);
-          }
+#pragma unroll 1
+          for (int tt = threadIdx.x >> 5; tt < nsec - 2; tt += blockDim.x >> 5)
+            copy_warp((longlong2*)ek + (size_t)wrap_slice(ifirst1 + 1 + tt, M) * totk,
+                      (const longlong2*)ekstage + (size_t)tt * totk, totk);
         }
         if (cache && mynode) {
           // The moved slices now hold the level evaluations; the entries that
@@ -1189,27 +1261,31 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
           const int nsm = s.ns_max;
           const double NaN = __longlong_as_double(0x7ff8000000000000LL);
           const bool sho = s.node_kind[msp] == PIMC_NODES_SHO;
+#pragma unroll 1
           for (int it = threadIdx.x; it < (nsec - 2) * n; it += blockDim.x) {
-            const int k = 1 + it / n, j = it % n;
+            const int k = 1 + it / n, j = it - (k - 1) * n;
             const int t1 = wrap_slice(ifirst1 + k, M);
             double* e = cache_entry(s, cache, msp, t1);
+            const double* nc = m.ncol + k * m.ncol_stride + j;
+            double c[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) c[q] = sho && q ? 0.0 : nc[q * n];
             e[2 + j] = m.ndist[(k * 2) * nsm + j];
             e[2 + n + j] = m.ndist[(k * 2 + 1) * nsm + j];
-            const double* nc = m.ncol + k * m.ncol_stride;
-            e[2 + 2 * n + jcol * n + j] = nc[j];
-            if (!sho)
-              for (int c = 1; c < 4; ++c) e[2 + 2 * n + c * n * n + jcol * n + j] = nc[c * n + j];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (!sho || q == 0) e[2 + 2 * n + q * n * n + jcol * n + j] = c[q];
           }
           if (sm_species(s, msp) && m.xstage) {
             // the moved slices' inverse blocks, as the level evaluations left them
             const int xw = n * n + 2, xs = cache_x_slot(s, msp);
-            for (int it = threadIdx.x; it < (nsec - 2) * xw; it += blockDim.x) {
-              const int k = 1 + it / xw, w = it - (k - 1) * xw;
-              cache_entry(s, cache, msp, wrap_slice(ifirst1 + k, M))[xs + w] =
-                  m.xstage[(size_t)k * m.xstage_stride + w];
-            }
+#pragma unroll 1
+            for (int k = 1 + (threadIdx.x >> 5); k < nsec - 1; k += blockDim.x >> 5)
+              copy_warp(cache_entry(s, cache, msp, wrap_slice(ifirst1 + k, M)) + xs,
+                        m.xstage + (size_t)k * m.xstage_stride, xw);
           }
           __syncthreads();
+#pragma unroll 1
           for (int k = 1 + threadIdx.x; k < nsec - 1; k += blockDim.x) {
             const int t1 = wrap_slice(ifirst1 + k, M);
             double* e = cache_entry(s, cache, msp, t1);
@@ -1246,6 +1322,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
           store_section(s, path, ifirst1, m.s1x, m.s1y, m.s1z);
         }
       } else if (reject < 0) {
+#pragma unroll 1
         for (int k = 1 + threadIdx.x; k < nsec - 1; k += blockDim.x) {
           const int islice = ifirst1 + k;
           if (islice < 0) continue;
@@ -1263,6 +1340,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
       P.state[r].status = status;
       P.state[r].accepted += nacc;
       P.state[r].attempted += nat;
+#pragma unroll 1
       for (int k = 0; k < kMaxSpecies; ++k) {
         P.state[r].node_scale[k] = scale[k];
         P.state[r].epoch[k] = epoch[k];

@@ -316,6 +316,8 @@ __device__ __forceinline__ double grid_log(const double* tab, double q, unsigned
   return __dadd_rn(__ldg(tab + kLogReciprocals + k), p);
 }
 
+static __device__ __noinline__ double log_call(double q) { return log(q); }  // (rare)
+
 // Pair-action table lookup on the logarithmic grid
 // (PairAction::u00 / uk0 / uk0CalcDerivatives, src/action/PairAction.cc:601-655).
 // Distances below the grid take its first point, those beyond it its last; a NaN or
@@ -327,7 +329,7 @@ __device__ __forceinline__ void tab_locate(const DevTable& t, double q, int& i, 
   if (k < (unsigned)kLogEntries) {
     x = grid_log(t.logtab, q, k) * t.logrratioinv;
   } else {  // below 1 (or negative: NaN paths), past 2^20, infinite or NaN
-    x = q >= 1 ? log(q) * t.logrratioinv : 0.0;
+    x = q >= 1 ? log_call(q) * t.logrratioinv : 0.0;
     if (!(x < 2e9)) x = 2e9;
   }
   i = max((int)x, 0);

@@ -50,7 +50,7 @@ struct Smem {
 
 
 enum {
-  C_IFIRST1 = 0, C_IFIRST2, C_IPART, C_REJECT, C_FLAG, C_SCANK, C_ERRS, C_NMISS, C_NCTL = 16
+  C_IFIRST1 = 0, C_IFIRST2, C_IPART, C_REJECT, C_FLAG, C_ERRS, C_NMISS, C_NCTL = 16
 };
 
 struct SectionSizes {
@@ -770,38 +770,27 @@ static __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
                       __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
 }
 
-static __device__ void ewald_bead_tables(const DevSys& s, double2* X, double2* Y, double2* Z,
-                                         int w, int col, double x, double y, double z) {
-  const int kx0 = s.ikmax[0], ky0 = s.ikmax[1], kz0 = s.ikmax[2];
-  X[col] = make_double2(1.0, 0.0);
-  Y[ky0 * w + col] = make_double2(1.0, 0.0);
-  Z[kz0 * w + col] = make_double2(1.0, 0.0);
-  double sn, cs;
-  if (kx0 > 0) {
-    sincos(__dmul_rn(s.deltak[0], x), &sn, &cs);
-    X[w + col] = make_double2(cs, sn);
-  }
-  if (ky0 > 0) {
-    sincos(__dmul_rn(s.deltak[1], y), &sn, &cs);
-    Y[(ky0 + 1) * w + col] = make_double2(cs, sn);
-    Y[(ky0 - 1) * w + col] = make_double2(cs, -sn);
-  }
-  if (kz0 > 0) {
-    sincos(__dmul_rn(s.deltak[2], z), &sn, &cs);
-    Z[(kz0 + 1) * w + col] = make_double2(cs, sn);
-    Z[(kz0 - 1) * w + col] = make_double2(cs, -sn);
-  }
-  const double2 x1 = X[w + col];
-  for (int k = 2; k <= kx0; ++k) X[k * w + col] = cmul_rn(X[(k - 1) * w + col], x1);
-  const double2 yp = Y[(ky0 + 1) * w + col], ym = Y[(ky0 - 1) * w + col];
-  for (int k = 2; k <= ky0; ++k) {
-    Y[(ky0 + k) * w + col] = cmul_rn(Y[(ky0 + k - 1) * w + col], yp);
-    Y[(ky0 - k) * w + col] = cmul_rn(Y[(ky0 - k + 1) * w + col], ym);
-  }
-  const double2 zp = Z[(kz0 + 1) * w + col], zm = Z[(kz0 - 1) * w + col];
-  for (int k = 2; k <= kz0; ++k) {
-    Z[(kz0 + k) * w + col] = cmul_rn(Z[(kz0 + k - 1) * w + col], zp);
-    Z[(kz0 - k) * w + col] = cmul_rn(Z[(kz0 - k + 1) * w + col], zm);
+static __device__ __noinline__ void ewald_bead_tables(const DevSys& s, double2* X, double2* Y,
+                                                      double2* Z, int w, int col, double x,
+                                                      double y, double z) {
+#pragma unroll 1
+  for (int a = 0; a < 3; ++a) {  // (one copy of the code for the three axes)
+    const int k0 = s.ikmax[a];
+    double2* T = a == 0 ? X + col : (a == 1 ? Y + k0 * w + col : Z + k0 * w + col);
+    T[0] = make_double2(1.0, 0.0);
+    if (k0 <= 0) continue;
+    double sn, cs;
+    sincos(__dmul_rn(s.deltak[a], a == 0 ? x : (a == 1 ? y : z)), &sn, &cs);
+    // the negative multiples of y and z are the conjugates: the recurrence of the
+    // conjugate gives exactly those
+    const double2 t1 = make_double2(cs, sn);
+    double2 t = t1;
+#pragma unroll 1
+    for (int k = 1; k <= k0; ++k) {
+      T[k * w] = t;
+      if (a > 0) T[-k * w] = make_double2(t.x, -t.y);
+      t = cmul_rn(t, t1);
+    }
   }
 }
 
