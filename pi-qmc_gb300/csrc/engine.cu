@@ -1462,6 +1462,7 @@ void fill_run_params(pimc_engine* e, RunParams& P, int nattempt, pimc_move_recor
   P.nattempt_r = nullptr;
   P.nrep = e->nrep;
   P.seed = e->seed;
+  P.wide = e->grid <= e->num_sms;
   P.lay = e->lay;
 }
 }  // namespace
@@ -2500,6 +2501,7 @@ int pimc_server_run(pimc_engine* e) {
   P.nattempt_r = e->d_slot_attempts.p;
   P.nrep = e->nactive;
   P.seed = e->seed;
+  P.wide = e->grid <= e->num_sms;
   P.lay = e->lay;
   CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
   CU(section_launch(e->minb, e->grid, e->block, e->lay.total * 8, e->stream, P));

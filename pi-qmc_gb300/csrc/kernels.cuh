@@ -44,12 +44,13 @@ struct RunParams {
   double* xstage;         // mixed form: per-CTA staging of changed slices' inverses (null: none)
   long long xstage_cta;   // doubles per CTA
   int nrep;
+  int wide;  // at most one CTA per SM
   uint64_t seed;
   Layout lay;
 };
 
 __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSys& s,
-                                      double* nodescr_g, double* xstage = nullptr) {
+                                      double* nodescr_g, double* xstage = nullptr, bool wide = false) {
   Smem m;
   // mixed form: this CTA's staging of the inverse blocks of an attempt's changed
   // slices ([nsec][2 + ns_max^2], global memory), committed to the cache on accept
@@ -91,6 +92,7 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
   m.ncol_stride = L.ncol_stride;
   m.nodescr_stride = L.nodescr_stride;
   m.nodescr = L.nodescr_in_smem ? base + L.nodescr : gbase;
+  m.wide = wide;
   m.act = L.act >= 0 ? base + L.act
                      : (L.act_global ? gbase + (L.gcta - nw * L.act_stride) : m.nodescr);
   m.act_stride = L.act_stride;
@@ -598,14 +600,19 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   __syncthreads();
   // warp tasks: each warp takes up to G misses of one species (lane groups of
   // a warp must run the same species so that they stay converged)
-  int ntask = 0, first[kMaxSpecies + 1];
+  int ntask = 0, first[kMaxSpecies + 1], wmin = m.wide ? 32 : 8;
 #pragma unroll 1
-  for (int sp = 0; sp < s.nspecies; ++sp) {
-    const int G = 32 / node_group_width(s.spec_count[sp]);
-    first[sp] = ntask;
-    ntask += (nmiss[sp] + G - 1) / G;
+  for (;; wmin >>= 1) {  // (wide: the widest groups that take no further round)
+    ntask = 0;
+#pragma unroll 1
+    for (int sp = 0; sp < s.nspecies; ++sp) {
+      const int G = 32 / max(wmin, node_group_width(s.spec_count[sp]));
+      first[sp] = ntask;
+      ntask += (nmiss[sp] + G - 1) / G;
+    }
+    first[s.nspecies] = ntask;
+    if (wmin == 8 || ntask <= nwarps) break;
   }
-  first[s.nspecies] = ntask;
   if (llt && warp == nwarps - 1) mover_all(s, m, ipart, seed, att, llt);
 #pragma unroll 1
   for (int wt = warp; wt < ntask; wt += nwarps) {
@@ -613,7 +620,7 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     while (wt >= first[sp + 1]) ++sp;
     const int n = s.spec_count[sp];
     const bool sho = s.node_kind[sp] == PIMC_NODES_SHO, mine = sp == msp;
-    const int W = node_group_width(n), G = 32 / W, gm = lane / W, glm = lane & (W - 1);
+    const int W = max(wmin, node_group_width(n)), G = 32 / W, gm = lane / W, glm = lane & (W - 1);
     const int base = (wt - first[sp]) * G;
     const int task = base + gm;
     const bool act = task < nmiss[sp];
@@ -816,8 +823,20 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   // lane groups of the species' width, packed (32 / W matrices a warp): the
   // SM's narrow FP64 pipe, shared by every resident warp, is the limit, and a
   // packed warp instruction serves several matrices
-  const int W = node_group_width(n), G = 32 / W, g = lane / W;
-  const int nodeW = min(nwarps, (ntask + G - 1) / G);
+  int W = node_group_width(n);
+  const int wantW = min(nwarps, (ntask * W + 31) / 32);
+  // (wantW, with the narrowest groups: the sums' shares do not depend on the launch)
+  const int a0 = 2 * wantW > nwarps ? 0 : (s.mixed ? nwarps / 2 : wantW), dmax = L - alo, dmin = ahi == L ? 0 : dmax;
+  // A CTA that has its SM to itself is bound by the chain of each matrix's operations,
+  // not by the pipe: it takes the widest groups that need no further round of the
+  // warps without action terms (128 mixed dots, one a CTA: 50.9 -> 44.9 ms a round, and
+  // 41.1 with half of the warps on the action; two CTAs per SM share the pipe, where
+  // narrow groups' fewer instructions count).
+  if (m.wide) {
+    const int most = a0 == 0 || alo > ahi ? nwarps : a0;
+    while (W < 32 && ntask * W <= 16 * most) W *= 2;
+  }
+  const int G = 32 / W, g = lane / W, nodeW = min(nwarps, (ntask + G - 1) / G);
   if (mynode) {
     if (threadIdx.x == 0) m.ictl[C_FLAG] = 0;
     if (hi == L) {
@@ -878,7 +897,6 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
       }
     }
   }
-  const int a0 = 2 * nodeW > nwarps ? 0 : nodeW, dmax = L - alo, dmin = ahi == L ? 0 : dmax;
   if (alo <= ahi) {
     if (warp >= a0) {
       double* buf = m.act + (size_t)warp * m.act_stride;
@@ -1050,7 +1068,7 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
     }
     if (threadIdx.x == 0) {
       M_ = carve(smem, P.lay, P.sys[r], P.nodescr_g,
-                 P.xstage ? P.xstage + (size_t)blockIdx.x * P.xstage_cta : nullptr);
+                 P.xstage ? P.xstage + (size_t)blockIdx.x * P.xstage_cta : nullptr, P.wide);
       status = P.state[r].status;
       nacc = 0;
 #pragma unroll 1

@@ -40,6 +40,7 @@ struct Smem {
   int ncol_stride;          // ns_max (SHO exp column) or 4 ns_max (free-particle values + gradients)
   double* nrm;              // [2^L - 1][3] the attempt's proposal normals
   int nodescr_stride;       // doubles per warp
+  bool wide;                // wider lane groups where warps would idle
   double* nodecold;         // cold parts of the node scratch when apart (global), or null
   int nodecold_stride;      // doubles per warp
   int node_cold_follows;    // each group's cold part follows its hot part
@@ -91,6 +92,36 @@ __device__ __forceinline__ int small_div(int a, int m) {
   return (int)(((unsigned)a * kSmallReciprocals.v[m]) >> 16);
 }
 
+// 1 / a, correctly rounded, on the integer pipe: Newton's iteration in fixed point
+// from the FP32 reciprocal (24 bits; then 44, then the 62 of the format).  With a =
+// 2^k d, d in (1/2, 1), the last step holds 2^62 / d to 2 units and the result
+// takes 10 fewer bits, so the rounding is certain unless the cut bits lie within 8
+// units of a tie; those 1.6% of values, powers of two, and results that are not
+// normal take the divide instruction sequence.  One FP64 instruction costs the SM
+// 19 clocks, so the 86 of __drcp_rn were a sixth of a factorisation's (n = 10).
+static __device__ __noinline__ double reciprocal_call(double a) { return __drcp_rn(a); }
+__device__ __forceinline__ double reciprocal(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = (hi >> 20) & 0x7ffu;
+  const unsigned long long M = (1ull << 63) | (b << 11);  // d
+  const float f = __uint_as_float(0x3f000000u | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const unsigned rb = __float_as_uint(__fdividef(1.0f, f));
+  const unsigned x0 = ((rb & 0x7fffffu) | 0x800000u) << ((rb >> 23) - 120u);  // 2^30 / d
+  const unsigned long long t =
+      (unsigned long long)(unsigned)(M >> 32) * x0 + (((unsigned long long)(unsigned)M * x0) >> 32);
+  const int e0 = (int)((long long)((1ull << 62) - t) >> 10);
+  const unsigned long long x1 = ((unsigned long long)x0 << 32) +
+                                (unsigned long long)(((long long)(int)(x0 >> 1) * e0) >> 19);
+  const int e1 = (int)((1ull << 62) - __umul64hi(M, x1));
+  const unsigned long long x2 =
+      x1 + (unsigned long long)(((long long)(int)(unsigned)(x1 >> 33) * e1) >> 29) + 512ull;
+  if ((((hi & 0xfffffu) | lo) == 0u) || e - 2u > 2042u || ((unsigned)x2 & 1023u) - 8u > 1008u)
+    return reciprocal_call(a);
+  return __longlong_as_double(
+      (long long)((((unsigned long long)(2045u - e) << 52) + (x2 >> 10) - (1ull << 52)) |
+                  (b & (1ull << 63))));
+}
+
 // ------------------------------------------------------------------ node model
 // The mixed form's Sherman-Morrison updates of cached inverses: at most
 // kSmRefresh updates between two factorisations of a slice pair's matrix, and
@@ -102,11 +133,14 @@ constexpr double kSmRefresh = 16.0;
 constexpr double kSmMinRatio = 0.05;
 constexpr double kSmMaxCond = 1e7;
 // Scratch doubles one lane group needs for an n-particle species: a hot part
-// (the LU and the inverse, rewritten at every elimination step, the reciprocal
-// pivots and the row order), and, for evaluations whose elements are not in a cache
+// (the LU and the inverse, rewritten at every elimination step (the inverse's place
+// later takes 8 n sums), the reciprocal pivots and the row order), and, for evaluations whose elements are not in a cache
 // entry, a cold part (the SHO exp matrix, or the free-particle gradient matrices:
 // written once, read once).
-__host__ __device__ constexpr int node_group_hot(int n) { return 2 * n * n + n + (n + 1) / 2 + 1; }
+__host__ __device__ constexpr int node_group_inverse(int n) { return (n < 8 ? 8 : n) * n; }
+__host__ __device__ constexpr int node_group_hot(int n) {
+  return n * n + node_group_inverse(n) + n + (n + 1) / 2 + 1;
+}
 __host__ __device__ constexpr int node_group_cold(int n, bool free_nodes = true) {
   return n * n + (free_nodes ? 3 * n * n : 0);
 }
@@ -221,7 +255,7 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   // hot part at scr; the cold part follows it unless given apart
   double* A = scr;          // n*n column-major, LU; after the inverse: work space
   double* X = A + n * n;    // n*n inverse, column-major
-  double* R = X + n * n;    // n reciprocals of the U diagonal
+  double* R = X + node_group_inverse(n);  // n reciprocals of the U diagonal
   int* order = (int*)(R + n + 1);  // the matrix row at each position; then its inverse
   double* E = cold ? cold : scr + node_group_hot(n);  // elements (and gradients) without a place
   constexpr bool sho = kSho;
@@ -439,7 +473,7 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
     __syncwarp();  // (every lane has it: the interchange moves it)
     if (regular) {
       // (the reciprocal starts on its way beside the interchange)
-      const double rinv = __drcp_rn(apj);  // 1 / a, correctly rounded
+      const double rinv = reciprocal(apj);
       if (p != j) {
         pivbits ^= 1u;
         if (gl < n) {  // rows j and p of columns j .. j + n - 1
@@ -617,30 +651,52 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
     // sum of w r and T that of w, S - ch r T
     const double c = s.node_c[sp], ch = s.node_cosh[sp];
     const double fac = 2 * c * scale;
+    double* S = X;
+    // (X, spent, takes the sums, one of the 8 n per lane and step, three steps at once)
+    if (ok)
+#pragma unroll 1
+      for (int q0 = gl; q0 < 8 * n; q0 += 3 * W) {
+        const double *w[3], *x[3];
+        double xm[3], sum[3];
+        int dw[3], im[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const int q = min(q0 + k * W, 8 * n - 1), c = q & 3, o = q >> 2;
+          const bool first = o < n;
+          const SliceView& v = first ? v2 : v1;
+          w[k] = A + (first ? o * n : o - n);
+          dw[k] = first ? 1 : n;
+          // (c = 3: the sum of the weights alone, a factor of one)
+          x[k] = (c == 0 ? v.sx : (c == 1 ? v.sy : v.sz)) + v.t * v.npart + f;
+          xm[k] = c == 0 ? v.mxv : (c == 1 ? v.myv : (c == 2 ? v.mzv : 1.0));
+          im[k] = c == 3 ? -1 : v.imov - f;
+          sum[k] = 0;
+        }
+        const bool one = (gl & 3) == 3;  // (W and q0 - gl are multiples of 4)
+#pragma unroll 1
+        for (int i = 0; i < n; ++i)
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            if (q0 + k * W < 8 * n) {
+              sum[k] = __fma_rn(*w[k], one || i == im[k] ? xm[k] : x[k][i], sum[k]);
+              w[k] += dw[k];
+            }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (q0 + k * W < 8 * n) S[q0 + k * W] = sum[k];
+      }
+    __syncwarp();
     if (ok)
 #pragma unroll 1
       for (int q = gl; q < 2 * n; q += W) {
         const bool first = q < n;
         const int p = first ? q : q - n;
-        const SliceView& v = first ? v2 : v1;
-        const int at = v.t * v.npart + f, im = v.imov - f;
-        const double* w = A + (first ? p * n : p);
-        const int dw = first ? 1 : n;
-        double sx = 0, sy = 0, sz = 0, tw = 0;
-#pragma unroll 4
-        for (int k = 0; k < n; ++k) {
-          const double wk = w[k * dw];
-          sx = __fma_rn(wk, k == im ? v.mxv : v.sx[at + k], sx);
-          sy = __fma_rn(wk, k == im ? v.myv : v.sy[at + k], sy);
-          sz = __fma_rn(wk, k == im ? v.mzv : v.sz[at + k], sz);
-          tw = __dadd_rn(tw, wk);
-        }
         double rx, ry, rz;
         (first ? v1 : v2).get(f + p, rx, ry, rz);
-        const double ct = __dmul_rn(ch, tw);
-        const double lx = __dmul_rn(fac, __fma_rn(-ct, rx, sx));
-        const double ly = __dmul_rn(fac, __fma_rn(-ct, ry, sy));
-        const double lz = __dmul_rn(fac, __fma_rn(-ct, rz, sz));
+        const double ct = __dmul_rn(ch, S[4 * q + 3]);
+        const double lx = __dmul_rn(fac, __fma_rn(-ct, rx, S[4 * q]));
+        const double ly = __dmul_rn(fac, __fma_rn(-ct, ry, S[4 * q + 1]));
+        const double lz = __dmul_rn(fac, __fma_rn(-ct, rz, S[4 * q + 2]));
         const double d = __dmul_rn(dk, rsqrt(__dadd_rn(dot3(lx, ly, lz, lx, ly, lz), 1e-15)));
         if (write) (first ? d1 : d2)[p] = d;
       }

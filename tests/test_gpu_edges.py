@@ -342,3 +342,32 @@ def test_pair_table_grid_edges(pimc, rmin, rmax, ngpts):
         ds = e.action_difference(level, sec, mov, np.zeros(len(r), np.int32))
         ref = np.array([port.action_diff(level, sec[b], mov[b], 0) for b in range(len(r))])
         assert np.all(np.abs(ds - ref) <= 1e-12 * size), level
+
+
+@pytest.mark.parametrize("mixed", [0, 1])
+@pytest.mark.parametrize("counts", [[1, 2], [4, 3], [8, 7], [9, 10], [16, 5]])
+def test_lane_group_widths(pimc, counts, mixed):
+    # A launch of at most one CTA per SM evaluates Slater matrices with wider lane
+    # groups than a fuller one: the same chains, bit for bit, and the oracle's.
+    kw = W.dot20_fn(counts=counts, nslice=64, beta=64 / 25.6, nlevel=4)
+    tabs, _ = pimc.coulomb_tables(kw)
+    cfg = O.make_config(**kw)
+    x = W.initial_path(cfg, "gauss", seed=3)
+    nrep, natt = 700, 24
+    few = pimc.Engine(kw, 2, tabs, seed=9, precision=mixed)
+    many = pimc.Engine(kw, nrep, tabs, seed=9, precision=mixed)
+    few.upload_paths([x] * 2)
+    many.upload_paths([x] * nrep)
+    a, b = few.run_sections(natt, records=True), many.run_sections(natt, records=True)
+    for k in a:
+        assert np.array_equal(a[k], b[k][:2], equal_nan=True), k
+    assert np.array_equal(few.download_paths()[1], many.download_paths()[1])
+    if not mixed:
+        port = O.PortOracle(cfg, tabs)
+        port.set_path(x)
+        ref = port.run(natt)
+        c = pimc.Engine(kw, 1, tabs)
+        c.upload_paths([x])
+        rec = c.run_sections(natt, records=True)
+        assert np.array_equal(rec["reject_level"][0], ref["reject_level"])
+        assert np.abs(c.download_paths()[0] - port.get_path()).max() <= 1e-10
