@@ -586,7 +586,7 @@ int ek_bits(const DevSys& d) {
 constexpr int kSmemLimit = 220 * 1024;
 
 Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutOpts opts = {}) {
-  int nsec = 0, np = 0, nsm = 1, per = 0;
+  int nsec = 0, np = 0, nsm = 1, per = 0, perxy = 0;
   bool fixed = false, ewald_full = false;
   for (const DevSys& d : sys) {
     nsec = std::max(nsec, d.nsec);
@@ -595,6 +595,7 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
     fixed |= d.fixed_node != 0;
     if (d.ewald) {
       per = std::max(per, d.ikmax[0] + 1 + 2 * d.ikmax[1] + 1 + 2 * d.ikmax[2] + 1);
+      perxy = std::max(perxy, (d.ikmax[0] + 1) * (2 * d.ikmax[1] + 1));
       ewald_full |= opts.full_ewald_tables || ek_bits(d) < 0;
     }
   }
@@ -620,7 +621,12 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
   L.ndm = take(nsec);
   L.dist = take(fixed ? nsec * 2 * nsm : 0);
   L.ndist = take(fixed ? nsec * 2 * nsm : 0);
-  L.ewt = take(2 * per * L.ewt_cols);
+  L.ewt_words = 2 * per * L.ewt_cols;
+  // without Slater scratch to share, room for the (kx, ky) products of eight slices
+  // (at 100 KB two CTAs fit an SM)
+  if (per && !ewald_full && !fixed && (off + 34 * (per + perxy)) * 8 <= 100 * 1024)
+    L.ewt_words = std::max(L.ewt_words, 34 * (per + perxy));
+  L.ewt = take(L.ewt_words);
   L.ictl = take((C_NCTL + 2 * kMaxSpecies * nsec + 1) / 2 + 1);
   bool sho = false;
   for (const DevSys& d : sys)

@@ -23,6 +23,7 @@ struct Layout {
   int ncol_global;      // the new-column buffer in the CTA's global area
   int gcta;             // doubles of global scratch per CTA
   int ewt_cols;         // bead columns of the Ewald tables area
+  int ewt_words;        // doubles of the tables area
   int ewxy;             // their (kx, ky) products (estimators; 0: none)
   int total;  // doubles
 };
@@ -93,6 +94,13 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
   m.nodescr_stride = L.nodescr_stride;
   m.nodescr = L.nodescr_in_smem ? base + L.nodescr : gbase;
   m.wide = wide;
+  // the level-0 Ewald term's tables: their own area, or the Slater scratch
+  m.ewx = m.ewt;
+  m.ewx_words = L.ewt_words;
+  if (L.nodescr_in_smem && nw * L.nodescr_stride > L.ewt_words) {
+    m.ewx = m.nodescr;
+    m.ewx_words = nw * L.nodescr_stride;
+  }
   m.act = L.act >= 0 ? base + L.act
                      : (L.act_global ? gbase + (L.gcta - nw * L.act_stride) : m.nodescr);
   m.act_stride = L.act_stride;
@@ -113,47 +121,84 @@ __device__ __forceinline__ int wrap_slice(int islice, int M) {
 // evalLongRange's difference is sum_k 2 v_k (|rho'_k|^2 - |rho_k|^2) / (2V)
 // (the self energy cancels).  O(totk) per slice instead of O(totk N) for each
 // of the two configurations.  rho'_k goes to `stage` for the accept step.
+// FP64 bound: 15 instructions and eight conversions per slice and k-vector with the
+// products q e^{i(kx x + ky y)} tabulated beside the axes' tables, over the Slater
+// scratch, which is free by then (53 and a third of the attempt without: N = 54,
+// totk = 257, XXX -> XXX clocks).
 static __device__ __noinline__ double ewald_level0_cached(const DevSys& s, const Smem& m, int ipart,
                                              int ifirst1, const long long* ek, long long* stage) {
   const int np = s.npart, nsec = s.nsec, M = s.nslice, totk = s.totk;
   const int ky0 = s.ikmax[1], kz0 = s.ikmax[2];
-  const int nx = s.ikmax[0] + 1, ny = 2 * ky0 + 1;
-  const int w = m.ewt_cols;  // bead columns of the tables area
-  const int chunk = w / 2;   // slices per pass: the old and the new bead of each
-  double2* X = (double2*)m.ewt;
+  const int nx = s.ikmax[0] + 1, ny = 2 * ky0 + 1, per = nx + ny + 2 * kz0 + 1;
+  // columns: a slice's old and new bead.  As many as the area holds of the three axes'
+  // tables and their (kx, ky) products (an odd row length against bank conflicts);
+  // where that is not one slice, the tables alone.
+  int w = m.ewx_words / (2 * (per + nx * ny));
+  const bool xy = w >= 3;
+  if (!xy) w = m.ewx_words / (2 * per);
+  w = w < 3 ? 2 : (min(w, 2 * (nsec - 2) + 1) - 1) | 1;
+  const int chunk = w / 2;  // slices per pass
+  double2* X = (double2*)m.ewx;
   double2* Y = X + nx * w;
   double2* Z = Y + ny * w;
-  const double q = m.qpart[ipart], is = 1.0 / s.ek_scale;
+  double2* XY = X + per * w;
+  const double qs = __dmul_rn(m.qpart[ipart], s.ek_scale);  // (exact: a power of two)
   double acc = 0.0;
 #pragma unroll 1
   for (int t0 = 1; t0 < nsec - 1; t0 += chunk) {
-    const int nt = min(chunk, nsec - 1 - t0);
+    const int nc = 2 * min(chunk, nsec - 1 - t0);
     __syncthreads();
 #pragma unroll 1
-    for (int c = threadIdx.x; c < 2 * nt; c += blockDim.x) {
-      const int t = t0 + (c >> 1), o = t * np + ipart;
-      ewald_bead_tables(s, X, Y, Z, w, c, c & 1 ? m.mx[t] : m.s1x[o], c & 1 ? m.my[t] : m.s1y[o],
-                        c & 1 ? m.mz[t] : m.s1z[o]);
+    for (int it = threadIdx.x; it < 3 * nc; it += blockDim.x) {
+      const int a = it / nc, c = it - a * nc, t = t0 + (c >> 1), o = t * np + ipart;
+      const double* bead = c & 1 ? (a == 0 ? m.mx : (a == 1 ? m.my : m.mz)) + t
+                                 : (a == 0 ? m.s1x : (a == 1 ? m.s1y : m.s1z)) + o;
+      ewald_axis_table(s, (a == 0 ? X : (a == 1 ? Y : Z)) + c, w, a, *bead);
     }
     __syncthreads();
+    if (xy) {
 #pragma unroll 1
-    for (int it = threadIdx.x; it < nt * totk; it += blockDim.x) {
+      for (int it = threadIdx.x; it < nx * ny * nc; it += blockDim.x) {
+        const int p = it / nc, c = it - p * nc, kx = p / ny;
+        const double2 a = X[kx * w + c];
+        XY[p * w + c] = cmul_rn(make_double2(__dmul_rn(qs, a.x), __dmul_rn(qs, a.y)),
+                                Y[(p - kx * ny) * w + c]);
+      }
+      __syncthreads();
+    }
+#pragma unroll 1
+    for (int it = threadIdx.x; 2 * it < nc * totk; it += blockDim.x) {
       const int tt = it / totk, k = it - tt * totk, t = t0 + tt;
-      const int kx = __ldg(s.kvec + 3 * k), ky = __ldg(s.kvec + 3 * k + 1) + ky0,
-                kz = __ldg(s.kvec + 3 * k + 2) + kz0;
       const longlong2 o =
           *(const longlong2*)(ek + ((size_t)wrap_slice(ifirst1 + t, M) * totk + k) * 2);
-      long long are, aim, bre, bim;
-      ewald_term_fixed(s, X, Y, Z, w, 2 * tt, kx, ky, kz, q, are, aim);
-      ewald_term_fixed(s, X, Y, Z, w, 2 * tt + 1, kx, ky, kz, q, bre, bim);
-      const long long nre = o.x + (bre - are), nim = o.y + (bim - aim);
-      *(longlong2*)(stage + ((size_t)(t - 1) * totk + k) * 2) = make_longlong2(nre, nim);
-      const double ore = __ll2double_rn(o.x) * is, oim = __ll2double_rn(o.y) * is;
-      const double rre = __ll2double_rn(nre) * is, rim = __ll2double_rn(nim) * is;
-      acc += 2 * __ldg(s.vk + k) * ((rre * rre + rim * rim) - (ore * ore + oim * oim));
+      const double vk = __ldg(s.vk + k);
+      const int kx = __ldg(s.kvec + 3 * k), ky = __ldg(s.kvec + 3 * k + 1) + ky0,
+                kz = __ldg(s.kvec + 3 * k + 2) + kz0;
+      longlong2 d = make_longlong2(0, 0);  // new - old
+#pragma unroll
+      for (int c = 2 * tt; c < 2 * tt + 2; ++c) {
+        double2 p;
+        if (xy) {
+          p = XY[(kx * ny + ky) * w + c];
+        } else {
+          const double2 a = X[kx * w + c];
+          p = cmul_rn(make_double2(__dmul_rn(qs, a.x), __dmul_rn(qs, a.y)), Y[ky * w + c]);
+        }
+        const double2 v = cmul_rn(p, Z[kz * w + c]);
+        d.x = __double2ll_rn(v.x) - d.x;
+        d.y = __double2ll_rn(v.y) - d.y;
+      }
+      const longlong2 n = make_longlong2(o.x + d.x, o.y + d.y);
+      *(longlong2*)(stage + ((size_t)(t - 1) * totk + k) * 2) = n;
+      // |rho'|^2 - |rho|^2 = (rho' - rho) . (rho' + rho)
+      acc = __fma_rn(vk,
+                     __fma_rn(__ll2double_rn(d.x), __ll2double_rn(o.x + n.x),
+                              __dmul_rn(__ll2double_rn(d.y), __ll2double_rn(o.y + n.y))),
+                     acc);
     }
   }
-  const double sum = block_sum(acc, m.red);
+  const double is = 1.0 / s.ek_scale;
+  const double sum = block_sum(acc, m.red) * (2 * is * is);
   return sum * s.one_over_2v * s.tau / s.epsilon;
 }
 

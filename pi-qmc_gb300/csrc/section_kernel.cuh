@@ -31,6 +31,8 @@ struct Smem {
   double* dist;             // [nsec][2][ns_max] distances at set-up (moving species)
   double* ndist;            // [nsec][2][ns_max] distances of the new path
   double* ewt;              // Ewald exp(ik.r) tables: [kx, ky, kz rows][ewt_cols]
+  double* ewx;              // the level-0 Ewald term's tables,
+  int ewx_words;            // and their room
   double* ewxy;             // estimators: [kx, ky][npart] products of the tables, or null
   double* qpart;            // [npart] charges
   int* ictl;                // control words
@@ -826,28 +828,32 @@ static __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
                       __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
 }
 
-static __device__ __noinline__ void ewald_bead_tables(const DevSys& s, double2* X, double2* Y,
-                                                      double2* Z, int w, int col, double x,
-                                                      double y, double z) {
+static __device__ __noinline__ void ewald_axis_table(const DevSys& s, double2* T, int w, int a,
+                                                     double x) {
+  const int k0 = s.ikmax[a];
+  if (a > 0) T += k0 * w;
+  T[0] = make_double2(1.0, 0.0);
+  if (k0 <= 0) return;
+  double sn, cs;
+  sincos(__dmul_rn(s.deltak[a], x), &sn, &cs);
+  // the negative multiples of y and z are the conjugates: the recurrence of the
+  // conjugate gives exactly those
+  const double2 t1 = make_double2(cs, sn);
+  double2 t = t1;
 #pragma unroll 1
-  for (int a = 0; a < 3; ++a) {  // (one copy of the code for the three axes)
-    const int k0 = s.ikmax[a];
-    double2* T = a == 0 ? X + col : (a == 1 ? Y + k0 * w + col : Z + k0 * w + col);
-    T[0] = make_double2(1.0, 0.0);
-    if (k0 <= 0) continue;
-    double sn, cs;
-    sincos(__dmul_rn(s.deltak[a], a == 0 ? x : (a == 1 ? y : z)), &sn, &cs);
-    // the negative multiples of y and z are the conjugates: the recurrence of the
-    // conjugate gives exactly those
-    const double2 t1 = make_double2(cs, sn);
-    double2 t = t1;
-#pragma unroll 1
-    for (int k = 1; k <= k0; ++k) {
-      T[k * w] = t;
-      if (a > 0) T[-k * w] = make_double2(t.x, -t.y);
-      t = cmul_rn(t, t1);
-    }
+  for (int k = 1; k <= k0; ++k) {
+    T[k * w] = t;
+    if (a > 0) T[-k * w] = make_double2(t.x, -t.y);
+    t = cmul_rn(t, t1);
   }
+}
+
+static __device__ __forceinline__ void ewald_bead_tables(const DevSys& s, double2* X, double2* Y,
+                                                         double2* Z, int w, int col, double x,
+                                                         double y, double z) {
+#pragma unroll 1
+  for (int a = 0; a < 3; ++a)
+    ewald_axis_table(s, (a == 0 ? X : (a == 1 ? Y : Z)) + col, w, a, a == 0 ? x : (a == 1 ? y : z));
 }
 
 // q e^{ik.r} of table column col for k-vector k, on the fixed-point grid of the
