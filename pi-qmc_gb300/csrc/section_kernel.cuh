@@ -163,6 +163,39 @@ __device__ __forceinline__ double* group_cold(const Smem& m, int slot, int G, in
                     : nullptr;
 }
 
+// *dst = *src, asynchronously where the hardware can (global to shared); complete
+// for the lane after copy_wait, for the others after a barrier too.
+__device__ __forceinline__ void copy_async(double* dst, const double* src) {
+#ifdef __CUDA_ARCH__
+  if (__isShared(dst) && __isGlobal(src)) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(__cvta_generic_to_global(src))
+                 : "memory");
+    return;
+  }
+#endif
+  *dst = *src;
+}
+__device__ __forceinline__ void copy_wait() {
+#ifdef __CUDA_ARCH__
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
+}
+
+__device__ __forceinline__ bool in_shared(const double* p) {
+#ifdef __CUDA_ARCH__
+  return __isShared(p);
+#else
+  return true;
+#endif
+}
+__device__ __forceinline__ void prefetch_l2(const double* p) {
+#ifdef __CUDA_ARCH__
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
+#endif
+}
+
 // One element rho(r1_j, r2_i) of a species' Slater matrix (unscaled), and for
 // free-particle nodes its gradient with respect to r1_j.  Rounded operations: the
 // same bits wherever it is computed.
@@ -290,6 +323,16 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
     }
     A[j * n + i] = scale * v.v;
   };
+  // (mixed form: the cached inverse is on its way to X meanwhile, the gradients to L2)
+  bool good = false;
+  if (kSm && xin) {
+    good = xin[0] == xepoch && xin[1] < kSmRefresh;
+#pragma unroll 4
+    for (int k = gl; k < nn; k += W) copy_async(X + k, xin + 2 + k);
+    if (!sho && ecache)
+#pragma unroll 1
+      for (int k = 16 * gl; k < 3 * nn; k += 16 * W) prefetch_l2(ecache + nn + k);
+  }
   {
     const int nrows = __popc(rows_new), ncols = ecache ? __popc(cols & nmask) : 0;
 #pragma unroll 1
@@ -316,19 +359,9 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
   // n/2 rows); otherwise, or when another writing group of the warp cannot,
   // the warp factorises as below.  Every lane takes part in the shuffles.
   bool use_sm = false;
-  bool good = kSm && xin != nullptr && xin[0] == xepoch && xin[1] < kSmRefresh;
   // (a warp none of whose writing groups can update factorises at once)
   if (kSm && __any_sync(FULL, good && write) && __all_sync(FULL, good || !write)) {
-    const double* xc = good ? xin + 2 : nullptr;
-#pragma unroll 1
-    for (int k0 = gl; k0 < nn; k0 += 8 * W) {  // (eight loads in flight a lane)
-      double v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = xc && k0 + q * W < nn ? xc[k0 + q * W] : 0.0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (k0 + q * W < nn) X[k0 + q * W] = v[q];
-    }
+    copy_wait();
     __syncwarp();
     double det = det_in;
     if (cols) {
@@ -398,6 +431,10 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
       det_out = det;
       err_out = 0;
     }
+  }
+  if (kSm && !use_sm) {  // (X is about to be overwritten)
+    copy_wait();
+    __syncwarp();
   }
   double amax = 0.0;  // max |a| of the matrix, for the conditioning estimate (mixed form)
   // every lane takes part in the shuffles
@@ -722,28 +759,36 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
     } else {
       const int tw = small_div(n, 3), nt = small_div(n + tw - 1, tw);  // 3 to 5 tiles of 3 tw <= W rows
       double l1[5] = {0, 0, 0, 0, 0};
+      const bool async = ecache && in_shared(A);
 #pragma unroll 1
       for (int t = 0; t < nt; ++t) {
         const int j0 = t * tw, wd = min(tw, n - j0);
         __syncwarp();
-        // row r = component * wd + column of the tile, element i on lane i; four rows'
-        // loads in flight
+        // row r = component * wd + column of the tile, element i on lane i: all rows'
+        // loads in flight, or four rows' where the scratch is not in shared memory
         const int i = min(gl, n - 1);
+        auto source = [&](int r) {
+          const int c = 1 + (r >= wd) + (r >= 2 * wd), j = j0 + r - (c - 1) * wd;
+          const double* from = (ecache ? ecache : E) + c * nn + j * n;
+          if (cols && (((cols >> j) | (rows_new >> i)) & 1u))
+            from = newcol ? newcol + c * n : E + c * nn + j * n;
+          return from + i;
+        };
+        if (async) {
+          if (gl < n)
 #pragma unroll 1
-        for (int r0 = 0; r0 < 3 * wd; r0 += 4) {
-          double v[4];
+            for (int r = 0; r < 3 * wd; ++r) copy_async(A + r * n + gl, source(r));
+          copy_wait();
+        } else {
+#pragma unroll 1
+          for (int r0 = 0; r0 < 3 * wd; r0 += 4) {
+            double v[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = min(r0 + q, 3 * wd - 1), c = 1 + (r >= wd) + (r >= 2 * wd);
-            const int j = j0 + r - (c - 1) * wd;
-            const double* from = (ecache ? ecache : E) + c * nn + j * n;
-            if (cols && (((cols >> j) | (rows_new >> i)) & 1u))
-              from = newcol ? newcol + c * n : E + c * nn + j * n;
-            v[q] = from[i];
+            for (int q = 0; q < 4; ++q) v[q] = *source(min(r0 + q, 3 * wd - 1));
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (r0 + q < 3 * wd && gl < n) A[(r0 + q) * n + gl] = v[q];
           }
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (r0 + q < 3 * wd && gl < n) A[(r0 + q) * n + gl] = v[q];
         }
         __syncwarp();
         if (gl < n)
