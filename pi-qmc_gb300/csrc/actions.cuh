@@ -154,7 +154,7 @@ __device__ __forceinline__ void link_terms(const DevSys& s, const Smem& m, int i
       double x = n1x, y = n1y, z = n1z;
       pbc(s, x, y, z);
       double x2 = x * x + y * y + z * z;
-      const double kt = s.tau * (1 << level);
+        const double kt = s.tau * pow2(level);
       const double nw = (s.prim_a[sp] * x2 + s.prim_b[sp] * x2 * x2) * kt;
       x = o1x;
       y = o1y;
@@ -166,21 +166,21 @@ __device__ __forceinline__ void link_terms(const DevSys& s, const Smem& m, int i
   }
 }
 
-// PairAction of one link from its two separations, times its length in slices.
+// PairAction of one link from its two separations, times its length in slices (2^shift).
 __device__ __forceinline__ double pair_term(const DevTable& t, const Sep& a, const Sep& b,
-                                            bool offdiag, int stride) {
+                                            bool offdiag, int shift) {
   const double qq = 0.5 * (a.r + b.r);
-  if (!offdiag) return tab_u00(t, qq) * stride;
+  if (!offdiag) return tab_u00(t, qq) * pow2(shift);
   const double sx = a.x - b.x, sy = a.y - b.y, sz = a.z - b.z;
-  const double qi = __drcp_rn(qq);
-  return tab_uk0(t, qq, dot3(sx, sy, sz, sx, sy, sz) * (qi * qi)) * stride;
+  const double qi = reciprocal(qq);
+  return tab_uk0(t, qq, dot3(sx, sy, sz, sx, sy, sz) * (qi * qi)) * pow2(shift);
 }
 __device__ __forceinline__ float pair_term(const DevTable& t, const SepF& a, const SepF& b,
-                                           bool offdiag, int stride) {
+                                           bool offdiag, int shift) {
   const float qq = 0.5f * (a.r + b.r);
   const float s2 =
       offdiag ? __fdividef(norm2_move_f(a.x - b.x, a.y - b.y, a.z - b.z), __fmul_rn(qq, qq)) : 0.f;
-  return tab_uk0_f(t, qq, s2, offdiag ? t.norder : 0) * (float)stride;
+  return tab_uk0_f(t, qq, s2, offdiag ? t.norder : 0) * __uint_as_float((127u + shift) << 23);
 }
 
 // Separations a warp holds at once (levels dmin .. dmax of the heap, below).
@@ -242,7 +242,7 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
         sep[e] = SepF{fx, fy, fz, sqrtf(norm2_move_f(fx, fy, fz))};
       } else {
         pbc(s, dx, dy, dz);
-        sep[e] = Sep{dx, dy, dz, sqrt(dot3(dx, dy, dz, dx, dy, dz))};
+        sep[e] = Sep{dx, dy, dz, square_root(dot3(dx, dy, dz, dx, dy, dz))};
       }
     }
     __syncwarp();
@@ -264,7 +264,7 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
       decltype(pair_term(t, n1, n0, offdiag, 1)) v[2];
 #pragma unroll 1
       for (int pass = 0; pass < 2; ++pass) {  // (one copy of the lookup's code)
-        const auto x = pair_term(t, pass ? b1 : n1, pass ? b0 : n0, offdiag, 1 << (L - d));
+        const auto x = pair_term(t, pass ? b1 : n1, pass ? b0 : n0, offdiag, L - d);
         v[1] = pass ? x : v[1];
         v[0] = pass ? v[0] : x;
       }

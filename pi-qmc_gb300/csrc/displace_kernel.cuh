@@ -191,13 +191,13 @@ static __device__ __noinline__ double displace_actions(const DevSys& s, const Mo
         nz -= mv.d[jm][2];
       }
       pbc(s, nx, ny, nz);
-      const Sep n1{nx, ny, nz, sqrt(dot3(nx, ny, nz, nx, ny, nz))};
-      const Sep o1{ox, oy, oz, sqrt(dot3(ox, oy, oz, ox, oy, oz))};
+      const Sep n1{nx, ny, nz, square_root(dot3(nx, ny, nz, nx, ny, nz))};
+      const Sep o1{ox, oy, oz, square_root(dot3(ox, oy, oz, ox, oy, oz))};
       const auto up = [](double v) { return __shfl_up_sync(0xffffffffu, v, 1); };
       const Sep n0{up(n1.x), up(n1.y), up(n1.z), up(n1.r)};
       const Sep o0{up(o1.x), up(o1.y), up(o1.z), up(o1.r)};
       if (lane > 0 && live)
-        part += pair_term(tb, n1, n0, tb.norder > 0, 1) - pair_term(tb, o1, o0, tb.norder > 0, 1);
+        part += pair_term(tb, n1, n0, tb.norder > 0, 0) - pair_term(tb, o1, o0, tb.norder > 0, 0);
     }
   }
   return part;

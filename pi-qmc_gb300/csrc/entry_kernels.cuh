@@ -101,7 +101,7 @@ struct PairSep<false> : Sep {
     x = dx;
     y = dy;
     z = dz;
-    r = sqrt(dot3(dx, dy, dz, dx, dy, dz));
+    r = square_root(dot3(dx, dy, dz, dx, dy, dz));
   }
 };
 template <>
@@ -284,7 +284,7 @@ __device__ __forceinline__ PairForce pair_force(const DevTable& tb, const double
   const double e2 = dot3(e[0], e[1], e[2], e[0], e[1], e[2]);
   const double p2 = dot3(p[0], p[1], p[2], p[0], p[1], p[2]);
   const double ri1 = rsqrt(e2), ri0 = rsqrt(p2);
-  const double q = 0.5 * (e2 * ri1 + p2 * ri0), qi = 1.0 / q;
+  const double q = 0.5 * (e2 * ri1 + p2 * ri0), qi = reciprocal(q);
   const double sv[3] = {e[0] - p[0], e[1] - p[1], e[2] - p[2]};
   const double s2 = dot3(sv[0], sv[1], sv[2], sv[0], sv[1], sv[2]) * (qi * qi);
   int i;
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kBlock) coulomb_kernel(EstimatorParams P) {
       const double* bj = path + ((size_t)t * np + j) * 3;
       double dx = bi[0] - bj[0], dy = bi[1] - bj[1], dz = bi[2] - bj[2];
       pbc(s, dx, dy, dz);
-      const double r = sqrt(dot3(dx, dy, dz, dx, dy, dz));
+      const double r = square_root(dot3(dx, dy, dz, dx, dy, dz));
       const double qq = s.charge[species_of(s, i)] * s.charge[species_of(s, j)];
       if (!ew) {
         part += qq / (eps * r);

@@ -126,6 +126,108 @@ __device__ __forceinline__ float f32_rn(double v) {
   return __uint_as_float(b | (hi & 0x80000000u));
 }
 
+// 1 / a, correctly rounded, on the integer pipe: Newton's iteration in fixed point
+// from the FP32 reciprocal (24 bits; then 44, then the 62 of the format).  With a =
+// 2^k d, d in (1/2, 1), the last step holds 2^62 / d to 2 units and the result
+// takes 10 fewer bits, so the rounding is certain unless the cut bits lie within 8
+// units of a tie; those 1.6% of values, powers of two, and results that are not
+// normal take the divide instruction sequence.  One FP64 instruction costs the SM
+// 19 clocks, so the 86 of __drcp_rn were a sixth of a factorisation's (n = 10).
+static __device__ __noinline__ double reciprocal_call(double a) { return __drcp_rn(a); }
+__device__ __forceinline__ double reciprocal(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = (hi >> 20) & 0x7ffu;
+  const unsigned long long M = (1ull << 63) | (b << 11);  // d
+  const float f = __uint_as_float(0x3f000000u | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const unsigned rb = __float_as_uint(__fdividef(1.0f, f));
+  const unsigned x0 = ((rb & 0x7fffffu) | 0x800000u) << ((rb >> 23) - 120u);  // 2^30 / d
+  const unsigned long long t =
+      (unsigned long long)(unsigned)(M >> 32) * x0 + (((unsigned long long)(unsigned)M * x0) >> 32);
+  const int e0 = (int)((long long)((1ull << 62) - t) >> 10);
+  const unsigned long long x1 = ((unsigned long long)x0 << 32) +
+                                (unsigned long long)(((long long)(int)(x0 >> 1) * e0) >> 19);
+  const int e1 = (int)((1ull << 62) - __umul64hi(M, x1));
+  const unsigned long long x2 =
+      x1 + (unsigned long long)(((long long)(int)(unsigned)(x1 >> 33) * e1) >> 29) + 512ull;
+  if ((((hi & 0xfffffu) | lo) == 0u) || e - 2u > 2042u || ((unsigned)x2 & 1023u) - 8u > 1008u)
+    return reciprocal_call(a);
+  return __longlong_as_double(
+      (long long)((((unsigned long long)(2045u - e) << 52) + (x2 >> 10) - (1ull << 52)) |
+                  (b & (1ull << 63))));
+}
+
+// sqrt(a), correctly rounded, likewise: a = 4^k d with d in [1, 4), s = d y with the FP32
+// reciprocal root y, then s += (d - s^2) y / 2 twice (22, 44, 61 bits).  143 clocks of
+// the FP64 pipe as an instruction sequence.
+static __device__ __noinline__ double square_root_call(double a) { return sqrt(a); }
+__device__ __forceinline__ double square_root(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
+  const bool even = (hi >> 20) & 1u;  // (of the exponent; the bias is odd)
+  const unsigned long long d = ((b & 0xfffffffffffffull) | (1ull << 52)) << (even ? 10 : 11);
+  const unsigned yb = __float_as_uint(rsqrtf(__uint_as_float(
+      (even ? 0x3f800000u : 0x40000000u) | ((hi & 0xfffffu) << 3) | (lo >> 29))));
+  const unsigned y = ((yb & 0x7fffffu) | 0x800000u) << ((yb >> 23) - 119u);  // 2^31 / sqrt(d)
+  const int y2 = (int)(y >> 1);
+  const unsigned long long s6 = ((unsigned long long)(unsigned)(d >> 32) * y) >> 30;
+  const unsigned s0 = s6 > 0xffffffffull ? 0xffffffffu : (unsigned)s6;
+  const long long e0 = (long long)(d - (unsigned long long)s0 * s0);
+  const unsigned long long s1 = ((unsigned long long)s0 << 31) +
+                                (unsigned long long)(((long long)(int)(e0 >> 14) * y2) >> 17);
+  const unsigned long long plo = s1 * s1, dlo = d << 62;
+  const unsigned long long ehi = (d >> 2) - __umul64hi(s1, s1) - (dlo < plo);
+  const int e1 = (int)((ehi << 10) | ((dlo - plo) >> 54));
+  const unsigned long long s2 = s1 + (unsigned long long)(((long long)e1 * y2) >> 39) + 512ull;
+  // (zero, subnormal, infinite, NaN and negative values)
+  if (hi - 0x00100000u >= 0x7fe00000u || ((unsigned)s2 & 1023u) - 8u > 1008u)
+    return square_root_call(a);
+  return __longlong_as_double((long long)(((unsigned long long)((hi + (1023u << 20)) >> 21) << 52) +
+                                          (s2 >> 10) - (1ull << 52)));
+}
+
+// 2^k, -1023 < k < 1024 (a conversion takes 16 clocks of the FP64 pipe)
+__device__ __forceinline__ double pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+
+// exp(x) by table (P. T. P. Tang, "Table-driven implementation of the exponential
+// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989): x = (64 e + j) ln2 / 64
+// + r, |r| <= ln2 / 128, exp x = 2^e 2^(j/64) (1 + p(r)) with the series to r^5 (r^6 / 720
+// < 2^-54).  Ten FP64 instructions where exp() takes sixteen; within 1 ulp too.
+static __device__ const double kExp2[64] = {
+    1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
+    1.0442737824274138, 1.0556451783605572, 1.0671404006768237, 1.0787607977571199,
+    1.0905077326652577, 1.102382583307841, 1.1143867425958924, 1.1265216186082418,
+    1.1387886347566916, 1.1511892299529827, 1.1637248587775775, 1.1763969916502812,
+    1.189207115002721, 1.202156731452703, 1.215247359980469, 1.22848053610687,
+    1.241857812073484, 1.255380757024691, 1.2690509571917332, 1.2828700160787783,
+    1.2968395546510096, 1.3109612115247644, 1.3252366431597413, 1.339667524053303,
+    1.3542555469368927, 1.3690024229745905, 1.383909881963832, 1.3989796725383112,
+    1.4142135623730951, 1.42961333839197, 1.4451808069770467, 1.460917794180647,
+    1.4768261459394993, 1.4929077282912648, 1.5091644275934228, 1.5255981507445384,
+    1.5422108254079407, 1.559004400237837, 1.5759808451078865, 1.593142151342267,
+    1.6104903319492543, 1.6280274218573478, 1.645755478153965, 1.6636765803267364,
+    1.681792830507429, 1.7001063537185235, 1.718619298122478, 1.7373338352737062,
+    1.7562521603732995, 1.7753764925265212, 1.7947090750031072, 1.8142521755003989,
+    1.8340080864093424, 1.8539791250833855, 1.8741676341103, 1.8945759815869656,
+    1.9152065613971474, 1.9360617934922943, 1.9571441241754002, 1.978456026387951};
+static __device__ __noinline__ double exp_call(double x) { return exp(x); }
+__device__ __forceinline__ double exp_table(double x) {
+  const unsigned m = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if (m >= 0x4085e000u) return exp_call(x);  // |x| >= 700, NaN
+  const double t = __fma_rn(x, 92.33248261689366, 6755399441055744.0);  // (3 2^51: rounds)
+  const double k = __dsub_rn(t, 6755399441055744.0);
+  const int n = __double2loint(t);
+  // ln2 / 64 in two parts, the first of 36 bits
+  double r = __fma_rn(-k, 0.010830424696223417, x);
+  r = __fma_rn(-k, 2.572804622327669e-14, r);
+  double p = __fma_rn(r, 1.0 / 120, 1.0 / 24);
+  p = __fma_rn(r, p, 1.0 / 6);
+  p = __fma_rn(r, p, 0.5);
+  p = __fma_rn(__dmul_rn(r, r), p, r);
+  const double c = __ldg(kExp2 + (n & 63));
+  p = __fma_rn(c, p, c);
+  return __hiloint2double(__double2hiint(p) + ((n >> 6) << 20), __double2loint(p));
+}
+
 // SuperCell::pbc (src/util/SuperCell.cc:25-34): minimum image, only applied
 // when |v|^2 exceeds a quarter of the shortest side squared.
 static __device__ __noinline__ double3 pbc_exact(const DevSys& s, double x, double y, double z) {
@@ -250,11 +352,11 @@ __device__ __forceinline__ double pg_eval(double nome, double pref, double k, in
 // relative to the Gaussian itself; returns 1 + r + rf and the bracket of the
 // derivative, (L - |x|) r - |x| - (L + |x|) rf.
 __device__ __forceinline__ double pg_axis(double al, double cell, double c, double ax, double& h) {
-  const double r = exp(__dmul_rn(-al, __fma_rn(-2.0, ax, cell)));
+  const double r = exp_table(__dmul_rn(-al, __fma_rn(-2.0, ax, cell)));
   double p = __dadd_rn(1.0, r);
   h = __fma_rn(__dsub_rn(cell, ax), r, -ax);
   if (c > 0.0) {
-    const double rf = __dmul_rn(c, __drcp_rn(r));  // r rf = exp(-2 alpha L^2)
+    const double rf = __dmul_rn(c, reciprocal(r));  // r rf = exp(-2 alpha L^2)
     p = __dadd_rn(p, rf);
     h = __fma_rn(-__dadd_rn(cell, ax), rf, h);
   }
@@ -282,7 +384,7 @@ __device__ __forceinline__ double with_sign_of(double v, double x) {
 __device__ __forceinline__ double pg_images_eval(const DevSys& s, int sp, double x, double y,
                                                  double z, double& gx, double& gy, double& gz) {
   const double al = s.pg_alpha[sp];
-  const double e = exp(__dmul_rn(-al, dot3(x, y, z, x, y, z)));
+  const double e = exp_table(__dmul_rn(-al, dot3(x, y, z, x, y, z)));
   double hx, hy, hz;
   const double px = pg_axis(s.pg_al[sp][0], s.cell[0], s.pg_c[sp][0], fabs(x), hx);
   const double py = pg_axis(s.pg_al[sp][1], s.cell[1], s.pg_c[sp][1], fabs(y), hy);
@@ -332,12 +434,22 @@ __device__ __forceinline__ void tab_locate(const DevTable& t, double q, int& i, 
     x = q >= 1 ? log_call(q) * t.logrratioinv : 0.0;
     if (!(x < 2e9)) x = 2e9;
   }
-  i = max((int)x, 0);
+  // the integer part by masks (x < 2^21; a conversion there and back takes 32 clocks)
+  const int hi = __double2hiint(x), e = (hi >> 20) - 1023;
+  double whole = 0.0;
+  i = 0;
+  if (hi >= 0x41400000) {
+    i = (int)x;
+    whole = i;
+  } else if (e >= 0) {  // (a negative x has a negative e)
+    i = ((hi & 0xfffff) | 0x100000) >> (20 - e);
+    whole = __hiloint2double(hi & ~(0xfffff >> e), 0);
+  }
   if (i > t.ngpts - 2) {
     i = t.ngpts - 2;
     x = 1;
   } else {
-    x -= i;
+    x -= whole;
   }
 }
 

@@ -94,36 +94,6 @@ __device__ __forceinline__ int small_div(int a, int m) {
   return (int)(((unsigned)a * kSmallReciprocals.v[m]) >> 16);
 }
 
-// 1 / a, correctly rounded, on the integer pipe: Newton's iteration in fixed point
-// from the FP32 reciprocal (24 bits; then 44, then the 62 of the format).  With a =
-// 2^k d, d in (1/2, 1), the last step holds 2^62 / d to 2 units and the result
-// takes 10 fewer bits, so the rounding is certain unless the cut bits lie within 8
-// units of a tie; those 1.6% of values, powers of two, and results that are not
-// normal take the divide instruction sequence.  One FP64 instruction costs the SM
-// 19 clocks, so the 86 of __drcp_rn were a sixth of a factorisation's (n = 10).
-static __device__ __noinline__ double reciprocal_call(double a) { return __drcp_rn(a); }
-__device__ __forceinline__ double reciprocal(double a) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = (hi >> 20) & 0x7ffu;
-  const unsigned long long M = (1ull << 63) | (b << 11);  // d
-  const float f = __uint_as_float(0x3f000000u | ((hi & 0xfffffu) << 3) | (lo >> 29));
-  const unsigned rb = __float_as_uint(__fdividef(1.0f, f));
-  const unsigned x0 = ((rb & 0x7fffffu) | 0x800000u) << ((rb >> 23) - 120u);  // 2^30 / d
-  const unsigned long long t =
-      (unsigned long long)(unsigned)(M >> 32) * x0 + (((unsigned long long)(unsigned)M * x0) >> 32);
-  const int e0 = (int)((long long)((1ull << 62) - t) >> 10);
-  const unsigned long long x1 = ((unsigned long long)x0 << 32) +
-                                (unsigned long long)(((long long)(int)(x0 >> 1) * e0) >> 19);
-  const int e1 = (int)((1ull << 62) - __umul64hi(M, x1));
-  const unsigned long long x2 =
-      x1 + (unsigned long long)(((long long)(int)(unsigned)(x1 >> 33) * e1) >> 29) + 512ull;
-  if ((((hi & 0xfffffu) | lo) == 0u) || e - 2u > 2042u || ((unsigned)x2 & 1023u) - 8u > 1008u)
-    return reciprocal_call(a);
-  return __longlong_as_double(
-      (long long)((((unsigned long long)(2045u - e) << 52) + (x2 >> 10) - (1ull << 52)) |
-                  (b & (1ull << 63))));
-}
-
 // ------------------------------------------------------------------ node model
 // The mixed form's Sherman-Morrison updates of cached inverses: at most
 // kSmRefresh updates between two factorisations of a slice pair's matrix, and
