@@ -742,7 +742,7 @@ def kernel_source_sha():
     below belongs to the kernel these files build."""
     d = os.path.join(REPO, "pi-qmc_gb300", "csrc")
     h = hashlib.sha256()
-    for f in ("section_kernel.cuh", "actions.cuh", "kernels.cuh", "pimc_device.cuh", "pimc_rng.h",
+    for f in ("section_kernel.cuh", "actions.cuh", "kernels.cuh", "pimc_device.cuh", "fixed_point.cuh", "pimc_rng.h",
               "section_variants.cu"):
         h.update(f.encode())
         h.update(open(os.path.join(d, f), "rb").read())

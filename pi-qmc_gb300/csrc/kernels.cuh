@@ -251,12 +251,13 @@ static __device__ __noinline__ void store_section(const DevSys& s, double* path,
 // pairs 2 ord and 2 ord + 1 and uses the first three values.  Both precision
 // forms draw the same FP64 normals, so a mixed-form chain makes the FP64
 // chain's proposals and its action differences can be compared with the FP64
-// form's on identical moves.  Whole warps draw the first or the second pairs.
+// form's on identical moves.
 static __device__ __noinline__ void attempt_normals(const DevSys& s, const Smem& m, uint64_t seed,
                                        uint32_t rep, uint32_t att) {
   // (with delayed rejection one more: the second proposal at level nlevel - 1
   // takes order 1, the slices after it one order later)
-  const int nord = (1 << s.nlevel) - 1 + (s.dr ? 1 : 0), pad = (nord + 31) & ~31;
+  // (the second pairs start on a half-warp: up to 16 slices' pairs take one warp)
+  const int nord = (1 << s.nlevel) - 1 + (s.dr ? 1 : 0), pad = (nord + 15) & ~15;
 #pragma unroll 1
   for (int it = threadIdx.x; it < 2 * pad; it += blockDim.x) {
     const int second = it >= pad, o = it - second * pad;

@@ -126,68 +126,6 @@ __device__ __forceinline__ float f32_rn(double v) {
   return __uint_as_float(b | (hi & 0x80000000u));
 }
 
-// 1 / a, correctly rounded, on the integer pipe: Newton's iteration in fixed point
-// from the FP32 reciprocal (24 bits; then 44, then the 62 of the format).  With a =
-// 2^k d, d in (1/2, 1), the last step holds 2^62 / d to 2 units and the result
-// takes 10 fewer bits, so the rounding is certain unless the cut bits lie within 8
-// units of a tie; those 1.6% of values, powers of two, and results that are not
-// normal take the divide instruction sequence.  One FP64 instruction costs the SM
-// 19 clocks, so the 86 of __drcp_rn were a sixth of a factorisation's (n = 10).
-static __device__ __noinline__ double reciprocal_call(double a) { return __drcp_rn(a); }
-__device__ __forceinline__ double reciprocal(double a) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b, e = (hi >> 20) & 0x7ffu;
-  const unsigned long long M = (1ull << 63) | (b << 11);  // d
-  const float f = __uint_as_float(0x3f000000u | ((hi & 0xfffffu) << 3) | (lo >> 29));
-  const unsigned rb = __float_as_uint(__fdividef(1.0f, f));
-  const unsigned x0 = ((rb & 0x7fffffu) | 0x800000u) << ((rb >> 23) - 120u);  // 2^30 / d
-  const unsigned long long t =
-      (unsigned long long)(unsigned)(M >> 32) * x0 + (((unsigned long long)(unsigned)M * x0) >> 32);
-  const int e0 = (int)((long long)((1ull << 62) - t) >> 10);
-  const unsigned long long x1 = ((unsigned long long)x0 << 32) +
-                                (unsigned long long)(((long long)(int)(x0 >> 1) * e0) >> 19);
-  const int e1 = (int)((1ull << 62) - __umul64hi(M, x1));
-  const unsigned long long x2 =
-      x1 + (unsigned long long)(((long long)(int)(unsigned)(x1 >> 33) * e1) >> 29) + 512ull;
-  if ((((hi & 0xfffffu) | lo) == 0u) || e - 2u > 2042u || ((unsigned)x2 & 1023u) - 8u > 1008u)
-    return reciprocal_call(a);
-  return __longlong_as_double(
-      (long long)((((unsigned long long)(2045u - e) << 52) + (x2 >> 10) - (1ull << 52)) |
-                  (b & (1ull << 63))));
-}
-
-// sqrt(a), correctly rounded, likewise: a = 4^k d with d in [1, 4), s = d y with the FP32
-// reciprocal root y, then s += (d - s^2) y / 2 twice (22, 44, 61 bits).  143 clocks of
-// the FP64 pipe as an instruction sequence.
-static __device__ __noinline__ double square_root_call(double a) { return sqrt(a); }
-__device__ __forceinline__ double square_root(double a) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
-  const bool even = (hi >> 20) & 1u;  // (of the exponent; the bias is odd)
-  const unsigned long long d = ((b & 0xfffffffffffffull) | (1ull << 52)) << (even ? 10 : 11);
-  const unsigned yb = __float_as_uint(rsqrtf(__uint_as_float(
-      (even ? 0x3f800000u : 0x40000000u) | ((hi & 0xfffffu) << 3) | (lo >> 29))));
-  const unsigned y = ((yb & 0x7fffffu) | 0x800000u) << ((yb >> 23) - 119u);  // 2^31 / sqrt(d)
-  const int y2 = (int)(y >> 1);
-  const unsigned long long s6 = ((unsigned long long)(unsigned)(d >> 32) * y) >> 30;
-  const unsigned s0 = s6 > 0xffffffffull ? 0xffffffffu : (unsigned)s6;
-  const long long e0 = (long long)(d - (unsigned long long)s0 * s0);
-  const unsigned long long s1 = ((unsigned long long)s0 << 31) +
-                                (unsigned long long)(((long long)(int)(e0 >> 14) * y2) >> 17);
-  const unsigned long long plo = s1 * s1, dlo = d << 62;
-  const unsigned long long ehi = (d >> 2) - __umul64hi(s1, s1) - (dlo < plo);
-  const int e1 = (int)((ehi << 10) | ((dlo - plo) >> 54));
-  const unsigned long long s2 = s1 + (unsigned long long)(((long long)e1 * y2) >> 39) + 512ull;
-  // (zero, subnormal, infinite, NaN and negative values)
-  if (hi - 0x00100000u >= 0x7fe00000u || ((unsigned)s2 & 1023u) - 8u > 1008u)
-    return square_root_call(a);
-  return __longlong_as_double((long long)(((unsigned long long)((hi + (1023u << 20)) >> 21) << 52) +
-                                          (s2 >> 10) - (1ull << 52)));
-}
-
-// 2^k, -1023 < k < 1024 (a conversion takes 16 clocks of the FP64 pipe)
-__device__ __forceinline__ double pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
-
 // exp(x) by table (P. T. P. Tang, "Table-driven implementation of the exponential
 // function in IEEE floating-point arithmetic", ACM TOMS 15, 1989): x = (64 e + j) ln2 / 64
 // + r, |r| <= ln2 / 128, exp x = 2^e 2^(j/64) (1 + p(r)) with the series to r^5 (r^6 / 720

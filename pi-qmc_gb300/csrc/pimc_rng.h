@@ -17,11 +17,14 @@
 // what lets the CPU oracle replay exactly the proposals a kernel made.
 // log() is the atanh series log(m) = 2 atanh((m-1)/(m+1)) (Abramowitz & Stegun
 // 4.1.27) after an exact power-of-two split; sin/cos are Taylor series after an
-// exact quarter-turn reduction of the uniform itself.
+// exact quarter-turn reduction of the uniform itself.  On the device the exact steps
+// (conversions, splits, the reduction) are integer arithmetic, and so are the
+// division and the square root: 83 FP64 instructions a pair -> 54.
 #pragma once
 #include <stdint.h>
 
 #if defined(__CUDACC__)
+#include "fixed_point.cuh"
 #define PIMC_HD __host__ __device__ __forceinline__
 #else
 #define PIMC_HD static inline
@@ -32,8 +35,8 @@
 #define PR_SUB(a, b) __dsub_rn((a), (b))
 #define PR_MUL(a, b) __dmul_rn((a), (b))
 #define PR_FMA(a, b, c) __fma_rn((a), (b), (c))
-#define PR_DIV(a, b) __ddiv_rn((a), (b))
-#define PR_SQRT(a) __dsqrt_rn(a)
+#define PR_DIV(a, b) divide((a), (b))
+#define PR_SQRT(a) square_root(a)
 #else
 #include <math.h>
 #define PR_ADD(a, b) ((a) + (b))
@@ -88,7 +91,11 @@ PIMC_HD Philox4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3
 // 53 random bits -> uniform double in [0, 1); exact.
 PIMC_HD double u53(uint32_t hi, uint32_t lo) {
   const uint64_t x = (((uint64_t)hi << 32) | (uint64_t)lo) >> 11;
+#if defined(__CUDA_ARCH__)
+  return scaled_integer(x, -53);
+#else
   return (double)x * 1.1102230246251565404e-16;  // 2^-53
+#endif
 }
 
 enum : uint32_t { kStreamUniform = 0u, kStreamNormal = 1u };
@@ -110,11 +117,11 @@ PIMC_HD double portable_log(double v) {
   c.d = v;
   int e = (int)((c.u >> 52) & 0x7ff) - 1023;
   c.u = (c.u & 0x000fffffffffffffull) | 0x3ff0000000000000ull;  // m in [1,2)
-  double m = c.d;
-  if (m > 1.4142135623730951) {
-    m = PR_MUL(m, 0.5);
+  if (c.u > 0x3ff6a09e667f3bcdull) {  // m > 1.4142135623730951: m / 2
+    c.u -= 1ull << 52;
     e += 1;
   }
+  const double m = c.d;
   const double s = PR_DIV(PR_SUB(m, 1.0), PR_ADD(m, 1.0));
   const double s2 = PR_MUL(s, s);
   double p = (1.0 / 23.0);
@@ -132,16 +139,26 @@ PIMC_HD double portable_log(double v) {
   const double logm = PR_FMA(PR_MUL(t, s2), p, t);        // 2s + 2s^3 p(s^2)
   const double LN2_HI = 6.93147180369123816490e-01;       // ln 2, high 32 bits
   const double LN2_LO = 1.90821492927058770002e-10;       // ln 2 - LN2_HI
+#if defined(__CUDA_ARCH__)
+  const double de = scaled_integer((unsigned)abs(e), 0, e < 0);
+#else
   const double de = (double)e;
+#endif
   return PR_ADD(PR_MUL(de, LN2_HI), PR_FMA(de, LN2_LO, logm));
 }
 
 // cos(2 pi u), sin(2 pi u) for u in [0,1): quarter-turn reduction is exact
 // because u is a multiple of 2^-53; |x| <= pi/4 after it.
-PIMC_HD void portable_cossin_2pi(double u, double* cs, double* sn) {
-  const double t = PR_MUL(u, 4.0);  // exact
-  double q = (double)(int)(PR_ADD(t, 0.5));
-  const double f = PR_SUB(t, q);    // exact, in [-0.5, 0.5]
+PIMC_HD void portable_cossin_2pi(uint64_t k, double* cs, double* sn) {  // u = k 2^-53
+#if defined(__CUDA_ARCH__)
+  const int iq = (int)((k + (1ull << 50)) >> 51);
+  const long long r = (long long)k - ((long long)iq << 51);
+  const double f = scaled_integer((unsigned long long)(r < 0 ? -r : r), -51, r < 0);
+#else
+  const double t = PR_MUL((double)k * 1.1102230246251565404e-16, 4.0);  // exact
+  const int iq = (int)(PR_ADD(t, 0.5));
+  const double f = PR_SUB(t, (double)iq);  // exact, in [-0.5, 0.5]
+#endif
   const double HALF_PI = 1.57079632679489661923;
   const double x = PR_MUL(f, HALF_PI);
   const double x2 = PR_MUL(x, x);
@@ -170,14 +187,13 @@ PIMC_HD void portable_cossin_2pi(double u, double* cs, double* sn) {
   pc = PR_FMA(pc, x2, (1.0 / 24.0));                    // 1/4!
   pc = PR_FMA(pc, x2, -0.5);
   const double c = PR_FMA(x2, pc, 1.0);
-  const int iq = ((int)q) & 3;
-  if (iq == 0) {
+  if ((iq & 3) == 0) {
     *cs = c;
     *sn = s;
-  } else if (iq == 1) {
+  } else if ((iq & 3) == 1) {
     *cs = -s;
     *sn = c;
-  } else if (iq == 2) {
+  } else if ((iq & 3) == 2) {
     *cs = -c;
     *sn = -s;
   } else {
@@ -191,11 +207,16 @@ PIMC_HD void stream_normal_pair(uint64_t seed, uint32_t replica, uint32_t attemp
                                 uint32_t pair, double* z0, double* z1) {
   const Philox4 b = philox4x32_10(pair, attempt, replica, kStreamNormal,
                                   (uint32_t)seed, (uint32_t)(seed >> 32));
-  const double u1 = u53(b.v[0], b.v[1]);
-  const double u2 = u53(b.v[2], b.v[3]);
-  const double rad = PR_SQRT(PR_MUL(-2.0, portable_log(PR_SUB(1.0, u1))));
+  const uint64_t k1 = (((uint64_t)b.v[0] << 32) | b.v[1]) >> 11;
+  const uint64_t k2 = (((uint64_t)b.v[2] << 32) | b.v[3]) >> 11;
+#if defined(__CUDA_ARCH__)
+  const double v1 = scaled_integer((1ull << 53) - k1, -53);
+#else
+  const double v1 = PR_SUB(1.0, (double)k1 * 1.1102230246251565404e-16);  // 1 - u1, exact
+#endif
+  const double rad = PR_SQRT(PR_MUL(-2.0, portable_log(v1)));
   double c, s;
-  portable_cossin_2pi(u2, &c, &s);
+  portable_cossin_2pi(k2, &c, &s);
   *z0 = PR_MUL(rad, c);
   *z1 = PR_MUL(rad, s);
 }
