@@ -21,7 +21,7 @@
 //    particles' rows and columns are new when the cached matrix is whole; an
 //    accepted move updates the cached entries instead of dropping them.
 // Four attempts of 19 electron gases (N = 54, M = 512, Ewald, 27 x 27 nodes): 504 ms
-// with one CTA per replica and full sums, 11.1 ms.
+// with one CTA per replica and full sums, now 9.4 ms.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -224,12 +224,13 @@ static __device__ __noinline__ double displace_ewald(const DevSys& s, const Move
   for (int t0 = gw * batch; t0 < M; t0 += ngw * batch) {
     const int nt = min(batch, M - t0);
     __syncwarp();
-    for (int c = lane; c < 2 * nmov * nt; c += 32) {
+    for (int it = lane; it < 6 * nmov * nt; it += 32) {  // (an axis per lane)
+      const int c = it / 3, a = it - 3 * c;
       const int t = t0 + c / (2 * nmov), k = (c % (2 * nmov)) >> 1;
       const double* b = path + ((size_t)t * s.npart + mv.p[k]) * 3;
       double x = b[0], y = b[1], z = b[2];
       if (c & 1) displaced_bead(s, mv, path, mv.p[k], t, x, y, z);
-      ewald_bead_tables(s, X, Y, Z, w, c, x, y, z);
+      ewald_axis_table(s, (a == 0 ? X : (a == 1 ? Y : Z)) + c, w, a, a == 0 ? x : (a == 1 ? y : z));
     }
     __syncwarp();
     for (int it = lane; it < nt * totk; it += 32) {
@@ -242,21 +243,24 @@ static __device__ __noinline__ double displace_ewald(const DevSys& s, const Move
       for (int im = 0; im < nmov; ++im) {
         const int col = (tt * nmov + im) * 2;
         long long are, aim, bre, bim;
-        ewald_term_fixed(s, X, Y, Z, w, col, kx, ky, kz, qpart[mv.p[im]], are, aim);
-        ewald_term_fixed(s, X, Y, Z, w, col + 1, kx, ky, kz, qpart[mv.p[im]], bre, bim);
+        const double qs = __dmul_rn(qpart[mv.p[im]], s.ek_scale);
+        ewald_term_fixed(s, X, Y, Z, w, col, kx, ky, kz, qs, are, aim);
+        ewald_term_fixed(s, X, Y, Z, w, col + 1, kx, ky, kz, qs, bre, bim);
         n.x += bre - are;
         n.y += bim - aim;
       }
       if (commit) {
         *at = n;
       } else {
-        const double ore = __ll2double_rn(o.x) * is, oim = __ll2double_rn(o.y) * is;
-        const double rre = __ll2double_rn(n.x) * is, rim = __ll2double_rn(n.y) * is;
-        acc += 2 * __ldg(s.vk + k) * ((rre * rre + rim * rim) - (ore * ore + oim * oim));
+        // |rho'|^2 - |rho|^2 = (rho' - rho) . (rho' + rho)
+        acc = __fma_rn(__ldg(s.vk + k),
+                       __fma_rn(__ll2double_rn(n.x - o.x), __ll2double_rn(n.x + o.x),
+                                __dmul_rn(__ll2double_rn(n.y - o.y), __ll2double_rn(n.y + o.y))),
+                       acc);
       }
     }
   }
-  return acc;
+  return acc * (2 * is * is);
 }
 
 // The same without cached structure factors: evalLongRange of both configurations

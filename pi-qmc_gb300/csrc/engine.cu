@@ -1803,13 +1803,21 @@ namespace {
 // warps, and when the whole scratch would keep fewer than 16 warps on an SM (the FP64
 // pipe wants as many), its cold part goes to global memory.
 struct NodeEvalShape {
+  int width;  // of the lane groups
   int grid, warps, stage, scratch, cold;  // cold: doubles per warp in global memory (0: none)
   size_t smem;
 };
 NodeEvalShape node_eval_shape(const DevSys& s, int ispec, int nbatch, int num_sms) {
-  const int n = s.spec_count[ispec], G = 32 / node_group_width(n);
+  const int n = s.spec_count[ispec];
   const bool fr = s.node_kind[ispec] == PIMC_NODES_FREE;
   NodeEvalShape r{};
+  // wider lane groups while every warp still has an SM's quarter to itself: the call
+  // then takes as long as one matrix's chain of operations (one 10 x 10: 56.8 -> 49.0 us a call)
+  r.width = node_group_width(n);
+  while (r.width < node_group_widest(n) &&
+         (long long)nbatch * 2 * r.width <= 32LL * 4 * num_sms)
+    r.width *= 2;
+  const int G = 32 / r.width;
   const long long warps = (nbatch + G - 1) / G;
   r.stage = G * 6 * n;
   r.scratch = (G * node_group_scratch(n, fr) + 1) & ~1;
@@ -1916,6 +1924,7 @@ int pimc_node_evaluate(pimc_engine* e, int ispec, int nbatch, const double* r1, 
   P.err = io.dev<int>(oerr);
   P.ispec = ispec;
   P.nbatch = nbatch;
+  P.width = sh.width;
   P.stage_stride = sh.stage;
   P.scratch_stride = sh.scratch;
   P.cold_stride = sh.cold;

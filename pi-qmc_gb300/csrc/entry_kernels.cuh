@@ -818,6 +818,7 @@ struct NodeEvalParams {
   int* err;
   int ispec;
   int nbatch;
+  int width;           // of the lane groups
   int stage_stride;    // doubles of staged beads per warp
   int scratch_stride;  // of Slater scratch per warp (its hot part when split)
   double* cold;        // the scratch's cold parts in global memory (null: not split)
@@ -840,7 +841,7 @@ __global__ void __launch_bounds__(kBlock) node_eval_kernel(NodeEvalParams P) {
   const DevSys& s = S;
   const int np = s.npart, sp = P.ispec, n = s.spec_count[sp], f = s.spec_first[sp];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const int W = node_group_width(n), G = 32 / W, g = lane / W, gl = lane & (W - 1);
+  const int W = P.width, G = 32 / W, g = lane / W, gl = lane & (W - 1);
   const bool free_nodes = s.node_kind[sp] != PIMC_NODES_SHO;
   const long long gw = (long long)blockIdx.x * nwarps + warp;
   double* st = smem + (size_t)warp * P.stage_stride + (size_t)g * 6 * n;

@@ -652,7 +652,8 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     ntask = 0;
 #pragma unroll 1
     for (int sp = 0; sp < s.nspecies; ++sp) {
-      const int G = 32 / max(wmin, node_group_width(s.spec_count[sp]));
+      const int n = s.spec_count[sp];
+      const int G = 32 / min(max(wmin, node_group_width(n)), node_group_widest(n));
       first[sp] = ntask;
       ntask += (nmiss[sp] + G - 1) / G;
     }
@@ -666,7 +667,8 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     while (wt >= first[sp + 1]) ++sp;
     const int n = s.spec_count[sp];
     const bool sho = s.node_kind[sp] == PIMC_NODES_SHO, mine = sp == msp;
-    const int W = max(wmin, node_group_width(n)), G = 32 / W, gm = lane / W, glm = lane & (W - 1);
+    const int W = min(max(wmin, node_group_width(n)), node_group_widest(n));
+    const int G = 32 / W, gm = lane / W, glm = lane & (W - 1);
     const int base = (wt - first[sp]) * G;
     const int task = base + gm;
     const bool act = task < nmiss[sp];
@@ -880,7 +882,7 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   // narrow groups' fewer instructions count).
   if (m.wide) {
     const int most = a0 == 0 || alo > ahi ? nwarps : a0;
-    while (W < 32 && ntask * W <= 16 * most) W *= 2;
+    while (W < node_group_widest(n) && ntask * W <= 16 * most) W *= 2;
   }
   const int G = 32 / W, g = lane / W, nodeW = min(nwarps, (ntask + G - 1) / G);
   if (mynode) {

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fixed_point.cuh"
 #include "pimc_rng.h"
 
 namespace pimc {
@@ -163,7 +164,7 @@ __device__ __forceinline__ double exp_table(double x) {
   p = __fma_rn(__dmul_rn(r, r), p, r);
   const double c = __ldg(kExp2 + (n & 63));
   p = __fma_rn(c, p, c);
-  return __hiloint2double(__double2hiint(p) + ((n >> 6) << 20), __double2loint(p));
+  return __hiloint2double(__double2hiint(p) + (int)((unsigned)(n >> 6) << 20), __double2loint(p));
 }
 
 // SuperCell::pbc (src/util/SuperCell.cc:25-34): minimum image, only applied

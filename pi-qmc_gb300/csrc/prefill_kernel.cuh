@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kBlock) ewald_prefill_kernel(EkPrefillParams P
     long long re = 0, im = 0;
     for (int j = 0; j < np; ++j) {
       long long a, b;
-      ewald_term_fixed(s, X, Y, Z, w, j, kx, ky, kz, q[j], a, b);
+      ewald_term_fixed(s, X, Y, Z, w, j, kx, ky, kz, __dmul_rn(q[j], s.ek_scale), a, b);
       re += a;
       im += b;
     }

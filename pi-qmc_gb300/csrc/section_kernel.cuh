@@ -812,6 +812,12 @@ static __device__ __noinline__ void node_eval_group(const DevSys& s, int sp, con
 __host__ __device__ __forceinline__ int node_group_width(int n) {
   return n <= 8 ? 8 : (n <= 16 ? 16 : 32);
 }
+// The widest lane group worth its longer reductions: one that n x n elements fill.
+__host__ __device__ __forceinline__ int node_group_widest(int n) {
+  int w = node_group_width(n);
+  while (w < 32 && n * n > 2 * w) w *= 2;
+  return w;
+}
 
 // One warp evaluates one slice pair (the entry-point kernels).
 static __device__ void node_eval_warp(const DevSys& s, int sp, const SliceView& v1, const SliceView& v2,
@@ -872,16 +878,17 @@ static __device__ __forceinline__ void ewald_bead_tables(const DevSys& s, double
 }
 
 // q e^{ik.r} of table column col for k-vector k, on the fixed-point grid of the
-// structure-factor cache (rounded to the nearest multiple of 1/ek_scale).
+// structure-factor cache (rounded to the nearest multiple of 1/ek_scale; qs = q ek_scale,
+// exact, as the scale is a power of two).
 static __device__ __forceinline__ void ewald_term_fixed(const DevSys& s, const double2* X,
                                                         const double2* Y, const double2* Z,
                                                         int w, int col, int kx, int ky, int kz,
-                                                        double q, long long& re, long long& im) {
+                                                        double qs, long long& re, long long& im) {
   const double2 a = X[kx * w + col];
-  const double2 t = make_double2(__dmul_rn(q, a.x), __dmul_rn(q, a.y));
+  const double2 t = make_double2(__dmul_rn(qs, a.x), __dmul_rn(qs, a.y));
   const double2 v = cmul_rn(cmul_rn(t, Y[ky * w + col]), Z[kz * w + col]);
-  re = __double2ll_rn(__dmul_rn(v.x, s.ek_scale));
-  im = __double2ll_rn(__dmul_rn(v.y, s.ek_scale));
+  re = __double2ll_rn(v.x);
+  im = __double2ll_rn(v.y);
 }
 
 // EwaldSum::evalLongRange (src/util/EwaldSum.cc:103-181) for the old and the

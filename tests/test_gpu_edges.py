@@ -371,3 +371,17 @@ def test_lane_group_widths(pimc, counts, mixed):
         rec = c.run_sections(natt, records=True)
         assert np.array_equal(rec["reject_level"][0], ref["reject_level"])
         assert np.abs(c.download_paths()[0] - port.get_path()).max() <= 1e-10
+
+
+@pytest.mark.parametrize("n", [3, 8, 9, 17])
+def test_node_evaluate_widths(pimc, n):
+    # Small batches take wider lane groups than large ones: the same values, bit for bit.
+    kw = W.dot20_fn(counts=[n, 1], nslice=64, beta=64 / 25.6, nlevel=4)
+    e = pimc.Engine(kw, 1, pimc.coulomb_tables(kw)[0])
+    rng = np.random.default_rng(n)
+    r1 = rng.normal(size=(5000, n + 1, 3))
+    r2 = r1 + 0.05 * rng.normal(size=r1.shape)
+    ref = e.node_evaluate(0, r1, r2)
+    for b in (1, 3, 150, 700, 1300):
+        for x, y in zip(e.node_evaluate(0, r1[:b], r2[:b]), ref):
+            assert np.array_equal(x, y[:b])
