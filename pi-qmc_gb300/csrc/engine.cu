@@ -195,7 +195,7 @@ struct pimc_engine {
   int graph_attempts = -1, graph_steps = -1;
   Layout lay{};
   Layout est_lay{};  // estimator kernels
-  bool half_block = false;  // the creation rule's choice, not a configured one
+  int displace_block = 0;  // displacements' block while none is configured
   LayoutOpts lay_opts{};
   int ctas_cap = 0;
   int minb = 2;  // register-budget variant of the section kernel
@@ -951,6 +951,11 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
       fixed |= d.fixed_node != 0;
     }
     e->block = fixed ? kBlock : (items <= 64 ? 64 : (items <= 128 ? 128 : kBlock));
+    e->displace_block = e->block;
+    // The smallest take one warp, without barriers between two, where replicas fill the
+    // SMs' 16 warps (32 attempts of 4864 dots of 2, 3 and 4 electrons, L = 4: 4.4, 7.7 and
+    // 8.9 ms with two, 4.0, 6.1 and 7.4 with one; 608 of two: 0.76 and 0.81).
+    if (!fixed && items <= 64 && nrep >= 8 * nsm) e->block = 32;
   }
   for (DevSys& d : e->hsys) d.mixed = precision == PIMC_PREC_MIXED;
   e->nodes = false;
@@ -1015,7 +1020,6 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
     const int hocc = ok ? section_occupancy(e->minb, half, hl.total * 8, e->nodes) : 0;
     if (hocc > 1 && hl.nodescr_in_smem) {
       e->block = half;
-      e->half_block = true;
       e->lay = hl;
       occ = hocc;
     }
@@ -1626,7 +1630,7 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
     if (d.fixed_node && (d.nslice % 2)) return fail(PIMC_ERR_INVALID, "odd nslice");
   }
   if (nattempt == 0) return PIMC_OK;
-  const int dthreads = e->half_block ? kBlock : std::min(e->block, kBlock), nwarps = dthreads / 32;
+  const int dthreads = std::min(e->displace_block ? e->displace_block : e->block, kBlock), nwarps = dthreads / 32;
   DisplaceLayout L;
   if (!displace_layout(e->hsys, nwarps, nmoving, L))
     return fail(PIMC_ERR_CAPACITY, "displacement working set too large");
@@ -2060,7 +2064,7 @@ int apply_config(pimc_engine* e, int block, LayoutOpts opts, int ctas_cap, int m
   e->ctas_cap = ctas_cap;
   e->minb = minb;
   e->block = block;
-  e->half_block = false;
+  e->displace_block = 0;
   e->grid = grid;
   if (e->graph) {  // captured with the old launch shape
     cudaGraphExecDestroy(e->graph);
