@@ -121,17 +121,17 @@ def sweep_attempts(kw):
 MEASURED_WORK = {
     # launch shape of the count (block, scratch placement, register variant):
     # the DRAM bytes depend on the scratch placement, the flops do not
-    ("dot20_fn", "mixed"): dict(fp64=3.220e5, fp32=1.895e5, dram=1.082e5, shape="256,0,2",
-                                sha="6f18248147df49dd"),
-    ("dot20_fn", "fp64"): dict(fp64=6.504e5, fp32=4.475e3, dram=1.141e5, shape="256,2,2",
-                               sha="6f18248147df49dd"),
+    ("dot20_fn", "mixed"): dict(fp64=2.346e5, fp32=1.716e5, dram=1.366e5, shape="256,0,2",
+                                sha="f954a30c7f94b354"),
+    ("dot20_fn", "fp64"): dict(fp64=3.786e5, fp32=1.916e4, dram=1.388e5, shape="256,0,2",
+                               sha="f954a30c7f94b354"),
     # counted on the first 1024 replicas of the mix
-    ("batch4096", "mixed"): dict(fp64=1.474e5, fp32=8.393e4, dram=3.358e4, shape="128,2,2",
-                                 sha="6f18248147df49dd"),
-    ("heg54", "mixed"): dict(fp64=1.891e6, fp32=5.344e5, dram=3.924e6, shape="512,1,1",
-                             sha="6f18248147df49dd"),
-    ("dot2", "fp64"): dict(fp64=1.760e4, fp32=164.4, dram=558.3, shape="32,0,3",
-                           sha="6f18248147df49dd"),
+    ("batch4096", "mixed"): dict(fp64=1.155e5, fp32=9.592e4, dram=3.481e4, shape="128,0,2",
+                                 sha="f954a30c7f94b354"),
+    ("heg54", "mixed"): dict(fp64=9.469e5, fp32=4.857e5, dram=2.198e6, shape="256,0,2",
+                             sha="f954a30c7f94b354"),
+    ("dot2", "fp64"): dict(fp64=9.148e3, fp32=1.167e3, dram=476.6, shape="32,0,2",
+                           sha="f954a30c7f94b354"),
 }
 
 
@@ -742,8 +742,8 @@ def kernel_source_sha():
     below belongs to the kernel these files build."""
     d = os.path.join(REPO, "pi-qmc_gb300", "csrc")
     h = hashlib.sha256()
-    for f in ("section_kernel.cuh", "actions.cuh", "kernels.cuh", "pimc_device.cuh", "fixed_point.cuh", "pimc_rng.h",
-              "section_variants.cu"):
+    for f in ("section_kernel.cuh", "actions.cuh", "kernels.cuh", "pimc_device.cuh",
+              "fixed_point.cuh", "pimc_rng.h", "section_variants.cu"):
         h.update(f.encode())
         h.update(open(os.path.join(d, f), "rb").read())
     return h.hexdigest()[:16]
