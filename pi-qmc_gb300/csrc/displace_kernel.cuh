@@ -463,6 +463,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
   const int cluster = blockIdx.x / C;
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gw = rank * nwarps + warp, ngw = C * nwarps;
+  cl.sync();  // every CTA has started: its shared memory may be written to
   for (int turn = 0;; ++turn) {
     if (threadIdx.x == 0 && rank == 0) {
       const int k = atomicAdd(P.next, 1);
