@@ -1,0 +1,55 @@
+"""What callers rely on beyond the values themselves: inputs that are accepted, and
+results that do not depend on what else a call or an engine holds."""
+import numpy as np
+import pytest
+
+import oracle_lib as O
+import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def pimc():
+    import pimc_gb300
+    pimc_gb300.build.build()
+    return pimc_gb300
+
+
+@pytest.mark.parametrize("sign", [1, -1])
+def test_infinite_table_entries(pimc, sign):
+    # A hard core: the potential's rows below a radius are infinite.  A move into it
+    # has an infinite action difference and is rejected, as with pi-qmc's
+    # interpolation (1 - x) g0 + x g1 (which is NaN at x = 0, below the grid); an
+    # infinite well at the Action-level call alone.
+    kw = W.dot2(counts=[2, 1], nslice=64, nlevel=4, beta=4.0, sho_omega=[1.0, 1.0])
+    tabs, _ = pimc.coulomb_tables(kw)
+    for t in tabs:
+        r = np.exp(np.arange(t["ngpts"]) / t["logrratioinv"]) / t["rgridinv"]
+        t["ugrid"][r < 0.8, 0, 0] = sign * np.inf
+    cfg = O.make_config(**kw)
+    port = O.PortOracle(cfg, tabs)
+    e = pimc.Engine(kw, 1, tabs)
+    x = np.tile(np.array([[1.0, 0, 0], [-0.6, 0.9, 0], [-0.6, -0.9, 0.1]]), (64, 1, 1))
+    if sign > 0:
+        port.set_path(x)
+        ref = port.run(400)
+        e.upload_paths([x])
+        rec = e.run_sections(400, records=True)
+        assert np.isinf(ref["ds"]).any() and (ref["reject_level"] < 0).any()
+        for k in ("ifirst1", "ipart", "reject_level"):
+            assert np.array_equal(rec[k][0], ref[k]), k
+        a, b = rec["ds"][0][:, :5], ref["ds"][:, :5]
+        assert np.array_equal(np.isinf(a), np.isinf(b))
+        assert np.abs(e.download_paths()[0] - port.get_path()).max() <= 1e-12
+    sec = np.tile(x[:17], (3, 1, 1, 1))
+    mov = sec[:, :, 0].copy()
+    mov[0, 1:-1] = x[0, 1] + [0.3, 0, 0]
+    mov[1, 1:-1] = x[0, 1] + [1e-4, 0, 0]  # below the grid
+    mov[2, 1:-1] += 0.1
+    for level in range(5):
+        ds = e.action_difference(level, sec, mov, np.zeros(3, np.int32))
+        ref = np.array([port.action_diff(level, sec[b], mov[b], 0) for b in range(3)])
+        assert level > 2 or ref[0] == sign * np.inf  # (longer links end outside)
+        assert np.isfinite(ref[2])
+        np.testing.assert_allclose(ds, ref, rtol=1e-12, atol=1e-12)  # (infinities, NaN alike)
