@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -411,8 +412,8 @@ const std::vector<double>& log_table() {
 }
 
 // The FP64 table a kernel reads: every coefficient g0 beside its difference to the next
-// grid point's, g1.  An infinite g0 (a hard core) has 0 or itself there, so that
-// g0 + x y is (1 - x) g0 + x g1: with the difference, inf + x (-inf), it would be NaN,
+// grid point's, g1.  An infinite g0 (a hard core) has itself there or the largest finite
+// difference, so that g0 + x y is (1 - x) g0 + x g1: with inf + x (-inf) it would be NaN,
 // which no Metropolis test rejects.
 void interleave_table(const pimc_pair_table& t, double* out) {
   const size_t row = 2 * (size_t)(t.norder + 1), n = row * t.ngpts;
@@ -421,7 +422,8 @@ void interleave_table(const pimc_pair_table& t, double* out) {
     const double next = k + row < n ? t.ugrid[k + row] : t.ugrid[k];
     out[2 * k + 1] = next - t.ugrid[k];
     if (std::isinf(t.ugrid[k])) {
-      if (std::isfinite(next)) out[2 * k + 1] = 0.0;
+      if (std::isfinite(next))
+        out[2 * k + 1] = -std::copysign(std::numeric_limits<double>::max(), t.ugrid[k]);
       if (next == t.ugrid[k]) out[2 * k + 1] = next;
     }
   }

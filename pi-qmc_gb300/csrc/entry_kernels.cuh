@@ -295,8 +295,6 @@ __device__ __forceinline__ PairForce pair_force(const DevTable& tb, const double
   for (int k = tb.norder; k >= 0; k--) {
     const double2 a = __ldg((const double2*)g + k);
     uq = uq * s2 + a.y;
-    // (an infinite coefficient's difference is not the table's)
-    if ((__double2hiint(a.x) & 0x7ff00000) == 0x7ff00000) uq -= a.x;
     if (k > 0) us2 = us2 * s2 + k * fma(x, a.y, a.x);
     vt = vt * s2 + tab_at(g + 2 * tb.ndata, k, x);
   }
