@@ -1582,8 +1582,14 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
   if (which == kEstVirial) {
     // forces of as many replicas at a time as fit 256 MB (one at least)
     long long stride = 0;
-    int per_warp = 1;
+    int per_warp = 1, passes = 1;
     for (const DevSys& d : e->hsys) {
+      for (int k = 0; k < d.ntab; ++k) {  // the most tables of one species pair
+        int same = 0;
+        for (int j = 0; j < d.ntab; ++j)
+          same += std::minmax(d.tab[j].s1, d.tab[j].s2) == std::minmax(d.tab[k].s1, d.tab[k].s2);
+        passes = std::max(passes, same);
+      }
       stride = std::max(stride, 6LL * d.nslice * d.npart);
       const int npair = (d.npart + 1) / 2, lpw = npair < 32 ? 32 / npair : 1;
       per_warp = std::max(per_warp, 6 * lpw * d.npart);
@@ -1602,9 +1608,12 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
     cudaFuncSetAttribute(virial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     for (P.rep0 = 0; P.rep0 < e->nrep; P.rep0 += pass) {
       const dim3 grid(kThermoChunks, std::min(pass, e->nrep - P.rep0));
-      virial_links_kernel<<<grid, 32 * warps, (size_t)warps * per_warp * 8, e->stream>>>(P);
+      for (P.pass = 0; P.pass < passes; ++P.pass) {
+        virial_links_kernel<<<grid, 32 * warps, (size_t)warps * per_warp * 8, e->stream>>>(P);
+        e->launches++;
+      }
       virial_kernel<<<grid, kBlock, L.total * 8, e->stream>>>(P);
-      e->launches += 2;
+      e->launches++;
     }
   } else {
     const dim3 grid(kThermoChunks, e->nrep);

@@ -323,6 +323,7 @@ struct EstimatorParams {
   // fm and fp on every bead, [replica of the pass][nslice_max][npart_max][6]
   int nwindow;
   int rep0;
+  int pass;                  // the pairs' first, second ... tables, adding up
   double* forces;
   long long forces_stride;   // doubles per replica
   const long long* ekcache;  // structure factors of Ewald replicas (null: none)
@@ -357,9 +358,11 @@ __global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P)
   const DevSys& s = S;
   if (threadIdx.x < kMaxSpecies * kMaxSpecies) {
     const int a = threadIdx.x / kMaxSpecies, b = threadIdx.x % kMaxSpecies;
-    int ti = -1;
+    int ti = -1, left = P.pass;
     for (int k = 0; k < s.ntab; ++k)
-      if ((s.tab[k].s1 == a && s.tab[k].s2 == b) || (s.tab[k].s1 == b && s.tab[k].s2 == a)) ti = k;
+      if (((s.tab[k].s1 == a && s.tab[k].s2 == b) || (s.tab[k].s1 == b && s.tab[k].s2 == a)) &&
+          left-- == 0)
+        ti = k;
     tabof[a][b] = (signed char)ti;
   }
   __syncthreads();
@@ -378,7 +381,8 @@ __global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P)
     const int nl = min(lpw, t1 - tw);
     __syncwarp();
     // the beads' own terms start the sums
-    for (int it = lane; it < nl * np; it += 32) {
+    for (int it = lane; P.pass && it < nl * np * 6; it += 32) F[it] = 0.0;
+    for (int it = lane; !P.pass && it < nl * np; it += 32) {
       const int t = tw + it / np, ip = it % np, tm = t == 0 ? M - 1 : t - 1;
       const double* b1 = path + ((size_t)t * np + ip) * 3;
       const double* b0 = path + ((size_t)tm * np + ip) * 3;
@@ -472,14 +476,17 @@ __global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P)
     for (int it = lane; it < nl * np * 3; it += 32) {
       const int q = it / 3, d = it - q * 3, t = tw + q / np, ip = q % np;
       const int tm = t == 0 ? M - 1 : t - 1;
-      forces[((size_t)t * np + ip) * 6 + d] = F[q * 6 + d];
-      forces[((size_t)tm * np + ip) * 6 + 3 + d] = F[q * 6 + 3 + d];
+      double* fm = forces + ((size_t)t * np + ip) * 6 + d;
+      double* fp = forces + ((size_t)tm * np + ip) * 6 + 3 + d;
+      *fm = P.pass ? *fm + F[q * 6 + d] : F[q * 6 + d];
+      *fp = P.pass ? *fp + F[q * 6 + 3 + d] : F[q * 6 + 3 + d];
     }
   }
   double tot = block_sum(part, red);
-  if (s.coulomb && s.ewald && P.ekcache && s.ek_offset >= 0)
+  if (!P.pass && s.coulomb && s.ewald && P.ekcache && s.ek_offset >= 0)
     tot += ewald_cached_energy(s, P.ekcache, t0, t1, red) / s.epsilon;
-  if (threadIdx.x == 0) P.partial[(size_t)rep * P.nchunk + blockIdx.x] = tot;
+  double* partial = P.partial + (size_t)rep * P.nchunk + blockIdx.x;
+  if (threadIdx.x == 0) *partial = P.pass ? *partial + tot : tot;
 }
 
 // VirialEnergyEstimator::handleLink / endCalc's windows.  One CTA per (chunk of

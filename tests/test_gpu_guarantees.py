@@ -53,3 +53,23 @@ def test_infinite_table_entries(pimc, sign):
         assert level > 2 or ref[0] == sign * np.inf  # (longer links end outside)
         assert np.isfinite(ref[2])
         np.testing.assert_allclose(ds, ref, rtol=1e-12, atol=1e-12)  # (infinities, NaN alike)
+
+
+def test_several_tables_of_one_pair(pimc):
+    # Two tables of the same species pair act together, in the virial estimator as in
+    # the moves: a table split in two halves is the whole one.
+    kw = W.dot2(counts=[3, 2], nslice=64, nlevel=3, beta=4.0)
+    tabs, _ = pimc.coulomb_tables(kw)
+    halves = [dict(t, ugrid=f * np.asarray(t["ugrid"])) for f in (0.25, 0.75) for t in tabs]
+    x = W.initial_path(dict(kw), "gauss", seed=3)
+    one, two = pimc.Engine(kw, 1, tabs), pimc.Engine(kw, 1, halves)
+    for e in (one, two):
+        e.upload_paths([x])
+    port = O.PortOracle(O.make_config(**kw), halves)
+    port.set_path(x)
+    for w in (1, 16):
+        a, b, ref = one.virial_energy(w)[0], two.virial_energy(w)[0], port.virial_energy(w)
+        scale = 1e-11 * max(1.0, abs(ref), abs(one.virial_energy(1)[0]))
+        assert abs(a - b) <= scale and abs(b - ref) <= scale, w
+    ra, rb = (e.run_sections(50, records=True) for e in (one, two))
+    assert np.array_equal(ra["reject_level"], rb["reject_level"])
