@@ -37,7 +37,8 @@ struct DisplaceLayout {
   int red, q, ictl;
   int sec;             // one staged slice, old and new, and
   int ewt, ewt_cols;   // its e^{ik.r} tables (replicas without cached structure factors)
-  int ek, ek_stride, ek_batch;  // per warp: tables of ek_batch slices' moved beads
+  int ek, ek_stride, ek_batch;  // per warp: tables of ek_batch slices' moved beads (-ek:
+                                // their place in the CTA's global area)
   int stage;           // per-group slice pairs [2][3][n]
   int nodescr, nodescr_stride, nodecold_stride, split, in_smem, gcta;
   int total;
@@ -494,6 +495,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
       m.ewt = smem + L.ewt;
       m.ewt_cols = L.ewt_cols;
       double* gbase = P.nodescr_g ? P.nodescr_g + (size_t)blockIdx.x * L.gcta : nullptr;
+      m.ewx = L.ek > 0 ? smem + L.ek : gbase - L.ek;
       m.nodescr = L.in_smem ? smem + L.nodescr : gbase;
       m.nodescr_stride = L.nodescr_stride;
       m.nodecold = L.split ? gbase : nullptr;
@@ -565,7 +567,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
       if (s.coulomb && s.ewald) {
         if (ek) {
           const double lr = displace_ewald(s, mv, path, m.qpart, ek,
-                                           smem + P.lay.ek + (size_t)warp * P.lay.ek_stride,
+                                           m.ewx + (size_t)warp * P.lay.ek_stride,
                                            P.lay.ek_batch, gw, ngw, false);
           ds += block_sum(lr, m.red) * s.one_over_2v * s.tau / s.epsilon;
         } else {
@@ -665,7 +667,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
         // ---- the accepted paths, their structure factors and Slater entries
         if (ek)
           displace_ewald(s, mv, path, m.qpart, ek,
-                         smem + P.lay.ek + (size_t)warp * P.lay.ek_stride, P.lay.ek_batch, gw,
+                         m.ewx + (size_t)warp * P.lay.ek_stride, P.lay.ek_batch, gw,
                          ngw, true);
         cl.sync();  // every CTA is done with the old path
         for (int it = threadIdx.x; it < nmov * (m1 - m0); it += blockDim.x) {

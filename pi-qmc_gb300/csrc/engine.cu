@@ -785,7 +785,8 @@ Layout estimator_layout(const std::vector<DevSys>& sys, const int* ikmax_extra) 
 // Shared memory of the displacement kernel: the Slater scratch of the node pass and
 // the Ewald tables share their space (a barrier lies between their phases); the
 // scratch goes to global memory, cold part first, and the tables' batch shrinks,
-// until it fits.
+// until it fits; tables of which one slice's a warp do not fit (wave vectors far up one
+// axis of a long box) go to global memory.
 bool displace_layout(const std::vector<DevSys>& sys, int nwarps, int nmoving, DisplaceLayout& out) {
   int np = 1, per = 0, perfull = 0, stage = 0, full = 0, hot = 0, cold = 0;
   for (const DevSys& d : sys) {
@@ -805,8 +806,9 @@ bool displace_layout(const std::vector<DevSys>& sys, int nwarps, int nmoving, Di
       }
   }
   const int limit = kSmemLimit / 8;
-  for (int place = 0; place < 3; ++place)
+  for (int place = 0; place < 4; ++place)
     for (int batch = 8; batch >= 1; batch /= 2) {
+      const bool ek_smem = place < 3;
       DisplaceLayout L{};
       int off = 0;
       auto take = [&](int n) {
@@ -829,7 +831,11 @@ bool displace_layout(const std::vector<DevSys>& sys, int nwarps, int nmoving, Di
       L.ek_batch = batch;
       L.ek_stride = 2 * per * 2 * nmoving * batch;
       L.nodescr = L.ek = off;
-      off += nwarps * std::max(L.in_smem ? L.nodescr_stride : 0, L.ek_stride);
+      off += nwarps * std::max(L.in_smem ? L.nodescr_stride : 0, ek_smem ? L.ek_stride : 0);
+      if (!ek_smem) {  // (after the Slater scratch)
+        L.ek = -L.gcta;
+        L.gcta += nwarps * L.ek_stride;
+      }
       L.total = off;
       if (off <= limit) {
         out = L;

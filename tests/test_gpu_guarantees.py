@@ -73,3 +73,33 @@ def test_several_tables_of_one_pair(pimc):
         assert abs(a - b) <= scale and abs(b - ref) <= scale, w
     ra, rb = (e.run_sections(50, records=True) for e in (one, two))
     assert np.array_equal(ra["reject_level"], rb["reject_level"])
+
+
+@pytest.mark.parametrize("nmoving", [1, 3])
+@pytest.mark.parametrize("nodes", [0, 2])
+def test_displacements_in_long_boxes(pimc, nodes, nmoving):
+    # A box ninety times as long as wide has wave vectors far up one axis: tables of a
+    # displaced bead that do not fit shared memory for every warp.
+    kw = W.heg54(n=10, cell=[10.0, 10.0, 900.0], nslice=16, nlevel=2, beta=1.6,
+                 ewald_kcut=5 * 2 * np.pi / 10.0, node_kind=[nodes, nodes])
+    tabs, ew = pimc.coulomb_tables(kw)
+    assert ew["ikmax"][2] > 400
+    rng = np.random.default_rng(3)
+    site = rng.uniform(-0.5, 0.5, size=(1, 10, 3)) * [10.0, 10.0, 900.0]
+    x = np.repeat(site, 16, axis=0)
+    cfg = O.make_config(**dict(kw, seed=4, cell=10.0))
+    cfg.cell[2] = 900.0
+    port = O.PortOracle(cfg, tabs, ew)
+    port.set_path(x)
+    ref = port.run_displace(6, [1.0, 1.0, 5.0], nmoving, -1)
+    e = pimc.Engine(kw, 1, tabs, ew, seed=4)
+    e.upload_paths([x])
+    d = e.run_displace(6, [1.0, 1.0, 5.0], nmoving, -1, records=True)
+    assert np.array_equal(d["accepted"][0], ref["accepted"]) and ref["accepted"].any()
+    for k, tol in (("ds", 1e-11), ("ds_node", 1e-9)):
+        assert np.all(np.abs(d[k][0] - ref[k]) <= tol * np.maximum(np.abs(ref[k]), 1.0)), k
+    assert np.abs(port.get_path() - e.download_paths()[0]).max() <= 1e-12
+    # the structure factors that the moves left are those of the paths
+    f = pimc.Engine(kw, 1, tabs, ew, seed=4)
+    f.upload_paths([e.download_paths()[0]])
+    assert e.thermo_energy()[0] == f.thermo_energy()[0]
