@@ -197,6 +197,16 @@ __host__ __device__ __forceinline__ int action_buffer(int nlevel, bool single_le
   return seps > sums ? seps : sums;
 }
 
+// The first of a CTA's warps that take action terms beside the Slater matrices of
+// `lanes` lanes: the others, or half of them in the mixed form, whose terms are cheap;
+// every warp, after its matrices, where those take more than half of the warps, and where
+// there are none (half of the warps left without work: a step of 152 mixed dots of 40
+// electrons without nodes, L = 4, 32 attempts: 1148 us, 862 with all).
+__host__ __device__ __forceinline__ int first_action_warp(int lanes, int nwarps, bool mixed) {
+  const int busy = (lanes + 31) / 32;
+  return lanes == 0 || 2 * busy > nwarps ? 0 : (mixed ? nwarps / 2 : busy);
+}
+
 // Warp w of the nw that share the work: the terms of heap depths 0 .. dmax (dmin =
 // 0) or of depth dmax alone (dmin = dmax).  The lanes' sums are left in the
 // warp's buffer: [0] slots 0 .. 31, or the one depth's; [32] depth 5; [64] depth 6.

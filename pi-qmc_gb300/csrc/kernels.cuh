@@ -872,9 +872,8 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   // SM's narrow FP64 pipe, shared by every resident warp, is the limit, and a
   // packed warp instruction serves several matrices
   int W = node_group_width(n);
-  const int wantW = min(nwarps, (ntask * W + 31) / 32);
-  // (wantW, with the narrowest groups: the sums' shares do not depend on the launch)
-  const int a0 = 2 * wantW > nwarps ? 0 : (s.mixed ? nwarps / 2 : wantW), dmax = L - alo, dmin = ahi == L ? 0 : dmax;
+  // (of the narrowest groups: the sums' shares do not depend on the launch)
+  const int a0 = first_action_warp(ntask * W, nwarps, s.mixed), dmax = L - alo, dmin = ahi == L ? 0 : dmax;
   // A CTA that has its SM to itself is bound by the chain of each matrix's operations,
   // not by the pipe: it takes the widest groups that need no further round of the
   // warps without action terms (128 mixed dots, one a CTA: 50.9 -> 44.9 ms a round, and

@@ -103,3 +103,27 @@ def test_displacements_in_long_boxes(pimc, nodes, nmoving):
     f = pimc.Engine(kw, 1, tabs, ew, seed=4)
     f.upload_paths([e.download_paths()[0]])
     assert e.thermo_energy()[0] == f.thermo_energy()[0]
+
+
+@pytest.mark.parametrize("block", [64, 128, 256])
+@pytest.mark.parametrize("counts", [[1, 1], [4, 3], [20, 21]])
+def test_mixed_sections_without_nodes(pimc, counts, block):
+    # Without Slater matrices every warp takes action terms in both precision forms: on
+    # the attempts that both chains make alike, ln T bit for bit and action
+    # differences within the mixed form's 1e-4 of max(|dS|, 1).
+    kw = W.dot2(counts=counts, nslice=64, beta=64 / 25.6, nlevel=4)
+    tabs, _ = pimc.coulomb_tables(kw)
+    x = W.initial_path(dict(kw), "gauss", seed=3)
+    rec = []
+    for precision in (0, 1):
+        e = pimc.Engine(kw, 4, tabs, seed=5, precision=precision)
+        e.configure(block, 0, 0, 2)
+        e.upload_paths([x] * 4)
+        rec.append(e.run_sections(40, records=True))
+    f, m = rec
+    alike = np.cumprod((f["reject_level"] == m["reject_level"]) & (f["ipart"] == m["ipart"]),
+                       axis=1).astype(bool)
+    assert alike.mean() > 0.5
+    assert np.array_equal(f["lnt"][alike][:, :5], m["lnt"][alike][:, :5])
+    a, b = m["ds"][alike][:, :5], f["ds"][alike][:, :5]
+    assert np.all(np.abs(a - b) <= 1e-4 * np.maximum(np.abs(b), 1.0))
