@@ -197,6 +197,21 @@ __host__ __device__ __forceinline__ int action_buffer(int nlevel, bool single_le
   return seps > sums ? seps : sums;
 }
 
+// The lowest level that is evaluated with those above it where an attempt has neither
+// Slater matrices nor Ewald sums: all together while their links fit a warp's lanes.  The
+// 32 and 64 links of the lowest levels of longer sections wait for the decisions above
+// them, which few attempts pass (32 attempts of 304 dots of 10 electrons, L = 6, 1 %
+// accepted: 2740 us together, 1270 so; of 100 electrons, L = 5, 14 % accepted: 6300
+// and 4280); but for up to 32 particles at L = 5, where they cost little and many
+// pass (152 dots of two, 60 % accepted: 734 us together, 811 apart).
+__host__ __device__ __forceinline__ int lowest_joint_level(int nlevel, int npart) {
+  return nlevel > 5 || (nlevel == 5 && npart > 32) ? nlevel - 4 : 0;
+}
+// Whether a system takes levels singly (the size of its action buffers).
+__host__ __device__ __forceinline__ bool takes_single_levels(const DevSys& s) {
+  return s.fixed_node || s.dr || s.ewald || lowest_joint_level(s.nlevel, s.npart) > 0;
+}
+
 // The first of a CTA's warps that take action terms beside the Slater matrices of
 // `lanes` lanes: the others, or half of them in the mixed form, whose terms are cheap;
 // every warp, after its matrices, where those take more than half of the warps, and where

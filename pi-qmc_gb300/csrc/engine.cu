@@ -708,7 +708,7 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
     int need = 0;
     for (const DevSys& d : sys) {
       // (a launch of all levels together alone needs no buffer for a single one)
-      const bool single = opts.single_levels || d.fixed_node || d.dr || d.ewald;
+      const bool single = opts.single_levels || takes_single_levels(d);
       need = std::max(need, action_buffer(d.nlevel, single, d.mixed != 0));
     }
     if (L.nodescr_in_smem && L.nodescr_stride >= need) {

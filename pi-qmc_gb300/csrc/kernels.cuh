@@ -1200,14 +1200,15 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
       // The top levels (L down to lb) are evaluated together, their Slater
       // matrices side by side; the decisions then follow level by level exactly as
       // below.  Work done for levels under a rejection is discarded.  Without node
-      // work or Ewald sums that is every level; else the lower levels, whose
+      // work or Ewald sums that is every level, or what fits a warp
+      // (lowest_joint_level); else the lower levels, whose
       // slices make up most of the work, wait for the decisions above them (the
       // mixed form's FP32 action terms are cheap and all come with the top ones).
       // (with delayed rejection every level is taken in turn: a second proposal
       // at level L - 1 changes the normals and uniforms of the levels under it)
-      const bool longr = s.ewald && s.coulomb;
-      const int lb = s.dr ? L + 1 : ((mynode || longr) ? max(1, L - 3) : 0);
-      const int alb = s.mixed ? 0 : lb;  // the lowest level whose action comes with them
+      const bool longr = s.ewald && s.coulomb, waits = mynode || longr;
+      const int lb = s.dr ? L + 1 : (waits ? max(1, L - 3) : lowest_joint_level(L, np));
+      const int alb = s.mixed && waits ? 0 : lb;  // the lowest level whose action comes with them
       if (lb <= L) {
         eval_levels(s, m, scale[msp], msp, ipart, lb, L, alb, L, mynode, cache, ifirst1,
                     epoch[msp], lds, lnd);

@@ -8,6 +8,7 @@ REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(REPO, "pi-qmc_gb300", "csrc")
 
 PROGRAM = r"""
+#include <algorithm>
 #include <cstdio>
 #include "kernels.cuh"
 using namespace pimc;
@@ -17,6 +18,17 @@ int main() {
       for (int lanes = 0; lanes <= 32 * 40; lanes += 8)
         std::printf("action %d %d %d %d\n", mixed, nwarps, lanes,
                     first_action_warp(lanes, nwarps, mixed));
+  static DevSys s;  // (no node models, no Ewald sums, no delayed rejection)
+  for (s.nlevel = 1; s.nlevel <= 6; ++s.nlevel)
+    for (s.npart = 1; s.npart <= 200; ++s.npart)
+      for (int mixed = 0; mixed < 2; ++mixed) {
+        const int low = lowest_joint_level(s.nlevel, s.npart);
+        int need = action_seps(0, s.nlevel - low);
+        for (int l = low - 1; l >= 0; --l)
+          need = std::max(need, action_seps(s.nlevel - l, s.nlevel - l));
+        std::printf("levels %d %d %d %d %d\n", s.nlevel, s.npart, low, (mixed ? 2 : 4) * need,
+                    action_buffer(s.nlevel, takes_single_levels(s), mixed));
+      }
 }
 """
 
@@ -51,3 +63,13 @@ def test_action_warps(rules):
             assert a0 >= busy
         seen.add((mixed, a0 > 0))
     assert len(seen) == 4
+
+
+def test_joint_levels(rules):
+    # Levels whose links fill more than a warp wait for the decisions above them in long
+    # sections, and the buffers hold every evaluation that is made.
+    for level, npart, low, need, room in (map(int, r[1:]) for r in rules if r[0] == "levels"):
+        assert 0 <= low < level and need <= room
+        assert low == 0 if level < 5 else level - low <= 5
+        if level == 6 or (level == 5 and npart > 32):
+            assert level - low == 4
