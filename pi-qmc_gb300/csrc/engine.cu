@@ -128,6 +128,7 @@ struct DevBuf {
 }  // namespace
 
 constexpr int kThermoChunks = 64;  // CTAs per replica of the estimators, at most
+constexpr int kThermoParts = 8;    // parts of a chunk, at most
 
 // Layout choices the autotuner varies.
 struct LayoutOpts {
@@ -531,12 +532,23 @@ void fill_sys(const pimc_system& s, DevSys& d) {
   d.rcut2_lo = (float)(d.rcut2 * (1.0 - 1e-5));
   d.rcut2_hi = (float)(d.rcut2 * (1.0 + 1e-5));
   for (int a = 0; a < 3; ++a) d.cellb_f[a] = (float)d.cellb[a];
-  // CTAs of the thermodynamic estimator by the system's own size (so that a value
-  // does not depend on what is measured beside it): 4096 bead or pair links each, 16
-  // per thread against the start-up of a CTA.  (64 CTAs for every system: a step of
-  // 9728 two-electron dots 29.4 ms, now 13.1.)
-  const long long links = (long long)s.nslice * s.npart * (s.npart + 1) / 2;
-  d.thermo_chunks = (int)std::max(1LL, std::min((long long)kThermoChunks, links / 4096));
+  // The thermodynamic estimator's chunks by the system's own size (so that a value does
+  // not depend on what is measured beside it): 4096 bead or pair links each, 16 per
+  // thread against the start-up of a CTA.  (64 CTAs for every system: a step of 9728
+  // two-electron dots 29.4 ms, now 13.1.)  A thread's links are runs of two items a
+  // thread; the runs of up to eight chunks (of all but 64 with Ewald sums) are cut into up to
+  // eight parts, which a launch that leaves SMs idle shares out to more CTAs.
+  {
+    const long long links = (long long)s.nslice * s.npart * (s.npart + 1) / 2;
+    const int nchunk = (int)std::max(1LL, std::min((long long)kThermoChunks, links / 4096));
+    const int ne = s.npart + (s.npart & 1), len = s.nslice / nchunk;
+    const long long items = s.coulomb && s.npart > 1 ? (long long)(ne - 1) * (ne / 2) : s.npart;
+    const int parts = std::max(1, std::min(kThermoParts, (s.ewald ? kThermoChunks : 16) / nchunk));
+    d.thermo_chunks = nchunk;
+    d.thermo_run = (int)std::max(1LL, std::min((long long)len, len * items / (2 * kBlock)));
+    d.thermo_sub = (d.thermo_run + parts - 1) / parts;
+    d.thermo_parts = (d.thermo_run + d.thermo_sub - 1) / d.thermo_sub;
+  }
   d.spring = s.spring;
   d.coulomb = s.coulomb;
   d.ewald = s.ewald;
@@ -771,6 +783,9 @@ Layout estimator_layout(const std::vector<DevSys>& sys, const int* ikmax_extra) 
   const int xy = 2 * (ik[0] + 1) * (2 * ik[1] + 1) * np;
   const bool ewald = ik[0] + ik[1] + ik[2] > 0;
   L.ewxy = ewald && (off + xy) * 8 <= 74 * 1024 ? take(xy) : 0;
+  int parts = 1;
+  for (const DevSys& d : sys) parts = std::max(parts, d.thermo_parts);
+  L.sums = take(parts > 1 ? parts * kBlock : 0);
   L.ictl = take(C_NCTL + 2);
   L.dm = L.ndm = L.dist = L.ndist = L.red;
   L.ecache = L.ncol = -1;
@@ -1448,11 +1463,21 @@ int pimc_set_replica_state(pimc_engine* e, int replica, const pimc_replica_state
 }
 
 namespace {
-// CTAs per replica of the largest thermodynamic measurement of an engine.
-int thermo_grid(const std::vector<DevSys>& sys) {
-  int n = 1;
-  for (const DevSys& d : sys) n = std::max(n, d.thermo_chunks);
-  return n;
+// The thermodynamic estimator over P.nrep systems, those of `slots` or all of the
+// engine's: the CTAs that share a chunk's parts are as many as fill the SMs with three each.
+void launch_thermo(pimc_engine* e, cudaStream_t st, ThermoParams P, const int* slots) {
+  long long all = 0;
+  int chunks[2] = {1, 0};  // the most, of systems with one part a chunk and several
+  for (int k = 0; k < P.nrep; ++k) {
+    const DevSys& d = e->hsys[slots ? slots[k] : k];
+    int& c = chunks[d.thermo_parts > 1];
+    c = std::max(c, d.thermo_chunks);
+    all += d.thermo_chunks;
+  }
+  P.split = (int)std::max(1LL, std::min((long long)kThermoParts, 3LL * e->num_sms / all));
+  const int grid = std::max(chunks[0], chunks[1] * P.split);
+  thermo_kernel<<<dim3(grid, P.nrep), kBlock, P.lay.total * 8, st>>>(P);
+  e->launches++;
 }
 
 // Enqueues the energy measurement of every replica into d_energy[row][*].
@@ -1475,11 +1500,11 @@ int enqueue_thermo(pimc_engine* e, cudaStream_t st, int row) {
   P.nchunk = kThermoChunks;
   P.nrep = e->nrep;
   P.lay = e->est_lay;
-  thermo_kernel<<<dim3(thermo_grid(e->hsys), e->nrep), kBlock, e->est_lay.total * 8, st>>>(P);
+  launch_thermo(e, st, P, nullptr);
   thermo_reduce_kernel<<<(e->nrep + 127) / 128, 128, 0, st>>>(
       e->d_sys.p, nullptr, e->d_partial.p, kThermoChunks, e->nrep,
       e->d_energy.p + (size_t)row * e->nrep, true);
-  e->launches += 2;
+  e->launches++;
   CU(cudaGetLastError());
   return PIMC_OK;
 }
@@ -2578,8 +2603,6 @@ int server_energy(pimc_engine* e, const std::vector<int>& slots, double* out) {
   // (a slot's chunks depend on its own system: its sum is grouped the same way
   // whatever the mix)
   const int nchunk = kThermoChunks;
-  int grid = 1;
-  for (int r : slots) grid = std::max(grid, e->hsys[r].thermo_chunks);
   std::vector<double> part((size_t)n * nchunk);
   EntryIo io(e);
   const int idx = io.in(slots.data(), sizeof(int) * (size_t)n);
@@ -2594,14 +2617,14 @@ int server_energy(pimc_engine* e, const std::vector<int>& slots, double* out) {
   P.nchunk = nchunk;
   P.nrep = n;
   P.lay = e->est_lay;
-  thermo_kernel<<<dim3(grid, n), kBlock, e->est_lay.total * 8, e->stream>>>(P);
-  e->launches++;
+  launch_thermo(e, e->stream, P, slots.data());
   CU(cudaGetLastError());
   if (int rc = io.close()) return rc;
   for (int k = 0; k < n; ++k) {
     double s = 0;
-    for (int c = 0; c < e->hsys[slots[k]].thermo_chunks; ++c) s += part[(size_t)k * nchunk + c];
-    out[k] = s / e->hsys[slots[k]].nslice;
+    const DevSys& d = e->hsys[slots[k]];
+    for (int c = 0; c < d.thermo_chunks * d.thermo_parts; ++c) s += part[(size_t)k * nchunk + c];
+    out[k] = s / d.nslice;
   }
   return PIMC_OK;
 }

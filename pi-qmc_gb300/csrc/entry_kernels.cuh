@@ -49,9 +49,10 @@ struct ThermoParams {
   const int* index;  // replicas to measure (null: all, blockIdx.y)
   const double* paths;
   const long long* ekcache;  // structure factors of Ewald replicas (null: none)
-  double* partial;  // [nrep][nchunk], the first thermo_chunks of each used
+  double* partial;  // [nrep][nchunk], the first thermo_chunks x thermo_parts of each used
   int nchunk;
   int nrep;
+  int split;  // CTAs that share a chunk's parts, at most
   Layout lay;
 };
 
@@ -144,10 +145,12 @@ __device__ __forceinline__ double pair_utau_link(const DevTable& tb, const PairS
 // adds 0.5 utau for each ordering (PairAction::getBeadAction runs over every partner
 // of every particle); the two orderings agree unless an image tie makes them
 // differ, so one evaluation usually stands for both, and the ordering (j, i) is
-// evaluated only on a tie.
-template <bool kMixed>
-__device__ __forceinline__ double pair_utau_run(const DevSys& s, const DevTable& tb,
-                                                const double* path, int i, int j, int t0, int t1) {
+// evaluated only on a tie.  kParts: every `sub` links' sum goes to add(k), add(k + 1) ...;
+// else all to add(k).
+template <bool kMixed, bool kParts, class Add>
+__device__ __forceinline__ void pair_utau_run(const DevSys& s, const DevTable& tb,
+                                              const double* path, int i, int j, int t0, int t1,
+                                              int sub, int k, Add add) {
   const int np = s.npart, M = s.nslice;
   const auto at = [&](int t, int a, int b, PairSep<kMixed>& sep) {
     const double* ba = path + ((size_t)t * np + a) * 3;
@@ -158,6 +161,7 @@ __device__ __forceinline__ double pair_utau_run(const DevSys& s, const DevTable&
     return tie;
   };
   double sum = 0.0;
+  int left = sub;
   PairSep<kMixed> p, e;
   int tm = t0 == 0 ? M - 1 : t0 - 1;
   bool tie0 = at(tm, i, j, p);
@@ -171,11 +175,16 @@ __device__ __forceinline__ double pair_utau_run(const DevSys& s, const DevTable&
       a = 0.5 * a + 0.5 * pair_utau_link(tb, re, rp);
     }
     sum += a;
+    if (kParts && --left == 0) {
+      add(k++, sum);
+      sum = 0.0;
+      left = sub;
+    }
     p = e;
     tie0 = tie1;
     tm = t;
   }
-  return sum;
+  if (!kParts || left < sub) add(k, sum);
 }
 
 // Pair k of round rd of the round-robin schedule over n (even) players: every
@@ -192,21 +201,24 @@ __device__ __forceinline__ void round_robin_pair(int n, int rd, int k, int& a, i
   }
 }
 
-// evalLongRange summed over slices [t0, t1) from the cached structure factors:
-// sum_k 2 v_k |rho_k|^2 / (2V) + the self energy.  All threads.
-static __device__ double ewald_cached_energy(const DevSys& s, const long long* ekcache, int t0,
-                                             int t1, double* red) {
+// evalLongRange summed over slices slice(0) .. slice(nt - 1) (the n of them that are >= 0)
+// from the cached structure factors: sum_k 2 v_k |rho_k|^2 / (2V) + the self energy.
+// All threads.
+template <class Slice>
+static __device__ double ewald_cached_energy(const DevSys& s, const long long* ekcache, int nt,
+                                             int n, Slice slice, double* red) {
   const long long* ek = ekcache + s.ek_offset;
   const double is = 1.0 / s.ek_scale;
-  const int nt = max(0, t1 - t0), totk = s.totk;
+  const int totk = s.totk;
   double lr = 0.0;
   for (int it = threadIdx.x; it < nt * totk; it += blockDim.x) {
-    const int t = t0 + it / totk, k = it % totk;
+    const int i = it / totk, k = it - i * totk, t = slice(i);
+    if (t < 0) continue;
     const longlong2 v = *(const longlong2*)(ek + ((size_t)t * totk + k) * 2);
     const double re = __ll2double_rn(v.x) * is, im = __ll2double_rn(v.y) * is;
     lr += 2 * __ldg(s.vk + k) * (re * re + im * im);
   }
-  return block_sum(lr, red) * s.one_over_2v + nt * s.self_energy;
+  return block_sum(lr, red) * s.one_over_2v + n * s.self_energy;
 }
 
 // evalLongRange of path slice t (EwaldSum::evalLongRange, src/util/EwaldSum.cc:103-181),
@@ -484,7 +496,9 @@ __global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P)
   }
   double tot = block_sum(part, red);
   if (!P.pass && s.coulomb && s.ewald && P.ekcache && s.ek_offset >= 0)
-    tot += ewald_cached_energy(s, P.ekcache, t0, t1, red) / s.epsilon;
+    tot += ewald_cached_energy(s, P.ekcache, t1 - t0, t1 - t0, [&](int i) { return t0 + i; },
+                               red) /
+           s.epsilon;
   double* partial = P.partial + (size_t)rep * P.nchunk + blockIdx.x;
   if (threadIdx.x == 0) *partial = P.pass ? *partial + tot : tot;
 }
@@ -624,36 +638,53 @@ __global__ void thermo_reduce_kernel(const DevSys* sys, const int* index, const 
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nrow) return;
   const int r = index ? index[k] : k;
-  const int used = thermo ? sys[r].thermo_chunks : nchunk;
+  const int used = thermo ? sys[r].thermo_chunks * sys[r].thermo_parts : nchunk;
   double s = 0.0;
   for (int c = 0; c < used; ++c) s = __dadd_rn(s, partial[(size_t)k * nchunk + c]);
   energy[r] = __ddiv_rn(s, (double)sys[r].nslice);
 }
 
-// One CTA per (chunk of slices, replica; a replica has DevSys::thermo_chunks): link
-// utau sums plus, for Coulomb with Ewald, the long-range energy of each slice (CoulombAction::getBeadAction adds
-// it at ipart == 0, src/action/CoulombAction.cc:165-171).
-__global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
+// Link utau sums plus, for Coulomb with Ewald, the long-range energy of each slice
+// (CoulombAction::getBeadAction adds it at ipart == 0, src/action/CoulombAction.cc:165-171).
+// A replica's CTAs share its chunks' parts; each part is summed apart (its share of the
+// chunk's links and slices, by the same threads in the same order), so the value does
+// not depend on the split.  Where the chunks fill the GPU a CTA takes a whole one,
+// whose runs share their links' separations; for a few small systems the parts go to
+// up to eight CTAs each (one dot of four electrons, M = 1024, from the host: 116 us on
+// two CTAs, 55 so; 2000 of them 1160 with whole chunks summed at once, 1220 so).  kParts: more than one part a chunk (with one, a leaner
+// form).
+template <bool kParts>
+__device__ __forceinline__ void thermo_chunk(const ThermoParams& P, const DevSys& s, int split) {
   extern __shared__ double smem[];
-  __shared__ DevSys S;
-  const int r = P.index ? P.index[blockIdx.y] : blockIdx.y;
-  if ((int)blockIdx.x >= P.sys[r].thermo_chunks) return;
-  {
-    const int* src = (const int*)(P.sys + r);
-    int* dst = (int*)&S;
-    for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x)
-      dst[i] = src[i];
-  }
-  __syncthreads();
-  const DevSys& s = S;
+  __shared__ signed char tabof[kMaxSpecies][kMaxSpecies];
   const double* path = P.paths + s.path_offset;
   const int M = s.nslice, np = s.npart;
-  const int nchunk = s.thermo_chunks;
-  const int t0 = (int)((long long)M * blockIdx.x / nchunk);
-  const int t1 = (int)((long long)M * (blockIdx.x + 1) / nchunk);
+  const int nchunk = s.thermo_chunks, run = s.thermo_run, sub = s.thermo_sub;
+  const int chunk = blockIdx.x / split, q = blockIdx.x - chunk * split;
+  const int k0 = kParts ? s.thermo_parts * q / split : 0;
+  const int k1 = kParts ? s.thermo_parts * (q + 1) / split : 1;
+  const int t0 = (int)((long long)M * chunk / nchunk);
+  const int t1 = (int)((long long)M * (chunk + 1) / nchunk);
+  const int nrun = (t1 - t0 + run - 1) / run;
   Smem m = carve(smem, P.lay, s, nullptr);
+  // this thread's sums, [part - k0][thread]; a single one in a register
+  double* sums = smem + P.lay.sums + threadIdx.x;
+  double part = 0.0;
+  if (kParts)
+    for (int k = k0; k < k1; ++k) sums[(k - k0) * kBlock] = 0.0;
+  const auto add = [&](int k, double v) {
+    if (kParts)
+      sums[(k - k0) * kBlock] += v;
+    else
+      part += v;
+  };
+  // the i-th slice of part k, or -1
+  const auto slice = [&](int k, int i) {
+    if (!kParts) return t0 + i < t1 ? t0 + i : -1;
+    const int j = i / sub, o = k * sub + (i - j * sub), t = t0 + j * run + o;
+    return o < run && t < t1 ? t : -1;
+  };
   // table of each species pair (pairs with no table contribute nothing)
-  __shared__ signed char tabof[kMaxSpecies][kMaxSpecies];
   if (threadIdx.x < kMaxSpecies * kMaxSpecies) {
     const int a = threadIdx.x / kMaxSpecies, b = threadIdx.x % kMaxSpecies;
     int ti = -1;
@@ -662,40 +693,65 @@ __global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
     tabof[a][b] = (signed char)ti;
   }
   __syncthreads();
-  double part = 0.0;
-  for (int it = threadIdx.x; it < (t1 - t0) * np; it += blockDim.x) {
-    const int t = t0 + it / np, ip = it % np;
-    part += link_utau(s, path, ip, t);
-  }
+  for (int k = k0; k < k1; ++k)
+    for (int it = threadIdx.x; it < nrun * sub * np; it += blockDim.x) {
+      const int i = it / np, t = slice(k, i);
+      if (t >= 0) add(k, link_utau(s, path, it - i * np, t));
+    }
   if (s.coulomb && np > 1) {
     // every pair once: rounds of the round-robin schedule (np rounded up to even).  A
-    // thread takes a run of a pair's links, as long as the threads all have one (a
-    // run of R links forms R + 1 separations).
+    // thread takes a run of a pair's links (a run of R links forms R + 1 separations).
     const int ne = np + (np & 1), per_round = ne / 2, nrd = ne - 1, pairs = nrd * per_round;
-    const int len = t1 - t0;
-    const int run = max(1, min(len, len * pairs / (2 * kBlock)));
-    const int items = ((len + run - 1) / run) * pairs;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int ta = t0 + it / pairs * run, tb = min(t1, ta + run);
+    for (int it = threadIdx.x; it < nrun * pairs; it += blockDim.x) {
+      const int ts = t0 + it / pairs * run;
+      const int ta = ts + k0 * sub, te = min(t1, ts + min(run, k1 * sub));
       const int rest = it % pairs;
       int a, b;
       round_robin_pair(ne, rest / per_round, rest % per_round, a, b);
-      if (a >= np || b >= np) continue;  // the bye of an odd count
+      if (a >= np || b >= np || ta >= te) continue;  // the bye of an odd count
       const int ti = tabof[species_of(s, a)][species_of(s, b)];
       if (ti < 0) continue;
-      part += s.mixed ? pair_utau_run<true>(s, s.tab[ti], path, a, b, ta, tb)
-                      : pair_utau_run<false>(s, s.tab[ti], path, a, b, ta, tb);
+      if (s.mixed)
+        pair_utau_run<true, kParts>(s, s.tab[ti], path, a, b, ta, te, sub, k0, add);
+      else
+        pair_utau_run<false, kParts>(s, s.tab[ti], path, a, b, ta, te, sub, k0, add);
     }
   }
-  double tot = block_sum(part, m.red);
-  if (s.coulomb && s.ewald && P.ekcache && s.ek_offset >= 0) {
-    // evalLongRange of every slice from its cached structure factors
-    tot += ewald_cached_energy(s, P.ekcache, t0, t1, m.red) / s.epsilon;
-  } else if (s.coulomb && s.ewald) {
+  const bool longr = s.coulomb && s.ewald, cached = longr && P.ekcache && s.ek_offset >= 0;
+  if (longr && !cached) {
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
-    for (int t = t0; t < t1; ++t) tot += ewald_staged_energy(s, m, path, t) / s.epsilon;
   }
-  if (threadIdx.x == 0) P.partial[(size_t)blockIdx.y * P.nchunk + blockIdx.x] = tot;
+  for (int k = k0; k < k1; ++k) {
+    double tot = block_sum(kParts ? sums[(k - k0) * kBlock] : part, m.red);
+    const auto at = [&](int i) { return slice(k, i); };
+    if (cached) {  // evalLongRange of every slice from its cached structure factors
+      const int full = (t1 - t0) / run, rest = (t1 - t0) - full * run, per = min(sub, run - k * sub);
+      const int n = full * per + max(0, min(per, rest - k * sub));
+      tot += ewald_cached_energy(s, P.ekcache, nrun * sub, n, at, m.red) / s.epsilon;
+    } else if (longr)
+      for (int i = 0; i < nrun * sub; ++i)
+        if (at(i) >= 0) tot += ewald_staged_energy(s, m, path, at(i)) / s.epsilon;
+    if (threadIdx.x == 0)
+      P.partial[(size_t)blockIdx.y * P.nchunk + chunk * s.thermo_parts + k] = tot;
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
+  __shared__ DevSys S;
+  const int r = P.index ? P.index[blockIdx.y] : blockIdx.y;
+  const int parts = P.sys[r].thermo_parts, split = min(P.split, parts);
+  if ((int)blockIdx.x >= P.sys[r].thermo_chunks * split) return;
+  {
+    const int* src = (const int*)(P.sys + r);
+    int* dst = (int*)&S;
+    for (int i = threadIdx.x; i < (int)(sizeof(DevSys) / sizeof(int)); i += blockDim.x)
+      dst[i] = src[i];
+  }
+  __syncthreads();
+  if (parts > 1)
+    thermo_chunk<true>(P, S, split);
+  else
+    thermo_chunk<false>(P, S, split);
 }
 
 // ------------------------------------------------------- Action-level entry

@@ -25,6 +25,7 @@ struct Layout {
   int ewt_cols;         // bead columns of the Ewald tables area
   int ewt_words;        // doubles of the tables area
   int ewxy;             // their (kx, ky) products (estimators; 0: none)
+  int sums;             // the thermodynamic estimator's sums by part and thread
   int total;  // doubles
 };
 

@@ -71,7 +71,10 @@ struct DevSys {
   double one_over_2v, self_energy, deltak[3];
   int ikmax[3];
   int ns_max;           // largest node-species count
-  int thermo_chunks;    // CTAs of the thermodynamic estimator (kThermoChunks at most)
+  // The thermodynamic estimator's sums, by the system alone: chunks of slices, cut into
+  // runs of thermo_run; part k of a chunk is the k-th thermo_sub links of every run.
+  // (chunks times parts: kThermoChunks at most)
+  int thermo_chunks, thermo_run, thermo_sub, thermo_parts;
   uint32_t stream_id;     // random stream of this replica (its replica or request id)
   long long nc_offset;    // doubles into the Slater-result cache pool (-1: no cache)
   int nc_stride;          // doubles per cache entry

@@ -127,3 +127,40 @@ def test_mixed_sections_without_nodes(pimc, counts, block):
     assert np.array_equal(f["lnt"][alike][:, :5], m["lnt"][alike][:, :5])
     a, b = m["ds"][alike][:, :5], f["ds"][alike][:, :5]
     assert np.all(np.abs(a - b) <= 1e-4 * np.maximum(np.abs(b), 1.0))
+
+
+THERMO = {
+    "dot4": W.dot2(counts=[2, 2], nslice=1024, beta=40.0),
+    "dot8_odd": W.dot2(counts=[5, 3], nslice=333, beta=13.0, nlevel=3),
+    "dot3_odd": W.dot2(counts=[2, 1], nslice=1237, beta=20.0, nlevel=2),
+    "dot20": W.dot2(counts=[10, 10], nslice=300, beta=12.0, nlevel=3),
+    "one": W.dot2(counts=[1], sho_omega=[1.0], nslice=9001, beta=90.0, nlevel=2, coulomb=0),
+    "heg8": W.heg54(n=8, nslice=520, nlevel=3, node_kind=[0, 0]),
+    "heg10_uncached": W.heg54(n=10, nslice=8, nlevel=2, t_over_tf=3.0, node_kind=[0, 0]),
+}
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", list(THERMO))
+def test_thermo_energy_of_one_and_many(pimc, case, precision):
+    # A replica's energy does not depend on how many are measured beside it, bit for
+    # bit, and is the restatement's.
+    kw = THERMO[case]
+    tabs, ew = pimc.coulomb_tables(kw) if kw["coulomb"] else ((), None)
+    rng = np.random.default_rng(1)
+    x = [W.initial_path(dict(kw), "grid" if kw.get("mover") else "gauss", seed=r) for r in range(3)]
+    x = [a + 0.2 * rng.normal(size=a.shape) for a in x]
+    want = None
+    for nrep in (1, 3, 40, 500):
+        e = pimc.Engine(kw, nrep, tabs, ew, precision=precision)
+        e.upload_paths([x[r % 3] for r in range(nrep)])
+        got = e.thermo_energy()
+        e.close()
+        assert np.array_equal(got, np.tile(got[:3], -(-nrep // 3))[:nrep])
+        if want is None:
+            want = got[0]
+            port = O.PortOracle(O.make_config(**kw), tabs, ew)
+            port.set_path(x[0])
+            ref = port.thermo_energy()
+            assert abs(want - ref) <= (1e-5 if precision else 1e-12) * max(1.0, abs(ref))
+        assert got[0] == want
