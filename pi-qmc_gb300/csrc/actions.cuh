@@ -188,13 +188,21 @@ __host__ __device__ __forceinline__ int action_seps(int dmin, int dmax) {
   const int nl = dmin ? 1 << dmax : 2 << dmax;
   return (nl < 32 ? 32 / nl : 1) * (2 << dmax);
 }
-// Doubles of a warp's work buffer: its separations, then its lanes' sums.
-__host__ __device__ __forceinline__ int action_buffer(int nlevel, bool single_levels, bool mixed) {
+// Doubles of a share's lane sums, and of a warp's separations.
+__host__ __device__ __forceinline__ int action_sum_words(int nlevel) {
+  return 32 * (nlevel >= 6 ? 3 : (nlevel >= 5 ? 2 : 1));
+}
+__host__ __device__ __forceinline__ int action_sep_words(int nlevel, bool single_levels, bool mixed) {
   int e = action_seps(0, nlevel);
   if (single_levels && e < 64) e = 64;
-  const int sums = 32 * (nlevel >= 6 ? 3 : (nlevel >= 5 ? 2 : 1));
-  const int seps = mixed ? 2 * e : 4 * e;
-  return seps > sums ? seps : sums;
+  return mixed ? 2 * e : 4 * e;
+}
+// Doubles of a warp's work buffer: its separations, then its lanes' sums over them; or
+// the sums of several shares after them.
+__host__ __device__ __forceinline__ int action_buffer(int nlevel, bool single_levels, bool mixed,
+                                                      int shares = 1) {
+  const int seps = action_sep_words(nlevel, single_levels, mixed), sums = action_sum_words(nlevel);
+  return shares > 1 ? seps + shares * sums : (seps > sums ? seps : sums);
 }
 
 // The lowest level that is evaluated with those above it where an attempt has neither
@@ -222,12 +230,26 @@ __host__ __device__ __forceinline__ int first_action_warp(int lanes, int nwarps,
   return lanes == 0 || 2 * busy > nwarps ? 0 : (mixed ? nwarps / 2 : busy);
 }
 
-// Warp w of the nw that share the work: the terms of heap depths 0 .. dmax (dmin =
-// 0) or of depth dmax alone (dmin = dmax).  The lanes' sums are left in the
-// warp's buffer: [0] slots 0 .. 31, or the one depth's; [32] depth 5; [64] depth 6.
+// The most shares of nshare warps' action terms that one of nwarps warps takes.
+__host__ __device__ __forceinline__ int action_shares_per_warp(int nwarps, int nshare) {
+  int most = 1;
+  for (int busy = 0; nwarps < nshare && busy <= nshare; ++busy)
+    for (int mixed = 0; mixed < 2; ++mixed) {
+      const int n = nshare - first_action_warp(32 * busy, nshare, mixed);
+      const int w = nwarps - first_action_warp(32 * busy, nwarps, mixed);
+      if ((n + w - 1) / w > most) most = (n + w - 1) / w;
+    }
+  return most;
+}
+
+// Share w of the nw of the work: the terms of heap depths 0 .. dmax (dmin = 0) or of
+// depth dmax alone (dmin = dmax), on the calling warp with its buffer.  The lanes'
+// sums go to sums (the buffer itself, or beyond its separations):
+// [0] slots 0 .. 31, or the one depth's; [32] depth 5; [64] depth 6.
 template <bool kMixed>
 static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, int ipart,
-                                                int dmin, int dmax, int w, int nw, double* buf) {
+                                                int dmin, int dmax, int w, int nw, double* buf,
+                                                double* sums) {
   using S = typename std::conditional<kMixed, SepF, Sep>::type;
   const int lane = threadIdx.x & 31, L = s.nlevel, np = s.npart;
   const int sh = L - dmax, nI = 2 << dmax, mid = 1 << dmax;
@@ -309,9 +331,9 @@ static __device__ __noinline__ void action_warp(const DevSys& s, const Smem& m, 
     }
   }
   __syncwarp();
-  buf[lane] = a0.value();
-  if (!dmin && dmax >= 5) buf[32 + lane] = a1.value();
-  if (!dmin && dmax >= 6) buf[64 + lane] = a2.value();
+  sums[lane] = a0.value();
+  if (!dmin && dmax >= 5) sums[32 + lane] = a1.value();
+  if (!dmin && dmax >= 6) sums[64 + lane] = a2.value();
 }
 
 // A heap's lane values (slot n of nI <= 32 on every lane congruent to it) folded by
@@ -334,17 +356,25 @@ __device__ __forceinline__ double fold_warp(double x) {
   return x;
 }
 
-// The action differences of action_warp's nw warps (buffers from buf0 on), per
-// level into lds[level].  Called by every warp after a barrier; the first ones work.
+// The action differences of action_warp's nshare shares, per level into lds[level]: share
+// k's sums are the k / nw-th (of `words`) from buf0 on in the buffer of the k % nw-th
+// of the nw warps.  Called by every warp after a barrier; the first ones work.
 __device__ __forceinline__ void action_reduce(const DevSys& s, const double* buf0, int stride,
-                                              int dmin, int dmax, int nw, double* lds) {
+                                              int dmin, int dmax, int nshare, int nw, int words,
+                                              double* lds) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int chunks = (dmin || dmax < 5) ? 1 : dmax - 3;
 #pragma unroll 1
   for (int c = warp; c < chunks; c += nwarps) {
     double x = 0.0;
 #pragma unroll 1
-    for (int w = 0; w < nw; ++w) x += buf0[(size_t)w * stride + 32 * c + lane];
+    for (int k = 0, w = 0, at = 32 * c + lane; k < nshare; ++k) {
+      x += buf0[(size_t)w * stride + at];
+      if (++w == nw) {
+        w = 0;
+        at += words;
+      }
+    }
     if (dmin || c > 0) {
       x = fold_warp(x);
       if (lane == 0) lds[s.nlevel - (dmin ? dmax : 4 + c)] = x;

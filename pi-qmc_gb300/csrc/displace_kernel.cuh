@@ -486,6 +486,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
       m.red = smem + L.red;
       m.qpart = smem + L.q;
       m.ictl = (int*)(smem + L.ictl);
+      m.nshare = nwarps;
       m.s1x = smem + L.sec;
       m.s1y = m.s1x + 2 * P.sys[r].npart;
       m.s1z = m.s1y + 2 * P.sys[r].npart;

@@ -136,6 +136,7 @@ struct LayoutOpts {
   bool cold_global = false;     // its cold parts in global memory even when all of it fits
   bool full_ewald_tables = false;  // Ewald tables for every bead (full evalLongRange sums)
   bool single_levels = false;      // action differences of one level at a time only
+  int nshare = 0;  // warps that sums are shared out to (0: the block's)
 };
 
 struct pimc_engine {
@@ -718,10 +719,11 @@ Layout make_layout(const std::vector<DevSys>& sys, int nwarps, bool& ok, LayoutO
   // shared memory (a warp is done with it by then), else their own
   {
     int need = 0;
+    const int per_warp = action_shares_per_warp(nwarps, std::max(nwarps, opts.nshare));
     for (const DevSys& d : sys) {
       // (a launch of all levels together alone needs no buffer for a single one)
       const bool single = opts.single_levels || takes_single_levels(d);
-      need = std::max(need, action_buffer(d.nlevel, single, d.mixed != 0));
+      need = std::max(need, action_buffer(d.nlevel, single, d.mixed != 0, per_warp));
     }
     if (L.nodescr_in_smem && L.nodescr_stride >= need) {
       L.act = -1;
@@ -985,13 +987,17 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
     // The smallest take one warp, without barriers between two, where replicas fill the
     // SMs' 16 warps (32 attempts of 4864 dots of 2, 3 and 4 electrons, L = 4: 4.4, 7.7 and
     // 8.9 ms with two, 4.0, 6.1 and 7.4 with one; 608 of two: 0.76 and 0.81).
-    if (!fixed && items <= 64 && nrep >= 8 * nsm) e->block = 32;
+    // (the sums stay those of two: chains do not depend on the number of replicas)
+    if (!fixed && items <= 64 && nrep >= 8 * nsm) {
+      e->block = 32;
+      e->lay_opts.nshare = 2;
+    }
   }
   for (DevSys& d : e->hsys) d.mixed = precision == PIMC_PREC_MIXED;
   e->nodes = false;
   for (const DevSys& d : e->hsys) e->nodes |= d.fixed_node != 0;
   bool ok = false;
-  e->lay = make_layout(e->hsys, e->block / 32, ok);
+  e->lay = make_layout(e->hsys, e->block / 32, ok, e->lay_opts);
   if (!ok) {
     delete e;
     return fail(PIMC_ERR_CAPACITY, "working set does not fit in shared memory");
@@ -1046,10 +1052,13 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
   // 32 particles: 14.7 -> 12.6 ms a loop).
   if (e->nodes && occ == 1 && nrep > nsm && e->block == kBlock) {
     const int half = kBlock / 2;
-    const Layout hl = make_layout(e->hsys, half / 32, ok);
+    LayoutOpts opts = e->lay_opts;
+    opts.nshare = kBlock / 32;  // (the sums stay those of eight warps)
+    const Layout hl = make_layout(e->hsys, half / 32, ok, opts);
     const int hocc = ok ? section_occupancy(e->minb, half, hl.total * 8, e->nodes) : 0;
     if (hocc > 1 && hl.nodescr_in_smem) {
       e->block = half;
+      e->lay_opts = opts;
       e->lay = hl;
       occ = hocc;
     }
@@ -1528,6 +1537,7 @@ void fill_run_params(pimc_engine* e, RunParams& P, int nattempt, pimc_move_recor
   P.nrep = e->nrep;
   P.seed = e->seed;
   P.wide = e->grid <= e->num_sms;
+  P.nshare = e->lay_opts.nshare ? e->lay_opts.nshare : e->block / 32;
   P.lay = e->lay;
 }
 }  // namespace
@@ -2586,6 +2596,7 @@ int pimc_server_run(pimc_engine* e) {
   P.nrep = e->nactive;
   P.seed = e->seed;
   P.wide = e->grid <= e->num_sms;
+  P.nshare = e->lay_opts.nshare ? e->lay_opts.nshare : e->block / 32;
   P.lay = e->lay;
   CU(cudaMemsetAsync(e->d_next.p, 0, sizeof(int), e->stream));
   CU(section_launch(e->minb, e->grid, e->block, e->lay.total * 8, e->stream, P));

@@ -859,12 +859,13 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   __syncthreads();
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, d = s.nlevel - P.level;
   double* lds = m.red + kWarps + 8;
+  double* buf = m.act + warp * m.act_stride;
   if (s.mixed)
-    action_warp<true>(s, m, ip, d, d, warp, nw, m.act + warp * m.act_stride);
+    action_warp<true>(s, m, ip, d, d, warp, nw, buf, buf);
   else
-    action_warp<false>(s, m, ip, d, d, warp, nw, m.act + warp * m.act_stride);
+    action_warp<false>(s, m, ip, d, d, warp, nw, buf, buf);
   __syncthreads();
-  action_reduce(s, m.act, m.act_stride, d, d, nw, lds);
+  action_reduce(s, m.act, m.act_stride, d, d, nw, nw, 0, lds);
   __syncthreads();
   if (threadIdx.x == 0) *out = lds[P.level];
 }

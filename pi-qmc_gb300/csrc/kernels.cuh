@@ -47,12 +47,14 @@ struct RunParams {
   long long xstage_cta;   // doubles per CTA
   int nrep;
   int wide;  // at most one CTA per SM
+  int nshare;  // warps that sums are shared out to, at least the block's
   uint64_t seed;
   Layout lay;
 };
 
 __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSys& s,
-                                      double* nodescr_g, double* xstage = nullptr, bool wide = false) {
+                                      double* nodescr_g, double* xstage = nullptr, bool wide = false,
+                                      int nshare = 0) {
   Smem m;
   // mixed form: this CTA's staging of the inverse blocks of an attempt's changed
   // slices ([nsec][2 + ns_max^2], global memory), committed to the cache on accept
@@ -105,6 +107,7 @@ __device__ __forceinline__ Smem carve(double* base, const Layout& L, const DevSy
   m.act = L.act >= 0 ? base + L.act
                      : (L.act_global ? gbase + (L.gcta - nw * L.act_stride) : m.nodescr);
   m.act_stride = L.act_stride;
+  m.nshare = nshare ? nshare : nw;
   return m;
 }
 
@@ -144,7 +147,10 @@ static __device__ __noinline__ double ewald_level0_cached(const DevSys& s, const
   double2* Z = Y + ny * w;
   double2* XY = X + per * w;
   const double qs = __dmul_rn(m.qpart[ipart], s.ek_scale);  // (exact: a power of two)
-  double acc = 0.0;
+  // (a term's place among all slices' decides whose share it is in: the sum does not
+  // depend on the passes or on the block)
+  const int nthr = 32 * m.nshare;
+  double acc[2] = {0.0, 0.0};
 #pragma unroll 1
   for (int t0 = 1; t0 < nsec - 1; t0 += chunk) {
     const int nc = 2 * min(chunk, nsec - 1 - t0);
@@ -167,8 +173,9 @@ static __device__ __noinline__ double ewald_level0_cached(const DevSys& s, const
       }
       __syncthreads();
     }
+    const int first = (threadIdx.x - (t0 - 1) * totk) & (blockDim.x - 1);
 #pragma unroll 1
-    for (int it = threadIdx.x; 2 * it < nc * totk; it += blockDim.x) {
+    for (int it = first; 2 * it < nc * totk; it += blockDim.x) {
       const int tt = it / totk, k = it - tt * totk, t = t0 + tt;
       const longlong2 o =
           *(const longlong2*)(ek + ((size_t)wrap_slice(ifirst1 + t, M) * totk + k) * 2);
@@ -192,14 +199,18 @@ static __device__ __noinline__ double ewald_level0_cached(const DevSys& s, const
       const longlong2 n = make_longlong2(o.x + d.x, o.y + d.y);
       *(longlong2*)(stage + ((size_t)(t - 1) * totk + k) * 2) = n;
       // |rho'|^2 - |rho|^2 = (rho' - rho) . (rho' + rho)
-      acc = __fma_rn(vk,
-                     __fma_rn(__ll2double_rn(d.x), __ll2double_rn(o.x + n.x),
-                              __dmul_rn(__ll2double_rn(d.y), __ll2double_rn(o.y + n.y))),
-                     acc);
+      const bool second = ((t0 - 1) * totk + it) & (nthr - 1) & blockDim.x;
+      const double a = __fma_rn(vk,
+                                __fma_rn(__ll2double_rn(d.x), __ll2double_rn(o.x + n.x),
+                                         __dmul_rn(__ll2double_rn(d.y), __ll2double_rn(o.y + n.y))),
+                                second ? acc[1] : acc[0]);
+      acc[0] = second ? acc[0] : a;
+      acc[1] = second ? a : acc[1];
     }
   }
   const double is = 1.0 / s.ek_scale;
-  const double sum = block_sum(acc, m.red) * (2 * is * is);
+  const double sum =
+      share_sum(m.nshare, m.red, [&](int h) { return h ? acc[1] : acc[0]; }) * (2 * is * is);
   return sum * s.one_over_2v * s.tau / s.epsilon;
 }
 
@@ -822,30 +833,32 @@ static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem&
 // (src/fixednode/FixedNodeAction.cc:96-131), after level 0's evaluations.
 static __device__ __noinline__ double nodal_action(const DevSys& s, const Smem& m, int n) {
   const int nsec = s.nsec, nsm = s.ns_max;
-  double part = 0.0;
-  FSum fpart;
+  return share_sum(m.nshare, m.red, [&](int h) {
+    double part = 0.0;
+    FSum fpart;
 #pragma unroll 1
-  for (int it = threadIdx.x; it < (nsec - 1) * n; it += blockDim.x) {
-    const int t = 1 + it / n, p = it - (t - 1) * n;
-    double num = 1.0, den = 1.0;
+    for (int it = threadIdx.x + h * blockDim.x; it < (nsec - 1) * n; it += 32 * m.nshare) {
+      const int t = 1 + it / n, p = it - (t - 1) * n;
+      double num = 1.0, den = 1.0;
 #pragma unroll 1
-    for (int side = 0; side < 2; ++side) {  // d1, then d2
-      const double* D = m.dist + (t * 2 + side) * nsm + p;
-      const double* N = m.ndist + (t * 2 + side) * nsm + p;
-      const double d = D[0] * D[-2 * nsm], e = N[0] * N[-2 * nsm];
-      if (s.mixed) {
-        // FP32 terms (1 - e^-x through expm1 keeps them accurate near the node),
-        // their sum compensated
-        const float a = -expm1f(-f32_rn(d)), b = -expm1f(-f32_rn(e));
-        fpart.add(logf(a) - logf(b));
-      } else {  // (one logarithm for both sides)
-        num *= 1 - exp(-d);
-        den *= 1 - exp(-e);
+      for (int side = 0; side < 2; ++side) {  // d1, then d2
+        const double* D = m.dist + (t * 2 + side) * nsm + p;
+        const double* N = m.ndist + (t * 2 + side) * nsm + p;
+        const double d = D[0] * D[-2 * nsm], e = N[0] * N[-2 * nsm];
+        if (s.mixed) {
+          // FP32 terms (1 - e^-x through expm1 keeps them accurate near the node),
+          // their sum compensated
+          const float a = -expm1f(-f32_rn(d)), b = -expm1f(-f32_rn(e));
+          fpart.add(logf(a) - logf(b));
+        } else {  // (one logarithm for both sides)
+          num *= 1 - exp(-d);
+          den *= 1 - exp(-e);
+        }
       }
+      if (!s.mixed) part += log(num / den);
     }
-    if (!s.mixed) part += log(num / den);
-  }
-  return block_sum(s.mixed ? fpart.value() : part, m.red);
+    return s.mixed ? fpart.value() : part;
+  });
 }
 
 // Bisection levels lo .. hi of the attempt at once, after its proposals (a
@@ -874,7 +887,9 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   // packed warp instruction serves several matrices
   int W = node_group_width(n);
   // (of the narrowest groups: the sums' shares do not depend on the launch)
-  const int a0 = first_action_warp(ntask * W, nwarps, s.mixed), dmax = L - alo, dmin = ahi == L ? 0 : dmax;
+  const int dmax = L - alo, dmin = ahi == L ? 0 : dmax;
+  const int shares = m.nshare - first_action_warp(ntask * W, m.nshare, s.mixed);
+  const int a0 = first_action_warp(ntask * W, nwarps, s.mixed);
   // A CTA that has its SM to itself is bound by the chain of each matrix's operations,
   // not by the pipe: it takes the widest groups that need no further round of the
   // warps without action terms (128 mixed dots, one a CTA: 50.9 -> 44.9 ms a round, and
@@ -946,15 +961,25 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
     }
   }
   if (alo <= ahi) {
+    // (the sums' shares are those of m.nshare warps, several to a warp here if need be)
+    const bool apart = m.nshare > nwarps;
+    const int words = apart ? action_sum_words(L) : 0;
+    const int off = apart ? action_sep_words(L, takes_single_levels(s), s.mixed) : 0;
     if (warp >= a0) {
       double* buf = m.act + (size_t)warp * m.act_stride;
-      if (s.mixed)
-        action_warp<true>(s, m, ipart, dmin, dmax, warp - a0, nwarps - a0, buf);
-      else
-        action_warp<false>(s, m, ipart, dmin, dmax, warp - a0, nwarps - a0, buf);
+      double* sums = buf + off;
+#pragma unroll 1
+      for (int w = warp - a0; w < shares; w += nwarps - a0) {
+        if (s.mixed)
+          action_warp<true>(s, m, ipart, dmin, dmax, w, shares, buf, sums);
+        else
+          action_warp<false>(s, m, ipart, dmin, dmax, w, shares, buf, sums);
+        sums += words;
+      }
     }
     __syncthreads();
-    action_reduce(s, m.act + (size_t)a0 * m.act_stride, m.act_stride, dmin, dmax, nwarps - a0, lds);
+    action_reduce(s, m.act + (size_t)a0 * m.act_stride + off, m.act_stride, dmin, dmax, shares,
+                  nwarps - a0, words, lds);
   }
   __syncthreads();
   const int flags = mynode ? m.ictl[C_FLAG] : 0;
@@ -1116,7 +1141,8 @@ __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
     }
     if (threadIdx.x == 0) {
       M_ = carve(smem, P.lay, P.sys[r], P.nodescr_g,
-                 P.xstage ? P.xstage + (size_t)blockIdx.x * P.xstage_cta : nullptr, P.wide);
+                 P.xstage ? P.xstage + (size_t)blockIdx.x * P.xstage_cta : nullptr, P.wide,
+                 P.nshare);
       status = P.state[r].status;
       nacc = 0;
 #pragma unroll 1

@@ -493,6 +493,28 @@ struct FSum {
   __device__ __forceinline__ double value() const { return (double)s + (double)c; }
 };
 
+// The sum of 32 nshare values, v(h) that of share warp + h nwarps (nwarps: the block's) on
+// this lane: the same tree whichever block the shares are dealt to.  All threads.
+template <class V>
+__device__ __forceinline__ double share_sum(int nshare, double* red, V v) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  __syncthreads();
+#pragma unroll 1
+  for (int h = 0; w + h * nw < nshare; ++h) {
+    double x = v(h);
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (l == 0) red[w + h * nw] = x;
+  }
+  __syncthreads();
+  if (w == 0) {
+    double x = (l < nshare) ? red[l] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (l == 0) red[kWarps] = x;
+  }
+  __syncthreads();
+  return red[kWarps];
+}
+
 // Deterministic block sum of one double per thread (fixed tree order).
 __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);

@@ -26,6 +26,8 @@ struct Smem {
   double* old;              // [2^L] the mover's terms of the old beads, by moved slice
   double* act;              // per-warp buffers of the action differences (actions.cuh)
   int act_stride;           // doubles per warp
+  int nshare;               // warps that sums are shared out to: the block's, or of a larger
+                            // block, whose shares this one takes several at a time
   double* dm;               // [nspecies][nsec] determinants at section set-up
   double* ndm;              // [nsec] determinants of the moving species' new slices
   double* dist;             // [nsec][2][ns_max] distances at set-up (moving species)
@@ -912,8 +914,10 @@ static __device__ void ewald_slice_sums(const DevSys& s, const Smem& m, int ipar
       ewald_bead_tables(s, X, Y, Z, w, p, m.mx[t], m.my[t], m.mz[t]);
   }
   __syncthreads();
-  double so = 0.0, sn_ = 0.0;
+  double so[2] = {0.0, 0.0}, sn_[2] = {0.0, 0.0};  // (of up to two shares)
+  const bool shares = m.nshare > (int)(blockDim.x >> 5);
   for (int k = threadIdx.x; k < s.totk; k += blockDim.x) {
+    const bool second = shares && ((k / blockDim.x) & 1);
     const int kx = __ldg(s.kvec + 3 * k), ky = __ldg(s.kvec + 3 * k + 1) + ky0,
               kz = __ldg(s.kvec + 3 * k + 2) + kz0;
     double cor = 0, coi = 0, cnr = 0, cni = 0;
@@ -944,11 +948,15 @@ static __device__ void ewald_slice_sums(const DevSys& s, const Smem& m, int ipar
       }
     }
     const double vk = __ldg(s.vk + k);
-    so += 2 * vk * (cor * cor + coi * coi);
-    sn_ += 2 * vk * (cnr * cnr + cni * cni);
+    const double o = (second ? so[1] : so[0]) + 2 * vk * (cor * cor + coi * coi);
+    const double n = (second ? sn_[1] : sn_[0]) + 2 * vk * (cnr * cnr + cni * cni);
+    so[0] = second ? so[0] : o;
+    so[1] = second ? o : so[1];
+    sn_[0] = second ? sn_[0] : n;
+    sn_[1] = second ? n : sn_[1];
   }
-  const double old_sum = block_sum(so, m.red);
-  const double new_sum = block_sum(sn_, m.red);
+  const double old_sum = share_sum(m.nshare, m.red, [&](int h) { return h ? so[1] : so[0]; });
+  const double new_sum = share_sum(m.nshare, m.red, [&](int h) { return h ? sn_[1] : sn_[0]; });
   eold = old_sum * s.one_over_2v + s.self_energy;
   enew = new_sum * s.one_over_2v + s.self_energy;
 }

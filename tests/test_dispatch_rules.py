@@ -18,6 +18,14 @@ int main() {
       for (int lanes = 0; lanes <= 32 * 40; lanes += 8)
         std::printf("action %d %d %d %d\n", mixed, nwarps, lanes,
                     first_action_warp(lanes, nwarps, mixed));
+  for (int nwarps = 1; nwarps <= 8; nwarps *= 2)
+    for (int nshare = nwarps; nshare <= 2 * nwarps; nshare *= 2)
+      for (int mixed = 0; mixed < 2; ++mixed)
+        for (int lanes = 0; lanes <= 32 * 20; lanes += 8)
+          std::printf("shares %d %d %d %d %d\n", nwarps, nshare,
+                      nshare - first_action_warp(lanes, nshare, mixed),
+                      nwarps - first_action_warp(lanes, nwarps, mixed),
+                      action_shares_per_warp(nwarps, nshare));
   static DevSys s;  // (no node models, no Ewald sums, no delayed rejection)
   for (s.nlevel = 1; s.nlevel <= 6; ++s.nlevel)
     for (s.npart = 1; s.npart <= 200; ++s.npart)
@@ -73,3 +81,12 @@ def test_joint_levels(rules):
         assert low == 0 if level < 5 else level - low <= 5
         if level == 6 or (level == 5 and npart > 32):
             assert level - low == 4
+
+
+def test_action_shares(rules):
+    # The shares of a larger block's action terms all have a warp and a place in its buffer.
+    for nwarps, nshare, shares, workers, most in (map(int, r[1:]) for r in rules
+                                                  if r[0] == "shares"):
+        assert 1 <= workers <= nwarps and 1 <= shares <= nshare
+        assert -(-shares // workers) <= most
+        assert nshare > nwarps or (shares == workers and most == 1)

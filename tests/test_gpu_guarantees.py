@@ -164,3 +164,41 @@ def test_thermo_energy_of_one_and_many(pimc, case, precision):
             ref = port.thermo_energy()
             assert abs(want - ref) <= (1e-5 if precision else 1e-12) * max(1.0, abs(ref))
         assert got[0] == want
+
+
+FEW_AND_MANY = {
+    # (system, paths, replicas of the larger engine): one warp a replica instead of two
+    # from eight replicas an SM on; four warps instead of eight, two CTAs an SM, for
+    # systems of which eight warps fill an SM, with more replicas than SMs
+    "dot2": (W.dot2(nslice=64, beta=2.5), "gauss", 1300),
+    "dot4_L3": (W.dot2(counts=[2, 2], nslice=64, beta=2.5, nlevel=3), "gauss", 1300),
+    "one_L6": (W.dot2(counts=[1], sho_omega=[1.0], nslice=64, beta=2.5, nlevel=6, coulomb=0),
+               "gauss", 1300),
+    "dot2_dr": (W.dot2(nslice=64, beta=2.5, delayed_rejection=1), "gauss", 1300),
+    "heg4": (W.heg54(n=4, nslice=1024, nlevel=4, node_kind=[0, 0]), "grid", 1300),
+    "heg4_uncached": (W.heg54(n=4, nslice=16, nlevel=4, beta=0.4, node_kind=[0, 0]), "grid", 1300),
+    "dot32_fn": (W.dot20_fn(counts=[16, 16], nslice=128, beta=5.0, node_temperature=0.25),
+                 "const", 170),
+    "heg54": (W.heg54(nslice=512, nlevel=4), "grid", 170),
+}
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", list(FEW_AND_MANY))
+def test_chains_of_few_and_many_replicas(pimc, case, precision):
+    # A replica's chain does not depend on how many replicas its engine has, bit for bit.
+    kw, kind, nrep = FEW_AND_MANY[case]
+    tabs, ew = pimc.coulomb_tables(kw) if kw["coulomb"] else ((), None)
+    x = [W.initial_path(dict(kw), kind, seed=r) for r in range(2)]
+    few = pimc.Engine(kw, 2, tabs, ew, seed=9, precision=precision)
+    many = pimc.Engine(kw, nrep, tabs, ew, seed=9, precision=precision)
+    few.upload_paths(x)
+    many.upload_paths([x[r % 2] for r in range(nrep)])
+    a, b = few.run_sections(30, records=True), many.run_sections(30, records=True)
+    if nrep == 1300:
+        assert (few.launch_config()["block"], many.launch_config()["block"]) == (64, 32)
+    for k in a:
+        assert np.array_equal(a[k], b[k][:2], equal_nan=True), k
+    for p, q in zip(few.download_paths(), many.download_paths()):
+        assert np.array_equal(p, q)
+    print(case, precision, few.launch_config()["block"], many.launch_config()["block"])
