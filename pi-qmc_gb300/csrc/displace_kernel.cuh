@@ -11,8 +11,9 @@
 // A replica's attempts follow one another, but the slices of an attempt are
 // independent, so a cluster of 1, 2, 4 or 8 CTAs takes a replica and shares its
 // slices: as many as keep the GPU busy with the replicas there are.  Every CTA
-// draws and decides the same from the CTAs' partial sums, exchanged through
-// distributed shared memory.  FP64 bound; what an attempt evaluates is
+// draws and decides the same from the partial sums, exchanged through distributed
+// shared memory: eight shares of every sum whatever the cluster, so that a replica's
+// decisions do not depend on how many there are.  FP64 bound; what an attempt evaluates is
 //  - the separations of the moved particles from the others, once per slice, each
 //    lane's neighbour supplying the previous slice;
 //  - with cached structure factors, the moved particles' terms alone (O(totk) per
@@ -71,9 +72,10 @@ __device__ __forceinline__ const double* bead_at(const double* path, int np, int
   return path + ((size_t)t * np + p) * 3;
 }
 
-// What the CTAs of a cluster exchange per attempt.
+// What the CTAs of a cluster exchange per attempt: its sums in kMaxDisplaceCluster shares,
+// of which a CTA computes as many as its part of the cluster.
 struct DisplaceShare {
-  double ds, node;
+  double ds[kMaxDisplaceCluster], node[kMaxDisplaceCluster];
   int bad, pad;
 };
 
@@ -117,10 +119,25 @@ __device__ __forceinline__ void displaced_bead(const DevSys& s, const Moved& mv,
   }
 }
 
+// The sums of an attempt, in nv shares: this warp's value of share v.  CTA rank of the
+// cluster's C has shares rank, rank + C, ... (the first of the work goes to all CTAs).
+struct DisplaceParts {
+  static constexpr int nv = kMaxDisplaceCluster;
+  double of[3][nv * (kBlock / 32)];  // action differences, Ewald terms, nodal actions
+  static __device__ __forceinline__ double warp_tree(double x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    return x;
+  }
+  __device__ __forceinline__ void put(int kind, int v, double x) {
+    x = warp_tree(x);
+    if ((threadIdx.x & 31) == 0) of[kind][v * (blockDim.x >> 5) + (threadIdx.x >> 5)] = x;
+  }
+};
+
 // SHOAction and PairAction over slices [0, i2] (and [half, half + i2]) of the whole
-// path, this thread's share (warp gw of the cluster's ngw).
-static __device__ __noinline__ double displace_actions(const DevSys& s, const Moved& mv,
-                                                       const double* path, int gw, int ngw) {
+// path, this thread's part of a share (warp gw of all shares' ngw).
+__device__ __forceinline__ double displace_actions_share(const DevSys& s, const Moved& mv,
+                                                         const double* path, int gw, int ngw) {
   const int np = s.npart, M = s.nslice, half = M / 2, lane = threadIdx.x & 31;
   const bool dbl = s.fixed_node != 0;
   const int nrange = dbl ? 2 : 1, len = dbl ? half : M;
@@ -202,6 +219,14 @@ static __device__ __noinline__ double displace_actions(const DevSys& s, const Mo
     }
   }
   return part;
+}
+static __device__ __noinline__ void displace_actions(const DevSys& s, const Moved& mv,
+                                                     const double* path, int rank, int C,
+                                                     DisplaceParts& parts) {
+  const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+#pragma unroll 1
+  for (int v = rank; v < parts.nv; v += C)
+    parts.put(0, v, displace_actions_share(s, mv, path, v * nwarps + warp, parts.nv * nwarps));
 }
 
 // CoulombAction's long-range term from the cached structure factors: per slice, the
@@ -457,6 +482,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
   __shared__ long long nacc;
   __shared__ int rnext[2], bad_, accept_;
   __shared__ DisplaceShare share[2];
+  __shared__ DisplaceParts parts;
   __shared__ int flip[kMaxSpecies], ovalid[kMaxSpecies];
   __shared__ Smem M_;  // carved pointers, shared so that callees read them from shared memory
   cg::cluster_group cl = cg::this_cluster();
@@ -464,6 +490,8 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
   const int cluster = blockIdx.x / C;
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int gw = rank * nwarps + warp, ngw = C * nwarps;
+  constexpr int nv = DisplaceParts::nv;
+  const int nvw = nv * nwarps;
   cl.sync();  // every CTA has started: its shared memory may be written to
   for (int turn = 0;; ++turn) {
     if (threadIdx.x == 0 && rank == 0) {
@@ -562,21 +590,21 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
         bad_ = 0;
       }
       __syncthreads();
-      // ---- Action differences, this CTA's share
-      double part = displace_actions(s, mv, path, gw, ngw);
-      double ds = block_sum(part, m.red);
-      if (s.coulomb && s.ewald) {
-        if (ek) {
-          const double lr = displace_ewald(s, mv, path, m.qpart, ek,
-                                           m.ewx + (size_t)warp * P.lay.ek_stride,
-                                           P.lay.ek_batch, gw, ngw, false);
-          ds += block_sum(lr, m.red) * s.one_over_2v * s.tau / s.epsilon;
-        } else {
-          ds += displace_ewald_full(s, m, mv, path, m0, m1);
+      // ---- Action differences, this CTA's shares
+      displace_actions(s, mv, path, rank, C, parts);
+      if (s.coulomb && s.ewald)
+        for (int v = rank; v < nv; v += C) {
+          if (ek) {
+            parts.put(1, v, displace_ewald(s, mv, path, m.qpart, ek,
+                                     m.ewx + (size_t)warp * P.lay.ek_stride, P.lay.ek_batch,
+                                     v * nwarps + warp, nvw, false));
+          } else {
+            const int e0 = (int)((long long)M * v / nv), e1 = (int)((long long)M * (v + 1) / nv);
+            const double lr = displace_ewald_full(s, m, mv, path, e0, e1);
+            parts.put(1, v, threadIdx.x == 0 ? lr : 0.0);
+          }
         }
-      }
       // ---- FixedNodeAction per node species holding a moving particle
-      double dsn = 0.0;
       if (dbl) {
         bool bad = false;
         for (int sp = 0; sp < s.nspecies; ++sp) {
@@ -593,49 +621,66 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
         }
         if (bad) bad_ = 1;
         cl.sync();  // the other CTAs' determinants and distances
-        double np_part = 0.0;
         bad = false;
-        for (int sp = 0; sp < s.nspecies; ++sp) {
-          if (!s.node_kind[sp] || !moved_mask(s, mv, sp)) continue;
-          const int n = s.spec_count[sp];
-          const double* ndet = scr + sp * spw;
-          const double* odist = ndet + half + (size_t)flip[sp] * half * 2 * nsm;
-          const double* ndist = ndet + half + (size_t)(flip[sp] ^ 1) * half * 2 * nsm;
-          // a sign change against the first slice rejects
-          for (int t = max(1, h0) + threadIdx.x; t < h1; t += blockDim.x)
-            bad |= ndet[t] * ndet[0] < 0.0;
-          // nodal action: -sum log(new) + sum log(old) over consecutive pairs
-          const int lo = max(1, h0);
-          for (int it = threadIdx.x; it < (h1 - lo) * n; it += blockDim.x) {
-            const int t = lo + it / n, p = it % n;
-            const double* a1 = ndist + (size_t)t * 2 * nsm;
-            const double* a0 = ndist + (size_t)(t - 1) * 2 * nsm;
-            const double* b1 = odist + (size_t)t * 2 * nsm;
-            const double* b0 = odist + (size_t)(t - 1) * 2 * nsm;
-            np_part -= log((1 - exp(-a1[p] * a0[p])) * (1 - exp(-a1[nsm + p] * a0[nsm + p])));
-            np_part += log((1 - exp(-b1[p] * b0[p])) * (1 - exp(-b1[nsm + p] * b0[nsm + p])));
+        for (int v = rank; v < nv; v += C) {
+          double np_part = 0.0;
+          const int first = 32 * (warp * nv + v) + (threadIdx.x & 31);
+          for (int sp = 0; sp < s.nspecies; ++sp) {
+            if (!s.node_kind[sp] || !moved_mask(s, mv, sp)) continue;
+            const int n = s.spec_count[sp];
+            const double* ndet = scr + sp * spw;
+            const double* odist = ndet + half + (size_t)flip[sp] * half * 2 * nsm;
+            const double* ndist = ndet + half + (size_t)(flip[sp] ^ 1) * half * 2 * nsm;
+            // a sign change against the first slice rejects
+            for (int t = first; t < half; t += 32 * nvw)
+              bad |= ndet[t] * ndet[0] < 0.0;
+            // nodal action: -sum log(new) + sum log(old) over consecutive pairs
+            for (int it = first; it < (half - 1) * n; it += 32 * nvw) {
+              const int t = 1 + it / n, p = it % n;
+              const double* a1 = ndist + (size_t)t * 2 * nsm;
+              const double* a0 = ndist + (size_t)(t - 1) * 2 * nsm;
+              const double* b1 = odist + (size_t)t * 2 * nsm;
+              const double* b0 = odist + (size_t)(t - 1) * 2 * nsm;
+              np_part -= log((1 - exp(-a1[p] * a0[p])) * (1 - exp(-a1[nsm + p] * a0[nsm + p])));
+              np_part += log((1 - exp(-b1[p] * b0[p])) * (1 - exp(-b1[nsm + p] * b0[nsm + p])));
+            }
           }
+          parts.put(2, v, np_part);
         }
         if (bad) bad_ = 1;
-        dsn = block_sum(np_part, m.red);  // (its barriers order bad_)
       }
-      // ---- the CTAs' shares, summed alike by every CTA
+      __syncthreads();
+      // ---- the shares, summed alike by every CTA
       DisplaceShare* mine = &share[a & 1];
-      if (threadIdx.x == 0) {
-        mine->ds = ds;
-        mine->node = dsn;
-        mine->bad = bad_;
-      }
-      cl.sync();
-      if (threadIdx.x == 0) {
-        double dst = 0.0, nodet = 0.0;
-        int bad = 0;
-        for (int c = 0; c < C; ++c) {
-          const DisplaceShare* o = cl.map_shared_rank(mine, c);
-          dst += o->ds;
-          nodet += o->node;
-          bad |= o->bad;
+      for (int v = rank + warp * C; v < nv; v += nwarps * C) {
+        const int l = threadIdx.x & 31, at = v * nwarps + l;
+        double x = parts.warp_tree(l < nwarps ? parts.of[0][at] : 0.0);
+        if (s.coulomb && s.ewald) {
+          const double lr = parts.warp_tree(l < nwarps ? parts.of[1][at] : 0.0);
+          x += ek ? lr * s.one_over_2v * s.tau / s.epsilon : lr;
         }
+        const double node = dbl ? parts.warp_tree(l < nwarps ? parts.of[2][at] : 0.0) : 0.0;
+        if (l == 0) {
+          mine->ds[v] = x;
+          mine->node[v] = node;
+        }
+      }
+      if (threadIdx.x == 0) mine->bad = bad_;
+      cl.sync();
+      double dst = 0.0, nodet = 0.0;
+      bool bad = false;
+      if (threadIdx.x < 32) {  // (a share per lane)
+        if (threadIdx.x < nv) {
+          const DisplaceShare* o = cl.map_shared_rank(mine, threadIdx.x % C);
+          dst = o->ds[threadIdx.x];
+          nodet = o->node[threadIdx.x];
+          bad = o->bad;
+        }
+        dst = parts.warp_tree(dst);
+        nodet = parts.warp_tree(nodet);
+        bad = __any_sync(0xffffffffu, bad);
+      }
+      if (threadIdx.x == 0) {
         if (bad) nodet = 2e100;
         // ---- Metropolis test
         const double total = dst + nodet;

@@ -202,3 +202,33 @@ def test_chains_of_few_and_many_replicas(pimc, case, precision):
     for p, q in zip(few.download_paths(), many.download_paths()):
         assert np.array_equal(p, q)
     print(case, precision, few.launch_config()["block"], many.launch_config()["block"])
+
+
+FEW_AND_MANY_DISPLACED = {
+    "dot2": (W.dot2(nslice=256, beta=10.0), "gauss"),
+    "dot5_fn": (W.dot20_fn(counts=[3, 2], nslice=40, beta=2.0, nlevel=2, node_temperature=0.5),
+                "const"),
+    "dot20_fn": (W.dot20_fn(nslice=128, beta=5.0, nlevel=4, node_temperature=0.25), "const"),
+    "heg10": (W.heg54(n=10, nslice=16, nlevel=2, t_over_tf=1.5), "grid"),
+    "heg10_uncached": (W.heg54(n=10, nslice=8, nlevel=2, t_over_tf=3.0), "grid"),
+}
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", list(FEW_AND_MANY_DISPLACED))
+def test_displacements_of_few_and_many_replicas(pimc, case, precision):
+    # The CTAs that share a replica are as many as the replicas leave room for: the
+    # decisions' sums do not depend on them, bit for bit.
+    kw, kind = FEW_AND_MANY_DISPLACED[case]
+    tabs, ew = pimc.coulomb_tables(kw)
+    x = W.initial_path(dict(kw), kind, seed=3)
+    want = None
+    for nrep in (1, 21, 60, 170, 700):
+        e = pimc.Engine(kw, nrep, tabs, ew, seed=99, precision=precision)
+        e.upload_paths([x] * nrep)
+        d = e.run_displace(12, [0.8, 0.8, 0.8], 1, -1, records=True)
+        got = [d[k][0] for k in sorted(d)] + [e.download_paths()[0]]
+        e.close()
+        want = want or got
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b), nrep
