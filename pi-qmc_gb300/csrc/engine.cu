@@ -1934,11 +1934,14 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   if (!lok) return fail(PIMC_ERR_CAPACITY, "working set does not fit in shared memory");
   const size_t nsecd = (size_t)nbatch * s.nsec * s.npart * 3, nmovd = (size_t)nbatch * s.nsec * 3;
   // with Ewald sums the section's slices go to CTAs of their own, as many per entry as
-  // a batch of this size leaves room for (two CTAs an SM), added up here in order
-  int parts = 1;
-  if (s.ewald && s.coulomb && level == 0)
+  // a batch of this size leaves room for (two CTAs an SM); the slices' terms are added up
+  // here in order, so that an entry's value does not depend on its batch
+  int parts = 1, terms = 1;
+  if (s.ewald && s.coulomb && level == 0) {
     parts = 1 + std::max(1, std::min(s.nsec - 2, 2 * e->num_sms / nbatch));
-  std::vector<double> share((size_t)nbatch * parts);
+    terms = s.nsec - 1;
+  }
+  std::vector<double> share((size_t)nbatch * terms);
   EntryIo io(e);
   const int sec = io.in(section, nsecd * 8), mov = io.in(moving, nmovd * 8);
   const int ip = io.in(ipart, nbatch * sizeof(int));
@@ -1952,6 +1955,7 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
   P.moving = io.dev<double>(mov);
   P.ipart = io.dev<int>(ip);
   P.ds = io.dev<double>(out);
+  P.terms = terms;
   P.level = level;
   P.lay = alay;
   P.scratch = alay.act_global ? io.dev<double>(scr) : nullptr;
@@ -1961,15 +1965,15 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
     Q.section += (size_t)b0 * s.nsec * s.npart * 3;
     Q.moving += (size_t)b0 * s.nsec * 3;
     Q.ipart += b0;
-    Q.ds += (size_t)b0 * parts;
+    Q.ds += (size_t)b0 * terms;
     action_diff_kernel<<<dim3(parts, nb), kBlock, P.lay.total * 8, e->stream>>>(Q);
     e->launches++;
   }
   CU(cudaGetLastError());
   if (int rc = io.close()) return rc;
   for (int b = 0; b < nbatch; ++b) {
-    double v = share[(size_t)b * parts];
-    for (int k = 1; k < parts; ++k) v += share[(size_t)b * parts + k];
+    double v = share[(size_t)b * terms];
+    for (int k = 1; k < terms; ++k) v += share[(size_t)b * terms + k];
     ds[b] = v;
   }
   return PIMC_OK;

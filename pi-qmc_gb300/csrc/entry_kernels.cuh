@@ -760,7 +760,8 @@ struct ActionDiffParams {
   const double* section;  // [nbatch][nsec][npart][3]
   const double* moving;   // [nbatch][nsec][3]
   const int* ipart;
-  double* ds;             // [nbatch][gridDim.x] shares, added by the caller
+  double* ds;             // [nbatch][terms], added by the caller: the links', every slice's
+  int terms;
   int level;
   Layout lay;
   double* scratch;  // the layout's global area per entry (null: none)
@@ -837,13 +838,13 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   const double* sec = P.section + (size_t)b * nsec * np * 3;
   const double* mov = P.moving + (size_t)b * nsec * 3;
   const int ip = P.ipart[b];
-  double* out = P.ds + (size_t)b * gridDim.x + blockIdx.x;
+  double* out = P.ds + (size_t)b * P.terms;
   if (blockIdx.x > 0) {
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
-    double ds = 0.0;
-    for (int t = blockIdx.x; t < nsec - 1; t += gridDim.x - 1)
-      ds += ewald_move_energy(s, m, sec + (size_t)t * np * 3, mov + (size_t)t * 3, ip);
-    if (threadIdx.x == 0) *out = ds * s.tau / s.epsilon;
+    for (int t = blockIdx.x; t < nsec - 1; t += gridDim.x - 1) {
+      const double de = ewald_move_energy(s, m, sec + (size_t)t * np * 3, mov + (size_t)t * 3, ip);
+      if (threadIdx.x == 0) out[t] = de * s.tau / s.epsilon;
+    }
     return;
   }
   for (int idx = threadIdx.x; idx < nsec * np; idx += blockDim.x) {
@@ -867,7 +868,7 @@ __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P)
   __syncthreads();
   action_reduce(s, m.act, m.act_stride, d, d, nw, nw, 0, lds);
   __syncthreads();
-  if (threadIdx.x == 0) *out = lds[P.level];
+  if (threadIdx.x == 0) out[0] = lds[P.level];
 }
 
 // ---------------------------------------------------- NodeModel-level entry

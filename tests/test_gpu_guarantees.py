@@ -232,3 +232,22 @@ def test_displacements_of_few_and_many_replicas(pimc, case, precision):
         want = want or got
         for a, b in zip(got, want):
             assert np.array_equal(a, b), nrep
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [10, 54])
+def test_action_difference_in_any_batch(pimc, n, precision):
+    # An entry's value does not depend on how many entries there are, bit for bit.
+    kw = W.heg54(n=n, nslice=512, nlevel=4)
+    tabs, ew = pimc.coulomb_tables(kw)
+    e = pimc.Engine(kw, 1, tabs, ew, precision=precision)
+    rng = np.random.default_rng(n)
+    nb = 300
+    sec = rng.uniform(-0.5, 0.5, size=(nb, 17, n, 3)) * kw["cell"]
+    ip = rng.integers(0, n, nb).astype(np.int32)
+    mov = sec[np.arange(nb), :, ip].copy()
+    mov[:, 1:-1] += 0.3 * rng.normal(size=mov[:, 1:-1].shape)
+    for level in (0, 1):
+        whole = e.action_difference(level, sec, mov, ip)
+        for b in (1, 3, 17, 40, 120):
+            assert np.array_equal(e.action_difference(level, sec[:b], mov[:b], ip[:b]), whole[:b]), b
