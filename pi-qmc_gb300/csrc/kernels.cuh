@@ -590,6 +590,14 @@ __device__ __forceinline__ int cache_mask_slot(const DevSys& s, int sp) {
 __host__ __device__ __forceinline__ bool sm_species(const DevSys& s, int sp) {
   return s.mixed && s.node_kind[sp] == PIMC_NODES_FREE;
 }
+// Lane-group width of a species' evaluations in a launch that asks for wmin lanes at
+// least: that of its size where it takes updates, which the matrices of a warp take
+// together or not at all (one matrix a warp instead of four would update others, and a
+// chain depend on the launch it runs in).
+__host__ __device__ __forceinline__ int node_launch_width(const DevSys& s, int sp, int wmin) {
+  const int n = s.spec_count[sp], w = node_group_width(n), most = node_group_widest(n);
+  return sm_species(s, sp) || wmin < w ? w : (wmin < most ? wmin : most);
+}
 // Mixed form: index of the entry's inverse block [epoch of its scale, updates
 // since the last factorisation, inverse (n*n, X layout)], after the stale-row word.
 __device__ __forceinline__ int cache_x_slot(const DevSys& s, int sp) {
@@ -659,15 +667,23 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   // warp tasks: each warp takes up to G misses of one species (lane groups of
   // a warp must run the same species so that they stay converged)
   int ntask = 0, first[kMaxSpecies + 1], wmin = m.wide ? 32 : 8;
+  unsigned narrow = 0, widest = 0;  // a byte per species: its groups' widths
+#pragma unroll 1
+  for (int sp = 0; sp < s.nspecies; ++sp) {
+    narrow |= (unsigned)node_launch_width(s, sp, 8) << (8 * sp);
+    widest |= (unsigned)node_launch_width(s, sp, wmin) << (8 * sp);
+  }
+  const auto width = [&](int sp) {
+    return min(max(wmin, (int)((narrow >> (8 * sp)) & 63u)), (int)((widest >> (8 * sp)) & 63u));
+  };
 #pragma unroll 1
   for (;; wmin >>= 1) {  // (wide: the widest groups that take no further round)
     ntask = 0;
 #pragma unroll 1
     for (int sp = 0; sp < s.nspecies; ++sp) {
-      const int n = s.spec_count[sp];
-      const int G = 32 / min(max(wmin, node_group_width(n)), node_group_widest(n));
+      const int shift = 6 - __ffs(width(sp));  // 32 / width groups a warp
       first[sp] = ntask;
-      ntask += (nmiss[sp] + G - 1) / G;
+      ntask += (nmiss[sp] + (1 << shift) - 1) >> shift;
     }
     first[s.nspecies] = ntask;
     if (wmin == 8 || ntask <= nwarps) break;
@@ -679,7 +695,7 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
     while (wt >= first[sp + 1]) ++sp;
     const int n = s.spec_count[sp];
     const bool sho = s.node_kind[sp] == PIMC_NODES_SHO, mine = sp == msp;
-    const int W = min(max(wmin, node_group_width(n)), node_group_widest(n));
+    const int W = width(sp);
     const int G = 32 / W, gm = lane / W, glm = lane & (W - 1);
     const int base = (wt - first[sp]) * G;
     const int task = base + gm;
@@ -895,9 +911,9 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   // warps without action terms (128 mixed dots, one a CTA: 50.9 -> 44.9 ms a round, and
   // 41.1 with half of the warps on the action; two CTAs per SM share the pipe, where
   // narrow groups' fewer instructions count).
-  if (m.wide) {
-    const int most = a0 == 0 || alo > ahi ? nwarps : a0;
-    while (W < node_group_widest(n) && ntask * W <= 16 * most) W *= 2;
+  if (m.wide && mynode) {
+    const int most = a0 == 0 || alo > ahi ? nwarps : a0, widest = node_launch_width(s, msp, 32);
+    while (W < widest && ntask * W <= 16 * most) W *= 2;
   }
   const int G = 32 / W, g = lane / W, nodeW = min(nwarps, (ntask + G - 1) / G);
   if (mynode) {

@@ -27,6 +27,17 @@ int main() {
                       nwarps - first_action_warp(lanes, nwarps, mixed),
                       action_shares_per_warp(nwarps, nshare));
   static DevSys s;  // (no node models, no Ewald sums, no delayed rejection)
+  for (int kind : {PIMC_NODES_SHO, PIMC_NODES_FREE})
+    for (int mixed = 0; mixed < 2; ++mixed)
+      for (int n = 1; n <= 32; ++n)
+        for (int wmin = 8; wmin <= 32; wmin *= 2) {
+          s.node_kind[0] = kind;
+          s.mixed = mixed;
+          s.spec_count[0] = n;
+          std::printf("width %d %d %d %d %d\n", kind == PIMC_NODES_FREE, mixed, n, wmin,
+                      node_launch_width(s, 0, wmin));
+        }
+  s = DevSys();
   for (s.nlevel = 1; s.nlevel <= 6; ++s.nlevel)
     for (s.npart = 1; s.npart <= 200; ++s.npart)
       for (int mixed = 0; mixed < 2; ++mixed) {
@@ -90,3 +101,18 @@ def test_action_shares(rules):
         assert 1 <= workers <= nwarps and 1 <= shares <= nshare
         assert -(-shares // workers) <= most
         assert nshare > nwarps or (shares == workers and most == 1)
+
+
+def test_lane_group_widths(rules):
+    # The groups that update matrices together are the same in every launch; the others
+    # may be wider in a launch that asks for it.
+    wider = 0
+    for free, mixed, n, wmin, w in (map(int, r[1:]) for r in rules if r[0] == "width"):
+        own = 8 if n <= 8 else 16 if n <= 16 else 32
+        assert w >= own and w in (8, 16, 32)
+        if free and mixed:
+            assert w == own
+        else:
+            assert w <= max(own, wmin)
+            wider += w > own
+    assert wider

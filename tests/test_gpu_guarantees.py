@@ -251,3 +251,23 @@ def test_action_difference_in_any_batch(pimc, n, precision):
         whole = e.action_difference(level, sec, mov, ip)
         for b in (1, 3, 17, 40, 120):
             assert np.array_equal(e.action_difference(level, sec[:b], mov[:b], ip[:b]), whole[:b]), b
+
+
+@pytest.mark.parametrize("n", [10, 14, 22, 30])
+def test_update_groups_of_few_and_many_replicas(pimc, n):
+    # Mixed form, free-particle nodes: whether a matrix is updated or factorised does not
+    # depend on how full the launch is, so neither does a replica's chain, bit for bit.
+    # (a short ring: entries reach their last update at different times)
+    kw = W.heg54(n=n, nslice=32, nlevel=3, t_over_tf=3.0, coulomb=0, ewald=0)
+    x = W.initial_path(dict(kw), "grid", seed=1)
+    # (the updates' rounding shows in few of the FP32 nodal terms)
+    few = pimc.Engine(kw, 150, seed=9, precision=1)
+    many = pimc.Engine(kw, 700, seed=9, precision=1)
+    few.upload_paths([x] * 150)
+    many.upload_paths([x] * 700)
+    for _ in range(4):
+        a, b = few.run_sections(100, records=True), many.run_sections(100, records=True)
+        for k in a:
+            assert np.array_equal(a[k], b[k][:150], equal_nan=True), k
+    for p, q in zip(few.download_paths(), many.download_paths()):
+        assert np.array_equal(p, q)
