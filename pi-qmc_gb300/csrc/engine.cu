@@ -8,7 +8,6 @@
 #include <cstring>
 #include <limits>
 #include <map>
-#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -127,6 +126,8 @@ struct DevBuf {
 
 }  // namespace
 
+#include "entry_io.h"
+
 constexpr int kThermoChunks = 64;  // CTAs per replica of the estimators, at most
 constexpr int kThermoParts = 8;    // parts of a chunk, at most
 
@@ -189,10 +190,8 @@ struct pimc_engine {
   DevBuf<double> d_dscratch;  // displacement moves: node dets and distances per CTA
   DevBuf<double> d_energy;   // [steps][nrep]
   DevBuf<double> d_forces;   // virial estimator: forces of a pass's replicas (bounded)
-  // host data of the calls that take or return arrays (EntryIo)
-  std::mutex io_mutex;
-  DevBuf<char> io_dev;
-  char* io_host = nullptr;
+  // host data of the calls that take or return arrays
+  IoBlocks io;
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   int graph_attempts = -1, graph_steps = -1;
@@ -213,8 +212,7 @@ struct pimc_engine {
     d_dscratch.free();
     d_energy.free();
     d_forces.free();
-    io_dev.free();
-    if (io_host) cudaFreeHost(io_host);
+    io.free();
     d_sys.free();
     d_state.free();
     d_paths.free();
@@ -240,103 +238,6 @@ struct pimc_engine {
 };
 
 namespace {
-
-// The arrays of one call between the caller's memory and the device.  A call names
-// its inputs, outputs and scratch, open() places them, dev() gives their device
-// addresses, and close() waits for the stream and delivers the outputs.  Small calls
-// (kIoMapped of inputs and outputs) run on a pinned host block of the engine that the
-// kernels read and write themselves: no copies are queued.  Larger ones copy from
-// and to the caller's memory through a device block, kept up to kIoKeep.  (Allocated
-// from the stream's pool in each call, which gives its memory back at every
-// synchronisation: a node evaluation of one pair took 275 us, now 61.)  The engine's
-// blocks serve one call at a time: a call holds the engine's mutex, and leaves with
-// the stream idle.
-constexpr size_t kIoMapped = 128 << 10, kIoKeep = 64 << 20;
-
-class EntryIo {
- public:
-  explicit EntryIo(pimc_engine* e) : eng_(e), lock_(e->io_mutex) {}
-  ~EntryIo() {
-    if (own_) cudaFreeAsync(own_, eng_->stream);
-  }
-  int in(const void* p, size_t bytes) { return add(const_cast<void*>(p), bytes, kIn); }
-  // (a table that every CTA reads: to device memory in either case)
-  int in_device(const void* p, size_t bytes) { return add(const_cast<void*>(p), bytes, kInDevice); }
-  int out(void* p, size_t bytes, bool zeroed = false) {
-    return add(p, bytes, zeroed ? kOutZero : kOut);
-  }
-  int scratch(size_t bytes) { return add(nullptr, bytes, kScratch); }
-  int open() {
-    size_t io = 0, tmp = 0;
-    for (const Part& p : parts_) (p.kind >= kInDevice ? tmp : io) += p.bytes;
-    mapped_ = io <= kIoMapped;
-    if (mapped_ && !eng_->io_host &&
-        cudaHostAlloc((void**)&eng_->io_host, kIoMapped, cudaHostAllocMapped) != cudaSuccess) {
-      cudaGetLastError();
-      eng_->io_host = nullptr;
-      mapped_ = false;
-    }
-    const size_t need = tmp + (mapped_ ? 0 : io);
-    char* dev = nullptr;
-    if (need > kIoKeep) {
-      CU(cudaMallocAsync(&own_, need, eng_->stream));
-      dev = own_;
-    } else if (need) {
-      if (eng_->io_dev.n < need) {
-        CU(cudaStreamSynchronize(eng_->stream));
-        if (eng_->io_dev.alloc(std::min(kIoKeep, std::max<size_t>(2 * eng_->io_dev.n, need))))
-          return fail(PIMC_ERR_CUDA, "cudaMalloc call buffers");
-      }
-      dev = eng_->io_dev.p;
-    }
-    size_t hoff = 0, doff = 0;
-    for (Part& p : parts_) {
-      const bool on_host = mapped_ && p.kind < kInDevice;
-      size_t& off = on_host ? hoff : doff;
-      p.dev = (on_host ? eng_->io_host : dev) + off;
-      off += p.bytes;
-      if (mapped_ && p.kind == kIn) memcpy(p.dev, p.host, p.size);
-      if (mapped_ && p.kind == kOutZero) memset(p.dev, 0, p.size);
-      if (((!mapped_ && p.kind == kIn) || p.kind == kInDevice) && p.size)
-        CU(cudaMemcpyAsync(p.dev, p.host, p.size, cudaMemcpyHostToDevice, eng_->stream));
-      if (!mapped_ && p.kind == kOutZero) CU(cudaMemsetAsync(p.dev, 0, p.size, eng_->stream));
-    }
-    return PIMC_OK;
-  }
-  template <class T>
-  T* dev(int k) const {
-    return (T*)parts_[k].dev;
-  }
-  int close() {
-    if (!mapped_)
-      for (const Part& p : parts_)
-        if (p.kind == kOut || p.kind == kOutZero)
-          CU(cudaMemcpyAsync(p.host, p.dev, p.size, cudaMemcpyDeviceToHost, eng_->stream));
-    CU(cudaStreamSynchronize(eng_->stream));
-    if (mapped_)
-      for (const Part& p : parts_)
-        if (p.kind == kOut || p.kind == kOutZero) memcpy(p.host, p.dev, p.size);
-    return PIMC_OK;
-  }
-
- private:
-  enum Kind { kIn, kOut, kOutZero, kInDevice, kScratch };
-  struct Part {
-    void* host;
-    size_t size, bytes;  // bytes: rounded up, so that the next part stays aligned
-    Kind kind;
-    char* dev;
-  };
-  int add(void* p, size_t size, Kind kind) {
-    parts_.push_back({p, size, (size + 255) & ~(size_t)255, kind, nullptr});
-    return (int)parts_.size() - 1;
-  }
-  pimc_engine* eng_;
-  std::lock_guard<std::mutex> lock_;
-  std::vector<Part> parts_;
-  char* own_ = nullptr;
-  bool mapped_ = false;
-};
 
 // PeriodicGaussian constructor constants (src/util/PeriodicGaussian.cc:7-18).
 void pg_params(double alpha, double length, double& nome, double& pref, double& k, int& nmax) {
@@ -1554,7 +1455,7 @@ int pimc_run_sections(pimc_engine* e, int nattempt, pimc_move_record* records) {
     return PIMC_OK;
   };
   if (!records) return launch(nullptr);
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int rec = io.out(records, sizeof(pimc_move_record) * (size_t)e->nrep * nattempt, true);
   if (int rc = io.open()) return rc;
   if (int rc = launch(io.dev<pimc_move_record>(rec))) return rc;
@@ -1670,7 +1571,7 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
 }
 // The same with nothing but the energies to return.
 int run_estimator_host(pimc_engine* e, int which, const EstimatorParams& P, double* host) {
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int out = io.out(host, e->nrep * sizeof(double));
   if (int rc = io.open()) return rc;
   if (int rc = run_estimator(e, which, P, e->est_lay, io.dev<double>(out))) return rc;
@@ -1772,7 +1673,7 @@ int pimc_run_displace(pimc_engine* e, int nattempt, const double* box, int nmovi
     return PIMC_OK;
   };
   if (!records) return launch(nullptr);
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int rec = io.out(records, sizeof(pimc_displace_record) * (size_t)e->nrep * nattempt, true);
   if (int rc = io.open()) return rc;
   if (int rc = launch(io.dev<pimc_displace_record>(rec))) return rc;
@@ -1800,7 +1701,7 @@ int pimc_ewald_coulomb_energy(pimc_engine* e, double epsilon, double rcut,
   if (!e || e->server || !(epsilon > 0) || !(rcut > 0) || !est || !vgrid || !host_energy ||
       est->totk < 0 || (est->totk > 0 && (!est->kvec || !est->vk)))
     return fail(PIMC_ERR_INVALID, "bad argument");
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int kv = io.in_device(est->kvec, 3 * est->totk * sizeof(int));
   const int vk = io.in_device(est->vk, est->totk * sizeof(double));
   const int vg = io.in_device(vgrid, 1001 * sizeof(double));
@@ -1942,7 +1843,7 @@ int pimc_action_difference(pimc_engine* e, int level, int nbatch, const double* 
     terms = s.nsec - 1;
   }
   std::vector<double> share((size_t)nbatch * terms);
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int sec = io.in(section, nsecd * 8), mov = io.in(moving, nmovd * 8);
   const int ip = io.in(ipart, nbatch * sizeof(int));
   const int out = io.out(share.data(), share.size() * 8);
@@ -1989,7 +1890,7 @@ int pimc_node_evaluate(pimc_engine* e, int ispec, int nbatch, const double* r1, 
   const int np = s.npart;
   const size_t nr = (size_t)nbatch * np * 3;
   const NodeEvalShape sh = node_eval_shape(s, ispec, nbatch, e->num_sms);
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int a1 = io.in(r1, nr * 8), a2 = io.in(r2, nr * 8);
   const int odet = io.out(det, nbatch * 8), oerr = io.out(err, nbatch * sizeof(int));
   const int od1 = io.out(d1, (size_t)nbatch * np * 8), od2 = io.out(d2, (size_t)nbatch * np * 8);
@@ -2619,7 +2520,7 @@ int server_energy(pimc_engine* e, const std::vector<int>& slots, double* out) {
   // whatever the mix)
   const int nchunk = kThermoChunks;
   std::vector<double> part((size_t)n * nchunk);
-  EntryIo io(e);
+  EntryIo io(e->io, e->stream);
   const int idx = io.in(slots.data(), sizeof(int) * (size_t)n);
   const int share = io.out(part.data(), part.size() * 8);
   if (int rc = io.open()) return rc;
