@@ -271,3 +271,52 @@ def test_update_groups_of_few_and_many_replicas(pimc, n):
             assert np.array_equal(a[k], b[k][:150], equal_nan=True), k
     for p, q in zip(few.download_paths(), many.download_paths()):
         assert np.array_equal(p, q)
+
+
+MIXED_DISPLACED = {
+    "heg10": (W.heg54(n=10, nslice=32, nlevel=3, t_over_tf=3.0), "grid"),
+    "heg26_free": (W.heg54(n=26, nslice=64, nlevel=3, t_over_tf=1.5, coulomb=0, ewald=0), "grid"),
+    "heg16_one_species": (dict(W.heg54(n=16, nslice=32, nlevel=3, t_over_tf=1.5),
+                               node_kind=[2, 0]), "grid"),
+    "dot8_fn": (W.dot20_fn(counts=[5, 3], nslice=32, beta=1.6, nlevel=3, node_temperature=0.5),
+                "const"),
+}
+
+
+@pytest.mark.parametrize("nmoving", [1, 2])
+@pytest.mark.parametrize("nrep", [1, 40, 170])
+@pytest.mark.parametrize("case", list(MIXED_DISPLACED))
+def test_mixed_displacements_then_sections(pimc, case, nrep, nmoving):
+    # Mixed form: after sections (whose matrices were updated) and displacements, the
+    # cached elements, determinants, distances, inverses and structure factors are those
+    # of the paths: the sections that follow are those of an engine that starts from
+    # them.  (The bars of the mixed form against FP64, as inverses here have been
+    # updated and there are fresh.)
+    kw, kind = MIXED_DISPLACED[case]
+    tabs, ew = pimc.coulomb_tables(kw) if kw["coulomb"] else ((), None)
+    x = W.initial_path(dict(kw), kind, seed=7)
+    a = pimc.Engine(kw, nrep, tabs, ew, seed=99, precision=1)
+    a.upload_paths([x] * nrep)
+    displaced = 0
+    for _ in range(4):
+        a.run_sections(25)
+        displaced += a.run_displace(6, [0.6] * 3, nmoving, -1, records=True)["accepted"].sum()
+        b = pimc.Engine(kw, nrep, tabs, ew, seed=99, precision=1)
+        b.upload_paths(a.download_paths())
+        for r in range(nrep):
+            b.set_replica_state(r, a.replica_state(r))
+        if ew is not None:
+            assert np.array_equal(a.thermo_energy(), b.thermo_energy())
+        ra, rb = a.run_sections(20, records=True), b.run_sections(20, records=True)
+        b.close()
+        alike = np.cumprod((ra["reject_level"] == rb["reject_level"]) & (ra["ipart"] == rb["ipart"]),
+                           axis=1).astype(bool)
+        assert alike.mean() > 0.95
+        nl = kw["nlevel"] + 1
+        for k in ("ds", "ds_node", "lnt"):
+            p, q = ra[k][alike][:, :nl], rb[k][alike][:, :nl]
+            assert np.array_equal(np.abs(p) >= 1e99, np.abs(q) >= 1e99)
+            fin = np.abs(q) < 1e99
+            tol = 1e-12 if k != "ds_node" else 1e-4
+            assert np.all(np.abs(p - q)[fin] <= tol * np.maximum(np.abs(q[fin]), 1.0)), k
+    assert displaced > 0
