@@ -948,10 +948,13 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
   int occ = 1;
   occ = section_occupancy(e->minb, e->block, e->lay.total * 8, e->nodes);
   occ = std::max(occ, 1);
-  // More replicas than SMs whose shared memory leaves room for one CTA of eight warps:
-  // two of four hide each other's barriers and serial parts (1024 mixed dots of up to
-  // 32 particles: 14.7 -> 12.6 ms a loop).
-  if (e->nodes && occ == 1 && nrep > nsm && e->block == kBlock) {
+  // Where shared memory leaves room for one CTA of eight warps, two of four may be faster.
+  int largest_sho = 0;
+  for (const DevSys& d : e->hsys)
+    for (int i = 0; i < d.nspecies; ++i)
+      if (d.node_kind[i] == PIMC_NODES_SHO) largest_sho = std::max(largest_sho, d.spec_count[i]);
+  if (e->nodes && occ == 1 && e->block == kBlock &&
+      prefers_two_ctas(nrep, nsm, largest_sho, uniform)) {
     const int half = kBlock / 2;
     LayoutOpts opts = e->lay_opts;
     opts.nshare = kBlock / 32;  // (the sums stay those of eight warps)

@@ -29,6 +29,23 @@ struct Layout {
   int total;  // doubles
 };
 
+// Whether systems of which a CTA of eight warps fills an SM run as two CTAs of four, which
+// hide each other's barriers and serial parts, but leave a replica half of the warps.
+// Free-particle nodes: where there are more replicas than SMs (12 attempts of 48
+// electrons, L = 3, mixed: 160 replicas 3.20 -> 2.66 ms, 608 7.46 -> 5.49).  SHO nodes,
+// whose matrices keep the warps busy: where the shorter chain of a replica does not
+// count, from four replicas an SM on (1024 uneven dots of up to 32 particles 7.73 -> 6.31 ms,
+// 608 4.68 -> 4.04, but 456 3.62 -> 3.91 and 240 2.38 -> 3.90), or where replicas of
+// one kind fill two CTAs an SM and no more (dots of 32: 304 replicas 5.60 -> 5.17, but
+// 240 4.86 -> 5.10 and 360 6.74 -> 7.42); and not for species that take a warp a
+// matrix (36 particles, 1000 replicas: 17.9 -> 18.9).
+// largest_sho: the largest species with SHO nodes (0: none).
+inline bool prefers_two_ctas(int nreplica, int nsm, int largest_sho, bool alike) {
+  if (!largest_sho) return nreplica > nsm;
+  const bool filled = alike && nreplica <= 2 * nsm && 10 * nreplica >= 19 * nsm;
+  return largest_sho <= 16 && (nreplica >= 4 * nsm || filled);
+}
+
 struct RunParams {
   const DevSys* sys;
   DevState* state;

@@ -18,6 +18,11 @@ int main() {
       for (int lanes = 0; lanes <= 32 * 40; lanes += 8)
         std::printf("action %d %d %d %d\n", mixed, nwarps, lanes,
                     first_action_warp(lanes, nwarps, mixed));
+  for (int sho : {0, 1, 16, 17, 32})
+    for (int nrep : {1, 152, 153, 280, 300, 304, 305, 607, 608, 5000})
+      for (int alike = 0; alike < 2; ++alike)
+        std::printf("ctas %d %d %d %d\n", sho, nrep, alike,
+                    prefers_two_ctas(nrep, 152, sho, alike));
   for (int nwarps = 1; nwarps <= 8; nwarps *= 2)
     for (int nshare = nwarps; nshare <= 2 * nwarps; nshare *= 2)
       for (int mixed = 0; mixed < 2; ++mixed)
@@ -116,3 +121,11 @@ def test_lane_group_widths(rules):
             assert w <= max(own, wmin)
             wider += w > own
     assert wider
+
+
+def test_two_ctas(rules):
+    # Half as many warps a replica: with SHO nodes only where replicas are many and their
+    # matrices share warps, with free-particle nodes wherever replicas wait for SMs.
+    for sho, nrep, alike, two in (map(int, r[1:]) for r in rules if r[0] == "ctas"):
+        many = nrep >= 608 or (alike and nrep in (300, 304))
+        assert two == (many and sho <= 16 if sho else nrep > 152)

@@ -178,8 +178,8 @@ FEW_AND_MANY = {
     "heg4": (W.heg54(n=4, nslice=1024, nlevel=4, node_kind=[0, 0]), "grid", 1300),
     "heg4_uncached": (W.heg54(n=4, nslice=16, nlevel=4, beta=0.4, node_kind=[0, 0]), "grid", 1300),
     "dot32_fn": (W.dot20_fn(counts=[16, 16], nslice=128, beta=5.0, node_temperature=0.25),
-                 "const", 170),
-    "heg54": (W.heg54(nslice=512, nlevel=4), "grid", 170),
+                 "const", 640),
+    "heg54": (W.heg54(nslice=256, nlevel=3), "grid", 170),
 }
 
 
@@ -195,13 +195,12 @@ def test_chains_of_few_and_many_replicas(pimc, case, precision):
     few.upload_paths(x)
     many.upload_paths([x[r % 2] for r in range(nrep)])
     a, b = few.run_sections(30, records=True), many.run_sections(30, records=True)
-    if nrep == 1300:
-        assert (few.launch_config()["block"], many.launch_config()["block"]) == (64, 32)
     for k in a:
         assert np.array_equal(a[k], b[k][:2], equal_nan=True), k
     for p, q in zip(few.download_paths(), many.download_paths()):
         assert np.array_equal(p, q)
-    print(case, precision, few.launch_config()["block"], many.launch_config()["block"])
+    blocks = few.launch_config()["block"], many.launch_config()["block"]
+    assert blocks == ((64, 32) if nrep == 1300 else (256, 128))
 
 
 FEW_AND_MANY_DISPLACED = {
