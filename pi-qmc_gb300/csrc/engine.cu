@@ -492,6 +492,16 @@ int ensure_xstage(pimc_engine* e, int grid) {
   return PIMC_OK;
 }
 
+// The precision form, and what follows from it.
+void set_precision(DevSys& d, int precision) {
+  d.mixed = precision == PIMC_PREC_MIXED;
+  d.node_widths = d.node_widest = 0;
+  for (int i = 0; i < d.nspecies; ++i) {
+    d.node_widths |= (unsigned)node_launch_width(d, i, 8) << (8 * i);
+    d.node_widest |= (unsigned)node_launch_width(d, i, 32) << (8 * i);
+  }
+}
+
 // Fixed-point exponent of a replica's structure-factor cache, or -1 when it
 // has none (no Ewald sum; fixed-node sections that can overlap; charges too
 // large for a fine grid): |rho_k| <= sum |q|, and an update adds at most
@@ -894,7 +904,7 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
       e->lay_opts.nshare = 2;
     }
   }
-  for (DevSys& d : e->hsys) d.mixed = precision == PIMC_PREC_MIXED;
+  for (DevSys& d : e->hsys) set_precision(d, precision);
   e->nodes = false;
   for (const DevSys& d : e->hsys) e->nodes |= d.fixed_node != 0;
   bool ok = false;
@@ -2364,7 +2374,7 @@ int pimc_server_admit(pimc_engine* e, const pimc_system* sys, const pimc_pair_ta
   if (r < 0) return fail(PIMC_ERR_CAPACITY, "no free slot");
   const long long pw = 3LL * sys->nslice * sys->npart;
   const bool cache = d.fixed_node && (1 << d.nlevel) < d.nslice / 2;
-  d.mixed = e->precision == PIMC_PREC_MIXED;
+  set_precision(d, e->precision);
   d.nc_stride = cache_entry_doubles(d);
   const long long cw = cache ? (long long)d.nspecies * d.nslice * d.nc_stride : 0;
   const long long po = pool_alloc(e, pw + cw);
@@ -2421,7 +2431,6 @@ int pimc_server_admit(pimc_engine* e, const pimc_system* sys, const pimc_pair_ta
     }
     d.ntab = ntables;
   }
-  d.mixed = e->precision == PIMC_PREC_MIXED;
   d.stream_id = stream_id;
   d.path_offset = po;
   d.nc_offset = cache ? po + pw : -1;

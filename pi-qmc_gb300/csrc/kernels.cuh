@@ -684,12 +684,7 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   // warp tasks: each warp takes up to G misses of one species (lane groups of
   // a warp must run the same species so that they stay converged)
   int ntask = 0, first[kMaxSpecies + 1], wmin = m.wide ? 32 : 8;
-  unsigned narrow = 0, widest = 0;  // a byte per species: its groups' widths
-#pragma unroll 1
-  for (int sp = 0; sp < s.nspecies; ++sp) {
-    narrow |= (unsigned)node_launch_width(s, sp, 8) << (8 * sp);
-    widest |= (unsigned)node_launch_width(s, sp, wmin) << (8 * sp);
-  }
+  const unsigned narrow = s.node_widths, widest = s.node_widest;
   const auto width = [&](int sp) {
     return min(max(wmin, (int)((narrow >> (8 * sp)) & 63u)), (int)((widest >> (8 * sp)) & 63u));
   };
@@ -929,7 +924,8 @@ static __device__ __noinline__ void eval_levels(const DevSys& s, const Smem& m, 
   // 41.1 with half of the warps on the action; two CTAs per SM share the pipe, where
   // narrow groups' fewer instructions count).
   if (m.wide && mynode) {
-    const int most = a0 == 0 || alo > ahi ? nwarps : a0, widest = node_launch_width(s, msp, 32);
+    const int most = a0 == 0 || alo > ahi ? nwarps : a0;
+    const int widest = (s.node_widest >> (8 * msp)) & 63u;
     while (W < widest && ntask * W <= 16 * most) W *= 2;
   }
   const int G = 32 / W, g = lane / W, nodeW = min(nwarps, (ntask + G - 1) / G);

@@ -62,6 +62,9 @@ struct DevSys {
   float rcut2_lo, rcut2_hi, cellb_f[3];
   int spring, coulomb, ewald, mover, fixed_node;
   int mixed;  // PIMC_PREC_MIXED: pair-action terms in FP32, accumulated in FP64
+  // lane-group widths of the species' Slater evaluations, a byte each: a full launch's,
+  // and the widest of one that leaves SMs room (node_launch_width)
+  unsigned node_widths, node_widest;
   double epsilon;
   int ntab;
   DevTable tab[kMaxTables];
