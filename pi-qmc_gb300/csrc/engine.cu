@@ -1537,7 +1537,8 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
   if (which == kEstVirial) {
     // forces of as many replicas at a time as fit 256 MB (one at least)
     long long stride = 0;
-    int per_warp = 1, passes = 1;
+    size_t smem = 8;
+    int passes = 1;
     for (const DevSys& d : e->hsys) {
       for (int k = 0; k < d.ntab; ++k) {  // the most tables of one species pair
         int same = 0;
@@ -1546,11 +1547,8 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
         passes = std::max(passes, same);
       }
       stride = std::max(stride, 6LL * d.nslice * d.npart);
-      const int npair = (d.npart + 1) / 2, lpw = npair < 32 ? 32 / npair : 1;
-      per_warp = std::max(per_warp, 6 * lpw * d.npart);
+      smem = std::max(smem, (size_t)virial_warps(d.npart) * virial_links(d.npart) * d.npart * 48);
     }
-    int warps = kBlock / 32;
-    while (warps > 1 && (size_t)warps * per_warp * 8 > (size_t)smem_max) warps /= 2;
     const int pass = (int)std::max(1LL, std::min((long long)std::min(e->nrep, 65535),
                                                  (256LL << 20) / (8 * stride)));
     if (e->d_forces.n < (size_t)pass * stride) {
@@ -1564,7 +1562,7 @@ int run_estimator(pimc_engine* e, int which, EstimatorParams P, const Layout& L,
     for (P.rep0 = 0; P.rep0 < e->nrep; P.rep0 += pass) {
       const dim3 grid(kThermoChunks, std::min(pass, e->nrep - P.rep0));
       for (P.pass = 0; P.pass < passes; ++P.pass) {
-        virial_links_kernel<<<grid, 32 * warps, (size_t)warps * per_warp * 8, e->stream>>>(P);
+        virial_links_kernel<<<grid, kBlock, smem, e->stream>>>(P);
         e->launches++;
       }
       virial_kernel<<<grid, kBlock, L.total * 8, e->stream>>>(P);

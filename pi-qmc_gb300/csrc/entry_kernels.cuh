@@ -351,6 +351,19 @@ struct EstimatorParams {
   int ikmax[3];
 };
 
+// Links a warp of virial_links_kernel takes at once, and the warps whose links' forces
+// (6 doubles a particle) fit shared memory, by the system alone.
+constexpr size_t kVirialSmem = 200 * 1024;
+__host__ __device__ __forceinline__ int virial_links(int np) {
+  const int npair = (np + 1) / 2;
+  return npair < 32 ? 32 / npair : 1;
+}
+__host__ __device__ __forceinline__ int virial_warps(int np) {
+  int w = kBlock / 32;
+  while (w > 1 && (size_t)w * virial_links(np) * np * 48 > kVirialSmem) w /= 2;
+  return w;
+}
+
 // One CTA per (chunk of links, replica); a warp takes as many links at a time as
 // their rounds of disjoint pairs fit its lanes, and keeps those links' forces in
 // shared memory: within a round every (link, particle) belongs to one lane.
@@ -381,15 +394,14 @@ __global__ void __launch_bounds__(kBlock) virial_links_kernel(EstimatorParams P)
   const double* path = P.paths + s.path_offset;
   double* forces = P.forces + blockIdx.y * P.forces_stride;
   const int M = s.nslice, np = s.npart, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
   const int nchunk = gridDim.x;
   const int t0 = (int)((long long)M * blockIdx.x / nchunk);
   const int t1 = (int)((long long)M * (blockIdx.x + 1) / nchunk);
   const int ne = np + (np & 1), npair = ne / 2, nrd = s.coulomb && np > 1 ? ne - 1 : 0;
-  const int lpw = npair < 32 ? 32 / npair : 1;  // links a warp takes at once
+  const int lpw = virial_links(np), nwarps = virial_warps(np);
   double* F = smem + (size_t)warp * lpw * np * 6;
   double part = 0.0;
-  for (int tw = t0 + warp * lpw; tw < t1; tw += nwarps * lpw) {
+  for (int tw = t0 + warp * lpw; warp < nwarps && tw < t1; tw += nwarps * lpw) {
     const int nl = min(lpw, t1 - tw);
     __syncwarp();
     // the beads' own terms start the sums

@@ -319,3 +319,23 @@ def test_mixed_displacements_then_sections(pimc, case, nrep, nmoving):
             tol = 1e-12 if k != "ds_node" else 1e-4
             assert np.all(np.abs(p - q)[fin] <= tol * np.maximum(np.abs(q[fin]), 1.0)), k
     assert displaced > 0
+
+
+def test_virial_energy_beside_a_large_system(pimc):
+    # A replica's value does not depend on the systems beside it (700 particles take fewer
+    # warps than five), bit for bit.
+    small = W.dot2(counts=[3, 2], nslice=6400, nlevel=1, beta=256.0)
+    large = W.dot2(counts=[350, 350], nslice=16, nlevel=1, beta=0.64)
+    tabs, _ = pimc.coulomb_tables(small)
+    x = [W.initial_path(dict(k), "gauss", seed=3) for k in (small, large)]
+    alone = pimc.Engine(small, 1, tabs)
+    alone.upload_paths([x[0]])
+    both = pimc.Engine.batch([small, large], [tabs, tabs])
+    both.upload_paths(x)
+    for w in (1, 16):
+        assert alone.virial_energy(w)[0] == both.virial_energy(w)[0]
+    port = O.PortOracle(O.make_config(**large), tabs)
+    port.set_path(x[1])
+    ref = port.virial_energy(4)
+    scale = max(1.0, abs(ref), abs(port.virial_energy(1)))
+    assert abs(both.virial_energy(4)[1] - ref) <= 1e-11 * scale
