@@ -327,15 +327,16 @@ def test_virial_energy_beside_a_large_system(pimc):
     small = W.dot2(counts=[3, 2], nslice=6400, nlevel=1, beta=256.0)
     large = W.dot2(counts=[350, 350], nslice=16, nlevel=1, beta=0.64)
     tabs, _ = pimc.coulomb_tables(small)
-    x = [W.initial_path(dict(k), "gauss", seed=3) for k in (small, large)]
-    alone = pimc.Engine(small, 1, tabs)
-    alone.upload_paths([x[0]])
-    both = pimc.Engine.batch([small, large], [tabs, tabs])
-    both.upload_paths(x)
+    x = [W.initial_path(dict(small), "gauss", seed=r) for r in range(12)]
+    y = W.initial_path(dict(large), "gauss", seed=3)
+    alone = pimc.Engine(small, 12, tabs)
+    alone.upload_paths(x)
+    both = pimc.Engine.batch([small] * 12 + [large], [tabs] * 13)
+    both.upload_paths(x + [y])
     for w in (1, 16):
-        assert alone.virial_energy(w)[0] == both.virial_energy(w)[0]
+        assert np.array_equal(alone.virial_energy(w), both.virial_energy(w)[:12])
     port = O.PortOracle(O.make_config(**large), tabs)
-    port.set_path(x[1])
+    port.set_path(y)
     ref = port.virial_energy(4)
     scale = max(1.0, abs(ref), abs(port.virial_energy(1)))
-    assert abs(both.virial_energy(4)[1] - ref) <= 1e-11 * scale
+    assert abs(both.virial_energy(4)[12] - ref) <= 1e-11 * scale
