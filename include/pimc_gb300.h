@@ -144,7 +144,14 @@ typedef struct pimc_engine pimc_engine;
  * tables and Ewald table), FixedNodeAction with SHONodes/FreeParticleNodes,
  * FreeMover/FreeMoverPBC, SectionChooser or DoubleSectionChooser, and a
  * MultiLevelSampler/DoubleMLSampler moving one particle chosen by
- * SimpleParticleChooser. */
+ * SimpleParticleChooser.
+ * A replica's moves and energies do not depend on how many replicas there are,
+ * bit for bit (in the default launch shape).
+ * Device memory besides paths and caches, kept until the engine is destroyed:
+ * the pair tables (FP64 coefficients beside their differences, and FP32); up to
+ * 64 MB of buffers for the calls that take or return host arrays (and 128 KB of
+ * pinned host memory); after a virial measurement the beads' forces, 48 bytes
+ * each, of as many replicas as fit 256 MB (of one at least). */
 int pimc_engine_create(const pimc_system* sys, int nreplica, const pimc_pair_table* tables,
                        int ntables, const pimc_ewald_table* ewald, uint64_t seed,
                        int precision, pimc_engine** out);
@@ -298,8 +305,10 @@ int pimc_ewald_coefficients(double* coef, int n);
  * many as fit) and the section
  * kernel's register-budget variant.  ms is the
  * time the autotuner measured for it (0 when not measured).  A configuration
- * changes how per-thread partial sums are grouped, so chains run under two
- * configurations agree to rounding, not bit for bit. */
+ * set here or by the autotuner changes how per-thread partial sums are grouped, so
+ * chains run under two configurations agree to rounding, not bit for bit.  (The
+ * default shape may take a smaller block for many replicas; its sums are those of
+ * the system's own.) */
 typedef struct {
   int block;
   int scratch_global;

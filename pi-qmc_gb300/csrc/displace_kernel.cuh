@@ -22,7 +22,7 @@
 //    particles' rows and columns are new when the cached matrix is whole; an
 //    accepted move updates the cached entries instead of dropping them.
 // Four attempts of 19 electron gases (N = 54, M = 512, Ewald, 27 x 27 nodes): 504 ms
-// with one CTA per replica and full sums, now 9.4 ms.
+// with one CTA per replica and full sums, 9.4 ms so.
 #pragma once
 #include <cooperative_groups.h>
 

@@ -437,7 +437,7 @@ void fill_sys(const pimc_system& s, DevSys& d) {
   // The thermodynamic estimator's chunks by the system's own size (so that a value does
   // not depend on what is measured beside it): 4096 bead or pair links each, 16 per
   // thread against the start-up of a CTA.  (64 CTAs for every system: a step of 9728
-  // two-electron dots 29.4 ms, now 13.1.)  A thread's links are runs of two items a
+  // two-electron dots 29.4 ms, 13.1 so.)  A thread's links are runs of two items a
   // thread; the runs of up to eight chunks (of all but 64 with Ewald sums) are cut into up to
   // eight parts, which a launch that leaves SMs idle shares out to more CTAs.
   {
@@ -978,7 +978,6 @@ int build_engine(const pimc_system* sys, int nrep, const pimc_pair_table* tables
     }
   }
   e->grid = std::min(nrep, nsm * occ);
-  for (DevSys& d : e->hsys) d.inv_offset = e->lay.gcta > 0 ? 0 : -1;
   if (e->lay.gcta > 0 && e->d_nodescr.alloc((size_t)e->grid * e->lay.gcta)) {
     delete e;
     return fail(PIMC_ERR_CUDA, "cudaMalloc node scratch");
@@ -2400,7 +2399,7 @@ int pimc_server_admit(pimc_engine* e, const pimc_system* sys, const pimc_pair_ta
       if (toff == (size_t)-1) {
         if (e->table_used + words > e->d_ugrid32.n) {
           pool_free(e, po, pw + cw);
-          return fail(PIMC_ERR_INVALID, "server table pool full (distinct pair tables exceed 32 MiB)");
+          return fail(PIMC_ERR_INVALID, "server table pool full (distinct pair tables exceed 4 Mi coefficients)");
         }
         toff = e->table_used;
         std::vector<float> f(t.ugrid, t.ugrid + words);
@@ -2432,7 +2431,6 @@ int pimc_server_admit(pimc_engine* e, const pimc_system* sys, const pimc_pair_ta
   d.stream_id = stream_id;
   d.path_offset = po;
   d.nc_offset = cache ? po + pw : -1;
-  d.inv_offset = e->lay.gcta > 0 ? 0 : -1;
   e->hsys[r] = d;
   e->hdesc[r] = *sys;
   e->slot_path[r] = po;

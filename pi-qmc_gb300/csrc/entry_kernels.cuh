@@ -832,7 +832,8 @@ static __device__ __noinline__ double ewald_move_energy(const DevSys& s, const S
 // Action differences of independent sections.  CTA (0, b) takes entry b's spring,
 // confinement and pair terms; with Ewald sums on level 0, CTAs (1 .., b) share the
 // section's slices.  (One CTA an entry, slice after slice, each with both sums in
-// full: 3440 us for one section of the electron gas from host arrays, now 312 us.)
+// full: 3440 us for one section of the electron gas from host arrays, 99 so and with the
+// call's arrays on a pinned block.)
 __global__ void __launch_bounds__(kBlock) action_diff_kernel(ActionDiffParams P) {
   extern __shared__ double smem[];
   __shared__ DevSys S;
@@ -904,7 +905,7 @@ struct NodeEvalParams {
 
 // Warps take as many pairs at a time as their lane groups (one of 32 lanes, two of
 // 16, four of 8 by the species' size).  (One pair a CTA of eight warps, seven of them
-// idle: 1024 27 x 27 evaluations from host arrays 1142 us, now 672 us.)
+// idle: 1024 27 x 27 evaluations from host arrays 1142 us, 672 so.)
 __global__ void __launch_bounds__(kBlock) node_eval_kernel(NodeEvalParams P) {
   extern __shared__ double smem[];
   __shared__ DevSys S;
@@ -987,9 +988,5 @@ __global__ void stream_sample_kernel(uint64_t seed, uint32_t rep, uint32_t att, 
   u[i] = stream_uniform(seed, rep, att, (uint32_t)i);
   z[i] = stream_normal(seed, rep, att, (uint32_t)i);
 }
-
-}  // namespace pimc
-
-namespace pimc {
 
 }  // namespace pimc

@@ -750,6 +750,12 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   __syncthreads();
 }
 
+// |x| < lo or |x| > hi (both normal; never for a NaN), on the integer pipe
+__device__ __forceinline__ bool outside_magnitudes(double x, double lo, double hi) {
+  const long long a = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+  return a < __double_as_longlong(lo) || (a > __double_as_longlong(hi) && a <= 0x7ff0000000000000LL);
+}
+
 // FixedNodeAction::initialize (src/fixednode/FixedNodeAction.cc:331-357) for every
 // species with a node model, reproducing NodeModel::evaluate's rescaling loop
 // (src/fixednode/SHONodes.cc:112-126): every species' slices are evaluated in
@@ -757,12 +763,6 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
 // other; they are independent); at a species' first slice whose determinant
 // leaves [1e-50, 1e50] its loop is replayed sequentially, and its later
 // slices are re-evaluated.
-// |x| < lo or |x| > hi (both normal; never for a NaN), on the integer pipe
-__device__ __forceinline__ bool outside_magnitudes(double x, double lo, double hi) {
-  const long long a = __double_as_longlong(x) & 0x7fffffffffffffffLL;
-  return a < __double_as_longlong(lo) || (a > __double_as_longlong(hi) && a <= 0x7ff0000000000000LL);
-}
-
 static __device__ __noinline__ void node_initialize(const DevSys& s, const Smem& m, double* scale, int* epoch,
                                 int msp, uint32_t* status, double* cache, int ifirst1, int ipart,
                                 uint64_t seed, uint32_t att, double* llt) {
@@ -1118,12 +1118,6 @@ static __device__ __noinline__ void delayed_rejection(const DevSys& s, const Sme
 }
 
 
-// NT (largest block) and MINB set the register budget, 65536 / (NT * MINB)
-// per thread; the variants are compiled in separate translation units
-// (section_variants.cu) and chosen at run time by the launch configuration.
-// kNodes = false: the variant for launches without node models, whose code
-// leaves the fixed-node phases out (a smaller kernel: fewer instruction-fetch
-// stalls when thousands of one-warp CTAs run different phases).
 // n values by a warp, eight loads in flight a lane
 template <class T>
 __device__ __forceinline__ void copy_warp(T* dst, const T* src, int n) {
@@ -1138,6 +1132,12 @@ __device__ __forceinline__ void copy_warp(T* dst, const T* src, int n) {
   }
 }
 
+// NT (largest block) and MINB set the register budget, 65536 / (NT * MINB)
+// per thread; the variants are compiled in separate translation units
+// (section_variants.cu) and chosen at run time by the launch configuration.
+// kNodes = false: the variant for launches without node models, whose code
+// leaves the fixed-node phases out (a smaller kernel: fewer instruction-fetch
+// stalls when thousands of one-warp CTAs run different phases).
 template <int NT, int MINB, bool kNodes = true>
 __global__ void __launch_bounds__(NT, MINB) section_moves_kernel(RunParams P) {
   extern __shared__ double smem[];

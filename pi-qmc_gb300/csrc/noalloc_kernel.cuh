@@ -6,10 +6,10 @@
 namespace pimc {
 
 // ------------------------------------------- allocation-free node evaluation
-// Scratch for node_eval_noalloc_kernel: one slot of 6 * 32 * 32 + 33 doubles
-// (rounded up to 6208: the LU, inverse and exp matrices, pivot reciprocals and
-// the three gradient matrices of free-particle nodes, for one Slater matrix of
-// up to 32 particles) per resident warp, kNoAllocSlots slots: 6.1 MiB, held by
+// Scratch for node_eval_noalloc_kernel: one slot of node_group_scratch(32) = 6193 doubles
+// (rounded up to 6208: the LU, inverse and element matrices, pivot reciprocals, the row
+// order and the three gradient matrices of free-particle nodes, for one Slater matrix
+// of up to 32 particles) per resident warp, kNoAllocSlots slots: 6.1 MiB, held by
 // every GPU that loads the library until exit.
 constexpr int kNoAllocSlots = 128;
 constexpr int kNoAllocSlot = (node_group_scratch(kMaxNs) + 31) / 32 * 32;

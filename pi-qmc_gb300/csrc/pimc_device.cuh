@@ -87,7 +87,6 @@ struct DevSys {
   long long ek_offset;    // int64 words into the structure-factor cache (-1: none)
   double ek_scale;        // grid spacing 1/ek_scale (a power of two)
   long long path_offset;  // doubles into the path pool
-  long long inv_offset;   // doubles into the node scratch pool (-1: shared memory)
 };
 
 // Mutable per-replica state kept on the device between launches.
@@ -474,13 +473,6 @@ __device__ __forceinline__ float tab_uk0d_tau_f(const DevTable& t, float q, floa
   float a = 0.f;
   for (int k = t.norder; k >= 0; k--) a = fmaf(a, s2, fmaf(x, __ldg(g1 + k) - __ldg(g0 + k), __ldg(g0 + k)));
   return a;
-}
-
-// Error-free sum of two doubles (Knuth TwoSum) for compensated accumulation.
-__device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
-  s = a + b;
-  const double bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
 }
 
 // A compensated FP32 sum (Knuth's TwoSum per term, the rounding errors

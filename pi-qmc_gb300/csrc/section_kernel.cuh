@@ -55,12 +55,7 @@ struct Smem {
 
 
 enum {
-  C_IFIRST1 = 0, C_IFIRST2, C_IPART, C_REJECT, C_FLAG, C_ERRS, C_NMISS, C_NCTL = 16
-};
-
-struct SectionSizes {
-  // all counts in doubles
-  static __host__ __device__ long long section(int nsec, int npart) { return 3LL * nsec * npart; }
+  C_IFIRST1 = 0, C_IFIRST2, C_IPART, C_REJECT, C_FLAG, C_NMISS, C_NCTL = 16
 };
 
 // Positions of particle p on section slice t, with the moving bead substituted.
