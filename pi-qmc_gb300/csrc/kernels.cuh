@@ -650,20 +650,37 @@ static __device__ __noinline__ void node_init_pass(const DevSys& s, const Smem& 
   int* miss = errs + kMaxSpecies * nsec;       // [kMaxSpecies][nsec] slices to evaluate
   int* nmiss = m.ictl + C_NMISS;               // [kMaxSpecies] (C_NMISS .. C_NMISS + 3)
   const double NaN = __longlong_as_double(0x7ff8000000000000LL);
-  if (threadIdx.x < kMaxSpecies) nmiss[threadIdx.x] = 0;
-  __syncthreads();
   const int nt = nsec - start;
+  // A warp lists a species' misses in the order of their slices: matrices that share a
+  // warp below are updated together or not at all, so a chain would follow the order.
 #pragma unroll 1
-  for (int it = threadIdx.x; it < s.nspecies * nt; it += blockDim.x) {
-    const int sp = it / nt, t = start + (it - sp * nt);
-    if (!s.node_kind[sp] || (only_sp >= 0 && sp != only_sp)) continue;
-    const double* e = cache ? cache_entry(s, cache, sp, wrap_slice(ifirst1 + t, M)) : nullptr;
-    if (e && e[0] == (double)epoch[sp]) {
-      m.dm[sp * nsec + t] = e[1];
-      errs[sp * nsec + t] = 0;
-    } else {
-      miss[sp * nsec + atomicAdd(&nmiss[sp], 1)] = t;
+  for (int sp = warp; sp < s.nspecies; sp += nwarps) {
+    const bool on = s.node_kind[sp] && (only_sp < 0 || sp == only_sp);
+    int count = 0;
+#pragma unroll 1
+    for (int t0 = start; on && t0 < nsec; t0 += 64) {  // (two slices' loads in flight)
+      double ep[2], det[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int t = min(t0 + 32 * q + lane, nsec - 1);
+        const double* e = cache ? cache_entry(s, cache, sp, wrap_slice(ifirst1 + t, M)) : nullptr;
+        ep[q] = e ? e[0] : NaN;
+        det[q] = e ? e[1] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int t = t0 + 32 * q + lane;
+        const bool hit = ep[q] == (double)epoch[sp], in = t < nsec;
+        if (in && hit) {
+          m.dm[sp * nsec + t] = det[q];
+          errs[sp * nsec + t] = 0;
+        }
+        const unsigned lost = __ballot_sync(0xffffffffu, in && !hit);
+        if (in && !hit) miss[sp * nsec + count + __popc(lost & ((1u << lane) - 1u))] = t;
+        count += __popc(lost);
+      }
     }
+    if (lane == 0) nmiss[sp] = count;
   }
   // the moving species' distances where the entry is valid (a particle per thread:
   // as a loop of the slice's own thread this took 8,000-21,000 clocks of load latency)
