@@ -129,7 +129,6 @@ struct DevBuf {
 #include "entry_io.h"
 
 constexpr int kThermoChunks = 64;  // CTAs per replica of the estimators, at most
-constexpr int kThermoParts = 8;    // parts of a chunk, at most
 
 // Layout choices the autotuner varies.
 struct LayoutOpts {
@@ -696,9 +695,11 @@ Layout estimator_layout(const std::vector<DevSys>& sys, const int* ikmax_extra) 
   const int xy = 2 * (ik[0] + 1) * (2 * ik[1] + 1) * np;
   const bool ewald = ik[0] + ik[1] + ik[2] > 0;
   L.ewxy = ewald && (off + xy) * 8 <= 74 * 1024 ? take(xy) : 0;
-  int parts = 1;
-  for (const DevSys& d : sys) parts = std::max(parts, d.thermo_parts);
-  L.sums = take(parts > 1 ? parts * kBlock : 0);
+  // (over the tables where those are as large: the sums are taken before them)
+  int parts = 0;
+  for (const DevSys& d : sys)
+    if (d.thermo_parts > 1) parts = std::max(parts, d.thermo_parts);
+  L.sums = off - L.ewt >= parts * kBlock ? L.ewt : take(parts * kBlock);
   L.ictl = take(C_NCTL + 2);
   L.dm = L.ndm = L.dist = L.ndist = L.red;
   L.ecache = L.ncol = -1;

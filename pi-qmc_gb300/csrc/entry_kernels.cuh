@@ -44,6 +44,8 @@ __device__ double link_utau(const DevSys& s, const double* path, int ip, int t) 
   return utau;
 }
 
+constexpr int kThermoParts = 8;  // parts of a chunk of the thermodynamic estimator, at most
+
 struct ThermoParams {
   const DevSys* sys;
   const int* index;  // replicas to measure (null: all, blockIdx.y)
@@ -733,22 +735,30 @@ __device__ __forceinline__ void thermo_chunk(const ThermoParams& P, const DevSys
   if (longr && !cached) {
     for (int i = threadIdx.x; i < np; i += blockDim.x) m.qpart[i] = s.charge[species_of(s, i)];
   }
+  // (every part's sums before the long-range terms, whose tables may lie over them)
+  __shared__ double links[kThermoParts];
   for (int k = k0; k < k1; ++k) {
-    double tot = block_sum(kParts ? sums[(k - k0) * kBlock] : part, m.red);
+    const double sum = block_sum(kParts ? sums[(k - k0) * kBlock] : part, m.red);
+    if (threadIdx.x == 0) links[k - k0] = sum;
+  }
+  for (int k = k0; k < k1; ++k) {
+    double lr = 0.0;
     const auto at = [&](int i) { return slice(k, i); };
     if (cached) {  // evalLongRange of every slice from its cached structure factors
       const int full = (t1 - t0) / run, rest = (t1 - t0) - full * run, per = min(sub, run - k * sub);
       const int n = full * per + max(0, min(per, rest - k * sub));
-      tot += ewald_cached_energy(s, P.ekcache, nrun * sub, n, at, m.red) / s.epsilon;
-    } else if (longr)
+      lr = ewald_cached_energy(s, P.ekcache, nrun * sub, n, at, m.red) / s.epsilon;
+    } else if (longr) {
       for (int i = 0; i < nrun * sub; ++i)
-        if (at(i) >= 0) tot += ewald_staged_energy(s, m, path, at(i)) / s.epsilon;
+        if (at(i) >= 0) lr += ewald_staged_energy(s, m, path, at(i)) / s.epsilon;
+    }
     if (threadIdx.x == 0)
-      P.partial[(size_t)blockIdx.y * P.nchunk + chunk * s.thermo_parts + k] = tot;
+      P.partial[(size_t)blockIdx.y * P.nchunk + chunk * s.thermo_parts + k] = links[k - k0] + lr;
   }
 }
 
-__global__ void __launch_bounds__(kBlock) thermo_kernel(ThermoParams P) {
+// (three CTAs an SM, 80 registers: 9728 dots of two 945 us; with the 128 that two leave, 996)
+__global__ void __launch_bounds__(kBlock, 3) thermo_kernel(ThermoParams P) {
   __shared__ DevSys S;
   const int r = P.index ? P.index[blockIdx.y] : blockIdx.y;
   const int parts = P.sys[r].thermo_parts, split = min(P.split, parts);
