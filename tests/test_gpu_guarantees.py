@@ -169,14 +169,14 @@ def test_thermo_energy_of_one_and_many(pimc, case, precision):
 def test_thermo_energy_in_a_long_box(pimc):
     # Wave vectors far up one axis: their tables fill the shared memory that the parts'
     # sums would take beside them.
-    kw = W.heg54(n=13, cell=[10.0, 10.0, 900.0], nslice=128, nlevel=2, beta=12.8,
+    kw = W.heg54(n=13, cell=[10.0, 10.0, 936.0], nslice=128, nlevel=2, beta=12.8,
                  ewald_kcut=5 * 2 * np.pi / 10.0, node_kind=[0, 0])
     tabs, ew = pimc.coulomb_tables(kw)
     rng = np.random.default_rng(3)
-    x = np.repeat(rng.uniform(-0.5, 0.5, size=(1, 13, 3)) * [10.0, 10.0, 900.0], 128, axis=0)
+    x = np.repeat(rng.uniform(-0.5, 0.5, size=(1, 13, 3)) * [10.0, 10.0, 936.0], 128, axis=0)
     x += 0.05 * rng.normal(size=x.shape)
     cfg = O.make_config(**dict(kw, cell=10.0))
-    cfg.cell[2] = 900.0
+    cfg.cell[2] = 936.0
     port = O.PortOracle(cfg, tabs, ew)
     port.set_path(x)
     e = pimc.Engine(kw, 1, tabs, ew)
