@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
             parts.put(1, v, threadIdx.x == 0 ? lr : 0.0);
           }
         }
+      __syncthreads();  // (the Slater scratch lies over the warps' Ewald tables)
       // ---- FixedNodeAction per node species holding a moving particle
       if (dbl) {
         bool bad = false;

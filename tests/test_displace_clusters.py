@@ -30,6 +30,43 @@ def test_clusters_start_before_remote_access():
         assert ".sync()" in body[:first], (f, name)
 
 
+def test_tables_and_scratch_share_memory_in_turn():
+    # The warps' Ewald tables and their Slater scratch are the same shared memory, split
+    # at different strides: a barrier lies between the two uses, in either order.
+    body = next(b for _, name, b in _kernels() if name == "displace_kernel")
+    uses = [(m.start(), m.group(1)) for m in re.finditer(r"\b(displace_ewald|displace_nodes)\(", body)]
+    assert [u for _, u in uses] == ["displace_ewald", "displace_nodes", "displace_nodes",
+                                    "displace_ewald"]
+    loop = uses + [(uses[0][0] + len(body), uses[0][1])]  # (and round to the next attempt)
+    for (a, first), (b, second) in zip(loop, loop[1:]):
+        if first != second:
+            assert re.search(r"__syncthreads\(\)|cl\.sync\(\)", (body + body)[a:b]), (first, second)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nrep,nmoving", [(1, 1), (21, 3), (320, 3)])
+def test_warps_at_different_speeds(nrep, nmoving):
+    # A short path leaves some warps without Ewald terms, which come to the Slater matrices
+    # before the others: many attempts against the restatement.
+    import oracle_lib as O
+    import pimc_gb300 as pimc
+    pimc.build.build()
+    kw = W.heg54(n=8, nslice=198, nlevel=5, beta=7.92, cell=15.0, node_temperature=0.2,
+                 ewald_kcut=3 * 2 * np.pi / 15.0)
+    tabs, ew = pimc.coulomb_tables(kw)
+    x = W.initial_path(dict(kw), "grid", seed=7)
+    e = pimc.Engine(kw, nrep, tabs, ew, seed=99)
+    e.upload_paths([x] * nrep)
+    d = e.run_displace(20, [0.7] * 3, nmoving, -1, records=True)
+    for r in {0, nrep - 1}:
+        port = O.PortOracle(O.make_config(**dict(kw, seed=99, replica=r)), tabs, ew)
+        port.set_path(x)
+        ref = port.run_displace(20, [0.7] * 3, nmoving, -1)
+        assert np.array_equal(d["accepted"][r], ref["accepted"])
+        for k, tol in (("ds", 1e-11), ("ds_node", 1e-9)):
+            assert np.all(np.abs(d[k][r] - ref[k]) <= tol * np.maximum(np.abs(ref[k]), 1.0)), k
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("nrep", [1, 21, 60, 170])
 def test_many_short_launches(nrep):
