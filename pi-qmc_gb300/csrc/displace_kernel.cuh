@@ -40,7 +40,7 @@ struct DisplaceLayout {
   int ewt, ewt_cols;   // its e^{ik.r} tables (replicas without cached structure factors)
   int ek, ek_stride, ek_batch;  // per warp: tables of ek_batch slices' moved beads (-ek:
                                 // their place in the CTA's global area)
-  int stage;           // per-group slice pairs [2][3][n]
+  int stage, stage_stride;  // slice pairs per warp, [lane group][2][3][n]
   int nodescr, nodescr_stride, nodecold_stride, split, in_smem, gcta;
   int total;
 };
@@ -329,14 +329,16 @@ static __device__ __noinline__ bool displace_nodes(const DevSys& s, const Smem& 
                                                    const Moved& mv, const double* path, int sp,
                                                    bool moved, int t0, int t1, double* cache,
                                                    double scale, int epoch, double* stage,
-                                                   double* det_out, double* dist) {
+                                                   int stage_stride, double* det_out,
+                                                   double* dist) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int n = s.spec_count[sp], f = s.spec_first[sp], half = s.nslice / 2, nsm = s.ns_max;
   const bool sho = s.node_kind[sp] == PIMC_NODES_SHO;
   const int W = node_group_width(n), G = 32 / W, g = lane / W, gl = lane & (W - 1);
   double* gscr = group_scr(m, warp * G + g, G, n, !sho);
   double* gcold = group_cold(m, warp * G + g, G, n, !sho);
-  double* st = stage + (size_t)(warp * G + g) * 6 * n;  // [2][3][n]
+  // (a warp's part is its own whatever the species: the next one's pass follows at once)
+  double* st = stage + (size_t)warp * stage_stride + (size_t)g * 6 * n;  // [2][3][n]
   const unsigned pm = moved_mask(s, mv, sp);
   bool bad = false;
   for (int base = t0 + warp * G; base < t1; base += nwarps * G) {
@@ -615,10 +617,10 @@ __global__ void __launch_bounds__(kBlock) displace_kernel(DisplaceParams P) {
           double* ndist = ndet + half + (size_t)(flip[sp] ^ 1) * half * 2 * nsm;
           if (!ovalid[sp])
             bad |= displace_nodes(s, m, mv, path, sp, false, h0, h1, cache, scale[sp], epoch[sp],
-                                  smem + P.lay.stage, ndet, odist);
+                                  smem + P.lay.stage, P.lay.stage_stride, ndet, odist);
           __syncthreads();  // (the old pass made the entries whole)
           bad |= displace_nodes(s, m, mv, path, sp, true, h0, h1, cache, scale[sp], epoch[sp],
-                                smem + P.lay.stage, ndet, ndist);
+                                smem + P.lay.stage, P.lay.stage_stride, ndet, ndist);
         }
         if (bad) bad_ = 1;
         cl.sync();  // the other CTAs' determinants and distances

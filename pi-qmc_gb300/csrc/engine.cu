@@ -752,6 +752,7 @@ bool displace_layout(const std::vector<DevSys>& sys, int nwarps, int nmoving, Di
       L.ewt_cols = perfull ? np + 1 : 0;
       L.ewt = take(2 * perfull * L.ewt_cols);
       L.stage = take(nwarps * stage);
+      L.stage_stride = stage;
       L.split = place == 1;
       L.in_smem = place < 2;
       L.nodescr_stride = ((place == 1 ? hot : full) + 1) & ~1;

@@ -84,3 +84,29 @@ def test_many_short_launches(nrep):
     for k in one:
         assert np.array_equal(one[k], np.concatenate([p[k] for p in parts], axis=1)), k
     assert np.array_equal(a.download_paths(flat=True), b.download_paths(flat=True))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nrep", [1, 40, 320])
+@pytest.mark.parametrize("counts", [[5, 3], [13, 4], [2, 9, 4]])
+def test_moves_in_species_of_different_size(counts, nrep):
+    # Moved particles in several node species, whose matrices a warp takes one species
+    # after the other without waiting for the other warps: against the restatement.
+    import oracle_lib as O
+    import pimc_gb300 as pimc
+    pimc.build.build()
+    ns = len(counts)
+    kw = W.dot20_fn(counts=counts, nslice=128, beta=5.0, nlevel=3, node_temperature=0.5,
+                    node_kind=[1] * ns, node_omega=[1.0] * ns, sho_omega=[1.0] * ns)
+    tabs, _ = pimc.coulomb_tables(kw)
+    x = W.initial_path(dict(kw), "const", seed=7)
+    e = pimc.Engine(kw, nrep, tabs, seed=99)
+    e.upload_paths([x] * nrep)
+    d = e.run_displace(25, [0.6] * 3, 4, -1, records=True)
+    for r in {0, nrep - 1}:
+        port = O.PortOracle(O.make_config(**dict(kw, seed=99, replica=r)), tabs)
+        port.set_path(x)
+        ref = port.run_displace(25, [0.6] * 3, 4, -1)
+        assert np.array_equal(d["accepted"][r], ref["accepted"])
+        for k, tol in (("ds", 1e-11), ("ds_node", 1e-8)):
+            assert np.all(np.abs(d[k][r] - ref[k]) <= tol * np.maximum(np.abs(ref[k]), 1.0)), k
