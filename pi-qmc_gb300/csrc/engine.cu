@@ -658,7 +658,8 @@ void set_smem_caps() {
   section_smem_cap_nf_v2(kSmemLimit);
   section_smem_cap_nf_v3(kSmemLimit);
   section_smem_cap_nf_v4(kSmemLimit);
-  cudaFuncSetAttribute(thermo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  cudaFuncSetAttribute(thermo_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  cudaFuncSetAttribute(thermo_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   cudaFuncSetAttribute(action_diff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        kSmemLimit);
   cudaFuncSetAttribute(node_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
@@ -1391,16 +1392,21 @@ namespace {
 // engine's: the CTAs that share a chunk's parts are as many as fill the SMs with three each.
 void launch_thermo(pimc_engine* e, cudaStream_t st, ThermoParams P, const int* slots) {
   long long all = 0;
-  int chunks[2] = {1, 0};  // the most, of systems with one part a chunk and several
+  int chunks[2] = {1, 0}, parts = 1;  // the most, of systems with one part a chunk and several
   for (int k = 0; k < P.nrep; ++k) {
     const DevSys& d = e->hsys[slots ? slots[k] : k];
     int& c = chunks[d.thermo_parts > 1];
     c = std::max(c, d.thermo_chunks);
+    parts = std::max(parts, d.thermo_parts);
     all += d.thermo_chunks;
   }
-  P.split = (int)std::max(1LL, std::min((long long)kThermoParts, 3LL * e->num_sms / all));
+  P.split = (int)std::max(1LL, std::min((long long)parts, 3LL * e->num_sms / all));
   const int grid = std::max(chunks[0], chunks[1] * P.split);
-  thermo_kernel<<<dim3(grid, P.nrep), kBlock, P.lay.total * 8, st>>>(P);
+  const dim3 ctas(grid, P.nrep);
+  if (all * P.split <= 2LL * e->num_sms)
+    thermo_kernel<2><<<ctas, kBlock, P.lay.total * 8, st>>>(P);
+  else
+    thermo_kernel<3><<<ctas, kBlock, P.lay.total * 8, st>>>(P);
   e->launches++;
 }
 

@@ -757,8 +757,11 @@ __device__ __forceinline__ void thermo_chunk(const ThermoParams& P, const DevSys
   }
 }
 
-// (three CTAs an SM, 80 registers: 9728 dots of two 945 us; with the 128 that two leave, 996)
-__global__ void __launch_bounds__(kBlock, 3) thermo_kernel(ThermoParams P) {
+// MINB: CTAs an SM.  Three (80 registers) for launches that fill them, two (128) for
+// smaller ones (9728 dots of two 945 us against 996; seven dots of 22, M = 114, 165
+// against 116).  The same bits.
+template <int MINB>
+__global__ void __launch_bounds__(kBlock, MINB) thermo_kernel(ThermoParams P) {
   __shared__ DevSys S;
   const int r = P.index ? P.index[blockIdx.y] : blockIdx.y;
   const int parts = P.sys[r].thermo_parts, split = min(P.split, parts);
