@@ -121,17 +121,17 @@ def sweep_attempts(kw):
 MEASURED_WORK = {
     # launch shape of the count (block, scratch placement, register variant):
     # the DRAM bytes depend on the scratch placement, the flops do not
-    ("dot20_fn", "mixed"): dict(fp64=2.346e5, fp32=1.716e5, dram=1.366e5, shape="256,0,2",
-                                sha="f954a30c7f94b354"),
-    ("dot20_fn", "fp64"): dict(fp64=3.786e5, fp32=1.916e4, dram=1.388e5, shape="256,0,2",
-                               sha="f954a30c7f94b354"),
+    ("dot20_fn", "mixed"): dict(fp64=2.346e5, fp32=1.736e5, dram=1.376e5, shape="256,0,2",
+                                sha="d2a64fb74459dc29"),
+    ("dot20_fn", "fp64"): dict(fp64=3.786e5, fp32=2.119e4, dram=1.394e5, shape="256,0,2",
+                               sha="d2a64fb74459dc29"),
     # counted on the first 1024 replicas of the mix
-    ("batch4096", "mixed"): dict(fp64=1.155e5, fp32=9.592e4, dram=3.481e4, shape="128,0,2",
-                                 sha="f954a30c7f94b354"),
-    ("heg54", "mixed"): dict(fp64=9.469e5, fp32=4.857e5, dram=2.198e6, shape="256,0,2",
-                             sha="f954a30c7f94b354"),
-    ("dot2", "fp64"): dict(fp64=9.148e3, fp32=1.167e3, dram=476.6, shape="32,0,2",
-                           sha="f954a30c7f94b354"),
+    ("batch4096", "mixed"): dict(fp64=1.155e5, fp32=9.668e4, dram=3.481e4, shape="128,0,2",
+                                 sha="d2a64fb74459dc29"),
+    ("heg54", "mixed"): dict(fp64=9.469e5, fp32=4.892e5, dram=2.200e6, shape="256,0,2",
+                             sha="d2a64fb74459dc29"),
+    ("dot2", "fp64"): dict(fp64=9.148e3, fp32=1.167e3, dram=477.4, shape="32,0,2",
+                           sha="d2a64fb74459dc29"),
 }
 
 
